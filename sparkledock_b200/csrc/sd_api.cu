@@ -67,20 +67,17 @@ void key_thresholds_host(double* t) {
 }
 
 // Spatial tiles of 32 receptor atoms: recursive bisection along the widest axis at a multiple
-// of 32, so that every tile except possibly the last is full and compact.
+// of 32, so that every tile except possibly the last is full and compact; inside a tile the same
+// at multiples of 8, so that each group of 8 slots is compact too.
 void build_tiles(const double* xyz, int n, std::vector<int>& slots) {
   std::vector<int> idx(n);
   std::iota(idx.begin(), idx.end(), 0);
   std::vector<std::pair<int, int>> stack = {{0, n}};
-  std::vector<std::pair<int, int>> leaves;
   while (!stack.empty()) {
     auto [a, b] = stack.back();
     stack.pop_back();
     const int m = b - a;
-    if (m <= SD_TILE) {
-      leaves.push_back({a, b});
-      continue;
-    }
+    if (m <= SD_GROUP) continue;
     double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
     for (int k = a; k < b; ++k)
       for (int d = 0; d < 3; ++d) {
@@ -90,17 +87,15 @@ void build_tiles(const double* xyz, int n, std::vector<int>& slots) {
     int ax = 0;
     for (int d = 1; d < 3; ++d)
       if (hi[d] - lo[d] > hi[ax] - lo[ax]) ax = d;
-    const int ntile = (m + SD_TILE - 1) / SD_TILE;
-    const int split = a + SD_TILE * ((ntile + 1) / 2);
+    const int unit = m > SD_TILE ? SD_TILE : SD_GROUP;
+    const int split = a + unit * (((m + unit - 1) / unit + 1) / 2);
     std::nth_element(idx.begin() + a, idx.begin() + split, idx.begin() + b,
                      [&](int u, int v) { return xyz[u * 3 + ax] < xyz[v * 3 + ax]; });
     stack.push_back({split, b});
     stack.push_back({a, split});
   }
-  std::sort(leaves.begin(), leaves.end());
-  slots.assign((size_t)leaves.size() * SD_TILE, -1);
-  for (size_t t = 0; t < leaves.size(); ++t)
-    for (int k = leaves[t].first; k < leaves[t].second; ++k) slots[t * SD_TILE + (k - leaves[t].first)] = idx[k];
+  slots.assign((size_t)((n + SD_TILE - 1) / SD_TILE) * SD_TILE, -1);
+  std::copy(idx.begin(), idx.end(), slots.begin());
 }
 
 }  // namespace sd
@@ -119,7 +114,6 @@ struct sd_ctx {
   DevComplex* d_cplx = nullptr;
   DevComplex* d_cplx_scratch = nullptr;
   double* d_table64 = nullptr;
-  double* d_tablek = nullptr;   // key-indexed copy [168][168][32] + 32 zeros
   double* d_lj_eps = nullptr;
   double* d_lj_sigma = nullptr;
   StepCtl* d_ctl = nullptr;
@@ -143,6 +137,7 @@ struct sd_ctx {
   size_t score_smem = 0;
   bool score_spill = false;  // the last configured scorer launch uses the spill instantiation
   size_t spill_stride = 0;
+  int score_poses = 1;       // poses per CTA of the last configured scorer launch
   // autotuner state (mixed-precision DFIRE kernel variants)
   int mixed_variant = 0;
   bool tuned = false;
@@ -222,6 +217,22 @@ float round_up_f(double v) {
   return f;
 }
 
+// modes [nm][n][3] of a molecule into slot order [nm][3][slots] (padded slots stay 0)
+void slot_modes(const double* modes, int nm, int n, const std::vector<int>& slots, std::vector<double>& out) {
+  const size_t ns = slots.size();
+  for (int m = 0; m < nm; ++m) {
+    const double* M = modes + (size_t)m * n * 3;
+    double* o = out.data() + (size_t)m * 3 * ns;
+    for (size_t s = 0; s < ns; ++s) {
+      if (slots[s] < 0) continue;
+      const double* v = M + (size_t)slots[s] * 3;
+      o[s] = v[0];
+      o[ns + s] = v[1];
+      o[2 * ns + s] = v[2];
+    }
+  }
+}
+
 int setup_complex(sd_ctx* c, const sd_complex_desc& d, ComplexHost& h, int gbase, int sbase) {
   DevComplex& D = h.d;
   memset(&D, 0, sizeof D);
@@ -243,22 +254,19 @@ int setup_complex(sd_ctx* c, const sd_complex_desc& d, ComplexHost& h, int gbase
   D.ntiles = nslots / SD_TILE;
   h.nslots = nslots;
   std::vector<double> rxyz((size_t)nslots * 3, 0.0), rmodes((size_t)std::max(1, D.nmr) * nslots * 3, 0.0);
-  std::vector<int> rmask(nslots, 0), rrow(nslots, 0), rrowk(nslots, 0), rlj(nslots, 0);
+  std::vector<int> rmask(nslots, 0), rrow(nslots, 0), rlj(nslots, 0);
   std::vector<float> rq(nslots, 0.f);
   std::vector<float4> tiles(D.ntiles);
   for (int s = 0; s < nslots; ++s) {
     const int i = slots[s];
     if (i < 0) continue;
-    for (int k = 0; k < 3; ++k) rxyz[(size_t)s * 3 + k] = d.rec_xyz[(size_t)i * 3 + k];
-    for (int m = 0; m < D.nmr; ++m)
-      for (int k = 0; k < 3; ++k)
-        rmodes[((size_t)m * nslots + s) * 3 + k] = d.rec_modes[((size_t)m * d.n_rec + i) * 3 + k];
+    for (int k = 0; k < 3; ++k) rxyz[(size_t)k * nslots + s] = d.rec_xyz[(size_t)i * 3 + k];
     rmask[s] = d.rec_mask[i];
     rrow[s] = d.rec_dfire_type[i] * SD_ROW;
-    rrowk[s] = d.rec_dfire_type[i] * SD_ROWK;
     if (d.rec_charge) rq[s] = (float)d.rec_charge[i];
     if (d.rec_lj_type) rlj[s] = d.rec_lj_type[i];
   }
+  slot_modes(d.rec_modes, D.nmr, d.n_rec, slots, rmodes);
   for (int t = 0; t < D.ntiles; ++t) {
     double ctr[3] = {0, 0, 0};
     int cnt = 0;
@@ -315,12 +323,11 @@ int setup_complex(sd_ctx* c, const sd_complex_desc& d, ComplexHost& h, int gbase
   if ((rc = upload(c, h, rmodes.data(), rmodes.size(), &D.r_modes))) return rc;
   if ((rc = upload(c, h, rmask.data(), rmask.size(), &D.r_mask))) return rc;
   if ((rc = upload(c, h, rrow.data(), rrow.size(), &D.r_row))) return rc;
-  if ((rc = upload(c, h, rrowk.data(), rrowk.size(), &D.r_rowk))) return rc;
   if ((rc = upload(c, h, tiles.data(), tiles.size(), &D.r_tile))) return rc;
   if ((rc = upload(c, h, rq.data(), rq.size(), &D.r_q))) return rc;
   if ((rc = upload(c, h, rlj.data(), rlj.size(), &D.r_lj))) return rc;
 
-  // ligand chunks (spatial order) for the mixed-precision kernel
+  // ligand chunks (spatial order)
   {
     std::vector<int> lslots;
     build_tiles(d.lig_xyz, d.n_lig, lslots);
@@ -352,41 +359,33 @@ int setup_complex(sd_ctx* c, const sd_complex_desc& d, ComplexHost& h, int gbase
     }
     const size_t nls = lslots.size();
     std::vector<double> cxyz(nls * 3, 0.0), cmodes((size_t)std::max(1, D.nml) * nls * 3, 0.0);
-    std::vector<int> cmask(nls, 0), ccolk(nls, 0);
+    std::vector<int> cmask(nls, 0), ccol(nls, 0), clj(nls, 0), slot_of(d.n_lig, 0);
+    std::vector<float> cq(nls, 0.f);
     for (size_t s = 0; s < nls; ++s) {
       const int j = lslots[s];
       if (j < 0) continue;
-      for (int k = 0; k < 3; ++k) cxyz[s * 3 + k] = d.lig_xyz[(size_t)j * 3 + k];
-      for (int m = 0; m < D.nml; ++m)
-        for (int k = 0; k < 3; ++k) cmodes[((size_t)m * nls + s) * 3 + k] = d.lig_modes[((size_t)m * d.n_lig + j) * 3 + k];
+      slot_of[j] = (int)s;
+      for (int k = 0; k < 3; ++k) cxyz[(size_t)k * nls + s] = d.lig_xyz[(size_t)j * 3 + k];
       cmask[s] = d.lig_mask[j];
-      ccolk[s] = d.lig_dfire_type[j] * SD_KEYS;
+      ccol[s] = d.lig_dfire_type[j] * SD_DFIRE_BINS;
+      if (d.lig_charge) cq[s] = (float)d.lig_charge[j];
+      if (d.lig_lj_type) clj[s] = d.lig_lj_type[j];
     }
+    slot_modes(d.lig_modes, D.nml, d.n_lig, lslots, cmodes);
     double lc[3] = {0, 0, 0};
     for (int j = 0; j < d.n_lig; ++j)
       for (int k = 0; k < 3; ++k) lc[k] += d.lig_xyz[(size_t)j * 3 + k];
     for (int k = 0; k < 3; ++k) D.lig_ctr[k] = (float)(lc[k] / std::max(1, d.n_lig));
-    int rc2;
-    if ((rc2 = upload(c, h, lslots.data(), lslots.size(), &D.l_perm))) return rc2;
-    if ((rc2 = upload(c, h, lch.data(), lch.size(), &D.l_chunk))) return rc2;
-    if ((rc2 = upload(c, h, cxyz.data(), cxyz.size(), &D.lc_xyz))) return rc2;
-    if ((rc2 = upload(c, h, cmodes.data(), cmodes.size(), &D.lc_modes))) return rc2;
-    if ((rc2 = upload(c, h, cmask.data(), cmask.size(), &D.lc_mask))) return rc2;
-    if ((rc2 = upload(c, h, ccolk.data(), ccolk.size(), &D.lc_colk))) return rc2;
+    if ((rc = upload(c, h, lslots.data(), lslots.size(), &D.l_perm))) return rc;
+    if ((rc = upload(c, h, slot_of.data(), slot_of.size(), &D.l_slot))) return rc;
+    if ((rc = upload(c, h, lch.data(), lch.size(), &D.l_chunk))) return rc;
+    if ((rc = upload(c, h, cxyz.data(), cxyz.size(), &D.l_xyz))) return rc;
+    if ((rc = upload(c, h, cmodes.data(), cmodes.size(), &D.l_modes))) return rc;
+    if ((rc = upload(c, h, cmask.data(), cmask.size(), &D.l_mask))) return rc;
+    if ((rc = upload(c, h, ccol.data(), ccol.size(), &D.l_col))) return rc;
+    if ((rc = upload(c, h, cq.data(), cq.size(), &D.l_q))) return rc;
+    if ((rc = upload(c, h, clj.data(), clj.size(), &D.l_lj))) return rc;
   }
-  std::vector<int> lcol(d.n_lig), llj(d.n_lig, 0);
-  std::vector<float> lq(d.n_lig, 0.f);
-  for (int j = 0; j < d.n_lig; ++j) {
-    lcol[j] = d.lig_dfire_type[j] * SD_DFIRE_BINS;
-    if (d.lig_charge) lq[j] = (float)d.lig_charge[j];
-    if (d.lig_lj_type) llj[j] = d.lig_lj_type[j];
-  }
-  if ((rc = upload(c, h, d.lig_xyz, (size_t)d.n_lig * 3, &D.l_xyz))) return rc;
-  if ((rc = upload(c, h, d.lig_modes, (size_t)D.nml * d.n_lig * 3, &D.l_modes))) return rc;
-  if ((rc = upload(c, h, d.lig_mask, (size_t)d.n_lig, &D.l_mask))) return rc;
-  if ((rc = upload(c, h, lcol.data(), lcol.size(), &D.l_col))) return rc;
-  if ((rc = upload(c, h, lq.data(), lq.size(), &D.l_q))) return rc;
-  if ((rc = upload(c, h, llj.data(), llj.size(), &D.l_lj))) return rc;
 
   const size_t n = (size_t)D.S * D.G;
   if ((rc = alloc_dev(h, n * D.pl, &D.pos))) return rc;
@@ -458,21 +457,40 @@ int grow_spill(sd_ctx* c, size_t bytes) {
 // a CTA may use, the spill instantiation is chosen (no dynamic shared memory) and the context's
 // spill scratch is sized to grid x per-CTA bytes; alloc = false refuses that instead of allocating.
 int configure_score_v(sd_ctx* c, int precision, int variant, int* grid, size_t* smem, bool alloc = true) {
-  const size_t need = score_smem_bytes(precision, c->scoring, c->max_nr, c->max_nl, variant);
+  const size_t need = score_smem_bytes(precision, c->scoring, c->max_nr, c->max_nl, 1);
   const void* k = score_kernel_ptr(precision, c->scoring, variant, false);
   cudaFuncAttributes fa;
   SD_CUDA(cudaFuncGetAttributes(&fa, k));
-  const bool spill = need + fa.sharedSizeBytes > (size_t)c->smem_optin;
-  size_t sm = need;
+  size_t sm = need + score_warp_bytes(precision, c->scoring, variant, false);
+  const bool spill = sm + fa.sharedSizeBytes > (size_t)c->smem_optin;
   int threads = score_threads_of(precision, c->scoring, variant);
   if (spill) {
     k = score_kernel_ptr(precision, c->scoring, variant, true);
-    sm = 0;
+    sm = score_warp_bytes(precision, c->scoring, variant, true);
     threads = score_threads_spill(precision, c->scoring);
   }
-  SD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(sm, 1)));
   int per_sm = 0;
-  SD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, sm));
+  auto occupancy = [&](size_t bytes) -> int {
+    SD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(bytes, 1)));
+    SD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, bytes));
+    return SD_OK;
+  };
+  int rc;
+  if ((rc = occupancy(sm))) return rc;
+  // two poses per CTA wherever their arrays leave as many CTAs resident as one pose's
+  c->score_poses = 1;
+  if (!spill && precision == SD_PREC_MIXED && c->scoring == SD_SCORING_DFIRE) {
+    const int one = per_sm;
+    const size_t two = sm - need + score_smem_bytes(precision, c->scoring, c->max_nr, c->max_nl, 2);
+    if (two + fa.sharedSizeBytes <= (size_t)c->smem_optin) {
+      if ((rc = occupancy(two))) return rc;
+      if (per_sm == one) {
+        c->score_poses = 2;
+        sm = two;
+      }
+    }
+    if (c->score_poses == 1 && (rc = occupancy(sm))) return rc;
+  }
   if (per_sm < 1) return fail(SD_ERR_ARG, "scoring kernel does not fit on an SM (shared memory)");
   *grid = per_sm * c->nsm;
   *smem = sm;
@@ -483,7 +501,7 @@ int configure_score_v(sd_ctx* c, int precision, int variant, int* grid, size_t* 
     if (c->s_spill.bytes < stride * (size_t)*grid) {
       if (!alloc) return fail(SD_ERR_NOTSUP, "complex too large for shared memory: its scorer needs the context's "
                                              "global scratch, which this call may not allocate");
-      int rc = grow_spill(c, stride * (size_t)*grid);
+      rc = grow_spill(c, stride * (size_t)*grid);
       if (rc) return rc;
     }
     c->spill_stride = stride;
@@ -497,6 +515,7 @@ int configure_score(sd_ctx* c, int precision, int* grid, size_t* smem, bool allo
 
 // the spill scratch of the last configured launch (null pointers when it uses shared memory)
 void set_spill(const sd_ctx* c, ScoreLaunch& L) {
+  L.poses_per_cta = c->score_poses;
   L.spill = c->score_spill ? (unsigned char*)c->s_spill.p : nullptr;
   L.spill_stride = c->score_spill ? c->spill_stride : 0;
 }
@@ -568,7 +587,6 @@ int autotune_mixed(sd_ctx* c) {
   L.ctl = c->d_ctl_scratch;
   L.work[0] = L.work[1] = (const int*)c->s_work.p;
   L.table64 = c->d_table64;
-  L.tablek = c->d_tablek;
   L.lj_eps = c->d_lj_eps;
   L.lj_sigma = c->d_lj_sigma;
   cudaEvent_t e0, e1;
@@ -588,6 +606,7 @@ int autotune_mixed(sd_ctx* c) {
       c->tune_ms[v] = -1;
       break;
     }
+    set_spill(c, L);
     double vbest = 1e300;
     for (int rep = 0; rep < 3; ++rep) {
       ctl.grab[0] = ctl.grab[1] = 0;
@@ -622,7 +641,6 @@ int enqueue_step(sd_ctx* c, int precision, int grid, size_t sm) {
   L.work[0] = c->d_work[0];
   L.work[1] = c->d_work[1];
   L.table64 = c->d_table64;
-  L.tablek = c->d_tablek;
   L.lj_eps = c->d_lj_eps;
   L.lj_sigma = c->d_lj_sigma;
   L.energy_out = nullptr;
@@ -673,7 +691,6 @@ int ctx_noalloc_view(sd_ctx* c, int ci, int precision, DevComplex* desc, ScoreLa
   memset(L, 0, sizeof *L);
   set_spill(c, *L);
   L->table64 = c->d_table64;
-  L->tablek = c->d_tablek;
   L->lj_eps = c->d_lj_eps;
   L->lj_sigma = c->d_lj_sigma;
   *device = c->device;
@@ -719,7 +736,7 @@ int sd_ctx_create(const sd_complex_desc* complexes, int n_complexes, const sd_ta
   // device memory the context will hold (tables, per-complex data, state, work lists), checked
   // against SPARKLE_DEVICE_BUDGET_MB when set (a forced budget, e.g. to test the OOM path)
   {
-    size_t bytes = (size_t)(SD_TABLE_SIZE + 32) * 12 + (size_t)(SD_TABLE_KEYS + 32) * 8 + 4096;
+    size_t bytes = (size_t)(SD_TABLE_SIZE + 32) * 12 + 4096;
     for (int i = 0; i < n_complexes; ++i) {
       const sd_complex_desc& d = complexes[i];
       const size_t nr = (size_t)((d.n_rec + SD_TILE - 1) / SD_TILE) * SD_TILE, nl = (size_t)d.n_lig;
@@ -783,7 +800,6 @@ int sd_ctx_create(const sd_complex_desc* complexes, int n_complexes, const sd_ta
   if ((rc = cu(cudaMalloc(&c->d_cplx, sizeof(DevComplex) * n_complexes), "cudaMalloc"))) return bail(rc);
   if ((rc = cu(cudaMalloc(&c->d_cplx_scratch, sizeof(DevComplex) * n_complexes), "cudaMalloc"))) return bail(rc);
   if ((rc = cu(cudaMalloc(&c->d_table64, sizeof(double) * (SD_TABLE_SIZE + 32)), "cudaMalloc"))) return bail(rc);
-  if ((rc = cu(cudaMalloc(&c->d_tablek, sizeof(double) * (SD_TABLE_KEYS + 32)), "cudaMalloc"))) return bail(rc);
   if ((rc = cu(cudaMalloc(&c->d_lj_eps, sizeof(double) * SD_LJ_TYPES), "cudaMalloc"))) return bail(rc);
   if ((rc = cu(cudaMalloc(&c->d_lj_sigma, sizeof(double) * SD_LJ_TYPES), "cudaMalloc"))) return bail(rc);
   if ((rc = cu(cudaMalloc(&c->d_ctl, sizeof(StepCtl)), "cudaMalloc"))) return bail(rc);
@@ -803,15 +819,6 @@ int sd_ctx_create(const sd_complex_desc* complexes, int n_complexes, const sd_ta
       if (!std::isfinite(tables->dfire_energy[i])) return bail(fail(SD_ERR_NUMERIC, "non-finite DFIRE table entry"));
       t64[i] = tables->dfire_energy[i];
     }
-    // key-indexed copy: entry [tR][tL][k] is what the reference reads for key k, the flat index
-    // tR*3360 + tL*20 + dist_to_bins[k]-1 (key 29, d^2 == 225, reads bin 20: the next ligand
-    // type's bin 0, or the zero padding after the last type pair)
-    static const int kBin[30] = {0, 0, 0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 13, 14, 14, 15, 15, 16, 16, 17, 17, 18, 18, 19, 19, 20};
-    std::vector<double> tk((size_t)SD_TABLE_KEYS + 32, 0.0);
-    for (int a = 0; a < SD_DFIRE_TYPES; ++a)
-      for (int b = 0; b < SD_DFIRE_TYPES; ++b)
-        for (int k = 0; k < 30; ++k)
-          tk[(size_t)a * SD_ROWK + b * SD_KEYS + k] = t64[(size_t)a * SD_ROW + b * SD_DFIRE_BINS + kBin[k]];
     std::vector<double> eps(SD_LJ_TYPES, 0.0), sig(SD_LJ_TYPES, 0.0);
     if (tables->lj_eps && tables->lj_sigma)
       for (int i = 0; i < SD_LJ_TYPES; ++i) {
@@ -824,7 +831,6 @@ int sd_ctx_create(const sd_complex_desc* complexes, int n_complexes, const sd_ta
     StepCtl ctl;
     memset(&ctl, 0, sizeof ctl);
     if ((rc = cu(cudaMemcpy(c->d_table64, t64.data(), t64.size() * 8, cudaMemcpyHostToDevice), "upload"))) return bail(rc);
-    if ((rc = cu(cudaMemcpy(c->d_tablek, tk.data(), tk.size() * 8, cudaMemcpyHostToDevice), "upload"))) return bail(rc);
     if ((rc = cu(cudaMemcpy(c->d_lj_eps, eps.data(), eps.size() * 8, cudaMemcpyHostToDevice), "upload"))) return bail(rc);
     if ((rc = cu(cudaMemcpy(c->d_lj_sigma, sig.data(), sig.size() * 8, cudaMemcpyHostToDevice), "upload"))) return bail(rc);
     if ((rc = cu(cudaMemcpy(c->d_swarm_map, smap.data(), smap.size() * 4, cudaMemcpyHostToDevice), "upload"))) return bail(rc);
@@ -843,7 +849,7 @@ int sd_ctx_destroy(sd_ctx* c) {
   if (c->graph) cudaGraphExecDestroy(c->graph);
   for (auto& h : c->cx)
     for (void* p : h.owned) cudaFree(p);
-  void* ps[] = {c->d_cplx, c->d_cplx_scratch, c->d_table64, c->d_tablek, c->d_lj_eps, c->d_lj_sigma, c->d_ctl,
+  void* ps[] = {c->d_cplx, c->d_cplx_scratch, c->d_table64, c->d_lj_eps, c->d_lj_sigma, c->d_ctl,
                 c->d_ctl_scratch, c->d_work[0], c->d_work[1], c->d_swarm_map, c->d_pos_prev, c->s_pose.p, c->s_score.p,
                 c->s_ref.p, c->s_energy.p, c->s_work.p, c->s_grad.p, c->s_bins.p, c->s_spill.p};
   for (void* p : ps)
@@ -1094,7 +1100,6 @@ int sd_score_poses(sd_ctx* c, int ci, const double* poses, int n, int precision,
   L.work[0] = (const int*)c->s_work.p;
   L.work[1] = (const int*)c->s_work.p;
   L.table64 = c->d_table64;
-  L.tablek = c->d_tablek;
   L.lj_eps = c->d_lj_eps;
   L.lj_sigma = c->d_lj_sigma;
   L.energy_out = (double*)c->s_energy.p;
@@ -1189,7 +1194,6 @@ int sd_pydock_grad(sd_ctx* c, int ci, const double* poses, int n, int precision,
   L.work[0] = (const int*)c->s_work.p;
   L.work[1] = (const int*)c->s_work.p;
   L.table64 = c->d_table64;
-  L.tablek = c->d_tablek;
   L.lj_eps = c->d_lj_eps;
   L.lj_sigma = c->d_lj_sigma;
   L.energy_out = (double*)c->s_energy.p;

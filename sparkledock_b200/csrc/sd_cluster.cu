@@ -47,7 +47,7 @@ __global__ void materialise_backbone_kernel(const DevComplex* cplx, int ci, int 
     } else {
       double q[4] = {pose[3], pose[4], pose[5], pose[6]}, qi[4];
       quat_inverse(q, qi);
-      ligand_exact(C, lb_idx[a - nbr], pose, q, qi, x, y, z);
+      ligand_exact(C, C.l_slot[lb_idx[a - nbr]], pose, q, qi, x, y, z);
     }
     double* o = out + (size_t)i * 3;
     o[0] = x;
@@ -147,7 +147,7 @@ __global__ void materialise_poses_kernel(const DevComplex* cplx, int ci, const i
     } else {
       double q[4] = {pose[3], pose[4], pose[5], pose[6]}, qi[4];
       quat_inverse(q, qi);
-      ligand_exact(C, a - nr, pose, q, qi, x, y, z);
+      ligand_exact(C, C.l_slot[a - nr], pose, q, qi, x, y, z);
       o = lig + ((size_t)k * nl + (a - nr)) * 3;
     }
     o[0] = x;

@@ -15,12 +15,10 @@
 
 #define SD_TABLE_SIZE (SD_DFIRE_TYPES * SD_DFIRE_TYPES * SD_DFIRE_BINS)
 #define SD_ROW (SD_DFIRE_TYPES * SD_DFIRE_BINS)  /* 3360 */
-#define SD_KEYS 32              /* bin keys per type pair in the key-indexed table (30 used) */
-#define SD_ROWK (SD_DFIRE_TYPES * SD_KEYS)        /* 5376 */
-#define SD_TABLE_KEYS (SD_DFIRE_TYPES * SD_ROWK)  /* key-indexed table entries, followed by 32 zeros */
 #define SD_CUTOFF2 225.0
 #define SD_MAX_COMPLEX 32
 #define SD_TILE 32              /* receptor atoms per tile (one warp lane each) */
+#define SD_GROUP 8              /* consecutive atoms of a tile that are compact by themselves */
 #define SD_MAX_LIG 65504        /* ligand atoms: the mixed scorer's 16-bit ligand slot indices */
 #define SD_MAX_REC (1 << 22)    /* receptor atoms */
 #define SD_MAX_G 1024           /* glowworms per swarm with one thread each (one CTA per swarm) */
@@ -65,30 +63,24 @@ struct DevComplex {
   int gbase, sbase;     // first global glowworm / swarm index of this complex
   // receptor in tile order (slot = tile*32 + lane); padded slots have orig = -1
   const int* r_orig;
-  const double* r_xyz;     // [nslots][3]
-  const double* r_modes;   // [nmr][nslots][3]
+  const double* r_xyz;     // [3][nslots]
+  const double* r_modes;   // [nmr][3][nslots]
   const int* r_mask;       // [nslots]
   const int* r_row;        // [nslots] DFIRE row base tR*3360
-  const int* r_rowk;       // [nslots] key-indexed row base tR*5376
   const float4* r_tile;    // [ntiles] centre (rest frame) + radius
   const float* r_q;        // [nslots] charge (pyDock)
   const int* r_lj;         // [nslots] LJ type (pyDock)
-  // ligand in original order
-  const double* l_xyz;     // [nl][3]
-  const double* l_modes;   // [nml][nl][3]
-  const int* l_mask;
-  const int* l_col;        // [nl] tL*20
-  const float* l_q;
-  const int* l_lj;
-  // ligand in spatial chunks of 32 (mixed precision only; order-free sums)
+  // ligand in spatial chunks of 32 (slot = chunk*32 + lane; padded slots 0, with l_perm = -1)
   int nlchunks;
-  const int* l_perm;       // [nlchunks*32] chunk slot -> original ligand index, or -1
+  const int* l_perm;       // [nlchunks*32] slot -> original ligand index, or -1
+  const int* l_slot;       // [nl] original ligand index -> slot
   const float4* l_chunk;   // [nlchunks] centre (ligand frame) + radius
-  // the ligand again in chunk-slot order (coalesced reads in the mixed kernels; padding slots 0)
-  const double* lc_xyz;    // [nlchunks*32][3]
-  const double* lc_modes;  // [nml][nlchunks*32][3]
-  const int* lc_mask;      // [nlchunks*32]
-  const int* lc_colk;      // [nlchunks*32] key-indexed column base tL*32
+  const double* l_xyz;     // [3][nlchunks*32]
+  const double* l_modes;   // [nml][3][nlchunks*32]
+  const int* l_mask;
+  const int* l_col;        // [nlchunks*32] tL*20
+  const float* l_q;        // [nlchunks*32] charge, LJ type (pyDock)
+  const int* l_lj;
   float lig_ctr[3];        // ligand centroid (ligand frame)
   float mnorm_r[SD_MAX_MODES], mnorm_l[SD_MAX_MODES];  // max per-atom mode norm (rounded up)
   float lig_radius;        // max |l0_j| (rounded up)
@@ -135,9 +127,9 @@ struct ScoreLaunch {
   StepCtl* ctl;
   const int* work[2];
   const double* table64;   // [SD_TABLE_SIZE + 32] zero padded
-  const double* tablek;    // [SD_TABLE_KEYS + 32] key-indexed: [tR][tL][key] = table64[tR*3360 + tL*20 + bin(key)]
   const double* lj_eps;    // [20] pyDock
   const double* lj_sigma;
+  int poses_per_cta;       // mixed DFIRE: 2 when two poses' arrays fit, else 1
   double* energy_out;      // nullable [local glowworm] raw energies (stateless scoring)
   // per-CTA global scratch that replaces the dynamic shared memory of the spill instantiations
   // (complexes whose per-pose arrays do not fit in shared memory); null otherwise
@@ -160,7 +152,8 @@ struct GsoLaunch {
 // spill: the instantiation that keeps its per-pose arrays in L.spill instead of shared memory
 int score_launch(const ScoreLaunch& L, int precision, int scoring, int grid, int threads, size_t smem,
                  cudaStream_t st, int variant, bool spill);
-size_t score_smem_bytes(int precision, int scoring, int max_nr, int max_nl, int variant);
+size_t score_smem_bytes(int precision, int scoring, int max_nr, int max_nl, int poses);
+size_t score_warp_bytes(int precision, int scoring, int variant, bool spill);
 int score_threads_of(int precision, int scoring, int variant);
 int score_threads_spill(int precision, int scoring);
 const void* score_kernel_ptr(int precision, int scoring, int variant, bool spill);

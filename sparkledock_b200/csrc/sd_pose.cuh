@@ -31,67 +31,67 @@ __device__ __forceinline__ void quat_rotate(const double* q, const double* qi, d
   pz = (d0 * qi[3] + d1 * qi[2] - d2 * qi[1] + d3 * qi[0]);
 }
 
+// one atom plus its masked mode displacements, each multiply and add rounded: coordinates [3][n] and
+// modes [nm][3][n] in slot order, so a warp's consecutive slots read full lines
+__device__ __forceinline__ void anm_exact(const double* xyz, const double* modes, const int* mask, int n, int nm,
+                                          const double* ext, int slot, double& x, double& y, double& z) {
+  const size_t st = n;
+  const double* p = xyz + slot;
+  x = p[0];
+  y = p[st];
+  z = p[2 * st];
+  if (mask[slot] != 1) return;
+  const double* M = modes + slot;
+#pragma unroll 2
+  for (int m = 0; m < nm; ++m, M += 3 * st) {
+    const double e = ext[m];
+    x += M[0] * e;
+    y += M[st] * e;
+    z += M[2 * st] * e;
+  }
+}
+
 // receptor atom in tile slot `slot`, extents e_rec = pose + 7
 __device__ __forceinline__ void receptor_exact(const DevComplex& C, int nslots, int slot, const double* pose,
                                                double& x, double& y, double& z) {
-  x = C.r_xyz[slot * 3];
-  y = C.r_xyz[slot * 3 + 1];
-  z = C.r_xyz[slot * 3 + 2];
-  const int mk = C.r_mask[slot];
-  for (int m = 0; m < C.nmr; ++m) {
-    const double e = pose[7 + m];
-    const double* M = C.r_modes + ((size_t)m * nslots + slot) * 3;
-    if (mk == 1) {
-      x += M[0] * e;
-      y += M[1] * e;
-      z += M[2] * e;
-    }
-  }
+  anm_exact(C.r_xyz, C.r_modes, C.r_mask, nslots, C.nmr, pose + 7, slot, x, y, z);
 }
 
-// ligand atom j (original order)
-__device__ __forceinline__ void ligand_exact(const DevComplex& C, int j, const double* pose, const double* q,
+// ligand atom in chunk slot s
+__device__ __forceinline__ void ligand_exact(const DevComplex& C, int s, const double* pose, const double* q,
                                              const double* qi, double& x, double& y, double& z) {
-  x = C.l_xyz[j * 3];
-  y = C.l_xyz[j * 3 + 1];
-  z = C.l_xyz[j * 3 + 2];
-  const int mk = C.l_mask[j];
-  for (int m = 0; m < C.nml; ++m) {
-    const double e = pose[7 + C.nmr + m];
-    const double* M = C.l_modes + ((size_t)m * C.nl + j) * 3;
-    if (mk == 1) {
-      x += M[0] * e;
-      y += M[1] * e;
-      z += M[2] * e;
-    }
-  }
+  anm_exact(C.l_xyz, C.l_modes, C.l_mask, C.nlchunks * SD_TILE, C.nml, pose + 7 + C.nmr, s, x, y, z);
   quat_rotate(q, qi, x, y, z);
   x += pose[0];
   y += pose[1];
   z += pose[2];
 }
 
-// ligand atom in chunk slot s (chunk-ordered copies, same arithmetic as ligand_exact)
-__device__ __forceinline__ void ligand_exact_chunk(const DevComplex& C, int s, const double* pose, const double* q,
-                                                   const double* qi, double& x, double& y, double& z) {
-  const int nls = C.nlchunks * SD_TILE;
-  x = C.lc_xyz[s * 3];
-  y = C.lc_xyz[s * 3 + 1];
-  z = C.lc_xyz[s * 3 + 2];
-  const int mk = C.lc_mask[s];
-  for (int m = 0; m < C.nml; ++m) {
-    const double e = pose[7 + C.nmr + m];
-    const double* M = C.lc_modes + ((size_t)m * nls + s) * 3;
-    if (mk == 1) {
-      x += M[0] * e;
-      y += M[1] * e;
-      z += M[2] * e;
+// the same displacement for kP poses (extents estride doubles apart) with fused multiply-adds (half
+// the FP64 instructions) and one read of the modes, for coordinates that are then rounded to FP32:
+// the difference is of the order of an FP64 rounding
+template <int kP>
+__device__ __forceinline__ void anm_fused(const double* xyz, const double* modes, const int* mask, int n, int nm,
+                                          const double* ext, int estride, int slot, double (&r)[kP][3]) {
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double v = xyz[slot + d * n];
+#pragma unroll
+    for (int p = 0; p < kP; ++p) r[p][d] = v;
+  }
+  if (mask[slot] != 1) return;
+  int o = slot;
+#pragma unroll 5
+  for (int m = 0; m < nm; ++m, o += 3 * n) {
+    const double M0 = modes[o], M1 = modes[o + n], M2 = modes[o + 2 * n];
+#pragma unroll
+    for (int p = 0; p < kP; ++p) {
+      const double e = ext[p * estride + m];
+      r[p][0] = fma(M0, e, r[p][0]);
+      r[p][1] = fma(M1, e, r[p][1]);
+      r[p][2] = fma(M2, e, r[p][2]);
     }
   }
-  quat_rotate(q, qi, x, y, z);
-  x += pose[0];
-  y += pose[1];
-  z += pose[2];
 }
 
 __device__ __forceinline__ int nslots_of(const DevComplex& C) { return C.ntiles * SD_TILE; }

@@ -94,9 +94,10 @@ __device__ __forceinline__ T warp_sum(T v) {
 
 // out_grad: nullable [n][6 + nmr + nml] (GRAD), energies go to C.scoring as score (-E) and to
 // L.energy_out (E) when set.  kSpill: the per-pose arrays live in this CTA's slice of the global
-// scratch L.spill instead of shared memory (ligands too large for it).
+// scratch L.spill instead of shared memory (ligands too large for it).  Four CTAs per SM (64
+// registers a thread) wherever the accumulators allow it: the pair terms are latency chains.
 template <class T, bool GRAD, bool kSpill>
-__global__ void __launch_bounds__(kPdWarps * 32) pydock_kernel(ScoreLaunch L, double* out_grad) {
+__global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4) pydock_kernel(ScoreLaunch L, double* out_grad) {
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   unsigned char* const smem = kSpill ? L.spill + (size_t)blockIdx.x * L.spill_stride : smem_dyn;
   __shared__ double sh_pose[7 + 2 * SD_MAX_MODES];
@@ -173,16 +174,13 @@ __global__ void __launch_bounds__(kPdWarps * 32) pydock_kernel(ScoreLaunch L, do
     T* fz = fy + (GRAD ? nls : 0);
     float4* chS = reinterpret_cast<float4*>(fz + (GRAD ? nls : 0));
     int* llj = reinterpret_cast<int*>(chS + nlc);
-    int* lorig = llj + nls;
-    int* tlist = lorig + nls;
+    int* tlist = llj + nls;
     for (int s = tid; s < nls; s += blockDim.x) {
-      const int j = C.l_perm[s];
-      lorig[s] = j;
-      if (j >= 0) {
+      if (C.l_perm[s] >= 0) {
         double x, y, z;
-        ligand_exact(C, j, sh_pose, sh_q, sh_qi, x, y, z);
-        la[s] = LigAtom<T>{(T)(x - tx), (T)(y - ty), (T)(z - tz), (T)(kKe * (double)C.l_q[j])};
-        llj[s] = C.l_lj[j] * SD_LJ_TYPES;
+        ligand_exact(C, s, sh_pose, sh_q, sh_qi, x, y, z);
+        la[s] = LigAtom<T>{(T)(x - tx), (T)(y - ty), (T)(z - tz), (T)(kKe * (double)C.l_q[s])};
+        llj[s] = C.l_lj[s] * SD_LJ_TYPES;
       } else {
         la[s] = LigAtom<T>{(T)1e18, (T)1e18, (T)1e18, T(0)};
         llj[s] = 0;
@@ -353,8 +351,8 @@ __global__ void __launch_bounds__(kPdWarps * 32) pydock_kernel(ScoreLaunch L, do
       }
       if (GRAD && active && C.r_mask[slot] == 1) {
         for (int m = 0; m < C.nmr; ++m) {
-          const double* M = C.r_modes + ((size_t)m * nslots + slot) * 3;
-          grec[m] += (T)M[0] * gx + (T)M[1] * gy + (T)M[2] * gz;
+          const double* M = C.r_modes + (size_t)m * 3 * nslots + slot;
+          grec[m] += (T)M[0] * gx + (T)M[nslots] * gy + (T)M[2 * (size_t)nslots] * gz;
         }
       }
     }
@@ -384,8 +382,7 @@ __global__ void __launch_bounds__(kPdWarps * 32) pydock_kernel(ScoreLaunch L, do
         Rm[8] = (w0 * w0 - x * x - y * y + z * z) / n2;
       }
       for (int s = tid; s < nls; s += blockDim.x) {
-        const int j = lorig[s];
-        if (j < 0) continue;
+        if (C.l_perm[s] < 0) continue;
         const double Fx = (double)fx[s], Fy = (double)fy[s], Fz = (double)fz[s];
         const double px = (double)la[s].x, py = (double)la[s].y, pz = (double)la[s].z;  // l_j - t
         acc[1] += Fx;
@@ -394,12 +391,13 @@ __global__ void __launch_bounds__(kPdWarps * 32) pydock_kernel(ScoreLaunch L, do
         acc[4] += py * Fz - pz * Fy;
         acc[5] += pz * Fx - px * Fz;
         acc[6] += px * Fy - py * Fx;
-        if (C.l_mask[j] == 1)
+        if (C.l_mask[s] == 1)
           for (int m = 0; m < C.nml; ++m) {
-            const double* M = C.l_modes + ((size_t)m * C.nl + j) * 3;
-            const double RMx = Rm[0] * M[0] + Rm[1] * M[1] + Rm[2] * M[2];
-            const double RMy = Rm[3] * M[0] + Rm[4] * M[1] + Rm[5] * M[2];
-            const double RMz = Rm[6] * M[0] + Rm[7] * M[1] + Rm[8] * M[2];
+            const double* M = C.l_modes + (size_t)m * 3 * nls + s;
+            const double M0 = M[0], M1 = M[nls], M2 = M[2 * (size_t)nls];
+            const double RMx = Rm[0] * M0 + Rm[1] * M1 + Rm[2] * M2;
+            const double RMy = Rm[3] * M0 + Rm[4] * M1 + Rm[5] * M2;
+            const double RMz = Rm[6] * M0 + Rm[7] * M1 + Rm[8] * M2;
             acc[1 + 6 + C.nmr + m] += RMx * Fx + RMy * Fy + RMz * Fz;
           }
       }
@@ -427,7 +425,7 @@ __global__ void __launch_bounds__(kPdWarps * 32) pydock_kernel(ScoreLaunch L, do
 size_t pydock_smem_bytes(int precision, bool grad, int max_nl, int max_nr) {
   const size_t nlc = (size_t)(max_nl + SD_TILE - 1) / SD_TILE, nls = nlc * SD_TILE;
   const size_t ts = precision == SD_PREC_MIXED ? 4 : 8;
-  return ts * nls * (4 + (grad ? 3 : 0)) + 16 * nlc + 4 * nls * 2 + 4 * ((max_nr + SD_TILE - 1) / SD_TILE) + 16;
+  return ts * nls * (4 + (grad ? 3 : 0)) + 16 * nlc + 4 * nls + 4 * ((max_nr + SD_TILE - 1) / SD_TILE) + 16;
 }
 
 const void* pydock_kernel_ptr(int precision, bool grad, bool spill) {

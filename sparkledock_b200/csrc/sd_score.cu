@@ -145,10 +145,12 @@ __global__ void __launch_bounds__(kFp64Threads) dfire_score_kernel(ScoreLaunch L
       sh_ntile = 0;
       sh_next = 0;
     }
-    for (int j = tid; j < nl; j += blockDim.x) {
+    for (int s = tid; s < C.nlchunks * SD_TILE; s += blockDim.x) {
+      const int j = C.l_perm[s];
+      if (j < 0) continue;
       double x, y, z;
-      ligand_exact(C, j, sh_pose, sh_q, sh_qi, x, y, z);
-      const int col = C.l_col[j];
+      ligand_exact(C, s, sh_pose, sh_q, sh_qi, x, y, z);
+      const int col = C.l_col[s];
       ligF[j] = make_float4((float)(x - tx), (float)(y - ty), (float)(z - tz), __int_as_float(col));
       ligD[j] = LigD{x, y, z, col, 0};
     }
@@ -312,28 +314,39 @@ struct MixedVariant {
   int min_blocks;
 };
 #define SD_MIXED(W, B) { (const void*)dfire_score_mixed_kernel<W, B, false>, W, B }
-// variant 0 (the default before the autotuner has run) is the fastest measured on the
-// 3002 / 1274-atom workload.  The variants give bit-identical energies (same per-tile work and
-// summation order), so the tuner's choice never changes a result.
+// 24 or 28 warps per SM in all of them (80 or 72 registers a thread).  Fewer and larger CTAs hold fewer
+// copies of the ligand in shared memory and leave L1 more room for gathers in flight; smaller ones
+// lose less at the end of a batch.  Measured (M poses/s for 12x2, 14x2, 8x3, 6x4): 757/481 atoms 7.2,
+// 7.0, 9.3, 9.6; 3002/1274 2.94, 2.98, 2.39, 2.78; 6032/1766 1.90, 1.50, 1.76, 1.41; 17307/1125 2.49,
+// 2.57, 2.04, 2.32.  Variant 0 is the default before the autotuner has run.  The variants give
+// bit-identical energies (same per-tile work and summation order), so the tuner's choice never changes
+// a result.
 static const MixedVariant kMixedVariants[] = {
-    SD_MIXED(8, 3), SD_MIXED(4, 5), SD_MIXED(4, 4), SD_MIXED(8, 2),
+    SD_MIXED(12, 2), SD_MIXED(14, 2), SD_MIXED(8, 3), SD_MIXED(6, 4),
 };
 // the spill instantiation of the mixed kernel: variant 0's shape (the per-tile work, and so every
 // energy, is the same in every variant)
-static const MixedVariant kMixedSpill = {(const void*)dfire_score_mixed_kernel<8, 3, true>, 8, 3};
+static const MixedVariant kMixedSpill = {(const void*)dfire_score_mixed_kernel<12, 2, true>, 12, 2};
 
 constexpr int kNumMixedVariants = sizeof(kMixedVariants) / sizeof(kMixedVariants[0]);
 static_assert(kNumMixedVariants <= SD_MAX_VARIANTS, "variant table");
 
 static const MixedVariant& mixed_variant(int v) { return kMixedVariants[v < 0 || v >= kNumMixedVariants ? 0 : v]; }
 
-size_t score_smem_bytes(int precision, int scoring, int max_nr, int max_nl, int variant) {
+// bytes of the mixed DFIRE scorer's per-warp buffers, in dynamic shared memory in front of the per-pose
+// arrays (alone there in the spill instantiation)
+size_t score_warp_bytes(int precision, int scoring, int variant, bool spill) {
+  if (scoring == SD_SCORING_PYDOCK || precision != SD_PREC_MIXED) return 0;
+  return sizeof(WarpBufs) * (spill ? kMixedSpill.warps : mixed_variant(variant).warps);
+}
+
+// bytes of a CTA's per-pose arrays; poses: of the mixed DFIRE scorer's batch (the others take one)
+size_t score_smem_bytes(int precision, int scoring, int max_nr, int max_nl, int poses) {
   if (scoring == SD_SCORING_PYDOCK) return pydock_smem_bytes(precision, false, max_nl, max_nr);
   if (precision == SD_PREC_MIXED) {
     const size_t nlc = (size_t)(max_nl + SD_TILE - 1) / SD_TILE;
     const size_t ntiles = (size_t)(max_nr + SD_TILE - 1) / SD_TILE;
-    (void)variant;  // every variant uses the same dynamic layout
-    return (size_t)8 * ((ntiles + 1) & ~(size_t)1) + (size_t)16 * (nlc * SD_TILE + nlc) + 4 * (3 * ntiles + nlc);
+    return poses * (8 * ((ntiles + 1) & ~(size_t)1) + 16 * (nlc * SD_TILE + 1 + nlc)) + 4 * (3 * ntiles + nlc);
   }
   return (size_t)16 * ((max_nl + 1) & ~1) + (size_t)32 * max_nl + (size_t)8 * max_nr +
          (size_t)12 * ((max_nr + SD_TILE - 1) / SD_TILE);
@@ -374,7 +387,7 @@ int score_launch(const ScoreLaunch& L, int precision, int scoring, int grid, int
                                                   : threads;
   ScoreLaunch l = L;
   void* args[] = {(void*)&l};
-  if (cudaLaunchKernel(fn, dim3(grid), dim3(nthreads), args, spill ? 0 : smem, st) != cudaSuccess) return SD_ERR_CUDA;
+  if (cudaLaunchKernel(fn, dim3(grid), dim3(nthreads), args, smem, st) != cudaSuccess) return SD_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? SD_OK : SD_ERR_CUDA;
 }
 
@@ -400,7 +413,7 @@ __global__ void dfire_bins_kernel(const DevComplex* cplx, int ci, const double* 
     if (orig < 0) continue;
     double rx, ry, rz, lx, ly, lz;
     receptor_exact(C, nslots, slot, pose, rx, ry, rz);
-    ligand_exact(C, j, pose, q, qi, lx, ly, lz);
+    ligand_exact(C, C.l_slot[j], pose, q, qi, lx, ly, lz);
     int bin = -1;
     if (precision != SD_PREC_MIXED) {
       const double ddx = rx - lx, ddy = ry - ly, ddz = rz - lz;

@@ -4,80 +4,150 @@
 // Same contract as the FP64 kernels: the energy of cdfire_calculate_dfire
 // (prepare_gso_tasks.cc:1522-1615) with every bin identical to the FP64 reference bin, FP64 sums
 // of FP64 table values, but in a free order, which the kernel uses:
-//  * persistent CTAs grab poses from the device work list; per pose the ligand is transformed
-//    (exact FP64, rounded to FP32 centred on the pose translation t) only for the spatial chunks
-//    of 32 atoms that some receptor tile within reach can reach, and the near receptor tiles are
-//    ordered largest-first (closest to the ligand centroid) so warps finish a pose together;
-//  * a warp takes a receptor tile (one lane per atom, FP64 ANM transform rounded to FP32),
-//    rejects ligand chunks by bounding spheres and ligand atoms by ballot, and stages the
-//    surviving candidates 32 at a time into one of two per-warp batch buffers, in the bit order
-//    of the stage-1 mask (candidate 2i at position i, 2i+1 at position 16+i);
-//  * stage 1 tests a pair with the dot-product form of the distance in packed FP16, three
-//    HFMA2 per two candidates: s = r.l - |l|^2/2 >= (|r|^2 - thr)/2, on coordinates centred on
-//    the tile centre.  thr is set per tile from a proven bound on the FP16 error (below), so
-//    every pair whose FP32 d^2 is within the cutoff passes; tiles or poses whose magnitudes
-//    would make the bound loose pass every candidate, and stage 2 filters exactly;
-//  * in-cutoff pairs are appended to a per-warp ring of 16-bit entries (buffer, position,
-//    receptor lane) by a warp scan; stage 2 drains it 64 entries per round (two per lane), reads
-//    the candidate and the receptor atom from 4-byte arrays and a float4 (mostly broadcast
-//    reads), recomputes the FP32 d^2 and takes the key from a fast reciprocal square root.  The
-//    key's edges ((k+1)/2)^2 and ((k+2)/2)^2 (the upper one stopped at the cutoff) are
-//    compared with d^2 - edge computed with one rounding against the FP32 error bound B, so a
-//    pair that is not near an edge has its FP64 bin proven; near pairs are recomputed from the
-//    exact FP64 transform (counted as fallbacks);
-//  * the table is gathered from a key-indexed copy [168][168][32] (entry k is the value the
-//    reference reads for key k, including the d^2 == 225 read of the next ligand type's bin 0),
-//    so no bin lookup is needed; a rejected or padding pair gathers a zero past the table instead
-//    of branching, and each round's gathers (through L2 only) are added by the next round, so
-//    they are in flight while the next round is evaluated.  Each lane sums its values in FP64
-//    (Kahan sums of an FP32-rounded table were measured to miss 1e-5 at 60k pairs per pose).
-//  * Fixed summation order: a tile's lane sums are reduced by warp shuffles when the tile is
-//    done and stored in a per-pose shared slot of that tile; at the pose end warp 0 adds the
-//    slots in a fixed order.  What happens inside a tile depends only on the pose and the tile,
-//    never on which warp took it or when, and no compiled variant changes it, so a pose's energy
-//    is the same bits in every run, every variant and every entry point.
+//  * persistent CTAs take poses from the device work list, two at a time while there are plenty
+//    (consecutive items are glowworms of one swarm, so they meet the same receptor tiles): one read
+//    of a tile's or chunk's modes serves both.  Per pose the ligand is transformed (FP64, rounded to
+//    FP32 centred on the pose translation t, stored negated) for the spatial chunks of 32 atoms that
+//    some receptor tile within reach can reach, and the near receptor tiles are ordered largest-first
+//    (closest to a ligand centroid) so warps finish a batch together;
+//  * a warp takes a receptor tile (one lane per atom, FP64 ANM transform rounded to FP32), rejects
+//    ligand chunks by bounding spheres and ligand atoms by the tile's sphere, and tests the survivors,
+//    32 at a time, against the bounding boxes of the tile's four groups of 8 atoms (boxes of the
+//    transformed atoms).  Each group has its own candidate list: the groups are small enough that 45 %
+//    of the pairs of a group and its candidates are inside the cutoff (21 % for a whole tile and its
+//    candidates), so every pair is evaluated where it stands, without a pre-filter or compaction;
+//  * a step evaluates 8 atoms x 8 candidates, two atoms per lane in packed FP32 (pair_terms): d^2, d by
+//    an approximate square root, the bin coordinate and its distance from the nearest edge.  A pair
+//    inside the cutoff and further from an edge than the proven FP32 error has its FP64 bin, and its
+//    value is gathered (through L2 only) and added by the next step, so that it is in flight while the
+//    next step is evaluated.  Pairs near an edge are found again after the group's loop and decided in
+//    FP64 from the exact transforms (counted as fallbacks).  Each lane sums its values in FP64 (Kahan
+//    sums of an FP32-rounded table were measured to miss 1e-5 at 60k pairs per pose);
+//  * fixed summation order: a tile's lane sums are reduced by warp shuffles when the tile is done and
+//    stored in a per-pose shared slot of that tile; at the end one warp per pose adds the slots in a
+//    fixed order.  What happens inside a tile depends only on the pose and the tile, never on which
+//    warp took it, when, or beside which other pose, and no compiled variant changes it, so a pose's
+//    energy is the same bits in every run, every variant and every entry point.
 //
-// FP16 bound (u = 2^-11, R >= |r - c| for the tile's atoms, Lb >= |l - c| for its candidates,
-// w = |l - c|^2 / 2):  |s_fp16 - (r.l - w)| <= u (2.001 R Lb + w) + 3u (1.002 R Lb + 1.001 w)
-// <= u (5.1 R Lb + 2.1 Lb^2) = Es, and the right-hand side rounds by at most u (R^2 + thr)/2 = Ea,
-// so thr = 225 + B + 2 Es + 2 Ea + 0.01 keeps every pair with FP32 d^2 <= 225 + B.
+// What bounds it: each gather is one sector from L2, and an SM receives about one per clock (random
+// 8-byte gathers alone measured 2.9e11/s on 148 SMs at 1965 MHz).  On 3002 / 1274 atoms (57 k pairs
+// in the cutoff per pose) it runs at 1.7e11 pairs/s, 0.58 of that; the modes' reads add a quarter to
+// the sectors (half of that before two poses shared them), and L1 must hold the gathers in flight, so
+// the shared memory a CTA takes costs speed too.  Measured on 8,000 to 20,000 poses, poses/s, against
+// the earlier kernel (FP16 pre-filter of tile x candidate pairs, a ring of in-cutoff pairs, one pose
+// per CTA): 3002/1274 2.36 M -> 2.97 M, 17307/1125 2.02 M -> 2.57 M, 6032/1766 1.34 M -> 1.90 M,
+// 757/481 6.9 M -> 9.5 M.
 #pragma once
 
 namespace sd {
 namespace {
 
-constexpr int kRingCap = 1088;  // < 64 left over + at most 32 x 32 from one batch
-constexpr int kZeroIdxKey = SD_TABLE_KEYS;   // a zero past the key-indexed table
+constexpr int kGroup = SD_GROUP;      // receptor atoms of a group (one row of 8 lanes)
+constexpr int kGroups = SD_TILE / kGroup;
+constexpr int kRow = 8;               // candidates of a step: 8 rows of 4 lanes, two atoms of the group per lane
+constexpr int kSteps = 1;             // steps in flight per block
+constexpr int kBlock = kSteps * kRow; // candidates of a block
+constexpr int kPoses = 2;             // poses of a batch: they share the reads of modes and tiles
+constexpr int kList = 160;            // candidates of a group between two drains of the lists
+constexpr int kNear = 16;             // pairs of a tile that may be decided in FP64 one by one
+constexpr float kMagic = 12582912.0f; // 1.5 * 2^23: adding it rounds to an integer in the low bits
+constexpr int kMagicBits = 0x4B400000;
 
-// exact FP64 key of one pair near a bin edge or the cutoff; -1 when the pair is outside the
-// cutoff; *edge = 1 for d^2 == 0, 2 for d^2 == 225 (inlined: measured fewer spills than a call)
-__device__ __forceinline__ int exact_pair_key(const DevComplex* C, int nslots, const double* pose,
-                                                     const double* q, const double* qi, const double* T, int slot,
-                                                     int j, int* edge) {
+// one pose of a CTA's batch
+struct __align__(16) PoseBufs {
+  double pose[7 + 2 * SD_MAX_MODES + 1];
+  double q[4], qi[4];
+  double rot[9 + 1];
+  float rotf[9];
+  float gc[3];                       // ligand centroid, rotated (centred on t)
+  float dR, dL, B;                   // bounds: receptor and ligand ANM displacement, FP32 error of d^2
+  float pad;
+};
+
+struct __align__(16) WarpBufs {
+  float4 rec[kPoses][SD_TILE];       // receptor atom of each lane centred on t, row bits
+  float4 box[2 * kGroups];           // centre and half extent of each group's bounding box
+  unsigned short list[kGroups][kList];  // each group's candidates: ligand slots
+  unsigned near[kNear];              // pairs to decide in FP64: ligand slot * 32 + receptor lane
+  unsigned short pend[64];           // pending candidate ligand slots of the tile (below SD_MAX_LIG)
+};
+
+// The table value of one pair decided in FP64 from the exact transforms (0 outside the cutoff); counts
+// the pair in cnt[0], d^2 == 0 in cnt[1], d^2 == 225 in cnt[2] and a pair inside the cutoff in cnt[3].
+// Not inlined: it is rare (about ten pairs of a pose), and inlined its registers slowed the pair loop.
+__device__ __noinline__ double decide_pair(const DevComplex& C, const double* pose, const double* q, const double* qi,
+                                           const double* T, const double* table, int slot, int s,
+                                           unsigned long long* cnt) {
   double rx, ry, rz, lx, ly, lz;
-  receptor_exact(*C, nslots, slot, pose, rx, ry, rz);
-  ligand_exact(*C, j, pose, q, qi, lx, ly, lz);
+  receptor_exact(C, nslots_of(C), slot, pose, rx, ry, rz);
+  ligand_exact(C, s, pose, q, qi, lx, ly, lz);
   const double dx = rx - lx, dy = ry - ly, dz = rz - lz;
   const double e2 = dx * dx + dy * dy + dz * dz;
-  *edge = 0;
-  if (!(e2 <= SD_CUTOFF2)) return -1;
+  atomicAdd(&cnt[0], 1ull);
+  if (!(e2 <= SD_CUTOFF2)) return 0.0;
+  atomicAdd(&cnt[3], 1ull);
+  int key = 0;
   if (e2 == 0.0) {
-    *edge = 1;
-    return 0;
+    atomicAdd(&cnt[1], 1ull);
+  } else {
+    key = exact_key(e2, T);
+    if (key == 29) atomicAdd(&cnt[2], 1ull);
   }
-  const int key = exact_key(e2, T);
-  if (key == 29) *edge = 2;
-  return key;
+  return table[C.r_row[slot] + C.l_col[s] + c_binlut[key]];
 }
 
-struct __align__(16) RingBufs {
-  float candf[4][64];        // x, y, z, col bits of [buffer][position]: ligand atom centred on t
-  __half candh[16][8];       // position pair i: {x(2i), x(2i+1), y.., y.., z.., z.., -w.., -w..}
-  float4 rec[32];            // receptor atom of each lane centred on t, row bits
-  unsigned short cslot[64];  // [buffer][position]: ligand chunk slot (exact fallback only)
-  unsigned short pend[64];   // pending candidate ligand slots (below SD_MAX_LIG)
-  unsigned short ring[kRingCap];  // (buffer << 10) | (position << 5) | lane
-};
+// two FP32 values in a 64-bit register, for the packed instructions of sm_100
+typedef unsigned long long float2x;
+__device__ __forceinline__ float2x pack2(float a, float b) {
+  float2x r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(float2x v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ float2x add2(float2x a, float2x b) {
+  float2x r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float2x mul2(float2x a, float2x b) {
+  float2x r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float2x fma2(float2x a, float2x b, float2x c) {
+  float2x r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Two pairs of a lane (two receptor atoms, one candidate l, coordinates negated): FP32 d^2, the
+// distance of the bin coordinate from the middle of its bin (0.5: on an edge) and the bin plus kMagicBits.
+// Bin coordinate of distance d: min(2d - 3, d + 5) (bins of 0.5 A below 8 A, of 1 A above; below 2 A all
+// bin 0), here less 0.5 so that rounding to the nearest integer is the floor, and no more than 20, so
+// that a pair well outside the cutoff (19.5) is not near an edge.
+__device__ __forceinline__ void pair_terms(float2x rx, float2x ry, float2x rz, const float4& l, float (&d2)[2],
+                                           float (&mid)[2], int (&bin)[2]) {
+  const float2x ex = add2(rx, pack2(l.x, l.x)), ey = add2(ry, pack2(l.y, l.y)), ez = add2(rz, pack2(l.z, l.z));
+  unpack2(fma2(ez, ez, fma2(ey, ey, mul2(ex, ex))), d2[0], d2[1]);
+  const float2x d = pack2(sqrt_approx(d2[0]), sqrt_approx(d2[1]));
+  float a0, a1, b0, b1;
+  unpack2(fma2(d, pack2(2.0f, 2.0f), pack2(-3.5f, -3.5f)), a0, a1);
+  unpack2(add2(d, pack2(4.5f, 4.5f)), b0, b1);
+  const float2x f = pack2(fminf(fminf(a0, b0), 20.0f), fminf(fminf(a1, b1), 20.0f));
+  const float2x fi = add2(f, pack2(kMagic, kMagic));
+  unpack2(add2(f, fma2(fi, pack2(-1.0f, -1.0f), pack2(kMagic, kMagic))), mid[0], mid[1]);
+  unpack2(fi, a0, a1);
+  bin[0] = max(__float_as_int(a0), kMagicBits);
+  bin[1] = max(__float_as_int(a1), kMagicBits);
+}
 
 }  // namespace
 
@@ -87,19 +157,14 @@ struct __align__(16) RingBufs {
 // scratch L.spill, for complexes too large for shared memory; the arithmetic is the same.
 template <int kWarps, int kMinBlocks, bool kSpill>
 __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) dfire_score_mixed_kernel(ScoreLaunch L) {
-  constexpr int kG = 64;  // entries per stage-2 round, two per lane
   constexpr int kSortMax = 512;        // near tiles ordered largest-first up to this many
   extern __shared__ __align__(16) unsigned char smem_dyn[];
-  unsigned char* const smem = kSpill ? L.spill + (size_t)blockIdx.x * L.spill_stride : smem_dyn;
-  __shared__ RingBufs wb[kWarps];
-  __shared__ double sh_pose[7 + 2 * SD_MAX_MODES];
-  __shared__ double sh_q[4], sh_qi[4];
+  WarpBufs* const wb = reinterpret_cast<WarpBufs*>(smem_dyn);
+  unsigned char* const smem =
+      kSpill ? L.spill + (size_t)blockIdx.x * L.spill_stride : smem_dyn + kWarps * sizeof(WarpBufs);
+  __shared__ PoseBufs sh_p[kPoses];
   __shared__ double sh_T[32];
-  __shared__ float sh_gc[3];      // ligand centroid, rotated (centred on t)
-  __shared__ double sh_red[1];
   __shared__ int sh_item, sh_ntile, sh_next;
-  __shared__ float sh_bound[4];
-  __shared__ float sh_rot[9];
   __shared__ unsigned long long sh_cnt[5];  // fallback, d2 == 0, d2 == 225, pairs, evaluations
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -111,414 +176,443 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) dfire_score_mixed_ker
   const int* work = L.work[parity];
   unsigned n_done = 0;
   const unsigned lt_mask = (1u << lane) - 1u;
-  RingBufs& W = wb[warp];
+  WarpBufs& W = wb[warp];
+  // the first n_pairs * 2 items are taken two at a time, the last ones (two rounds of the grid) one
+  // at a time, so that the CTAs finish together
+  const int n_pairs = L.poses_per_cta > 1 ? max(0, (count - 2 * (int)gridDim.x) / 2) : 0;
 
   for (;;) {
     __syncthreads();
     if (tid == 0) sh_item = atomicAdd(&ctl->grab[parity], 1);
     __syncthreads();
-    const int item = sh_item;
+    int item = sh_item < n_pairs ? 2 * sh_item : sh_item + n_pairs;
+    const int item_end = sh_item < n_pairs ? item + 2 : item + 1;
     if (item >= count) break;
-    const int w = work[item];
-    const int ci = wi_complex(w), p = wi_local(w);
-    const DevComplex& C = L.cplx[ci];
-    const int nslots = nslots_of(C), pl = C.pl, nlc = C.nlchunks;
-    const double* pose_g = C.pos + (size_t)p * pl;
-    if (tid < pl) sh_pose[tid] = pose_g[tid];
-    __syncthreads();
-    if (warp == 0) {
-      // pose prologue spread over warp 0: quaternion inverse (one division per lane, bit-identical
-      // to quat_inverse), FP32 rotation for culling, ANM displacement bounds, reference point
-      if (lane < 4) {
-        const double w0 = sh_pose[3], x = sh_pose[4], y = sh_pose[5], z = sh_pose[6];
+    while (item < item_end) {
+      const int ci = wi_complex(work[item]);
+      const int np = item + 1 < item_end && wi_complex(work[item + 1]) == ci ? 2 : 1;  // poses of this batch
+      const int first = wi_local(work[item]), second = wi_local(work[item + np - 1]);
+      item += np;
+      const DevComplex& C = L.cplx[ci];
+      const int nslots = nslots_of(C), pl = C.pl, nlc = C.nlchunks;
+      if (warp < np) {
+        // pose prologue, one warp per pose: quaternion inverse (one division per lane, bit-identical to
+        // quat_inverse), rotation matrix, ANM displacement bounds, reference point
+        PoseBufs& Q = sh_p[warp];
+        const int p = warp == 0 ? first : second;
+        const double* pose_g = C.pos + (size_t)p * pl;
+        if (lane < pl) Q.pose[lane] = pose_g[lane];
+        __syncwarp();
+        const double w0 = Q.pose[3], x = Q.pose[4], y = Q.pose[5], z = Q.pose[6];
         const double n2 = w0 * w0 + x * x + y * y + z * z;
-        const double qv = sh_pose[3 + lane];
-        sh_q[lane] = qv;
-        sh_qi[lane] = (lane == 0 ? qv : -qv) / n2;
-      }
-      {
-        const float qw = (float)sh_pose[3], qx = (float)sh_pose[4], qy = (float)sh_pose[5], qz = (float)sh_pose[6];
-        const float in = rsqrtf(qw * qw + qx * qx + qy * qy + qz * qz);
-        const float w0 = qw * in, x = qx * in, y = qy * in, z = qz * in;
-        float rv = 0.f;
-        switch (lane) {
-          case 0: rv = 1 - 2 * (y * y + z * z); break;
-          case 1: rv = 2 * (x * y - w0 * z); break;
-          case 2: rv = 2 * (x * z + w0 * y); break;
-          case 3: rv = 2 * (x * y + w0 * z); break;
-          case 4: rv = 1 - 2 * (x * x + z * z); break;
-          case 5: rv = 2 * (y * z - w0 * x); break;
-          case 6: rv = 2 * (x * z - w0 * y); break;
-          case 7: rv = 2 * (y * z + w0 * x); break;
-          case 8: rv = 1 - 2 * (x * x + y * y); break;
-          default: break;
+        if (lane < 4) {
+          const double qv = Q.pose[3 + lane];
+          Q.q[lane] = qv;
+          Q.qi[lane] = (lane == 0 ? qv : -qv) / n2;
         }
-        if (lane < 9) sh_rot[lane] = rv;
-      }
-      float tR = lane < C.nmr ? fabsf((float)sh_pose[7 + lane]) * C.mnorm_r[lane] : 0.f;
-      float tL = lane < C.nml ? fabsf((float)sh_pose[7 + C.nmr + lane]) * C.mnorm_l[lane] : 0.f;
-      for (int o = 16; o > 0; o >>= 1) {
-        tR += __shfl_xor_sync(0xffffffffu, tR, o);
-        tL += __shfl_xor_sync(0xffffffffu, tL, o);
-      }
-      __syncwarp();
-      if (lane < 3)
-        sh_gc[lane] = sh_rot[3 * lane] * C.lig_ctr[0] + sh_rot[3 * lane + 1] * C.lig_ctr[1] +
-                      sh_rot[3 * lane + 2] * C.lig_ctr[2];
-      if (lane == 0) {
-        const float dR = tR * 1.0001f + 1e-4f, dL = tL * 1.0001f + 1e-4f;
-        sh_bound[0] = dR;
-        sh_bound[1] = dL;
-        // bound of |FP32 d2 - FP64 d2| for pairs within 15.1 A (coordinates centred on t)
-        const float RL = C.lig_radius + dL;
-        const float u32 = 5.9604645e-8f;
-        sh_bound[2] = 2.0f * (2.02f * u32 * (26.2f * (2.0f * RL + 15.1f) + 228.0f) + 3.0f * u32 * 228.0f) + 1e-6f;
-        // ligand reference point (prepare_gso_tasks.cc:460, :513, :524-526)
-        double rx = C.lig_ref[0], ry = C.lig_ref[1], rz = C.lig_ref[2];
-        quat_rotate(sh_q, sh_qi, rx, ry, rz);
-        double* ref = C.ref + (size_t)p * 3;
-        ref[0] = rx + sh_pose[0];
-        ref[1] = ry + sh_pose[1];
-        ref[2] = rz + sh_pose[2];
-        sh_ntile = 0;
-        sh_next = 0;
-      }
-    }
-    __syncthreads();
-    const double tx = sh_pose[0], ty = sh_pose[1], tz = sh_pose[2];
-    const float dR = sh_bound[0], dL = sh_bound[1], B = sh_bound[2];
-    const int nls = nlc * SD_TILE, ntiles = C.ntiles;
-    double* tsum = reinterpret_cast<double*>(smem);  // [ntiles] FP64 energy of each tile of the pose
-    float4* ligS = reinterpret_cast<float4*>(tsum + ((ntiles + 1) & ~1));  // [nls] centred on t, col bits
-    float4* chS = ligS + nls;                        // [nlc] centre + radius
-    int* tlist = reinterpret_cast<int*>(chS + nlc);  // [ntiles] tiles within reach
-    int* tord = tlist + ntiles;                      // [ntiles] the same, largest first
-    float* tdist = reinterpret_cast<float*>(tord + ntiles);  // [ntiles]
-    int* cneed = reinterpret_cast<int*>(tdist + ntiles);     // [nlc] chunk within reach of a near tile
-    for (int c = tid; c < nlc; c += blockDim.x) {
-      const float4 cc = C.l_chunk[c];
-      const float X = sh_rot[0] * cc.x + sh_rot[1] * cc.y + sh_rot[2] * cc.z;
-      const float Y = sh_rot[3] * cc.x + sh_rot[4] * cc.y + sh_rot[5] * cc.z;
-      const float Z = sh_rot[6] * cc.x + sh_rot[7] * cc.y + sh_rot[8] * cc.z;
-      chS[c] = make_float4(X, Y, Z, cc.w + dL);
-      cneed[c] = 0;
-    }
-    for (int k = tid; k < ntiles; k += blockDim.x) tsum[k] = 0.0;
-    const float lig_reach = C.lig_radius + dL;
-    for (int k = tid; k < ntiles; k += blockDim.x) {
-      const float4 tile = C.r_tile[k];
-      const float cx = (float)((double)tile.x - tx), cy = (float)((double)tile.y - ty),
-                  cz = (float)((double)tile.z - tz);
-      const float reach = 15.0f + dR + SD_CULL_MARGIN + tile.w + lig_reach;
-      if (cx * cx + cy * cy + cz * cz <= reach * reach) {
-        // distance from the ligand centroid: the closest tiles have the most pairs
-        const int at = atomicAdd(&sh_ntile, 1);
-        const float ex = cx - sh_gc[0], ey = cy - sh_gc[1], ez = cz - sh_gc[2];
-        tlist[at] = k;
-        // a NaN distance (non-finite quaternion) ranks last: the ranking below must stay a strict
-        // total order, or tord would not be a permutation of the near tiles
-        const float dd = ex * ex + ey * ey + ez * ez;
-        tdist[at] = dd == dd ? dd : 3.0e38f;
-      }
-    }
-    __syncthreads();
-    const int ntile = sh_ntile;
-    const bool sorted = ntile <= kSortMax;
-    // which ligand chunks any near tile can reach (the same test as the per-tile one below, with
-    // 0.01 A to spare, so a chunk that is not needed is never read)
-    for (int t = warp; t < ntile; t += kWarps) {
-      const float4 tile = C.r_tile[tlist[t]];
-      const float cx = (float)((double)tile.x - tx), cy = (float)((double)tile.y - ty),
-                  cz = (float)((double)tile.z - tz);
-      const float rt = 15.0f + dR + SD_CULL_MARGIN + tile.w;
-      for (int c = lane; c < nlc; c += 32) {
-        const float4 ch = chS[c];
-        const float ex = ch.x - cx, ey = ch.y - cy, ez = ch.z - cz, r = rt + ch.w + 0.01f;
-        if (ex * ex + ey * ey + ez * ez <= r * r) cneed[c] = 1;
-      }
-    }
-    if (sorted) {
-      for (int t = tid; t < ntile; t += blockDim.x) {
-        const float d = tdist[t];
-        int rank = 0;
-        for (int u = 0; u < ntile; ++u) {
-          const float e = tdist[u];
-          rank += (e < d || (e == d && u < t)) ? 1 : 0;
+        {
+          // rotation matrix of the (possibly not normalised) quaternion, one element per lane
+          double rv = 0.0;
+          switch (lane) {
+            case 0: rv = w0 * w0 + x * x - y * y - z * z; break;
+            case 1: rv = 2 * (x * y - w0 * z); break;
+            case 2: rv = 2 * (x * z + w0 * y); break;
+            case 3: rv = 2 * (x * y + w0 * z); break;
+            case 4: rv = w0 * w0 - x * x + y * y - z * z; break;
+            case 5: rv = 2 * (y * z - w0 * x); break;
+            case 6: rv = 2 * (x * z - w0 * y); break;
+            case 7: rv = 2 * (y * z + w0 * x); break;
+            case 8: rv = w0 * w0 - x * x - y * y + z * z; break;
+            default: break;
+          }
+          rv /= n2;
+          if (lane < 9) {
+            Q.rot[lane] = rv;
+            Q.rotf[lane] = (float)rv;
+          }
         }
-        tord[rank] = tlist[t];
+        float tR = lane < C.nmr ? fabsf((float)Q.pose[7 + lane]) * C.mnorm_r[lane] : 0.f;
+        float tL = lane < C.nml ? fabsf((float)Q.pose[7 + C.nmr + lane]) * C.mnorm_l[lane] : 0.f;
+        for (int o = 16; o > 0; o >>= 1) {
+          tR += __shfl_xor_sync(0xffffffffu, tR, o);
+          tL += __shfl_xor_sync(0xffffffffu, tL, o);
+        }
+        __syncwarp();
+        if (lane < 3)
+          Q.gc[lane] = Q.rotf[3 * lane] * C.lig_ctr[0] + Q.rotf[3 * lane + 1] * C.lig_ctr[1] +
+                       Q.rotf[3 * lane + 2] * C.lig_ctr[2];
+        if (lane == 0) {
+          const float dR = tR * 1.0001f + 1e-4f, dL = tL * 1.0001f + 1e-4f;
+          Q.dR = dR;
+          Q.dL = dL;
+          // bound of |FP32 d2 - FP64 d2| for pairs within 15.1 A (coordinates centred on t)
+          const float RL = C.lig_radius + dL;
+          const float u32 = 5.9604645e-8f;
+          Q.B = 2.0f * (2.02f * u32 * (26.2f * (2.0f * RL + 15.1f) + 228.0f) + 3.0f * u32 * 228.0f) + 1e-6f;
+          // ligand reference point (prepare_gso_tasks.cc:460, :513, :524-526)
+          double rx = C.lig_ref[0], ry = C.lig_ref[1], rz = C.lig_ref[2];
+          quat_rotate(Q.q, Q.qi, rx, ry, rz);
+          double* ref = C.ref + (size_t)p * 3;
+          ref[0] = rx + Q.pose[0];
+          ref[1] = ry + Q.pose[1];
+          ref[2] = rz + Q.pose[2];
+          if (warp == 0) {
+            sh_ntile = 0;
+            sh_next = 0;
+          }
+        }
       }
-    }
-    __syncthreads();
-    auto lig_atom = [&](int s) {
-      if (s >= nls || !cneed[s >> 5]) return;
-      if (C.l_perm[s] >= 0) {
-        double x, y, z;
-        ligand_exact_chunk(C, s, sh_pose, sh_q, sh_qi, x, y, z);
-        ligS[s] = make_float4((float)(x - tx), (float)(y - ty), (float)(z - tz), __int_as_float(C.lc_colk[s]));
-      } else {
-        ligS[s] = make_float4(1e18f, 1e18f, 1e18f, __int_as_float(0));
+      __syncthreads();
+      const int nls = nlc * SD_TILE, ntiles = C.ntiles, tstride = (ntiles + 1) & ~1;
+      double* tsum = reinterpret_cast<double*>(smem);  // [np][tstride] FP64 energy of each tile of each pose
+      // [np][nls + 1] ligand atoms centred on t and negated, col bits; [nls] a far atom, the padding
+      float4* ligS = reinterpret_cast<float4*>(tsum + np * tstride);
+      float4* chS = ligS + np * (nls + 1);             // [np][nlc] centre + radius
+      int* tlist = reinterpret_cast<int*>(chS + np * nlc);  // [ntiles] tiles within reach: tile * 4 + poses (bits)
+      int* tord = tlist + ntiles;                      // [ntiles] the same, largest first
+      float* tdist = reinterpret_cast<float*>(tord + ntiles);  // [ntiles]
+      int* cneed = reinterpret_cast<int*>(tdist + ntiles);     // [nlc] chunk within reach of a near tile
+      for (int c = tid; c < nlc; c += blockDim.x) {
+        const float4 cc = C.l_chunk[c];
+        for (int p = 0; p < np; ++p) {
+          const float* R = sh_p[p].rotf;
+          const float X = R[0] * cc.x + R[1] * cc.y + R[2] * cc.z;
+          const float Y = R[3] * cc.x + R[4] * cc.y + R[5] * cc.z;
+          const float Z = R[6] * cc.x + R[7] * cc.y + R[8] * cc.z;
+          chS[p * nlc + c] = make_float4(X, Y, Z, cc.w + sh_p[p].dL);
+        }
+        cneed[c] = 0;
       }
-    };
-    for (int s = tid; s < nls; s += 2 * kWarps * 32) {
-      lig_atom(s);
-      lig_atom(s + kWarps * 32);
-    }
-    __syncthreads();
-    const int* tl = sorted ? tord : tlist;
-    const float cut2 = 225.0f + B;
-    double acc = 0.0;               // per-lane FP64 sum of table values
-    double pv0 = 0.0, pv1 = 0.0;    // values gathered by the previous round, added by the next
-    const double* table = L.tablek;
-    unsigned npairs = 0, nevals = 0;
-
-    for (;;) {
-      int ti = 0;
-      if (lane == 0) ti = atomicAdd(&sh_next, 1);
-      ti = __shfl_sync(0xffffffffu, ti, 0);
-      if (ti >= ntile) break;
-      const int k = tl[ti];
-      const float4 tile = C.r_tile[k];
-      const float cx = (float)((double)tile.x - tx), cy = (float)((double)tile.y - ty),
-                  cz = (float)((double)tile.z - tz);
-      const float reach = 15.0f + dR + SD_CULL_MARGIN + tile.w;
-      const float reach2 = reach * reach;
-      const int slot = k * SD_TILE + lane;
-      const bool active = C.r_orig[slot] >= 0;
-      float fx = 1e18f, fy = 1e18f, fz = 1e18f;
-      int row = 0;
-      if (active) {
-        double rx, ry, rz;
-        receptor_exact(C, nslots, slot, sh_pose, rx, ry, rz);
-        fx = (float)(rx - tx);
-        fy = (float)(ry - ty);
-        fz = (float)(rz - tz);
-        row = C.r_rowk[slot];
+      if (tid < np) ligS[tid * (nls + 1) + nls] = make_float4(3e18f, 3e18f, 3e18f, 0.f);
+      for (int k = tid; k < np * tstride; k += blockDim.x) tsum[k] = 0.0;
+      for (int k = tid; k < ntiles; k += blockDim.x) {
+        const float4 tile = C.r_tile[k];
+        int bits = 0;
+        float dmin = 3.0e38f;
+        for (int p = 0; p < np; ++p) {
+          const PoseBufs& Q = sh_p[p];
+          const float cx = (float)((double)tile.x - Q.pose[0]), cy = (float)((double)tile.y - Q.pose[1]),
+                      cz = (float)((double)tile.z - Q.pose[2]);
+          const float reach = 15.0f + Q.dR + SD_CULL_MARGIN + tile.w + (C.lig_radius + Q.dL);
+          if (cx * cx + cy * cy + cz * cz <= reach * reach) {
+            bits |= 1 << p;
+            // distance from the ligand centroid: the closest tiles have the most pairs; a NaN
+            // (non-finite quaternion) leaves 3e38, so the ranking below stays a strict total order
+            const float ex = cx - Q.gc[0], ey = cy - Q.gc[1], ez = cz - Q.gc[2];
+            dmin = fminf(dmin, ex * ex + ey * ey + ez * ez);
+          }
+        }
+        if (bits) {
+          const int at = atomicAdd(&sh_ntile, 1);
+          tlist[at] = k * 4 + bits;
+          tdist[at] = dmin;
+        }
       }
-      W.rec[lane] = make_float4(fx, fy, fz, __int_as_float(row));
-      const unsigned act_mask = __ballot_sync(0xffffffffu, active);
-      const int nact = __popc(act_mask);
-      // stage-1 constants of this lane
-      __half2 rx2, ry2, rz2, a2;
-      const float R = tile.w + dR + SD_CULL_MARGIN, Lb = reach + 0.01f;
-      const bool tight = R <= 40.0f && Lb <= 80.0f;  // warp-uniform
-      {
-        const float u16 = 4.8828125e-4f;
-        const float Es = u16 * (5.1f * R * Lb + 2.1f * Lb * Lb);
-        const float thr0 = 225.0f + B + 1e-3f + 2.0f * Es;
-        const float thr = thr0 + u16 * (R * R + thr0 + 10.0f) + 2e-4f + 0.01f;
-        const float ux = fx - cx, uy = fy - cy, uz = fz - cz;
-        const float a = 0.5f * (ux * ux + uy * uy + uz * uz) - 0.5f * thr;
-        const bool use = active && tight;
-        rx2 = __float2half2_rn(use ? ux : 0.f);
-        ry2 = __float2half2_rn(use ? uy : 0.f);
-        rz2 = __float2half2_rn(use ? uz : 0.f);
-        // loose tile: every candidate passes (s = 0 > -65504); inactive lane: none does
-        a2 = __float2half2_rn(!active ? 65504.f : (tight ? a : -65504.f));
+      __syncthreads();
+      const int ntile = sh_ntile;
+      const bool sorted = ntile <= kSortMax;
+      // which ligand chunks any near tile can reach (the same test as the per-tile one below, with
+      // 0.01 A to spare, so a chunk that is not needed is never read)
+      for (int t = warp; t < ntile; t += kWarps) {
+        const int kb = tlist[t];
+        const float4 tile = C.r_tile[kb >> 2];
+        for (int p = 0; p < np; ++p) {
+          if (!(kb >> p & 1)) continue;
+          const PoseBufs& Q = sh_p[p];
+          const float cx = (float)((double)tile.x - Q.pose[0]), cy = (float)((double)tile.y - Q.pose[1]),
+                      cz = (float)((double)tile.z - Q.pose[2]);
+          const float rt = 15.0f + Q.dR + SD_CULL_MARGIN + tile.w;
+          for (int c = lane; c < nlc; c += 32) {
+            const float4 ch = chS[p * nlc + c];
+            const float ex = ch.x - cx, ey = ch.y - cy, ez = ch.z - cz, r = rt + ch.w + 0.01f;
+            if (ex * ex + ey * ey + ez * ez <= r * r) cneed[c] = 1;
+          }
+        }
       }
-      int ncand = 0, head = 0, par = 0, oldL = 0;  // ring holds entries [0, head)
-      int cb = 0;
-      unsigned cm = 0;
+      if (sorted) {
+        for (int t = tid; t < ntile; t += blockDim.x) {
+          const float d = tdist[t];
+          int rank = 0;
+          for (int u = 0; u < ntile; ++u) {
+            const float e = tdist[u];
+            rank += (e < d || (e == d && u < t)) ? 1 : 0;
+          }
+          tord[rank] = tlist[t];
+        }
+      }
+      __syncthreads();
+      // the ligand of each pose (both from one read of its modes)
+      for (int s = tid; s < nls; s += kWarps * 32) {
+        if (!cneed[s >> 5]) continue;
+        if (C.l_perm[s] >= 0) {
+          double l[kPoses][3];
+          anm_fused<kPoses>(C.l_xyz, C.l_modes, C.l_mask, nls, C.nml, &sh_p[0].pose[7 + C.nmr],
+                            (int)(sizeof(PoseBufs) / sizeof(double)), s, l);
+          const float col = __int_as_float(C.l_col[s]);
+#pragma unroll
+          for (int p = 0; p < kPoses; ++p) {
+            if (p >= np) break;
+            const double* R = sh_p[p].rot;
+            ligS[p * (nls + 1) + s] = make_float4(-(float)fma(R[0], l[p][0], fma(R[1], l[p][1], R[2] * l[p][2])),
+                                                  -(float)fma(R[3], l[p][0], fma(R[4], l[p][1], R[5] * l[p][2])),
+                                                  -(float)fma(R[6], l[p][0], fma(R[7], l[p][1], R[8] * l[p][2])), col);
+          }
+        } else {
+          for (int p = 0; p < np; ++p) ligS[p * (nls + 1) + s] = make_float4(1e18f, 1e18f, 1e18f, __int_as_float(0));
+        }
+      }
+      __syncthreads();
+      const int* tl = sorted ? tord : tlist;
+      double acc = 0.0;           // per-lane FP64 sum of table values
+      double pv[2 * kSteps];      // values gathered by the previous block, added by the next
+#pragma unroll
+      for (int u = 0; u < 2 * kSteps; ++u) pv[u] = 0.0;
+      const double* table = L.table64;
+      unsigned pose_pairs = 0, pose_evals = 0;  // of this warp's tiles (pairs per lane)
 
       for (;;) {
-        // collect candidates until a batch is full or the ligand is exhausted
-        while (ncand < 32) {
-          if (cm == 0) {
-            if (cb >= nlc) break;
-            const int c = cb + lane;
-            bool cnear = false;
-            if (c < nlc) {
-              const float4 ch = chS[c];
-              const float ex = ch.x - cx, ey = ch.y - cy, ez = ch.z - cz, r = reach + ch.w;
-              cnear = ex * ex + ey * ey + ez * ez <= r * r;  // same expression as the cneed test
-            }
-            cm = __ballot_sync(0xffffffffu, cnear);
-            cb += 32;
-            continue;
+        int ti = 0;
+        if (lane == 0) ti = atomicAdd(&sh_next, 1);
+        ti = __shfl_sync(0xffffffffu, ti, 0);
+        if (ti >= ntile) break;
+        const int kb = tl[ti], k = kb >> 2;
+        const int slot = k * SD_TILE + lane;
+        const bool active = C.r_orig[slot] >= 0;
+        const unsigned act_mask = __ballot_sync(0xffffffffu, active);
+        {
+          // the tile's atoms in each pose, from one read of their modes
+          const int row = active ? C.r_row[slot] - kMagicBits : 0;
+          double r[kPoses][3];
+          anm_fused<kPoses>(C.r_xyz, C.r_modes, C.r_mask, nslots, C.nmr, &sh_p[0].pose[7],
+                            (int)(sizeof(PoseBufs) / sizeof(double)), slot, r);
+#pragma unroll
+          for (int p = 0; p < kPoses; ++p) {
+            const double* t = sh_p[p].pose;
+            W.rec[p][lane] = active ? make_float4((float)(r[p][0] - t[0]), (float)(r[p][1] - t[1]),
+                                                  (float)(r[p][2] - t[2]), __int_as_float(row))
+                                    : make_float4(1e18f, 1e18f, 1e18f, 0.f);
           }
-          const int sb = (cb - 32 + __ffs(cm) - 1) * SD_TILE;
-          cm &= cm - 1;
-          const float4 la = ligS[sb + lane];
-          const float ax = la.x - cx, ay = la.y - cy, az = la.z - cz;
-          const bool cand = fmaf(az, az, fmaf(ay, ay, ax * ax)) <= reach2;
-          const unsigned am = __ballot_sync(0xffffffffu, cand);
-          if (cand) W.pend[ncand + __popc(am & lt_mask)] = (unsigned short)(sb + lane);
-          ncand += __popc(am);
         }
-        const bool exhausted = cm == 0 && cb >= nlc;
-        if (ncand == 0 && head == 0) break;
-        const int nb = min(ncand, 32);
-        const bool final_batch = exhausted && ncand <= 32;
-        if (nb > 0) {
-          // stage the batch into buffer par, in mask bit order
+        for (int p = 0; p < np; ++p) {
+          if (!(kb >> p & 1)) continue;
+          const PoseBufs& Q = sh_p[p];
+          const float4 tile = C.r_tile[k];
+          const float cx = (float)((double)tile.x - Q.pose[0]), cy = (float)((double)tile.y - Q.pose[1]),
+                      cz = (float)((double)tile.z - Q.pose[2]);
+          const float reach = 15.0f + Q.dR + SD_CULL_MARGIN + tile.w;
+          const float reach2 = reach * reach;
+          const float cut2 = 225.0f + Q.B;
+          const float box_cut = 225.1f + Q.B;
+          // the bin coordinate's error: |d_fp32 - d| <= B / 30 inside the cutoff (B bounds d^2 there, its
+          // leading term is 2 d |error of the difference vector|), times the slope 2, plus FP32 roundings
+          // (square root 2^-22, coordinate up to 20).  If it reaches 0.5 no pair is settled in FP32
+          const float inner = 0.5f - (Q.B * 0.0673f + 2e-5f);
+          const float4* const lig = ligS + p * (nls + 1);
+          const float4* const rec = W.rec[p];
           __syncwarp();
-          const int pos = (lane >> 1) | ((lane & 1) << 4);
-          float4 l4 = make_float4(-1e18f, -1e18f, -1e18f, 0.f);
-          int s = 0;
-          if (lane < nb) {
-            s = W.pend[lane];
-            l4 = ligS[s];
-          }
-          W.candf[0][par * 32 + pos] = l4.x;
-          W.candf[1][par * 32 + pos] = l4.y;
-          W.candf[2][par * 32 + pos] = l4.z;
-          W.candf[3][par * 32 + pos] = l4.w;
-          W.cslot[par * 32 + pos] = (unsigned short)s;
           {
-            // unused place: s = -60000, never in range; loose tile: every place passes
-            float lx = 0.f, ly = 0.f, lz = 0.f, nw = tight ? -60000.f : 0.f;
-            if (lane < nb && tight) {
-              lx = l4.x - cx;
-              ly = l4.y - cy;
-              lz = l4.z - cz;
-              nw = fmaxf(-0.5f * (lx * lx + ly * ly + lz * lz), -60000.f);
+            // bounding box of each group of 8 lanes (an empty group's half extent is -inf: no candidate)
+            const float4 own = rec[lane];
+            float lo[3] = {own.x, own.y, own.z}, hi[3] = {own.x, own.y, own.z};
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+              if (!active) {
+                lo[d] = 3e38f;
+                hi[d] = -3e38f;
+              }
+#pragma unroll
+              for (int o = 1; o < kGroup; o <<= 1) {
+                lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+                hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+              }
             }
-            // lanes 2i and 2i+1 fill candh[i] with one 8-byte store each: the even lane the x and y
-            // pairs, the odd lane the z and w pairs (conflict-free, where 16-bit stores collide)
-            const __half2 xy = __floats2half2_rn(lx, ly), zw = __floats2half2_rn(lz, nw);
-            const bool odd = lane & 1;
-            const __half2 other = __shfl_xor_sync(0xffffffffu, odd ? xy : zw, 1);
-            const __half2 mine = odd ? zw : xy;
-            const __half2 lo = odd ? other : mine, hi = odd ? mine : other;  // even lane's, odd lane's
-            const __half2 o0 = __lows2half2(lo, hi), o1 = __highs2half2(lo, hi);
-            uint2 u;
-            u.x = reinterpret_cast<const unsigned&>(o0);
-            u.y = reinterpret_cast<const unsigned&>(o1);
-            *reinterpret_cast<uint2*>(reinterpret_cast<unsigned char*>(W.candh[lane >> 1]) + 8 * (lane & 1)) = u;
-          }
-          __syncwarp();
-          // stage 1: bit b of m <=> (this lane's receptor atom, candidate at position b) in range
-          unsigned M = 0;
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const uint4 qq = *reinterpret_cast<const uint4*>(W.candh[i]);
-            __half2 sv = __hfma2(rx2, *reinterpret_cast<const __half2*>(&qq.x), *reinterpret_cast<const __half2*>(&qq.w));
-            sv = __hfma2(ry2, *reinterpret_cast<const __half2*>(&qq.y), sv);
-            sv = __hfma2(rz2, *reinterpret_cast<const __half2*>(&qq.z), sv);
-            M |= __hge2_mask(sv, a2) & (0x00010001u << i);
-          }
-          const unsigned lo = (1u << ((nb + 1) >> 1)) - 1u, hi = (1u << (nb >> 1)) - 1u;
-          unsigned m = M & (lo | (hi << 16)) & (active ? 0xffffffffu : 0u);
-          nevals += lane == 0 ? (unsigned)(nb * nact) : 0u;
-          // append this lane's pairs to the ring
-          const int cnt = __popc(m);
-          int incl = cnt;
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-          }
-          const int total = __shfl_sync(0xffffffffu, incl, 31);
-          int at = head + incl - cnt;
-          const unsigned tag = ((unsigned)par << 10) | (unsigned)lane;
-          // two entries per iteration: the highest and the lowest bit left
-          while (m) {
-            const int b = 31 - __clz(m);
-            const unsigned low = m & (0u - m);
-            const int b2 = 31 - __clz(low);
-            m &= ~((1u << b) | low);
-            W.ring[at] = (unsigned short)(tag | ((unsigned)b << 5));
-            if (b2 != b) W.ring[at + 1] = (unsigned short)(tag | ((unsigned)b2 << 5));
-            at += b2 != b ? 2 : 1;
-          }
-          head += total;
-          // keep the candidates beyond the first 32
-          const int rest = ncand - nb;
-          int carry = 0;
-          if (lane < rest) carry = W.pend[32 + lane];
-          __syncwarp();
-          if (lane < rest) W.pend[lane] = (unsigned short)carry;
-          ncand = rest;
-          par ^= 1;
-        }
-        __syncwarp();
-        // stage 2: drain whole rounds of kG; everything at the end of the tile, or when entries
-        // of the previous batch would otherwise outlive its buffer
-        const int upto = (final_batch || (oldL > 0 && head < kG)) ? head : (head & ~(kG - 1));
-        auto pair = [&](int t0, int h, int n) -> int {
-          const unsigned e = W.ring[t0 + h * 32 + lane];
-          const int cix = (int)(e >> 5) & 63, rl = (int)e & 31;
-          const float4 rr = W.rec[rl];
-          const float ex = rr.x - W.candf[0][cix], ey = rr.y - W.candf[1][cix], ez = rr.z - W.candf[2][cix];
-          const int col = __float_as_int(W.candf[3][cix]);
-          const float d2 = fmaf(ez, ez, fmaf(ey, ey, ex * ex));
-          bool ok = (h * 32 + lane < n) && d2 <= cut2;
-          // key estimate; d2 == 0 gives NaN -> 0 and lies within B of edge 0 (exact path)
-          const float r = d2 * rsqrtf(d2);
-          const int key = (int)fmaf(r, 2.0f, -1.0f) & 31;
-          // key edges ((key+1)/2)^2 and ((key+2)/2)^2, differences with one rounding; the upper
-          // edge stops at the cutoff 15^2, so key 29 (d^2 == 225 only) always takes the exact
-          // path: the FP32 cut2 = 225 + B may round above 225 + B
-          int idx = __float_as_int(rr.w) + col + key;
-          const float hk = fmaf((float)key, 0.5f, 0.5f), hk1 = fminf(hk + 0.5f, 15.0f);
-          const bool near = fmaf(-hk, hk, d2) <= B || fmaf(hk1, hk1, -d2) <= B;
-          if (ok && near) {
-            atomicAdd(&sh_cnt[0], 1ull);
-            int edge;
-            const int kx = exact_pair_key(&C, nslots, sh_pose, sh_q, sh_qi, sh_T, k * SD_TILE + rl,
-                                          C.l_perm[W.cslot[cix]], &edge);
-            if (kx < 0) {
-              ok = false;
-            } else {
-              idx = __float_as_int(rr.w) + col + kx;
-              if (edge) atomicAdd(&sh_cnt[edge], 1ull);
+            if ((lane & (kGroup - 1)) == 0) {
+              W.box[2 * (lane / kGroup)] =
+                  make_float4(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2]), 0.f);
+              W.box[2 * (lane / kGroup) + 1] =
+                  make_float4(0.5f * (hi[0] - lo[0]), 0.5f * (hi[1] - lo[1]), 0.5f * (hi[2] - lo[2]), 0.f);
             }
           }
-          npairs += ok ? 1u : 0u;
-          return ok ? idx : kZeroIdxKey;
-        };
-        // the gathers go through L2 only (ld.global.cg): each is used once, and cached in L1 they
-        // would evict the receptor / ligand atom and mode lines that the next tiles read again
-        for (int t0 = 0; t0 < upto; t0 += kG) {
-          const int n = min(kG, upto - t0);
-          acc += pv0;
-          pv0 = __ldcg(table + pair(t0, 0, n));
-          acc += pv1;
-          pv1 = __ldcg(table + pair(t0, 1, n));
+          __syncwarp();
+
+          unsigned nnear = 0, npairs = 0, nevals = 0;
+          int ncand = 0, cb = 0;
+          unsigned cm = 0;
+          bool more = true;
+          do {
+            // fill each group's list until the ligand is exhausted or a list may overflow
+            unsigned cnt[kGroups];
+#pragma unroll
+            for (int g = 0; g < kGroups; ++g) cnt[g] = 0;
+            unsigned longest = 0;
+            do {
+              // collect candidates until a round is full or the ligand is exhausted
+              while (ncand < 32) {
+                if (cm == 0) {
+                  if (cb >= nlc) break;
+                  const int c = cb + lane;
+                  bool cnear = false;
+                  if (c < nlc) {
+                    const float4 ch = chS[p * nlc + c];
+                    const float ex = ch.x - cx, ey = ch.y - cy, ez = ch.z - cz, r = reach + ch.w;
+                    cnear = ex * ex + ey * ey + ez * ez <= r * r;  // same expression as the cneed test
+                  }
+                  cm = __ballot_sync(0xffffffffu, cnear);
+                  cb += 32;
+                  continue;
+                }
+                const int sb = (cb - 32 + __ffs(cm) - 1) * SD_TILE;
+                cm &= cm - 1;
+                const float4 la = lig[sb + lane];
+                const float ax = la.x + cx, ay = la.y + cy, az = la.z + cz;
+                const bool cand = fmaf(az, az, fmaf(ay, ay, ax * ax)) <= reach2;
+                const unsigned am = __ballot_sync(0xffffffffu, cand);
+                if (cand) W.pend[ncand + __popc(am & lt_mask)] = (unsigned short)(sb + lane);
+                ncand += __popc(am);
+              }
+              __syncwarp();
+              const int nb = min(ncand, 32);
+              const int s = lane < nb ? W.pend[lane] : nls;
+              const float4 l4 = lig[s];
+#pragma unroll
+              for (int g = 0; g < kGroups; ++g) {
+                const float4 bc = W.box[2 * g], bh = W.box[2 * g + 1];
+                const float ex = fmaxf(fabsf(l4.x + bc.x) - bh.x, 0.f), ey = fmaxf(fabsf(l4.y + bc.y) - bh.y, 0.f),
+                            ez = fmaxf(fabsf(l4.z + bc.z) - bh.z, 0.f);
+                const bool in = fmaf(ez, ez, fmaf(ey, ey, ex * ex)) <= box_cut;
+                const unsigned am = __ballot_sync(0xffffffffu, in);
+                if (in) W.list[g][cnt[g] + __popc(am & lt_mask)] = (unsigned short)s;
+                cnt[g] += __popc(am);
+                longest = max(longest, cnt[g]);
+              }
+              // keep the candidates beyond the first 32
+              const int rest = ncand - nb;
+              int carry = 0;
+              if (lane < rest) carry = W.pend[32 + lane];
+              __syncwarp();
+              if (lane < rest) W.pend[lane] = (unsigned short)carry;
+              ncand = rest;
+              __syncwarp();
+              more = ncand > 0 || cm != 0 || cb < nlc;
+            } while (more && longest <= kList - 32 - kBlock);
+            // each list is padded with the far atom to whole blocks
+#pragma unroll
+            for (int g = 0; g < kGroups; ++g) {
+              if (lane < kBlock) W.list[g][cnt[g] + lane] = (unsigned short)nls;
+              nevals += cnt[g] * __popc((act_mask >> (g * kGroup)) & 255u);
+            }
+            __syncwarp();
+            unsigned counts = cnt[0] | cnt[1] << 8 | cnt[2] << 16 | cnt[3] << 24;
+            for (int g = 0; g < kGroups; ++g, counts >>= 8) {
+              const float4 r0 = rec[g * kGroup + (lane & 3)], r1 = rec[g * kGroup + (lane & 3) + 4];
+              const float2x rx = pack2(r0.x, r1.x), ry = pack2(r0.y, r1.y), rz = pack2(r0.z, r1.z);
+              const double* row0 = table + __float_as_int(r0.w);
+              const double* row1 = table + __float_as_int(r1.w);
+              const unsigned short* list = W.list[g] + lane / 4;
+              const int n = (int)(counts & 255u);
+              float far = 0.f;
+              for (int c = 0; c < n; c += kBlock) {
+                float d2[kSteps][2], mid[kSteps][2];
+                const double* at[kSteps][2];
+#pragma unroll
+                for (int u = 0; u < kSteps; ++u) {
+                  const float4 l = lig[list[c + u * kRow]];
+                  int bin[2];
+                  pair_terms(rx, ry, rz, l, d2[u], mid[u], bin);
+                  far = fmaxf(far, fmaxf(fabsf(mid[u][0]), fabsf(mid[u][1])));
+                  at[u][0] = row0 + (__float_as_int(l.w) + bin[0]);
+                  at[u][1] = row1 + (__float_as_int(l.w) + bin[1]);
+                }
+#pragma unroll
+                for (int u = 0; u < 2 * kSteps; ++u) {
+                  acc += pv[u];
+                  // a pair inside the cutoff and away from a bin's edge: its value, through L2 only (each
+                  // is used once, and cached in L1 it would evict the atom and mode lines that the next
+                  // tiles read again)
+                  asm("{\n\t.reg .pred p;\n\t.reg .f32 m;\n\t"
+                      "abs.f32 m, %4;\n\t"
+                      "setp.le.f32 p, %2, %3;\n\t"
+                      "setp.lt.and.f32 p, m, %5, p;\n\t"
+                      "mov.f64 %0, 0d0000000000000000;\n\t"
+                      "@p ld.global.cg.f64 %0, [%6];\n\t"
+                      "@p add.u32 %1, %1, 1;\n\t}"
+                      : "=&d"(pv[u]), "+r"(npairs)
+                      : "f"(d2[u >> 1][u & 1]), "f"(cut2), "f"(mid[u >> 1][u & 1]), "f"(inner), "l"(at[u >> 1][u & 1]));
+                }
+              }
+              if (__any_sync(0xffffffffu, far >= inner)) {
+                // some pair of the group is near an edge (one group in about ten): find such pairs again
+                for (int c = 0; c < n; c += kRow) {
+                  const int s = list[c];
+                  const float4 l = lig[s];
+                  float d2[2], mid[2];
+                  int bin[2];
+                  pair_terms(rx, ry, rz, l, d2, mid, bin);
+#pragma unroll
+                  for (int h = 0; h < 2; ++h) {
+                    const bool near = d2[h] <= cut2 && fabsf(mid[h]) >= inner;
+                    const unsigned nm = __ballot_sync(0xffffffffu, near);
+                    const unsigned place = nnear + __popc(nm & lt_mask);
+                    if (near && place < kNear)
+                      W.near[place] = (unsigned)s * 32u + (unsigned)(g * kGroup + (lane & 3) + 4 * h);
+                    nnear += __popc(nm);
+                  }
+                }
+              }
+            }
+            __syncwarp();
+          } while (more);
+          __syncwarp();
+          if (nnear <= kNear) {
+            for (int i = lane; i < (int)nnear; i += 32) {
+              const unsigned e = W.near[i];
+              acc += decide_pair(C, Q.pose, Q.q, Q.qi, sh_T, table, k * SD_TILE + (int)(e & 31), (int)(e >> 5), sh_cnt);
+            }
+          } else {
+            // coordinates so large that FP32 decides nothing: the whole tile in FP64
+            npairs = 0;
+            acc = 0.0;
+#pragma unroll
+            for (int u = 0; u < 2 * kSteps; ++u) pv[u] = 0.0;
+            if (active)
+              for (int s = 0; s < nls; ++s)
+                if (C.l_perm[s] >= 0) acc += decide_pair(C, Q.pose, Q.q, Q.qi, sh_T, table, slot, s, sh_cnt);
+          }
+          __syncwarp();
+          // the tile's energy: the last block's gathers, then the lane sums in a fixed shuffle order,
+          // into the tile's slot
+#pragma unroll
+          for (int u = 0; u < 2 * kSteps; ++u) {
+            acc += pv[u];
+            pv[u] = 0.0;
+          }
+          double v = acc;
+          for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+          if (lane == 0) tsum[p * tstride + k] = v;
+          pose_pairs += npairs;
+          pose_evals += nevals;
+          acc = 0.0;
         }
-        // move the leftover (< kG) entries to the front
-        const int left = head - upto;
-        unsigned short e0 = 0, e1 = 0;
-        if (lane < left) e0 = W.ring[upto + lane];
-        if (lane + 32 < left) e1 = W.ring[upto + 32 + lane];
-        __syncwarp();
-        if (lane < left) W.ring[lane] = e0;
-        if (lane + 32 < left) W.ring[lane + 32] = e1;
-        head = left;
-        oldL = left;
-        if (final_batch) break;
       }
-      __syncwarp();
-      // the tile's energy: the last round's gathers, then the lane sums in a fixed shuffle order,
-      // into the tile's slot
-      acc += pv0;
-      acc += pv1;
-      pv0 = 0.0;
-      pv1 = 0.0;
-      double v = acc;
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-      if (lane == 0) tsum[k] = v;
-      acc = 0.0;
-    }
-    // counters, then the pose energy: warp 0 adds the tile slots in a fixed order
-    const unsigned wp = __reduce_add_sync(0xffffffffu, npairs);
-    if (lane == 0) {
-      if (wp) atomicAdd(&sh_cnt[3], (unsigned long long)wp);
-      if (nevals) atomicAdd(&sh_cnt[4], (unsigned long long)nevals);
-    }
-    __syncthreads();
-    if (warp == 0) {
-      double v = 0.0;
-      for (int k = lane; k < ntiles; k += 32) v += tsum[k];
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-      if (lane == 0) sh_red[0] = v;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      const double E = sh_red[0];
-      const double score = ((E)*0.0157 - 4.7) * -1;
-      C.scoring[p] = score;
-      if (L.energy_out) L.energy_out[p] = E;
-      ++n_done;
+      // counters, then the pose energy: warp 0 adds the tile slots in a fixed order
+      const unsigned wp = __reduce_add_sync(0xffffffffu, pose_pairs);
+      if (lane == 0) {
+        if (wp) atomicAdd(&sh_cnt[3], (unsigned long long)wp);
+        if (pose_evals) atomicAdd(&sh_cnt[4], (unsigned long long)pose_evals);
+      }
+      __syncthreads();
+      if (warp < np) {
+        double v = 0.0;
+        for (int k = lane; k < ntiles; k += 32) v += tsum[warp * tstride + k];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0) {
+          const int p = warp == 0 ? first : second;
+          C.scoring[p] = ((v)*0.0157 - 4.7) * -1;
+          if (L.energy_out) L.energy_out[p] = v;
+        }
+      }
+      n_done += np;
+      if (item < item_end) __syncthreads();
     }
   }
   __syncthreads();
