@@ -1177,8 +1177,9 @@ int sd_pydock_grad(sd_ctx* c, int ci, const double* poses, int n, int precision,
   cudaFuncAttributes fa;
   SD_CUDA(cudaFuncGetAttributes(&fa, k));
   // a ligand too large for shared memory: the spill instantiation, per-CTA arrays in global scratch
-  const bool spill = need + fa.sharedSizeBytes > (size_t)c->smem_optin;
-  const size_t sm = spill ? 0 : need;
+  const size_t warp_bytes = pydock_warp_bytes(precision);
+  const bool spill = warp_bytes + need + fa.sharedSizeBytes > (size_t)c->smem_optin;
+  const size_t sm = warp_bytes + (spill ? 0 : need);
   if (spill) k = pydock_kernel_ptr(precision, true, true);
   SD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(sm, 1)));
   int per_sm = 0;

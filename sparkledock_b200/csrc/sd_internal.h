@@ -166,6 +166,7 @@ int gso_prepare_large();
 int bins_launch(const DevComplex* cplx, int c, const double* d_pose, int precision, int* d_bins, int nr, int nl,
                 int* d_fallback, cudaStream_t st);
 size_t pydock_smem_bytes(int precision, bool grad, int max_nl, int max_nr);
+size_t pydock_warp_bytes(int precision);
 const void* pydock_kernel_ptr(int precision, bool grad, bool spill);
 int pydock_launch(const ScoreLaunch& L, int precision, bool grad, double* out_grad, int grid, size_t smem,
                   cudaStream_t st, bool spill);

@@ -13,11 +13,13 @@
 //   dE/de_rec_m = sum_i mask_i M_mi.G_i, with F_j = dE/dl_j, G_i = dE/dr_i (pair forces).
 //
 // Kernel: one CTA (8 warps) per pose at a time, persistent over a work list; receptor tiles of
-// 32 (one lane per atom) culled against the ligand sphere and against spatial ligand chunks;
-// per candidate ligand atom every lane evaluates its pair.  GRAD adds per-lane receptor force
-// accumulators (projected onto the receptor modes at the end of each tile) and per-ligand-atom
-// force accumulators in shared memory (one warp reduction + one shared atomic per component
-// and ligand atom), projected onto t, w and the ligand modes at the end of the pose.
+// 32 (one lane per atom) culled against the ligand sphere and against spatial ligand chunks, and
+// each tile's candidate ligand atoms against the bounding boxes of its four groups of 8 atoms.  A
+// step evaluates 8 receptor atoms x 4 candidates of one group, one pair per lane.  GRAD adds
+// per-lane receptor force accumulators (summed over the four rows at the end of a group, projected
+// onto the receptor modes at the end of each tile) and per-ligand-atom force accumulators in shared
+// memory (a row's three components reduced together in four shuffles, one shared atomic), projected
+// onto t, w and the ligand modes at the end of the pose.
 #include <cuda_runtime.h>
 
 #include "sd_internal.h"
@@ -84,6 +86,19 @@ __device__ __forceinline__ T pd_pair(T x, T qq, T eps, T sig2, T& dedx) {
   return e;
 }
 
+constexpr int kRows = SD_TILE / SD_GROUP;  // groups of a tile; candidates of a step (one row of 8 lanes each)
+constexpr int kPdList = 128;               // candidates of a group between two drains of the lists
+
+// a warp's tile
+template <class T>
+struct PdWarp {
+  LigAtom<T> rec[SD_TILE];           // receptor atoms (position relative to t, charge)
+  float4 box[2 * kRows];             // centre and half extent of each group's bounding box
+  int lj[SD_TILE];
+  unsigned short list[kRows][kPdList];  // each group's candidates: ligand slots
+  unsigned short pend[64];           // pending candidate ligand slots of the tile
+};
+
 template <class T>
 __device__ __forceinline__ T warp_sum(T v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -99,7 +114,9 @@ __device__ __forceinline__ T warp_sum(T v) {
 template <class T, bool GRAD, bool kSpill>
 __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4) pydock_kernel(ScoreLaunch L, double* out_grad) {
   extern __shared__ __align__(16) unsigned char smem_dyn[];
-  unsigned char* const smem = kSpill ? L.spill + (size_t)blockIdx.x * L.spill_stride : smem_dyn;
+  PdWarp<T>& W = reinterpret_cast<PdWarp<T>*>(smem_dyn)[threadIdx.x >> 5];
+  unsigned char* const smem =
+      kSpill ? L.spill + (size_t)blockIdx.x * L.spill_stride : smem_dyn + kPdWarps * sizeof(PdWarp<T>);
   __shared__ double sh_pose[7 + 2 * SD_MAX_MODES];
   __shared__ double sh_q[4], sh_qi[4];
   __shared__ LjPair<T> sh_lj[SD_LJ_TYPES * SD_LJ_TYPES];
@@ -109,6 +126,8 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
   __shared__ int sh_item, sh_ntile, sh_next;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  const int atom = lane & (SD_GROUP - 1), crow = lane / SD_GROUP;  // a step's atom and candidate row
   for (int k = tid; k < SD_LJ_TYPES * SD_LJ_TYPES; k += blockDim.x) {
     const int a = k / SD_LJ_TYPES, b = k % SD_LJ_TYPES;
     sh_lj[k].eps = (T)sqrt(L.lj_eps[a] * L.lj_eps[b]);
@@ -166,15 +185,23 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
     __syncthreads();
     const double tx = sh_pose[0], ty = sh_pose[1], tz = sh_pose[2];
     const float dR = sh_bound[0], dL = sh_bound[1];
-    // shared layout: ligand atoms [nls] (LigAtom<T>), llj [nls] (int), chunk spheres [nlc] (float4),
-    // tile list [ntiles] (int), GRAD: fx, fy, fz [nls] (T)
+    // per-pose arrays: ligand atoms [nls + 1] (LigAtom<T>; the last a far atom, the padding), GRAD: fx,
+    // fy, fz [nls + 1] (T), chunk spheres [nlc] (float4), llj [nls + 1], near tiles [ntiles] as found,
+    // in order of distance, and their distances
     LigAtom<T>* la = reinterpret_cast<LigAtom<T>*>(smem);
-    T* fx = reinterpret_cast<T*>(la + nls);  // GRAD only
-    T* fy = fx + (GRAD ? nls : 0);
-    T* fz = fy + (GRAD ? nls : 0);
-    float4* chS = reinterpret_cast<float4*>(fz + (GRAD ? nls : 0));
+    T* fx = reinterpret_cast<T*>(la + nls + 1);  // GRAD only: [3][nls + 4]
+    const int fstride = nls + 4;
+    float4* chS = reinterpret_cast<float4*>(fx + (GRAD ? 3 * fstride : 0));
     int* llj = reinterpret_cast<int*>(chS + nlc);
-    int* tlist = llj + nls;
+    int* tlist = llj + nls + 1;
+    int* tord = tlist + C.ntiles;
+    float* tdist = reinterpret_cast<float*>(tord + C.ntiles);
+    if (tid == 0) {
+      la[nls] = LigAtom<T>{(T)3e18, (T)3e18, (T)3e18, T(0)};
+      llj[nls] = 0;
+    }
+    if (GRAD)
+      for (int s = tid; s < 3 * fstride; s += blockDim.x) fx[s] = T(0);
     for (int s = tid; s < nls; s += blockDim.x) {
       if (C.l_perm[s] >= 0) {
         double x, y, z;
@@ -185,7 +212,6 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
         la[s] = LigAtom<T>{(T)1e18, (T)1e18, (T)1e18, T(0)};
         llj[s] = 0;
       }
-      if (GRAD) fx[s] = fy[s] = fz[s] = T(0);
     }
     for (int c = tid; c < nlc; c += blockDim.x) {
       const float4 cc = C.l_chunk[c];
@@ -200,10 +226,31 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
       const float cx = (float)((double)tile.x - tx), cy = (float)((double)tile.y - ty),
                   cz = (float)((double)tile.z - tz);
       const float reach = 15.0f + dR + SD_CULL_MARGIN + tile.w + lig_reach;
-      if (cx * cx + cy * cy + cz * cz <= reach * reach) tlist[atomicAdd(&sh_ntile, 1)] = k;
+      const float dd = cx * cx + cy * cy + cz * cz;
+      if (dd <= reach * reach) {
+        const int at = atomicAdd(&sh_ntile, 1);
+        tlist[at] = k;
+        tdist[at] = dd;
+      }
     }
     __syncthreads();
     const int ntile = sh_ntile;
+    // the tiles closest to the ligand centre (t) have the most pairs: taken first, the warps finish a
+    // pose together
+    const bool sorted = ntile <= 512;
+    if (sorted) {
+      for (int t = tid; t < ntile; t += blockDim.x) {
+        const float d = tdist[t];
+        int rank = 0;
+        for (int u = 0; u < ntile; ++u) {
+          const float e = tdist[u];
+          rank += (e < d || (e == d && u < t)) ? 1 : 0;
+        }
+        tord[rank] = tlist[t];
+      }
+      __syncthreads();
+    }
+    const int* tl = sorted ? tord : tlist;
     double es = 0.0;  // energy: FP64 per-lane sum of the pair terms
     T grec[SD_MAX_MODES];
     for (int m = 0; m < SD_MAX_MODES; ++m) grec[m] = T(0);
@@ -213,7 +260,7 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
       if (lane == 0) ti = atomicAdd(&sh_next, 1);
       ti = __shfl_sync(0xffffffffu, ti, 0);
       if (ti >= ntile) break;
-      const int k = tlist[ti];
+      const int k = tl[ti];
       const float4 tile = C.r_tile[k];
       const float cx = (float)((double)tile.x - tx), cy = (float)((double)tile.y - ty),
                   cz = (float)((double)tile.z - tz);
@@ -221,134 +268,160 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
       const float reach2 = reach * reach;
       const int slot = k * SD_TILE + lane;
       const bool active = C.r_orig[slot] >= 0;
-      T rx = (T)1e18, ry = (T)1e18, rz = (T)1e18, rq = T(0);
-      int rlj = 0;
+      LigAtom<T> own{(T)1e18, (T)1e18, (T)1e18, T(0)};
       if (active) {
         double x, y, z;
         receptor_exact(C, nslots, slot, sh_pose, x, y, z);
-        rx = (T)(x - tx);
-        ry = (T)(y - ty);
-        rz = (T)(z - tz);
-        rq = (T)C.r_q[slot];
-        rlj = C.r_lj[slot];
+        own = LigAtom<T>{(T)(x - tx), (T)(y - ty), (T)(z - tz), (T)C.r_q[slot]};
       }
-      T gx = T(0), gy = T(0), gz = T(0);  // dE/dr_i
-      for (int cb = 0; cb < nlc; cb += 32) {
-        const int c = cb + lane;
-        bool cnear = false;
-        if (c < nlc) {
-          const float4 ch = chS[c];
-          const float ex = ch.x - cx, ey = ch.y - cy, ez = ch.z - cz, r = reach + ch.w;
-          cnear = ex * ex + ey * ey + ez * ez <= r * r;
+      __syncwarp();
+      W.rec[lane] = own;
+      W.lj[lane] = active ? C.r_lj[slot] : 0;
+      {
+        // bounding box of each group of 8 lanes (an empty group's half extent is -inf: no candidate)
+        float lo[3] = {(float)own.x, (float)own.y, (float)own.z}, hi[3] = {lo[0], lo[1], lo[2]};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          if (!active) {
+            lo[d] = 3e38f;
+            hi[d] = -3e38f;
+          }
+#pragma unroll
+          for (int o = 1; o < SD_GROUP; o <<= 1) {
+            lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+            hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+          }
         }
-        unsigned cm = __ballot_sync(0xffffffffu, cnear);
-        while (cm) {
-          const int cc = cb + __ffs(cm) - 1;
-          cm &= cm - 1;
-          const int sb = cc * SD_TILE;
-          const LigAtom<T> ca = la[sb + lane];
-          const float ax = (float)ca.x - cx, ay = (float)ca.y - cy, az = (float)ca.z - cz;
-          unsigned am = __ballot_sync(0xffffffffu, ax * ax + ay * ay + az * az <= reach2);
-          // this lane's pair with candidate slot s: energy, dE/dr_i into (gx, gy, gz), and the
-          // force on the ligand atom into f
-          auto pair = [&](int s, T f[3]) {
+        if (atom == 0) {
+          W.box[2 * crow] = make_float4(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2]), 0.f);
+          W.box[2 * crow + 1] =
+              make_float4(0.5f * (hi[0] - lo[0]), 0.5f * (hi[1] - lo[1]), 0.5f * (hi[2] - lo[2]), 0.f);
+        }
+      }
+      __syncwarp();
+      T gx = T(0), gy = T(0), gz = T(0);  // dE/dr of this lane's atom of the tile
+      int ncand = 0, cb = 0;
+      unsigned cm = 0;
+      bool more = true;
+      do {
+        // fill each group's list until the ligand is exhausted or a list may overflow
+        unsigned cnt[kRows];
+#pragma unroll
+        for (int g = 0; g < kRows; ++g) cnt[g] = 0;
+        unsigned longest = 0;
+        do {
+          // collect candidates until a round is full or the ligand is exhausted
+          while (ncand < 32) {
+            if (cm == 0) {
+              if (cb >= nlc) break;
+              const int c = cb + lane;
+              bool cnear = false;
+              if (c < nlc) {
+                const float4 ch = chS[c];
+                const float ex = ch.x - cx, ey = ch.y - cy, ez = ch.z - cz, r = reach + ch.w;
+                cnear = ex * ex + ey * ey + ez * ez <= r * r;
+              }
+              cm = __ballot_sync(0xffffffffu, cnear);
+              cb += 32;
+              continue;
+            }
+            const int sb = (cb - 32 + __ffs(cm) - 1) * SD_TILE;
+            cm &= cm - 1;
+            const LigAtom<T> ca = la[sb + lane];
+            const float ax = (float)ca.x - cx, ay = (float)ca.y - cy, az = (float)ca.z - cz;
+            const bool cand = ax * ax + ay * ay + az * az <= reach2;
+            const unsigned am = __ballot_sync(0xffffffffu, cand);
+            if (cand) W.pend[ncand + __popc(am & lt_mask)] = (unsigned short)(sb + lane);
+            ncand += __popc(am);
+          }
+          __syncwarp();
+          const int nb = min(ncand, 32);
+          const int s = lane < nb ? W.pend[lane] : nls;
+          const LigAtom<T> c = la[s];
+          const float x = (float)c.x, y = (float)c.y, z = (float)c.z;
+#pragma unroll
+          for (int g = 0; g < kRows; ++g) {
+            const float4 bc = W.box[2 * g], bh = W.box[2 * g + 1];
+            const float ex = fmaxf(fabsf(x - bc.x) - bh.x, 0.f), ey = fmaxf(fabsf(y - bc.y) - bh.y, 0.f),
+                        ez = fmaxf(fabsf(z - bc.z) - bh.z, 0.f);
+            const bool in = fmaf(ez, ez, fmaf(ey, ey, ex * ex)) <= 225.1f;
+            const unsigned am = __ballot_sync(0xffffffffu, in);
+            if (in) W.list[g][cnt[g] + __popc(am & lt_mask)] = (unsigned short)s;
+            cnt[g] += __popc(am);
+            longest = max(longest, cnt[g]);
+          }
+          // keep the candidates beyond the first 32
+          const int rest = ncand - nb;
+          int carry = 0;
+          if (lane < rest) carry = W.pend[32 + lane];
+          __syncwarp();
+          if (lane < rest) W.pend[lane] = (unsigned short)carry;
+          ncand = rest;
+          __syncwarp();
+          more = ncand > 0 || cm != 0 || cb < nlc;
+        } while (more && longest <= kPdList - 32 - kRows);
+        // each list is padded with the far atom to whole steps
+#pragma unroll
+        for (int g = 0; g < kRows; ++g)
+          if (lane < kRows) W.list[g][cnt[g] + lane] = (unsigned short)nls;
+        __syncwarp();
+        unsigned counts = cnt[0] | cnt[1] << 8 | cnt[2] << 16 | cnt[3] << 24;
+        for (int g = 0; g < kRows; ++g, counts >>= 8) {
+          const LigAtom<T> r = W.rec[g * SD_GROUP + atom];
+          const LjPair<T>* ljrow = sh_lj + W.lj[g * SD_GROUP + atom];
+          const unsigned short* list = W.list[g] + crow;
+          const int n = (int)(counts & 255u);
+          T hx = T(0), hy = T(0), hz = T(0);  // dE/dr of this lane's pairs
+          for (int c = 0; c < n; c += kRows) {
+            const int s = list[c];
             const LigAtom<T> a = la[s];
-            const T dx = rx - a.x, dy = ry - a.y, dz = rz - a.z;
+            const T dx = r.x - a.x, dy = r.y - a.y, dz = r.z - a.z;
             const T x = dx * dx + dy * dy + dz * dz;
+            T f0 = T(0), f1 = T(0), f2 = T(0);
             if (x < T(225)) {
               T dedx;
-              // the table is symmetric (products and sums of the two types' parameters), so it is
-              // read as [ligand type][receptor type]: the lanes of one candidate read consecutive
-              // entries instead of entries 20 apart that meet in a few banks
-              const LjPair<T> lj = sh_lj[llj[s] + rlj];
-              const T e = pd_pair<T>(x, rq * a.q, lj.eps, lj.sig2, dedx);
+              // the table is symmetric (products and sums of the two types' parameters), so it is read as
+              // [ligand type][receptor type]: the lanes of one candidate read entries of one row
+              const LjPair<T> lj = ljrow[llj[s]];
+              const T e = pd_pair<T>(x, r.q * a.q, lj.eps, lj.sig2, dedx);
               es += (double)e;
               if (GRAD) {
                 const T g2 = T(2) * dedx;
-                gx += g2 * dx;
-                gy += g2 * dy;
-                gz += g2 * dz;
-                f[0] = -g2 * dx;
-                f[1] = -g2 * dy;
-                f[2] = -g2 * dz;
+                f0 = g2 * dx;
+                f1 = g2 * dy;
+                f2 = g2 * dz;
+                hx += f0;
+                hy += f1;
+                hz += f2;
               }
             }
-          };
-          if (!GRAD) {
-            while (am) {
-              const int b = __ffs(am) - 1;
-              am &= am - 1;
-              T f[3];
-              pair(sb + b, f);
+            if (GRAD) {
+              // the row's forces on its candidate: lanes 0, 2 and 4 of the row end with x, y and z
+              const bool h4 = (lane & 4) != 0, h2 = (lane & 2) != 0;
+              const T k0 = (h4 ? f2 : f0) + __shfl_xor_sync(0xffffffffu, h4 ? f0 : f2, 4);
+              const T k1 = (h4 ? T(0) : f1) + __shfl_xor_sync(0xffffffffu, h4 ? f1 : T(0), 4);
+              T v = (h2 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, h2 ? k0 : k1, 2);
+              v += __shfl_xor_sync(0xffffffffu, v, 1);
+              if ((lane & 1) == 0 && atom < 6) atomicAdd(&fx[(atom >> 1) * fstride + s], -v);
             }
-          } else {
-            // candidates several at a time share one warp reduction of their ligand forces
-            const bool h16 = (lane & 16) != 0, h8 = (lane & 8) != 0;
-            if constexpr (sizeof(T) == 8) {
-              // FP64 (registers to spare), four: an exchange across the half-warps and one across
-              // the quarter-warps leave candidate A's partial forces in lanes 0-7, B's in 8-15,
-              // C's in 16-23 and D's in 24-31; three more levels finish all four
-              while (am) {
-                int b[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                  b[q] = am ? __ffs(am) - 1 : -1;
-                  if (am) am &= am - 1;
-                }
-                T f[4][3];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                  f[q][0] = f[q][1] = f[q][2] = T(0);
-                  if (b[q] >= 0) pair(sb + b[q], f[q]);
-                }
-                T r[3];
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                  T k0 = h16 ? f[2][k] : f[0][k], k1 = h16 ? f[3][k] : f[1][k];
-                  k0 += __shfl_xor_sync(0xffffffffu, h16 ? f[0][k] : f[2][k], 16);
-                  k1 += __shfl_xor_sync(0xffffffffu, h16 ? f[1][k] : f[3][k], 16);
-                  T v = (h8 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, h8 ? k0 : k1, 8);
-                  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                  r[k] = v;
-                }
-                const int bq = b[(h16 ? 2 : 0) + (h8 ? 1 : 0)];
-                if ((lane & 7) == 0 && bq >= 0) {
-                  atomicAdd(&fx[sb + bq], r[0]);
-                  atomicAdd(&fy[sb + bq], r[1]);
-                  atomicAdd(&fz[sb + bq], r[2]);
-                }
-              }
-            } else {
-              // FP32, two: one exchange across the half-warps leaves candidate A's partial forces
-              // in lanes 0-15 and B's in 16-31; four more levels finish both
-              while (am) {
-                const int b0 = __ffs(am) - 1;
-                am &= am - 1;
-                int b1 = -1;
-                if (am) {
-                  b1 = __ffs(am) - 1;
-                  am &= am - 1;
-                }
-                T fa[3] = {T(0), T(0), T(0)}, fb[3] = {T(0), T(0), T(0)};
-                pair(sb + b0, fa);
-                if (b1 >= 0) pair(sb + b1, fb);
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                  T v = (h16 ? fb[k] : fa[k]) + __shfl_xor_sync(0xffffffffu, h16 ? fa[k] : fb[k], 16);
-                  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                  fa[k] = v;
-                }
-                const int s = sb + (h16 ? b1 : b0);
-                if ((lane & 15) == 0 && (!h16 || b1 >= 0)) {
-                  atomicAdd(&fx[s], fa[0]);
-                  atomicAdd(&fy[s], fa[1]);
-                  atomicAdd(&fz[s], fa[2]);
-                }
-              }
+          }
+          if (GRAD) {
+            // sum over the rows; the lanes of the group's own row keep it
+            hx += __shfl_xor_sync(0xffffffffu, hx, 8);
+            hy += __shfl_xor_sync(0xffffffffu, hy, 8);
+            hz += __shfl_xor_sync(0xffffffffu, hz, 8);
+            hx += __shfl_xor_sync(0xffffffffu, hx, 16);
+            hy += __shfl_xor_sync(0xffffffffu, hy, 16);
+            hz += __shfl_xor_sync(0xffffffffu, hz, 16);
+            if (crow == g) {
+              gx += hx;
+              gy += hy;
+              gz += hz;
             }
           }
         }
-      }
+        __syncwarp();
+      } while (more);
       if (GRAD && active && C.r_mask[slot] == 1) {
         for (int m = 0; m < C.nmr; ++m) {
           const double* M = C.r_modes + (size_t)m * 3 * nslots + slot;
@@ -383,7 +456,7 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
       }
       for (int s = tid; s < nls; s += blockDim.x) {
         if (C.l_perm[s] < 0) continue;
-        const double Fx = (double)fx[s], Fy = (double)fy[s], Fz = (double)fz[s];
+        const double Fx = (double)fx[s], Fy = (double)fx[fstride + s], Fz = (double)fx[2 * fstride + s];
         const double px = (double)la[s].x, py = (double)la[s].y, pz = (double)la[s].z;  // l_j - t
         acc[1] += Fx;
         acc[2] += Fy;
@@ -422,10 +495,15 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
   if (tid == 0 && n_done) atomicAdd(&ctl->stats[ST_SCORED], n_done);
 }
 
+// bytes of a CTA's per-pose arrays, and of its warps' buffers in front of them (always shared memory)
 size_t pydock_smem_bytes(int precision, bool grad, int max_nl, int max_nr) {
   const size_t nlc = (size_t)(max_nl + SD_TILE - 1) / SD_TILE, nls = nlc * SD_TILE;
   const size_t ts = precision == SD_PREC_MIXED ? 4 : 8;
-  return ts * nls * (4 + (grad ? 3 : 0)) + 16 * nlc + 4 * nls + 4 * ((max_nr + SD_TILE - 1) / SD_TILE) + 16;
+  return ts * (4 * (nls + 1) + (grad ? 3 * (nls + 4) : 0)) + 16 * nlc + 4 * (nls + 1) +
+         12 * ((max_nr + SD_TILE - 1) / SD_TILE) + 16;
+}
+size_t pydock_warp_bytes(int precision) {
+  return kPdWarps * (precision == SD_PREC_MIXED ? sizeof(PdWarp<float>) : sizeof(PdWarp<double>));
 }
 
 const void* pydock_kernel_ptr(int precision, bool grad, bool spill) {
@@ -442,7 +520,7 @@ int pydock_launch(const ScoreLaunch& L, int precision, bool grad, double* out_gr
   ScoreLaunch l = L;
   void* args[] = {(void*)&l, (void*)&out_grad};
   if (cudaLaunchKernel(pydock_kernel_ptr(precision, grad, spill), dim3(grid), dim3(kPdWarps * 32), args,
-                       spill ? 0 : smem, st) != cudaSuccess)
+                       smem, st) != cudaSuccess)
     return SD_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? SD_OK : SD_ERR_CUDA;
 }

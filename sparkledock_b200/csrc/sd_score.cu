@@ -333,10 +333,11 @@ static_assert(kNumMixedVariants <= SD_MAX_VARIANTS, "variant table");
 
 static const MixedVariant& mixed_variant(int v) { return kMixedVariants[v < 0 || v >= kNumMixedVariants ? 0 : v]; }
 
-// bytes of the mixed DFIRE scorer's per-warp buffers, in dynamic shared memory in front of the per-pose
-// arrays (alone there in the spill instantiation)
+// bytes of the scorer's per-warp buffers, in dynamic shared memory in front of the per-pose arrays
+// (alone there in the spill instantiation)
 size_t score_warp_bytes(int precision, int scoring, int variant, bool spill) {
-  if (scoring == SD_SCORING_PYDOCK || precision != SD_PREC_MIXED) return 0;
+  if (scoring == SD_SCORING_PYDOCK) return pydock_warp_bytes(precision);
+  if (precision != SD_PREC_MIXED) return 0;
   return sizeof(WarpBufs) * (spill ? kMixedSpill.warps : mixed_variant(variant).warps);
 }
 
