@@ -137,6 +137,7 @@ struct sd_ctx {
   size_t score_smem = 0;
   bool score_spill = false;  // the last configured scorer launch uses the spill instantiation
   size_t spill_stride = 0;
+  float force_scale = 1.f;   // pyDock: fixed-point units of FP32 ligand forces
   int score_poses = 1;       // poses per CTA of the last configured scorer launch
   // autotuner state (mixed-precision DFIRE kernel variants)
   int mixed_variant = 0;
@@ -825,6 +826,14 @@ int sd_ctx_create(const sd_complex_desc* complexes, int n_complexes, const sd_ta
         eps[i] = tables->lj_eps[i];
         sig[i] = tables->lj_sigma[i];
       }
+    if (scoring == SD_SCORING_PYDOCK) {
+      double qr = 0, ql = 0;
+      for (int i = 0; i < n_complexes; ++i) {
+        for (int k = 0; k < complexes[i].n_rec; ++k) qr = std::max(qr, std::fabs(complexes[i].rec_charge[k]));
+        for (int k = 0; k < complexes[i].n_lig; ++k) ql = std::max(ql, std::fabs(complexes[i].lig_charge[k]));
+      }
+      c->force_scale = pydock_force_scale(qr, ql, eps.data(), sig.data(), c->max_nr);
+    }
     std::vector<int> smap(c->total_swarms);
     for (int ci = 0, s0 = 0; ci < n_complexes; ++ci)
       for (int s = 0; s < complexes[ci].n_swarms; ++s) smap[s0++] = wi_pack(ci, s);
@@ -1177,19 +1186,20 @@ int sd_pydock_grad(sd_ctx* c, int ci, const double* poses, int n, int precision,
   cudaFuncAttributes fa;
   SD_CUDA(cudaFuncGetAttributes(&fa, k));
   // a ligand too large for shared memory: the spill instantiation, per-CTA arrays in global scratch
-  const size_t warp_bytes = pydock_warp_bytes(precision);
+  const size_t warp_bytes = pydock_warp_bytes(precision, true);
   const bool spill = warp_bytes + need + fa.sharedSizeBytes > (size_t)c->smem_optin;
   const size_t sm = warp_bytes + (spill ? 0 : need);
   if (spill) k = pydock_kernel_ptr(precision, true, true);
   SD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(sm, 1)));
   int per_sm = 0;
-  SD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, pydock_threads(), sm));
+  SD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, pydock_threads(precision, true), sm));
   if (per_sm < 1) return fail(SD_ERR_ARG, "pyDock gradient kernel does not fit on an SM");
   const size_t stride = (need + 255) & ~(size_t)255;
   if (spill && (rc = grow_spill(c, stride * (size_t)per_sm * c->nsm))) return rc;
   ScoreLaunch L{};
   L.spill = spill ? (unsigned char*)c->s_spill.p : nullptr;
   L.spill_stride = spill ? stride : 0;
+  L.force_scale = c->force_scale;
   L.cplx = c->d_cplx_scratch;
   L.ctl = c->d_ctl_scratch;
   L.work[0] = (const int*)c->s_work.p;

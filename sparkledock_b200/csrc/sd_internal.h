@@ -129,6 +129,7 @@ struct ScoreLaunch {
   const double* table64;   // [SD_TABLE_SIZE + 32] zero padded
   const double* lj_eps;    // [20] pyDock
   const double* lj_sigma;
+  float force_scale;       // pyDock gradients in FP32: units of the ligand forces' fixed point
   int poses_per_cta;       // mixed DFIRE: 2 when two poses' arrays fit, else 1
   double* energy_out;      // nullable [local glowworm] raw energies (stateless scoring)
   // per-CTA global scratch that replaces the dynamic shared memory of the spill instantiations
@@ -166,11 +167,12 @@ int gso_prepare_large();
 int bins_launch(const DevComplex* cplx, int c, const double* d_pose, int precision, int* d_bins, int nr, int nl,
                 int* d_fallback, cudaStream_t st);
 size_t pydock_smem_bytes(int precision, bool grad, int max_nl, int max_nr);
-size_t pydock_warp_bytes(int precision);
+size_t pydock_warp_bytes(int precision, bool grad);
+float pydock_force_scale(double max_q_rec, double max_q_lig, const double* eps, const double* sigma, int max_nr);
 const void* pydock_kernel_ptr(int precision, bool grad, bool spill);
 int pydock_launch(const ScoreLaunch& L, int precision, bool grad, double* out_grad, int grid, size_t smem,
                   cudaStream_t st, bool spill);
-int pydock_threads();
+int pydock_threads(int precision, bool grad);
 void set_key_thresholds(const double* t64);
 size_t cluster_smem_bytes(int G, int nbb);
 int materialise_launch(const DevComplex* d_cplx, int ci, const int* d_poses, int n, const int* d_rslot, int nr, int nl,

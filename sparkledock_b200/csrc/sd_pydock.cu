@@ -14,25 +14,38 @@
 //
 // Kernel: one CTA (8 warps) per pose at a time, persistent over a work list; receptor tiles of
 // 32 (one lane per atom) culled against the ligand sphere and against spatial ligand chunks, and
-// each tile's candidate ligand atoms against the bounding boxes of its four groups of 8 atoms.  A
-// step evaluates 8 receptor atoms x 4 candidates of one group, one pair per lane.  GRAD adds
-// per-lane receptor force accumulators (summed over the four rows at the end of a group, projected
-// onto the receptor modes at the end of each tile) and per-ligand-atom force accumulators in shared
-// memory (a row's three components reduced together in four shuffles, one shared atomic), projected
+// each tile's candidate ligand atoms against the bounding boxes of its four groups of 8 atoms (45 %
+// of a group's listed pairs are inside the cutoff, 21 % of a tile's).  A step evaluates 8 receptor
+// atoms x 8 candidates of one group, two atoms per lane (FP32 in packed instructions).  GRAD adds
+// per-lane receptor force accumulators (summed over the rows at the end of a group, projected onto
+// the receptor modes at the end of each tile) and per-ligand-atom force accumulators in shared
+// memory (a row's three components reduced together in three shuffles, one shared atomic), projected
 // onto t, w and the ligand modes at the end of the pose.
+//
+// What bounds it: instruction issue (0.7 of the slots) and, with forces, the latency of the shuffles
+// and shared atomics; memory traffic is small.  Measured on 3002 / 1274 atoms, 4,096 poses, the whole
+// call, against the earlier kernel (one candidate of a tile over all its lanes, 15 shuffles and 3
+// atomics for two candidates): FP32 gradients 6.1 -> 4.0 ms, FP32 energies 3.6 -> 2.0 ms, FP64 energies
+// 4.0 -> 2.6 ms, 2,000 FP64 gradients 4.7 -> 2.5 ms.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
+
 #include "sd_internal.h"
+#include "sd_packed.cuh"
 #include "sd_pose.cuh"
 
 namespace sd {
 
 namespace {
 
-constexpr int kPdWarps = 8;
+// warps of a CTA: FP32 gradients 12, two CTAs per SM (their ligand forces take 24 bytes an atom, and
+// three CTAs of 8 warps would not fit beside ligands over 1,270 atoms); else 8, as many as fit
+__host__ __device__ constexpr int pd_warps(bool fp64, bool grad) { return grad && !fp64 ? 12 : 8; }
 constexpr double kKe = 332.0636 / 4.0;
 
-// a ligand atom in shared memory (position relative to t, charge): one 16-byte load in FP32
+// an atom in shared memory (position relative to t, the ligand's negated, charge): one 16-byte load in FP32
 template <class T>
 struct alignas(16) LigAtom {
   T x, y, z, q;
@@ -43,59 +56,145 @@ struct alignas(2 * sizeof(T)) LjPair {
   T eps, sig2;
 };
 
-// the switch with its constant 1 / (off2 - on2)^3 passed in (both widths are fixed)
+// two values of T, one per receptor atom of a lane; FP32 in packed instructions
 template <class T>
-__device__ __forceinline__ void pd_switch(T x, T on2, T off2, T rden, T& s, T& ds) {
-  if (x <= on2) {
-    s = T(1);
-    ds = T(0);
-    return;
-  }
-  if (x >= off2) {
-    s = T(0);
-    ds = T(0);
-    return;
-  }
-  const T a = off2 - x;
-  s = a * a * (off2 + T(2) * x - T(3) * on2) * rden;
-  ds = T(6) * a * (on2 - x) * rden;
+struct V2 {
+  T a, b;
+  __device__ __forceinline__ V2() {}
+  __device__ __forceinline__ V2(T x, T y) : a(x), b(y) {}
+  __device__ __forceinline__ explicit V2(T x) : a(x), b(x) {}
+  __device__ __forceinline__ T first() const { return a; }
+  __device__ __forceinline__ T second() const { return b; }
+};
+template <class T>
+__device__ __forceinline__ V2<T> operator+(V2<T> x, V2<T> y) { return V2<T>(x.a + y.a, x.b + y.b); }
+template <class T>
+__device__ __forceinline__ V2<T> operator-(V2<T> x, V2<T> y) { return V2<T>(x.a - y.a, x.b - y.b); }
+template <class T>
+__device__ __forceinline__ V2<T> operator*(V2<T> x, V2<T> y) { return V2<T>(x.a * y.a, x.b * y.b); }
+template <>
+struct V2<float> {
+  float2x v;
+  __device__ __forceinline__ V2() {}
+  __device__ __forceinline__ V2(float x, float y) : v(pack2(x, y)) {}
+  __device__ __forceinline__ explicit V2(float x) : v(pack2(x, x)) {}
+  __device__ __forceinline__ float first() const { float x, y; unpack2(v, x, y); return x; }
+  __device__ __forceinline__ float second() const { float x, y; unpack2(v, x, y); return y; }
+};
+__device__ __forceinline__ V2<float> operator+(V2<float> x, V2<float> y) { x.v = add2(x.v, y.v); return x; }
+// -0 read at run time: x y + (-0) is the product rounded once, and cannot be contracted with an addition
+// that follows (a packed multiply followed by a packed add was, measured, whatever -fmad says)
+__constant__ float c_minus_zero[2] = {-0.f, -0.f};
+__device__ __forceinline__ V2<float> operator*(V2<float> x, V2<float> y) {
+  x.v = fma2(x.v, y.v, pack2(c_minus_zero[0], c_minus_zero[1]));
+  return x;
+}
+// x - y as x + (-1) y: the product is exact, so the difference is rounded once
+__device__ __forceinline__ V2<float> operator-(V2<float> x, V2<float> y) { x.v = fma2(y.v, pack2(-1.f, -1.f), x.v); return x; }
+
+// the switch at x with its constant 1 / (off2 - on2)^3 passed in, from its polynomial's value v and slope dv
+template <class T>
+__device__ __forceinline__ void pd_switch(T x, T on2, T off2, T v, T dv, T& s, T& ds) {
+  const bool in = x > on2 && x < off2;
+  s = in ? v : (x <= on2 ? T(1) : T(0));
+  ds = in ? dv : T(0);
 }
 
-// pair energy and dE/dx for x < 225; two divisions per pair (1 / (x + 1) and, inside 8 A,
-// 1 / (x + sig2 / 2)), every other quotient a product with them
+// the LJ term of a pair inside 8 A added to its energy and dE/dx
 template <class T>
-__device__ __forceinline__ T pd_pair(T x, T qq, T eps, T sig2, T& dedx) {
-  T s, ds;
-  const T inv = T(1) / (x + T(1));
-  const T el = qq * inv;
-  pd_switch<T>(x, T(196), T(225), T(1) / T(24389), s, ds);  // (225 - 196)^3
-  T e = el * s;
-  T de = -el * inv * s + el * ds;
+__device__ __forceinline__ void pd_lj(T x, const LjPair<T>* pl, T& e, T& de) {
   if (x < T(64)) {
-    const T rden = T(1) / (x + T(0.5) * sig2);
-    const T sv = sig2 * rden;
+    const LjPair<T> p = *pl;
+    const T rden = T(1) / (x + T(0.5) * p.sig2);
+    const T sv = p.sig2 * rden;
     const T s2 = sv * sv, s3 = s2 * sv, s6 = s3 * s3;
-    const T lj = T(4) * eps * (s6 - s3);
+    const T v = T(4) * p.eps * (s6 - s3);
     const T dsv = -sv * rden;
-    const T dlj = T(4) * eps * (T(6) * s3 * s2 - T(3) * s2) * dsv;  // d(s^6 - s^3)/ds = 6 s^5 - 3 s^2
-    pd_switch<T>(x, T(49), T(64), T(1) / T(3375), s, ds);  // (64 - 49)^3
-    e += T(0.1) * (lj * s);
-    de += T(0.1) * (dlj * s + lj * ds);
+    const T dv = T(4) * p.eps * (T(6) * s3 * s2 - T(3) * s2) * dsv;  // d(s^6 - s^3)/ds = 6 s^5 - 3 s^2
+    const T a = T(64) - x, c = T(1) / T(3375);                       // (64 - 49)^3
+    T s, ds;
+    pd_switch<T>(x, T(49), T(64), a * a * (T(64) + T(2) * x - T(147)) * c, T(6) * a * (T(49) - x) * c, s, ds);
+    e += T(0.1) * (v * s);
+    de += T(0.1) * (dv * s + v * ds);
   }
-  dedx = de;
-  return e;
 }
 
-constexpr int kRows = SD_TILE / SD_GROUP;  // groups of a tile; candidates of a step (one row of 8 lanes each)
+// energies e and dE/dx of two pairs at squared distances x (both 0 from 225 on, where the switch is);
+// two divisions per pair (1 / (x + 1) and, inside 8 A, 1 / (x + sig2 / 2)), every other quotient a
+// product with them.  The LJ terms stand behind a branch of the whole warp: neighbours in a list are
+// neighbours in space, so many steps have no pair inside 8 A
+template <class T>
+__device__ __forceinline__ void pd_pairs(V2<T> x, V2<T> qq, const LjPair<T>* l0, const LjPair<T>* l1, T (&e)[2],
+                                         V2<T>& dedx) {
+  const V2<T> y = x + V2<T>(T(1));
+  const V2<T> inv(T(1) / y.first(), T(1) / y.second());
+  const V2<T> el = qq * inv;
+  const V2<T> a = V2<T>(T(225)) - x, c(T(1) / T(24389));  // (225 - 196)^3
+  const V2<T> v = a * a * (V2<T>(T(225)) + V2<T>(T(2)) * x - V2<T>(T(588))) * c;
+  const V2<T> dv = V2<T>(T(6)) * a * (V2<T>(T(196)) - x) * c;
+  const T x0 = x.first(), x1 = x.second();
+  T s[2], ds[2];
+  pd_switch<T>(x0, T(196), T(225), v.first(), dv.first(), s[0], ds[0]);
+  pd_switch<T>(x1, T(196), T(225), v.second(), dv.second(), s[1], ds[1]);
+  const V2<T> S(s[0], s[1]), E = el * S;
+  const V2<T> D = el * V2<T>(ds[0], ds[1]) - el * inv * S;
+  e[0] = E.first();
+  e[1] = E.second();
+  dedx = D;
+  if (__any_sync(0xffffffffu, x0 < T(64) || x1 < T(64))) {
+    T d0 = D.first(), d1 = D.second();
+    pd_lj<T>(x0, l0, e[0], d0);
+    pd_lj<T>(x1, l1, e[1], d1);
+    dedx = V2<T>(d0, d1);
+  }
+}
+
+// The force on a ligand atom, summed by all warps.  FP32: a 64-bit fixed-point number in units of
+// 1 / scale (a power of two that the host derives from the largest possible pair force, so the sum
+// cannot overflow), as two 32-bit words added by integer shared atomics, which the hardware has (an FP32
+// shared atomic is a compare-and-swap loop).  The sum is exact, so it does not depend on the order.  A
+// value that is not finite (a charge or parameter was not) sets *bad.  FP64 keeps its own type: fixed
+// point would be coarser than it.
+template <class T>
+struct Force {
+  T v;
+  static constexpr int kWords = 1;
+};
+template <>
+struct Force<float> {
+  unsigned v;
+  static constexpr int kWords = 2;
+};
+__device__ __forceinline__ void add_force(Force<float>* f, int words, int i, float v, float scale, int* bad) {
+  const float q = v * scale;
+  if (!(fabsf(q) < 9.0e18f)) *bad = 1;
+  const long long n = __float2ll_rn(q);
+  const unsigned lo = (unsigned)n;
+  const unsigned old = atomicAdd(&f[i].v, lo);
+  const unsigned hi = (unsigned)(n >> 32) + (old + lo < lo ? 1u : 0u);
+  if (hi) atomicAdd(&f[words + i].v, hi);
+}
+__device__ __forceinline__ double force_of(const Force<float>* f, int words, int i, float scale) {
+  const long long n = (long long)((unsigned long long)f[words + i].v << 32 | f[i].v);
+  return (double)n / (double)scale;
+}
+__device__ __forceinline__ void add_force(Force<double>* f, int, int i, double v, float, int*) {
+  atomicAdd(&f[i].v, v);
+}
+__device__ __forceinline__ double force_of(const Force<double>* f, int, int i, float) { return f[i].v; }
+
+constexpr int kGroups = SD_TILE / SD_GROUP;
+constexpr int kRow = SD_GROUP / 2;         // lanes of a row: one candidate, two atoms of the group per lane
+constexpr int kRows = 32 / kRow;           // candidates of a step
 constexpr int kPdList = 128;               // candidates of a group between two drains of the lists
 
 // a warp's tile
 template <class T>
 struct PdWarp {
   LigAtom<T> rec[SD_TILE];           // receptor atoms (position relative to t, charge)
-  float4 box[2 * kRows];             // centre and half extent of each group's bounding box
+  float4 box[2 * kGroups];           // centre and half extent of each group's bounding box
   int lj[SD_TILE];
-  unsigned short list[kRows][kPdList];  // each group's candidates: ligand slots
+  unsigned short list[kGroups][kPdList];  // each group's candidates: ligand slots
   unsigned short pend[64];           // pending candidate ligand slots of the tile
 };
 
@@ -110,24 +209,26 @@ __device__ __forceinline__ T warp_sum(T v) {
 // out_grad: nullable [n][6 + nmr + nml] (GRAD), energies go to C.scoring as score (-E) and to
 // L.energy_out (E) when set.  kSpill: the per-pose arrays live in this CTA's slice of the global
 // scratch L.spill instead of shared memory (ligands too large for it).  Four CTAs per SM (64
-// registers a thread) wherever the accumulators allow it: the pair terms are latency chains.
+// registers a thread) without forces: the pair terms are latency chains.
 template <class T, bool GRAD, bool kSpill>
-__global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4) pydock_kernel(ScoreLaunch L, double* out_grad) {
+__global__ void __launch_bounds__(pd_warps(sizeof(T) == 8, GRAD) * 32, GRAD ? 2 : 4)
+pydock_kernel(ScoreLaunch L, double* out_grad) {
+  constexpr int kWarps = pd_warps(sizeof(T) == 8, GRAD);
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   PdWarp<T>& W = reinterpret_cast<PdWarp<T>*>(smem_dyn)[threadIdx.x >> 5];
   unsigned char* const smem =
-      kSpill ? L.spill + (size_t)blockIdx.x * L.spill_stride : smem_dyn + kPdWarps * sizeof(PdWarp<T>);
+      kSpill ? L.spill + (size_t)blockIdx.x * L.spill_stride : smem_dyn + kWarps * sizeof(PdWarp<T>);
   __shared__ double sh_pose[7 + 2 * SD_MAX_MODES];
   __shared__ double sh_q[4], sh_qi[4];
   __shared__ LjPair<T> sh_lj[SD_LJ_TYPES * SD_LJ_TYPES];
-  __shared__ double sh_red[kPdWarps][32];
+  __shared__ double sh_red[kWarps][32];
   __shared__ float sh_rot[9];
   __shared__ float sh_bound[2];
-  __shared__ int sh_item, sh_ntile, sh_next;
+  __shared__ int sh_item, sh_ntile, sh_next, sh_bad;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned lt_mask = (1u << lane) - 1u;
-  const int atom = lane & (SD_GROUP - 1), crow = lane / SD_GROUP;  // a step's atom and candidate row
+  const int atom = lane & (kRow - 1), crow = lane / kRow;  // a step's first atom (the other: + kRow) and row
   for (int k = tid; k < SD_LJ_TYPES * SD_LJ_TYPES; k += blockDim.x) {
     const int a = k / SD_LJ_TYPES, b = k % SD_LJ_TYPES;
     sh_lj[k].eps = (T)sqrt(L.lj_eps[a] * L.lj_eps[b]);
@@ -175,6 +276,7 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
       sh_rot[8] = 1 - 2 * (x * x + y * y);
       sh_ntile = 0;
       sh_next = 0;
+      sh_bad = 0;
       double rx = C.lig_ref[0], ry = C.lig_ref[1], rz = C.lig_ref[2];
       quat_rotate(sh_q, sh_qi, rx, ry, rz);
       double* ref = C.ref + (size_t)p * 3;
@@ -185,29 +287,29 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
     __syncthreads();
     const double tx = sh_pose[0], ty = sh_pose[1], tz = sh_pose[2];
     const float dR = sh_bound[0], dL = sh_bound[1];
-    // per-pose arrays: ligand atoms [nls + 1] (LigAtom<T>; the last a far atom, the padding), GRAD: fx,
-    // fy, fz [nls + 1] (T), chunk spheres [nlc] (float4), llj [nls + 1], near tiles [ntiles] as found,
-    // in order of distance, and their distances
+    // per-pose arrays: ligand atoms [nls + 1] (the last a far atom, the padding), GRAD: their forces
+    // [words][3][nls + 4], chunk spheres [nlc], near tiles [ntiles] as found, in order of distance, and
+    // their distances, LJ types [nls + 1]
     LigAtom<T>* la = reinterpret_cast<LigAtom<T>*>(smem);
-    T* fx = reinterpret_cast<T*>(la + nls + 1);  // GRAD only: [3][nls + 4]
+    Force<T>* fx = reinterpret_cast<Force<T>*>(la + nls + 1);  // GRAD only
     const int fstride = nls + 4;
-    float4* chS = reinterpret_cast<float4*>(fx + (GRAD ? 3 * fstride : 0));
-    int* llj = reinterpret_cast<int*>(chS + nlc);
-    int* tlist = llj + nls + 1;
+    float4* chS = reinterpret_cast<float4*>(fx + (GRAD ? Force<T>::kWords * 3 * fstride : 0));
+    int* tlist = reinterpret_cast<int*>(chS + nlc);
     int* tord = tlist + C.ntiles;
     float* tdist = reinterpret_cast<float*>(tord + C.ntiles);
+    unsigned char* llj = reinterpret_cast<unsigned char*>(tdist + C.ntiles);
     if (tid == 0) {
-      la[nls] = LigAtom<T>{(T)3e18, (T)3e18, (T)3e18, T(0)};
+      la[nls] = LigAtom<T>{(T)1e17, (T)1e17, (T)1e17, T(0)};
       llj[nls] = 0;
     }
     if (GRAD)
-      for (int s = tid; s < 3 * fstride; s += blockDim.x) fx[s] = T(0);
+      for (int s = tid; s < Force<T>::kWords * 3 * fstride; s += blockDim.x) fx[s].v = 0;
     for (int s = tid; s < nls; s += blockDim.x) {
       if (C.l_perm[s] >= 0) {
         double x, y, z;
         ligand_exact(C, s, sh_pose, sh_q, sh_qi, x, y, z);
-        la[s] = LigAtom<T>{(T)(x - tx), (T)(y - ty), (T)(z - tz), (T)(kKe * (double)C.l_q[s])};
-        llj[s] = C.l_lj[s] * SD_LJ_TYPES;
+        la[s] = LigAtom<T>{-(T)(x - tx), -(T)(y - ty), -(T)(z - tz), (T)(kKe * (double)C.l_q[s])};
+        llj[s] = (unsigned char)C.l_lj[s];
       } else {
         la[s] = LigAtom<T>{(T)1e18, (T)1e18, (T)1e18, T(0)};
         llj[s] = 0;
@@ -292,9 +394,10 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
             hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
           }
         }
-        if (atom == 0) {
-          W.box[2 * crow] = make_float4(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2]), 0.f);
-          W.box[2 * crow + 1] =
+        if (lane % SD_GROUP == 0) {
+          W.box[2 * (lane / SD_GROUP)] =
+              make_float4(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2]), 0.f);
+          W.box[2 * (lane / SD_GROUP) + 1] =
               make_float4(0.5f * (hi[0] - lo[0]), 0.5f * (hi[1] - lo[1]), 0.5f * (hi[2] - lo[2]), 0.f);
         }
       }
@@ -305,9 +408,9 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
       bool more = true;
       do {
         // fill each group's list until the ligand is exhausted or a list may overflow
-        unsigned cnt[kRows];
+        unsigned cnt[kGroups];
 #pragma unroll
-        for (int g = 0; g < kRows; ++g) cnt[g] = 0;
+        for (int g = 0; g < kGroups; ++g) cnt[g] = 0;
         unsigned longest = 0;
         do {
           // collect candidates until a round is full or the ligand is exhausted
@@ -328,7 +431,7 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
             const int sb = (cb - 32 + __ffs(cm) - 1) * SD_TILE;
             cm &= cm - 1;
             const LigAtom<T> ca = la[sb + lane];
-            const float ax = (float)ca.x - cx, ay = (float)ca.y - cy, az = (float)ca.z - cz;
+            const float ax = (float)ca.x + cx, ay = (float)ca.y + cy, az = (float)ca.z + cz;
             const bool cand = ax * ax + ay * ay + az * az <= reach2;
             const unsigned am = __ballot_sync(0xffffffffu, cand);
             if (cand) W.pend[ncand + __popc(am & lt_mask)] = (unsigned short)(sb + lane);
@@ -340,10 +443,10 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
           const LigAtom<T> c = la[s];
           const float x = (float)c.x, y = (float)c.y, z = (float)c.z;
 #pragma unroll
-          for (int g = 0; g < kRows; ++g) {
+          for (int g = 0; g < kGroups; ++g) {
             const float4 bc = W.box[2 * g], bh = W.box[2 * g + 1];
-            const float ex = fmaxf(fabsf(x - bc.x) - bh.x, 0.f), ey = fmaxf(fabsf(y - bc.y) - bh.y, 0.f),
-                        ez = fmaxf(fabsf(z - bc.z) - bh.z, 0.f);
+            const float ex = fmaxf(fabsf(x + bc.x) - bh.x, 0.f), ey = fmaxf(fabsf(y + bc.y) - bh.y, 0.f),
+                        ez = fmaxf(fabsf(z + bc.z) - bh.z, 0.f);
             const bool in = fmaf(ez, ez, fmaf(ey, ey, ex * ex)) <= 225.1f;
             const unsigned am = __ballot_sync(0xffffffffu, in);
             if (in) W.list[g][cnt[g] + __popc(am & lt_mask)] = (unsigned short)s;
@@ -362,61 +465,58 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
         } while (more && longest <= kPdList - 32 - kRows);
         // each list is padded with the far atom to whole steps
 #pragma unroll
-        for (int g = 0; g < kRows; ++g)
+        for (int g = 0; g < kGroups; ++g)
           if (lane < kRows) W.list[g][cnt[g] + lane] = (unsigned short)nls;
         __syncwarp();
         unsigned counts = cnt[0] | cnt[1] << 8 | cnt[2] << 16 | cnt[3] << 24;
-        for (int g = 0; g < kRows; ++g, counts >>= 8) {
-          const LigAtom<T> r = W.rec[g * SD_GROUP + atom];
-          const LjPair<T>* ljrow = sh_lj + W.lj[g * SD_GROUP + atom];
+        for (int g = 0; g < kGroups; ++g, counts >>= 8) {
+          const LigAtom<T> ra = W.rec[g * SD_GROUP + atom], rb = W.rec[g * SD_GROUP + atom + kRow];
+          const V2<T> rx(ra.x, rb.x), ry(ra.y, rb.y), rz(ra.z, rb.z), rq(ra.q, rb.q);
+          // the LJ table is symmetric (products and sums of the two types' parameters), so it is read as
+          // [ligand type][receptor type]: the lanes of one candidate read entries of one row
+          const LjPair<T>* lja = sh_lj + W.lj[g * SD_GROUP + atom];
+          const LjPair<T>* ljb = sh_lj + W.lj[g * SD_GROUP + atom + kRow];
           const unsigned short* list = W.list[g] + crow;
           const int n = (int)(counts & 255u);
-          T hx = T(0), hy = T(0), hz = T(0);  // dE/dr of this lane's pairs
+          V2<T> hx(T(0)), hy(T(0)), hz(T(0));  // dE/dr of this lane's pairs
           for (int c = 0; c < n; c += kRows) {
             const int s = list[c];
-            const LigAtom<T> a = la[s];
-            const T dx = r.x - a.x, dy = r.y - a.y, dz = r.z - a.z;
-            const T x = dx * dx + dy * dy + dz * dz;
-            T f0 = T(0), f1 = T(0), f2 = T(0);
-            if (x < T(225)) {
-              T dedx;
-              // the table is symmetric (products and sums of the two types' parameters), so it is read as
-              // [ligand type][receptor type]: the lanes of one candidate read entries of one row
-              const LjPair<T> lj = ljrow[llj[s]];
-              const T e = pd_pair<T>(x, r.q * a.q, lj.eps, lj.sig2, dedx);
-              es += (double)e;
-              if (GRAD) {
-                const T g2 = T(2) * dedx;
-                f0 = g2 * dx;
-                f1 = g2 * dy;
-                f2 = g2 * dz;
-                hx += f0;
-                hy += f1;
-                hz += f2;
-              }
-            }
+            const LigAtom<T> l = la[s];
+            const int lj = llj[s] * SD_LJ_TYPES;
+            const V2<T> dx = rx + V2<T>(l.x), dy = ry + V2<T>(l.y), dz = rz + V2<T>(l.z);
+            const V2<T> x = dx * dx + dy * dy + dz * dz;
+            T e[2];
+            V2<T> dedx;
+            pd_pairs<T>(x, rq * V2<T>(l.q), lja + lj, ljb + lj, e, dedx);
+            es += (double)e[0];
+            es += (double)e[1];
             if (GRAD) {
-              // the row's forces on its candidate: lanes 0, 2 and 4 of the row end with x, y and z
-              const bool h4 = (lane & 4) != 0, h2 = (lane & 2) != 0;
-              const T k0 = (h4 ? f2 : f0) + __shfl_xor_sync(0xffffffffu, h4 ? f0 : f2, 4);
-              const T k1 = (h4 ? T(0) : f1) + __shfl_xor_sync(0xffffffffu, h4 ? f1 : T(0), 4);
-              T v = (h2 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, h2 ? k0 : k1, 2);
-              v += __shfl_xor_sync(0xffffffffu, v, 1);
-              if ((lane & 1) == 0 && atom < 6) atomicAdd(&fx[(atom >> 1) * fstride + s], -v);
+              const V2<T> g2 = V2<T>(T(2)) * dedx;
+              const V2<T> fx2 = g2 * dx, fy2 = g2 * dy, fz2 = g2 * dz;
+              hx = hx + fx2;
+              hy = hy + fy2;
+              hz = hz + fz2;
+              // the row's forces on its candidate: lanes 0, 1 and 2 of the row end with x, y and z
+              const T f0 = fx2.first() + fx2.second(), f1 = fy2.first() + fy2.second(), f2 = fz2.first() + fz2.second();
+              const bool h2 = (lane & 2) != 0, h1 = (lane & 1) != 0;
+              const T k0 = (h2 ? f2 : f0) + __shfl_xor_sync(0xffffffffu, h2 ? f0 : f2, 2);
+              const T k1 = (h2 ? T(0) : f1) + __shfl_xor_sync(0xffffffffu, h2 ? f1 : T(0), 2);
+              const T v = (h1 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, h1 ? k0 : k1, 1);
+              if (atom < 3) add_force(fx, 3 * fstride, atom * fstride + s, -v, L.force_scale, &sh_bad);
             }
           }
           if (GRAD) {
-            // sum over the rows; the lanes of the group's own row keep it
-            hx += __shfl_xor_sync(0xffffffffu, hx, 8);
-            hy += __shfl_xor_sync(0xffffffffu, hy, 8);
-            hz += __shfl_xor_sync(0xffffffffu, hz, 8);
-            hx += __shfl_xor_sync(0xffffffffu, hx, 16);
-            hy += __shfl_xor_sync(0xffffffffu, hy, 16);
-            hz += __shfl_xor_sync(0xffffffffu, hz, 16);
-            if (crow == g) {
-              gx += hx;
-              gy += hy;
-              gz += hz;
+            // sum over the rows; the lanes of the group's own atoms keep it
+            T a[6] = {hx.first(), hy.first(), hz.first(), hx.second(), hy.second(), hz.second()};
+#pragma unroll
+            for (int k = 0; k < 6; ++k)
+#pragma unroll
+              for (int o = kRow; o < 32; o <<= 1) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
+            if (lane / SD_GROUP == g) {
+              const bool second = (lane & kRow) != 0;
+              gx += second ? a[3] : a[0];
+              gy += second ? a[4] : a[1];
+              gz += second ? a[5] : a[2];
             }
           }
         }
@@ -435,7 +535,7 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
     const int ng = GRAD ? 6 + C.nmr + C.nml : 0;
     acc[0] = es;
     if (GRAD) {
-      for (int k = 1; k <= ng; ++k) acc[k] = 0.0;
+      for (int k = 1; k <= ng; ++k) acc[k] = sh_bad ? nan("") : 0.0;
       for (int m = 0; m < C.nmr; ++m) acc[1 + 6 + m] = (double)grec[m];
       // ligand side: F_j projected on t, w, ligand modes
       double Rm[9];
@@ -456,8 +556,10 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
       }
       for (int s = tid; s < nls; s += blockDim.x) {
         if (C.l_perm[s] < 0) continue;
-        const double Fx = (double)fx[s], Fy = (double)fx[fstride + s], Fz = (double)fx[2 * fstride + s];
-        const double px = (double)la[s].x, py = (double)la[s].y, pz = (double)la[s].z;  // l_j - t
+        const double Fx = force_of(fx, 3 * fstride, s, L.force_scale),
+                     Fy = force_of(fx, 3 * fstride, fstride + s, L.force_scale),
+                     Fz = force_of(fx, 3 * fstride, 2 * fstride + s, L.force_scale);
+        const double px = -(double)la[s].x, py = -(double)la[s].y, pz = -(double)la[s].z;  // l_j - t
         acc[1] += Fx;
         acc[2] += Fy;
         acc[3] += Fz;
@@ -482,7 +584,7 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
     __syncthreads();
     if (tid <= ng) {
       double v = 0.0;
-      for (int i = 0; i < kPdWarps; ++i) v += sh_red[i][tid];
+      for (int i = 0; i < kWarps; ++i) v += sh_red[i][tid];
       if (tid == 0) {
         C.scoring[p] = -v;
         if (L.energy_out) L.energy_out[p] = v;
@@ -499,11 +601,30 @@ __global__ void __launch_bounds__(kPdWarps * 32, GRAD && sizeof(T) == 8 ? 2 : 4)
 size_t pydock_smem_bytes(int precision, bool grad, int max_nl, int max_nr) {
   const size_t nlc = (size_t)(max_nl + SD_TILE - 1) / SD_TILE, nls = nlc * SD_TILE;
   const size_t ts = precision == SD_PREC_MIXED ? 4 : 8;
-  return ts * (4 * (nls + 1) + (grad ? 3 * (nls + 4) : 0)) + 16 * nlc + 4 * (nls + 1) +
+  // forces: 24 bytes an atom in both types
+  return ts * 4 * (nls + 1) + (grad ? 24 * (nls + 4) : 0) + 16 * nlc + (nls + 1) +
          12 * ((max_nr + SD_TILE - 1) / SD_TILE) + 16;
 }
-size_t pydock_warp_bytes(int precision) {
-  return kPdWarps * (precision == SD_PREC_MIXED ? sizeof(PdWarp<float>) : sizeof(PdWarp<double>));
+size_t pydock_warp_bytes(int precision, bool grad) {
+  const bool fp64 = precision != SD_PREC_MIXED;
+  return pd_warps(fp64, grad) * (fp64 ? sizeof(PdWarp<double>) : sizeof(PdWarp<float>));
+}
+
+// the scale of FP32 ligand forces: pair forces are at most 0.7 kKe q q' (electrostatics) plus 1.6 eps
+// (3072 / sig^2 + 26) (LJ: |6 s^5 - 3 s^2| <= 192, s^2 <= 4, within 8 A), times the receptor's atoms
+float pydock_force_scale(double max_q_rec, double max_q_lig, const double* eps, const double* sigma, int max_nr) {
+  double f = 0.7 * kKe * max_q_rec * max_q_lig;
+  double lj = 0;
+  for (int a = 0; a < SD_LJ_TYPES; ++a)
+    for (int b = 0; b < SD_LJ_TYPES; ++b) {
+      const double e = std::sqrt(eps[a] * eps[b]), sg = 0.5 * (sigma[a] + sigma[b]);
+      const double v = 1.6 * e * ((sg != 0 ? 3072.0 / (sg * sg) : 0.0) + 26.0);
+      if (std::isfinite(v)) lj = std::max(lj, v);
+    }
+  f = (f + lj) * std::max(8, max_nr);
+  if (!std::isfinite(f)) f = 1e30;
+  const int k = (int)std::floor(61.0 - std::log2(std::max(f, 1e-9)));
+  return std::ldexp(1.0f, std::min(100, std::max(-100, k)));
 }
 
 const void* pydock_kernel_ptr(int precision, bool grad, bool spill) {
@@ -519,12 +640,12 @@ int pydock_launch(const ScoreLaunch& L, int precision, bool grad, double* out_gr
                   cudaStream_t st, bool spill) {
   ScoreLaunch l = L;
   void* args[] = {(void*)&l, (void*)&out_grad};
-  if (cudaLaunchKernel(pydock_kernel_ptr(precision, grad, spill), dim3(grid), dim3(kPdWarps * 32), args,
+  if (cudaLaunchKernel(pydock_kernel_ptr(precision, grad, spill), dim3(grid), dim3(pydock_threads(precision, grad)), args,
                        smem, st) != cudaSuccess)
     return SD_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? SD_OK : SD_ERR_CUDA;
 }
 
-int pydock_threads() { return kPdWarps * 32; }
+int pydock_threads(int precision, bool grad) { return pd_warps(precision != SD_PREC_MIXED, grad) * 32; }
 
 }  // namespace sd

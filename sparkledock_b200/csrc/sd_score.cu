@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include "sd_internal.h"
+#include "sd_packed.cuh"
 #include "sd_pose.cuh"
 
 namespace sd {
@@ -336,7 +337,7 @@ static const MixedVariant& mixed_variant(int v) { return kMixedVariants[v < 0 ||
 // bytes of the scorer's per-warp buffers, in dynamic shared memory in front of the per-pose arrays
 // (alone there in the spill instantiation)
 size_t score_warp_bytes(int precision, int scoring, int variant, bool spill) {
-  if (scoring == SD_SCORING_PYDOCK) return pydock_warp_bytes(precision);
+  if (scoring == SD_SCORING_PYDOCK) return pydock_warp_bytes(precision, false);
   if (precision != SD_PREC_MIXED) return 0;
   return sizeof(WarpBufs) * (spill ? kMixedSpill.warps : mixed_variant(variant).warps);
 }
@@ -358,12 +359,12 @@ int mixed_variant_warps(int v) { return mixed_variant(v).warps; }
 int mixed_variant_min_blocks(int v) { return mixed_variant(v).min_blocks; }
 
 int score_threads_of(int precision, int scoring, int variant) {
-  if (scoring == SD_SCORING_PYDOCK) return pydock_threads();
+  if (scoring == SD_SCORING_PYDOCK) return pydock_threads(precision, false);
   return precision == SD_PREC_MIXED ? mixed_variant_warps(variant) * 32 : kFp64Threads;
 }
 
 int score_threads_spill(int precision, int scoring) {
-  if (scoring == SD_SCORING_PYDOCK) return pydock_threads();
+  if (scoring == SD_SCORING_PYDOCK) return pydock_threads(precision, false);
   return precision == SD_PREC_MIXED ? kMixedSpill.warps * 32 : kFp64Threads;
 }
 
