@@ -132,7 +132,6 @@ struct sd_ctx {
   // step graph
   cudaGraphExec_t graph = nullptr;
   int graph_precision = -1;
-  int score_threads = 256;
   int score_grid = 0;
   size_t score_smem = 0;
   bool score_spill = false;  // the last configured scorer launch uses the spill instantiation
@@ -141,6 +140,7 @@ struct sd_ctx {
   int score_poses = 1;       // poses per CTA of the last configured scorer launch
   // autotuner state (mixed-precision DFIRE kernel variants)
   int mixed_variant = 0;
+  int smem_sm = 0;         // shared memory of an SM
   bool tuned = false;
   double tune_ms[SD_MAX_VARIANTS] = {};
 };
@@ -457,18 +457,18 @@ int grow_spill(sd_ctx* c, size_t bytes) {
 // memory, threads.  When the per-pose arrays of the largest complex do not fit in the shared memory
 // a CTA may use, the spill instantiation is chosen (no dynamic shared memory) and the context's
 // spill scratch is sized to grid x per-CTA bytes; alloc = false refuses that instead of allocating.
-int configure_score_v(sd_ctx* c, int precision, int variant, int* grid, size_t* smem, bool alloc = true) {
+int configure_score(sd_ctx* c, int precision, int variant, int* grid, size_t* smem, bool alloc = true) {
   const size_t need = score_smem_bytes(precision, c->scoring, c->max_nr, c->max_nl, 1);
   const void* k = score_kernel_ptr(precision, c->scoring, variant, false);
   cudaFuncAttributes fa;
   SD_CUDA(cudaFuncGetAttributes(&fa, k));
   size_t sm = need + score_warp_bytes(precision, c->scoring, variant, false);
   const bool spill = sm + fa.sharedSizeBytes > (size_t)c->smem_optin;
-  int threads = score_threads_of(precision, c->scoring, variant);
+  int threads = score_threads_of(precision, c->scoring, variant, false);
   if (spill) {
     k = score_kernel_ptr(precision, c->scoring, variant, true);
     sm = score_warp_bytes(precision, c->scoring, variant, true);
-    threads = score_threads_spill(precision, c->scoring);
+    threads = score_threads_of(precision, c->scoring, variant, true);
   }
   int per_sm = 0;
   auto occupancy = [&](size_t bytes) -> int {
@@ -495,7 +495,6 @@ int configure_score_v(sd_ctx* c, int precision, int variant, int* grid, size_t* 
   if (per_sm < 1) return fail(SD_ERR_ARG, "scoring kernel does not fit on an SM (shared memory)");
   *grid = per_sm * c->nsm;
   *smem = sm;
-  c->score_threads = threads;
   c->score_spill = spill;
   if (spill) {
     const size_t stride = (need + 255) & ~(size_t)255;
@@ -510,8 +509,14 @@ int configure_score_v(sd_ctx* c, int precision, int variant, int* grid, size_t* 
   return SD_OK;
 }
 
-int configure_score(sd_ctx* c, int precision, int* grid, size_t* smem, bool alloc = true) {
-  return configure_score_v(c, precision, c->mixed_variant, grid, smem, alloc);
+// the compiled variant of a precision's DFIRE kernel for a launch of at most `poses` poses; stateless:
+// not a GSO step, whose mixed variant the autotuner chose on its own poses
+int score_variant(const sd_ctx* c, int precision, int poses, bool stateless) {
+  if (precision == SD_PREC_FP64) return fp64_shape(c->max_nr, c->max_nl, c->smem_sm, poses, c->nsm);
+  if (precision != SD_PREC_MIXED || !stateless || poses > c->nsm) return c->mixed_variant;
+  const size_t cta = score_smem_bytes(precision, SD_SCORING_DFIRE, c->max_nr, c->max_nl, 1) +
+                     score_warp_bytes(precision, SD_SCORING_DFIRE, SD_MIXED_FEW, false) + 2048;
+  return cta <= (size_t)c->smem_optin ? SD_MIXED_FEW : c->mixed_variant;
 }
 
 // the spill scratch of the last configured launch (null pointers when it uses shared memory)
@@ -598,7 +603,7 @@ int autotune_mixed(sd_ctx* c) {
   for (int v = 0; v < nv && v < SD_MAX_VARIANTS; ++v) {
     int grid;
     size_t sm;
-    if (configure_score_v(c, SD_PREC_MIXED, v, &grid, &sm) != SD_OK) {
+    if (configure_score(c, SD_PREC_MIXED, v, &grid, &sm) != SD_OK) {
       c->tune_ms[v] = -1;
       continue;
     }
@@ -613,7 +618,7 @@ int autotune_mixed(sd_ctx* c) {
       ctl.grab[0] = ctl.grab[1] = 0;
       SD_CUDA(cudaMemcpyAsync(c->d_ctl_scratch, &ctl, sizeof ctl, cudaMemcpyHostToDevice, c->stream));
       SD_CUDA(cudaEventRecord(e0, c->stream));
-      if ((rc = score_launch(L, SD_PREC_MIXED, c->scoring, grid, c->score_threads, sm, c->stream, v, false)))
+      if ((rc = score_launch(L, SD_PREC_MIXED, c->scoring, grid, sm, c->stream, v, false)))
         return fail(rc, std::string("autotune launch: ") + cudaGetErrorString(cudaGetLastError()));
       SD_CUDA(cudaEventRecord(e1, c->stream));
       SD_CUDA(cudaEventSynchronize(e1));
@@ -634,7 +639,7 @@ int autotune_mixed(sd_ctx* c) {
   return SD_OK;
 }
 
-int enqueue_step(sd_ctx* c, int precision, int grid, size_t sm) {
+int enqueue_step(sd_ctx* c, int precision, int variant, int grid, size_t sm) {
   int rc;
   ScoreLaunch L{};
   L.cplx = c->d_cplx;
@@ -646,8 +651,7 @@ int enqueue_step(sd_ctx* c, int precision, int grid, size_t sm) {
   L.lj_sigma = c->d_lj_sigma;
   L.energy_out = nullptr;
   set_spill(c, L);
-  if ((rc = score_launch(L, precision, c->scoring, grid, c->score_threads, sm, c->stream, c->mixed_variant,
-                         c->score_spill)))
+  if ((rc = score_launch(L, precision, c->scoring, grid, sm, c->stream, variant, c->score_spill)))
     return fail(rc, std::string("score kernel launch: ") + cudaGetErrorString(cudaGetLastError()));
   GsoLaunch G{};
   G.cplx = c->d_cplx;
@@ -678,7 +682,7 @@ namespace sd {
 // Read-only view of a context for sd_score_poses_noalloc (sd_noalloc.cu): the device
 // descriptor of one complex, table pointers and the launch shape of the scoring kernel.
 // Makes the context's device current; allocates nothing.
-int ctx_noalloc_view(sd_ctx* c, int ci, int precision, DevComplex* desc, ScoreLaunch* L, int* grid, size_t* smem,
+int ctx_noalloc_view(sd_ctx* c, int ci, int precision, int n, DevComplex* desc, ScoreLaunch* L, int* grid, size_t* smem,
                      int* device, cudaStream_t* stream, int* scoring, int* variant) {
   if (!c || ci < 0 || ci >= c->ncplx) return fail(SD_ERR_ARG, "sd_score_poses_noalloc: bad context or complex");
   if (precision < SD_PREC_FP64_REF || precision > SD_PREC_MIXED)
@@ -686,7 +690,8 @@ int ctx_noalloc_view(sd_ctx* c, int ci, int precision, DevComplex* desc, ScoreLa
   SD_CUDA(cudaSetDevice(c->device));
   // a complex too large for shared memory uses the context's spill scratch, allocated by an
   // earlier allocating call; this call only uses it when it is already large enough
-  int rc = configure_score(c, precision, grid, smem, false);
+  *variant = score_variant(c, precision, n, true);
+  int rc = configure_score(c, precision, *variant, grid, smem, false);
   if (rc) return rc;
   *desc = c->cx[ci].d;
   memset(L, 0, sizeof *L);
@@ -697,7 +702,6 @@ int ctx_noalloc_view(sd_ctx* c, int ci, int precision, DevComplex* desc, ScoreLa
   *device = c->device;
   *stream = c->stream;
   *scoring = c->scoring;
-  *variant = c->mixed_variant;
   return SD_OK;
 }
 }  // namespace sd
@@ -767,6 +771,7 @@ int sd_ctx_create(const sd_complex_desc* complexes, int n_complexes, const sd_ta
   c->device = device;
   c->nsm = prop.multiProcessorCount;
   c->smem_optin = (int)prop.sharedMemPerBlockOptin;
+  c->smem_sm = (int)prop.sharedMemPerMultiprocessor;
   c->ncplx = n_complexes;
   c->scoring = scoring;
   c->precision = precision;
@@ -1004,11 +1009,12 @@ int sd_step(sd_ctx* c, int n_steps, int sync) {
     }
     int grid;
     size_t sm;
-    int rc = configure_score(c, c->precision, &grid, &sm);
+    const int variant = score_variant(c, c->precision, c->total_glowworms, false);
+    int rc = configure_score(c, c->precision, variant, &grid, &sm);
     if (rc) return rc;
     cudaGraph_t g;
     SD_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-    rc = enqueue_step(c, c->precision, grid, sm);
+    rc = enqueue_step(c, c->precision, variant, grid, sm);
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     if (rc) {
       if (e == cudaSuccess) cudaGraphDestroy(g);
@@ -1102,7 +1108,8 @@ int sd_score_poses(sd_ctx* c, int ci, const double* poses, int n, int precision,
   SD_CUDA(cudaMemcpyAsync(c->d_ctl_scratch, &ctl, sizeof ctl, cudaMemcpyHostToDevice, c->stream));
   int grid;
   size_t sm;
-  if ((rc = configure_score(c, precision, &grid, &sm))) return rc;
+  const int variant = score_variant(c, precision, n, true);
+  if ((rc = configure_score(c, precision, variant, &grid, &sm))) return rc;
   ScoreLaunch L{};
   L.cplx = c->d_cplx_scratch;
   L.ctl = c->d_ctl_scratch;
@@ -1113,8 +1120,7 @@ int sd_score_poses(sd_ctx* c, int ci, const double* poses, int n, int precision,
   L.lj_sigma = c->d_lj_sigma;
   L.energy_out = (double*)c->s_energy.p;
   set_spill(c, L);
-  if ((rc = score_launch(L, precision, c->scoring, grid, c->score_threads, sm, c->stream, c->mixed_variant,
-                         c->score_spill)))
+  if ((rc = score_launch(L, precision, c->scoring, grid, sm, c->stream, variant, c->score_spill)))
     return fail(rc, std::string("score kernel: ") + cudaGetErrorString(cudaGetLastError()));
   SD_CUDA(cudaMemcpyAsync(score_out, c->s_score.p, (size_t)n * 8, cudaMemcpyDeviceToHost, c->stream));
   if (energy_out)

@@ -25,6 +25,7 @@
 #define SD_MAX_GLOWWORMS 6144   /* glowworms per swarm: luciferin + reference points in shared memory */
 #define SD_CULL_MARGIN 0.05f    /* A, covers FP32 rounding of the conservative culling tests */
 #define SD_MAX_VARIANTS 16      /* compiled variants of the mixed DFIRE kernel (autotuner) */
+#define SD_MIXED_FEW SD_MAX_VARIANTS  /* the mixed variant for stateless calls with few poses (not tuned) */
 #define SD_NOALLOC_MAX_POSES 65536           /* poses per sd_score_poses_noalloc call */
 #define SD_NOALLOC_SCRATCH_BYTES (288 * 1024) /* its file-scope device scratch array */
 
@@ -151,12 +152,12 @@ struct GsoLaunch {
 
 // kernel launchers (sd_score.cu, sd_gso.cu)
 // spill: the instantiation that keeps its per-pose arrays in L.spill instead of shared memory
-int score_launch(const ScoreLaunch& L, int precision, int scoring, int grid, int threads, size_t smem,
-                 cudaStream_t st, int variant, bool spill);
+int score_launch(const ScoreLaunch& L, int precision, int scoring, int grid, size_t smem, cudaStream_t st, int variant,
+                 bool spill);
 size_t score_smem_bytes(int precision, int scoring, int max_nr, int max_nl, int poses);
 size_t score_warp_bytes(int precision, int scoring, int variant, bool spill);
-int score_threads_of(int precision, int scoring, int variant);
-int score_threads_spill(int precision, int scoring);
+int score_threads_of(int precision, int scoring, int variant, bool spill);
+int fp64_shape(int max_nr, int max_nl, int smem_sm, int poses, int nsm);
 const void* score_kernel_ptr(int precision, int scoring, int variant, bool spill);
 int mixed_variant_count();
 int mixed_variant_warps(int v);

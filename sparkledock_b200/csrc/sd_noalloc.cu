@@ -27,7 +27,7 @@
 
 namespace sd {
 // defined in sd_api.cu: the parts of a context this call reads (no allocation)
-int ctx_noalloc_view(sd_ctx* c, int ci, int precision, DevComplex* desc, ScoreLaunch* L, int* grid, size_t* smem,
+int ctx_noalloc_view(sd_ctx* c, int ci, int precision, int n, DevComplex* desc, ScoreLaunch* L, int* grid, size_t* smem,
                      int* device, cudaStream_t* stream, int* scoring, int* variant);
 }  // namespace sd
 
@@ -125,7 +125,7 @@ extern "C" int sd_score_poses_noalloc(sd_ctx* ctx, int complex_idx, const double
   int grid = 0, device = 0, scoring = SD_SCORING_DFIRE, variant = 0;
   size_t smem = 0;
   cudaStream_t stream = nullptr;
-  int rc = ctx_noalloc_view(ctx, complex_idx, precision, &desc, &L, &grid, &smem, &device, &stream, &scoring, &variant);
+  int rc = ctx_noalloc_view(ctx, complex_idx, precision, n, &desc, &L, &grid, &smem, &device, &stream, &scoring, &variant);
   if (rc) return rc;
   if (n == 0) return SD_OK;
   if (device < 0 || device >= 64) return fail(SD_ERR_ARG, "sd_score_poses_noalloc: device index above 63");
@@ -175,9 +175,7 @@ extern "C" int sd_score_poses_noalloc(sd_ctx* ctx, int complex_idx, const double
   L.work[1] = L.work[0];
   L.energy_out = d_energy;
   const bool spill = L.spill != nullptr;
-  if ((rc = score_launch(L, precision, scoring, grid,
-                         spill ? score_threads_spill(precision, scoring) : score_threads_of(precision, scoring, variant),
-                         smem, stream, variant, spill)))
+  if ((rc = score_launch(L, precision, scoring, grid, smem, stream, variant, spill)))
     return fail(rc, std::string("sd_score_poses_noalloc: scoring kernel: ") + cudaGetErrorString(cudaGetLastError()));
   if (sync) {
     unsigned long long bad = 0;

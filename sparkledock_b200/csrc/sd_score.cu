@@ -6,21 +6,14 @@
 //   E = sum_i ( sum_j [d2_ij <= 225] table[tR_i][tL_j][dist_to_bins[(int)(2 sqrt(d2)-1)]-1] )
 //   score = -(0.0157 E - 4.7)
 //
-// Design (one persistent kernel, one CTA per pose at a time, dynamic work grabbing):
-//  * the ligand of the pose is transformed once into shared memory (exact FP64 transform);
-//  * receptor atoms are pre-sorted into spatial tiles of 32 (one warp lane per atom); a warp
-//    takes a tile, skips it when its bounding sphere (inflated by the pose's ANM displacement
-//    bound) is beyond 15 A of the ligand's sphere, and otherwise builds ballot masks of the
-//    ligand atoms that can reach the tile, 32 at a time, visiting them in ascending j;
-//  * FP64 modes: each lane's partial v_i sums its pairs in ascending j exactly as the
-//    reference, and the pose energy adds the v_i in ascending original i (zeros skipped:
-//    adding +0.0 never changes a sum), so energies are bit-identical to the reference
-//    order with or without culling;
-//  * MIXED (sd_score_mixed.cuh): distances from FP32 coordinates centred on the pose
-//    translation, an exact per-pair bin unless d2 lies within a proven error bound B of a bin
-//    or cutoff edge, in which case the pair is recomputed in FP64 exactly (counted); FP64 sums
-//    of the FP64 table values.
-#include <cuda_fp16.h>
+// Persistent kernels, one or two poses per CTA at a time, dynamic work grabbing:
+//  * FP64_REF (here): every pair in FP64, each receptor atom's partial v_i summed in ascending j and
+//    the pose energy over the v_i in ascending i, as the reference;
+//  * FP64 (sd_score_fp64.cuh): the same sums, so the same bits, over the pairs that culling leaves;
+//  * MIXED (sd_score_mixed.cuh): the same table values in another order of summation.
+// FP64 and MIXED take distances from FP32 coordinates centred on the pose translation: an exact
+// per-pair bin unless the distance lies within a proven error bound of a bin or cutoff edge, in which
+// case the pair is decided in FP64 from the exact transforms.
 #include <cuda_runtime.h>
 
 #include "sd_internal.h"
@@ -64,36 +57,30 @@ __device__ __forceinline__ int exact_key(double d2, const double* T) {
   return k;
 }
 
-// PREC: SD_PREC_FP64_REF (no culling) or SD_PREC_FP64 (culled); the mixed-precision kernel is
-// in sd_score_mixed.cuh.  16 warps per CTA: the per-pose shared memory (receptor accumulators,
-// ligand atoms) allows two CTAs per SM, so the warps per CTA set the SM's residency.
-// kSpill: the per-pose arrays live in this CTA's slice of the global scratch L.spill instead
-// (complexes too large for shared memory); the arithmetic is the same.
-constexpr int kFp64Threads = 512;
+// SD_PREC_FP64_REF: all Nr*Nl pairs in FP64, one lane per receptor atom, ligand atoms in order.  16
+// warps per CTA: the per-pose shared memory (receptor accumulators, ligand atoms) allows two CTAs per
+// SM, so the warps per CTA set the SM's residency.  kSpill: the per-pose arrays live in this CTA's slice
+// of the global scratch L.spill instead (complexes too large for shared memory); the arithmetic is the
+// same.
+constexpr int kRefThreads = 512;
 
-template <int PREC, bool kSpill>
-__global__ void __launch_bounds__(kFp64Threads) dfire_score_kernel(ScoreLaunch L) {
+template <bool kSpill>
+__global__ void __launch_bounds__(kRefThreads) dfire_score_ref_kernel(ScoreLaunch L) {
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   unsigned char* const smem = kSpill ? L.spill + (size_t)blockIdx.x * L.spill_stride : smem_dyn;
   __shared__ double sh_pose[7 + 2 * SD_MAX_MODES];
   __shared__ double sh_q[4], sh_qi[4];
   __shared__ double sh_T[32];
-  __shared__ float sh_Tf[32];
   __shared__ int sh_lut[32];
-  __shared__ int sh_item;
-  __shared__ int sh_ntile, sh_next;
-  __shared__ float sh_bound[4];  // dR, dL
-  __shared__ unsigned long long sh_fallback, sh_z, sh_cut, sh_pairs, sh_evals;
+  __shared__ int sh_item, sh_next;
+  __shared__ unsigned long long sh_z, sh_cut, sh_pairs, sh_evals;
 
-  constexpr bool kCull = PREC != SD_PREC_FP64_REF;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid < 32) {
     sh_T[tid] = c_T[tid];
-    sh_Tf[tid] = c_Tf[tid];
     sh_lut[tid] = c_binlut[tid];
   }
   if (tid == 0) {
-    sh_fallback = 0;
     sh_z = 0;
     sh_cut = 0;
     sh_pairs = 0;
@@ -125,35 +112,19 @@ __global__ void __launch_bounds__(kFp64Threads) dfire_score_kernel(ScoreLaunch L
       sh_q[2] = sh_pose[5];
       sh_q[3] = sh_pose[6];
       quat_inverse(sh_q, sh_qi);
-      float dR = 0.f, dL = 0.f;
-      for (int m = 0; m < C.nmr; ++m) dR += fabsf((float)sh_pose[7 + m]) * C.mnorm_r[m];
-      for (int m = 0; m < C.nml; ++m) dL += fabsf((float)sh_pose[7 + C.nmr + m]) * C.mnorm_l[m];
-      dR = dR * 1.0001f + 1e-4f;
-      dL = dL * 1.0001f + 1e-4f;
-      sh_bound[0] = dR;
-      sh_bound[1] = dL;
+      sh_next = 0;
     }
     __syncthreads();
     // ---- ligand of this pose into shared memory ----
     const double tx = sh_pose[0], ty = sh_pose[1], tz = sh_pose[2];
-    float4* ligF = reinterpret_cast<float4*>(smem);  // centred FP32 (x,y,z, col bits)
-    LigD* ligD = reinterpret_cast<LigD*>(smem + (size_t)16 * ((nl + 1) & ~1));
-    double* vacc = reinterpret_cast<double*>(reinterpret_cast<unsigned char*>(ligD) + (size_t)32 * nl);
-    int* tlist = reinterpret_cast<int*>(vacc + nr);  // tiles within reach of the ligand
-    int* tord = tlist + C.ntiles;                    // the same, closest to t first
-    float* tdist = reinterpret_cast<float*>(tord + C.ntiles);
-    if (tid == 0) {
-      sh_ntile = 0;
-      sh_next = 0;
-    }
+    LigD* ligD = reinterpret_cast<LigD*>(smem);
+    double* vacc = reinterpret_cast<double*>(ligD + nl);
     for (int s = tid; s < C.nlchunks * SD_TILE; s += blockDim.x) {
       const int j = C.l_perm[s];
       if (j < 0) continue;
       double x, y, z;
       ligand_exact(C, s, sh_pose, sh_q, sh_qi, x, y, z);
-      const int col = C.l_col[s];
-      ligF[j] = make_float4((float)(x - tx), (float)(y - ty), (float)(z - tz), __int_as_float(col));
-      ligD[j] = LigD{x, y, z, col, 0};
+      ligD[j] = LigD{x, y, z, C.l_col[s], 0};
     }
     for (int i = tid; i < nr; i += blockDim.x) vacc[i] = 0.0;
     if (tid == 0) {
@@ -166,118 +137,49 @@ __global__ void __launch_bounds__(kFp64Threads) dfire_score_kernel(ScoreLaunch L
       ref[2] = z + tz;
     }
     __syncthreads();
-    const float dR = sh_bound[0], dL = sh_bound[1];
-    const float tile_reach_base = 15.0f + dR + SD_CULL_MARGIN;
-    const float lig_reach = C.lig_radius + dL;
-    for (int k = tid; k < C.ntiles; k += blockDim.x) {
-      bool keep = true;
-      if (kCull) {
-        const float4 tile = C.r_tile[k];
-        const float cx = (float)((double)tile.x - tx), cy = (float)((double)tile.y - ty),
-                    cz = (float)((double)tile.z - tz);
-        const float reach = tile_reach_base + tile.w + lig_reach;
-        keep = cx * cx + cy * cy + cz * cz <= reach * reach;
-        if (keep) {
-          const int at = atomicAdd(&sh_ntile, 1);
-          tlist[at] = k;
-          // a NaN distance (non-finite pose) ranks last: the ranking below must stay a strict total
-          // order, or tord would not be a permutation of the kept tiles
-          const float dd = cx * cx + cy * cy + cz * cz;
-          tdist[at] = dd == dd ? dd : 3.0e38f;
-        }
-      } else {
-        tlist[atomicAdd(&sh_ntile, 1)] = k;
-      }
-    }
-    __syncthreads();
-    const int ntile = sh_ntile;
-    // culled: the tiles closest to the ligand centre (t) have the most pairs; taking them first
-    // lets the warps finish a pose together (the tile order does not touch the summation order)
-    const bool sorted = kCull && ntile <= 512;
-    if (sorted) {
-      for (int t = tid; t < ntile; t += blockDim.x) {
-        const float d = tdist[t];
-        int rank = 0;
-        for (int u = 0; u < ntile; ++u) {
-          const float e = tdist[u];
-          rank += (e < d || (e == d && u < t)) ? 1 : 0;
-        }
-        tord[rank] = tlist[t];
-      }
-      __syncthreads();
-    }
-    const int* tl = sorted ? tord : tlist;
-
     for (;;) {
-      int ti = 0;
-      if (lane == 0) ti = atomicAdd(&sh_next, 1);
-      ti = __shfl_sync(0xffffffffu, ti, 0);
-      if (ti >= ntile) break;
-      const int k = tl[ti];
-      const float4 tile = C.r_tile[k];
-      const float cx = (float)((double)tile.x - tx), cy = (float)((double)tile.y - ty),
-                  cz = (float)((double)tile.z - tz);
-      const float reach = tile_reach_base + tile.w;
-      const float reach2 = reach * reach;
+      int k = 0;
+      if (lane == 0) k = atomicAdd(&sh_next, 1);
+      k = __shfl_sync(0xffffffffu, k, 0);
+      if (k >= C.ntiles) break;
       const int slot = k * SD_TILE + lane;
       const int orig = C.r_orig[slot];
-      const bool active = orig >= 0;
-      double rx = 0, ry = 0, rz = 0;
-      int row = 0;
-      if (active) {
-        receptor_exact(C, nslots, slot, sh_pose, rx, ry, rz);
-        row = C.r_row[slot];
-      }
+      if (orig < 0) continue;  // padding of the last tile
+      double rx, ry, rz;
+      receptor_exact(C, nslots, slot, sh_pose, rx, ry, rz);
+      const int row = C.r_row[slot];
       double v = 0.0;  // FP64 partial of receptor atom `orig`
-      for (int base = 0; base < nl; base += 32) {
-        const int j = base + lane;
-        bool cand = j < nl;
-        if (kCull && cand) {
-          const float4 lj = ligF[j];
-          const float ex = lj.x - cx, ey = lj.y - cy, ez = lj.z - cz;
-          cand = ex * ex + ey * ey + ez * ez <= reach2;
-        }
-        unsigned mask = __ballot_sync(0xffffffffu, cand);
-        while (mask) {
-          const int b = __ffs(mask) - 1;
-          mask &= mask - 1;
-          const int jj = base + b;
-          n_evals += active;
-          {
-            const LigD l = ligD[jj];
-            const double ddx = rx - l.x, ddy = ry - l.y, ddz = rz - l.z;
-            const double d2 = ddx * ddx + ddy * ddy + ddz * ddz;
-            if (active && d2 <= SD_CUTOFF2) {
-              int key;
-              if (d2 == 0.0) {
-                key = 0;
-                atomicAdd(&sh_z, 1ull);
-              } else {
-                key = exact_key(d2, sh_T);
-                if (key == 29) atomicAdd(&sh_cut, 1ull);
-              }
-              v += L.table64[row + l.col + sh_lut[key]];
-              ++n_pairs;
-            }
+      for (int j = 0; j < nl; ++j) {
+        const LigD l = ligD[j];
+        const double ddx = rx - l.x, ddy = ry - l.y, ddz = rz - l.z;
+        const double d2 = ddx * ddx + ddy * ddy + ddz * ddz;
+        if (d2 <= SD_CUTOFF2) {
+          int key;
+          if (d2 == 0.0) {
+            key = 0;
+            atomicAdd(&sh_z, 1ull);
+          } else {
+            key = exact_key(d2, sh_T);
+            if (key == 29) atomicAdd(&sh_cut, 1ull);
           }
+          v += L.table64[row + l.col + sh_lut[key]];
+          ++n_pairs;
         }
       }
-      if (active) vacc[orig] = v;
+      n_evals += nl;
+      vacc[orig] = v;
     }
     __syncthreads();
-    double E;
-    {
-      // reference order: E += v_i for i ascending (zero partials skipped)
-      E = 0.0;
-      if (warp == 0) {
-        for (int base = 0; base < nr; base += 32) {
-          const double vv = base + lane < nr ? vacc[base + lane] : 0.0;
-          unsigned m = __ballot_sync(0xffffffffu, vv != 0.0);
-          while (m) {
-            const int b = __ffs(m) - 1;
-            m &= m - 1;
-            E += __shfl_sync(0xffffffffu, vv, b);
-          }
+    // reference order: E += v_i for i ascending (zero partials skipped)
+    double E = 0.0;
+    if (warp == 0) {
+      for (int base = 0; base < nr; base += 32) {
+        const double vv = base + lane < nr ? vacc[base + lane] : 0.0;
+        unsigned m = __ballot_sync(0xffffffffu, vv != 0.0);
+        while (m) {
+          const int b = __ffs(m) - 1;
+          m &= m - 1;
+          E += __shfl_sync(0xffffffffu, vv, b);
         }
       }
     }
@@ -295,7 +197,6 @@ __global__ void __launch_bounds__(kFp64Threads) dfire_score_kernel(ScoreLaunch L
     if (sh_pairs) atomicAdd(&ctl->stats[ST_PAIRS], sh_pairs);
     if (sh_evals) atomicAdd(&ctl->stats[ST_EVALS], sh_evals);
     if (n_done) atomicAdd(&ctl->stats[ST_SCORED], n_done);
-    if (sh_fallback) atomicAdd(&ctl->stats[ST_FALLBACK], sh_fallback);
     if (sh_z) atomicAdd(&ctl->stats[ST_D2ZERO], sh_z);
     if (sh_cut) atomicAdd(&ctl->stats[ST_D2CUT], sh_cut);
   }
@@ -304,6 +205,7 @@ __global__ void __launch_bounds__(kFp64Threads) dfire_score_kernel(ScoreLaunch L
 }  // namespace sd
 
 #include "sd_score_mixed.cuh"
+#include "sd_score_fp64.cuh"
 
 namespace sd {
 
@@ -327,18 +229,42 @@ static const MixedVariant kMixedVariants[] = {
 };
 // the spill instantiation of the mixed kernel: variant 0's shape (the per-tile work, and so every
 // energy, is the same in every variant)
+// stateless calls with at most one pose per SM: one CTA per SM with as many warps as fit, for a pose's
+// time (16 poses of 3002 / 1274 atoms, the whole call: 193 us with 12 warps, 164 us with 24)
+static const MixedVariant kMixedFew = {(const void*)dfire_score_mixed_kernel<24, 1, false>, 24, 1};
 static const MixedVariant kMixedSpill = {(const void*)dfire_score_mixed_kernel<12, 2, true>, 12, 2};
+
+// shapes of the culled FP64 kernel, the smallest CTAs first: they lose least where warps wait for each
+// other at a pose's end, and the first whose CTAs are all resident for the context's largest complex is
+// taken (the v_i of a large receptor fill the shared memory; when none fits, the spill instantiation).
+// Measured (M poses/s for 4x6, 8x3, 12x2): 757/481 atoms 5.7, 5.2, 4.0; 1200/1400 - (does not fit), 1.90,
+// 1.86; 2516/1061 -, 1.98, 2.01; 3002/1274 -, -, 1.74.  With too few poses to fill the GPU the shape with
+// the most warps is taken instead: a pose's time counts then.
+static const MixedVariant kFp64Shapes[] = {
+    {(const void*)dfire_score_fp64_kernel<4, 6, false>, 4, 6},
+    {(const void*)dfire_score_fp64_kernel<6, 4, false>, 6, 4},
+    {(const void*)dfire_score_fp64_kernel<8, 3, false>, 8, 3},
+    {(const void*)dfire_score_fp64_kernel<12, 2, false>, 12, 2},
+    {(const void*)dfire_score_fp64_kernel<24, 1, false>, 24, 1},
+    {(const void*)dfire_score_fp64_kernel<16, 1, false>, 16, 1},
+    {(const void*)dfire_score_fp64_kernel<8, 1, false>, 8, 1},
+};
+static const MixedVariant kFp64Spill = {(const void*)dfire_score_fp64_kernel<12, 2, true>, 12, 2};
+constexpr int kNumFp64Shapes = sizeof(kFp64Shapes) / sizeof(kFp64Shapes[0]);
 
 constexpr int kNumMixedVariants = sizeof(kMixedVariants) / sizeof(kMixedVariants[0]);
 static_assert(kNumMixedVariants <= SD_MAX_VARIANTS, "variant table");
 
-static const MixedVariant& mixed_variant(int v) { return kMixedVariants[v < 0 || v >= kNumMixedVariants ? 0 : v]; }
+static const MixedVariant& mixed_variant(int v) {
+  return v == SD_MIXED_FEW ? kMixedFew : kMixedVariants[v < 0 || v >= kNumMixedVariants ? 0 : v];
+}
 
 // bytes of the scorer's per-warp buffers, in dynamic shared memory in front of the per-pose arrays
 // (alone there in the spill instantiation)
 size_t score_warp_bytes(int precision, int scoring, int variant, bool spill) {
   if (scoring == SD_SCORING_PYDOCK) return pydock_warp_bytes(precision, false);
-  if (precision != SD_PREC_MIXED) return 0;
+  if (precision == SD_PREC_FP64_REF) return 0;
+  if (precision == SD_PREC_FP64) return sizeof(OrdBufs) * (spill ? kFp64Spill : kFp64Shapes[variant]).warps;
   return sizeof(WarpBufs) * (spill ? kMixedSpill.warps : mixed_variant(variant).warps);
 }
 
@@ -350,46 +276,55 @@ size_t score_smem_bytes(int precision, int scoring, int max_nr, int max_nl, int 
     const size_t ntiles = (size_t)(max_nr + SD_TILE - 1) / SD_TILE;
     return poses * (8 * ((ntiles + 1) & ~(size_t)1) + 16 * (nlc * SD_TILE + 1 + nlc)) + 4 * (3 * ntiles + nlc);
   }
-  return (size_t)16 * ((max_nl + 1) & ~1) + (size_t)32 * max_nl + (size_t)8 * max_nr +
-         (size_t)12 * ((max_nr + SD_TILE - 1) / SD_TILE);
+  if (precision == SD_PREC_FP64) {
+    const size_t nls = (size_t)(max_nl + SD_TILE - 1) / SD_TILE * SD_TILE;
+    return (size_t)8 * ((max_nr + 1) & ~1) + 16 * (nls + 1) + (size_t)12 * ((max_nr + SD_TILE - 1) / SD_TILE);
+  }
+  return (size_t)32 * max_nl + (size_t)8 * max_nr;
 }
 
+// the culled FP64 kernel's shape for these sizes and at most `poses` poses (1 KiB of each CTA is the
+// system's, 1 KiB covers the static arrays); the last one when none fits (the caller then spills)
+int fp64_shape(int max_nr, int max_nl, int smem_sm, int poses, int nsm) {
+  int best = kNumFp64Shapes - 1;
+  for (int v = kNumFp64Shapes - 1; v >= 0; --v) {
+    const size_t cta = score_smem_bytes(SD_PREC_FP64, SD_SCORING_DFIRE, max_nr, max_nl, 1) +
+                       score_warp_bytes(SD_PREC_FP64, SD_SCORING_DFIRE, v, false) + 2048;
+    const bool few = poses <= kFp64Shapes[v].min_blocks * nsm;
+    if (cta * kFp64Shapes[v].min_blocks > (size_t)smem_sm) continue;
+    if (!few || kFp64Shapes[v].warps > kFp64Shapes[best].warps) best = v;
+  }
+  return best;
+}
 int mixed_variant_count() { return kNumMixedVariants; }
 int mixed_variant_warps(int v) { return mixed_variant(v).warps; }
 int mixed_variant_min_blocks(int v) { return mixed_variant(v).min_blocks; }
 
-int score_threads_of(int precision, int scoring, int variant) {
+int score_threads_of(int precision, int scoring, int variant, bool spill) {
   if (scoring == SD_SCORING_PYDOCK) return pydock_threads(precision, false);
-  return precision == SD_PREC_MIXED ? mixed_variant_warps(variant) * 32 : kFp64Threads;
-}
-
-int score_threads_spill(int precision, int scoring) {
-  if (scoring == SD_SCORING_PYDOCK) return pydock_threads(precision, false);
-  return precision == SD_PREC_MIXED ? kMixedSpill.warps * 32 : kFp64Threads;
+  if (precision == SD_PREC_FP64_REF) return kRefThreads;
+  if (precision == SD_PREC_FP64) return (spill ? kFp64Spill : kFp64Shapes[variant]).warps * 32;
+  return (spill ? kMixedSpill : mixed_variant(variant)).warps * 32;
 }
 
 const void* score_kernel_ptr(int precision, int scoring, int variant, bool spill) {
   if (scoring == SD_SCORING_PYDOCK) return pydock_kernel_ptr(precision, false, spill);
   switch (precision) {
     case SD_PREC_FP64_REF:
-      return spill ? (const void*)dfire_score_kernel<SD_PREC_FP64_REF, true>
-                   : (const void*)dfire_score_kernel<SD_PREC_FP64_REF, false>;
-    case SD_PREC_FP64:
-      return spill ? (const void*)dfire_score_kernel<SD_PREC_FP64, true>
-                   : (const void*)dfire_score_kernel<SD_PREC_FP64, false>;
-    default: return spill ? kMixedSpill.fn : mixed_variant(variant).fn;
+      return spill ? (const void*)dfire_score_ref_kernel<true> : (const void*)dfire_score_ref_kernel<false>;
+    case SD_PREC_FP64: return (spill ? kFp64Spill : kFp64Shapes[variant]).fn;
+    default: return (spill ? kMixedSpill : mixed_variant(variant)).fn;
   }
 }
 
-int score_launch(const ScoreLaunch& L, int precision, int scoring, int grid, int threads, size_t smem,
-                 cudaStream_t st, int variant, bool spill) {
+int score_launch(const ScoreLaunch& L, int precision, int scoring, int grid, size_t smem, cudaStream_t st, int variant,
+                 bool spill) {
   if (scoring == SD_SCORING_PYDOCK) return pydock_launch(L, precision, false, nullptr, grid, smem, st, spill);
-  const void* fn = score_kernel_ptr(precision, scoring, variant, spill);
-  const int nthreads = precision == SD_PREC_MIXED ? (spill ? kMixedSpill.warps : mixed_variant(variant).warps) * 32
-                                                  : threads;
   ScoreLaunch l = L;
   void* args[] = {(void*)&l};
-  if (cudaLaunchKernel(fn, dim3(grid), dim3(nthreads), args, smem, st) != cudaSuccess) return SD_ERR_CUDA;
+  if (cudaLaunchKernel(score_kernel_ptr(precision, scoring, variant, spill), dim3(grid),
+                       dim3(score_threads_of(precision, scoring, variant, spill)), args, smem, st) != cudaSuccess)
+    return SD_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? SD_OK : SD_ERR_CUDA;
 }
 

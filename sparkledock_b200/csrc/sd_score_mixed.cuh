@@ -123,6 +123,103 @@ __device__ __forceinline__ void pair_terms(float2x rx, float2x ry, float2x rz, c
   bin[1] = max(__float_as_int(a1), kMagicBits);
 }
 
+// prologue of pose p by one warp: quaternion inverse (one division per lane, bit-identical to
+// quat_inverse), rotation matrix, ANM displacement bounds, reference point
+__device__ __forceinline__ void pose_prologue(const DevComplex& C, int p, PoseBufs& Q, int lane) {
+  if (lane < C.pl) Q.pose[lane] = C.pos[(size_t)p * C.pl + lane];
+  __syncwarp();
+  const double w0 = Q.pose[3], x = Q.pose[4], y = Q.pose[5], z = Q.pose[6];
+  const double n2 = w0 * w0 + x * x + y * y + z * z;
+  if (lane < 4) {
+    const double qv = Q.pose[3 + lane];
+    Q.q[lane] = qv;
+    Q.qi[lane] = (lane == 0 ? qv : -qv) / n2;
+  }
+  {
+    // rotation matrix of the (possibly not normalised) quaternion, one element per lane
+    double rv = 0.0;
+    switch (lane) {
+      case 0: rv = w0 * w0 + x * x - y * y - z * z; break;
+      case 1: rv = 2 * (x * y - w0 * z); break;
+      case 2: rv = 2 * (x * z + w0 * y); break;
+      case 3: rv = 2 * (x * y + w0 * z); break;
+      case 4: rv = w0 * w0 - x * x + y * y - z * z; break;
+      case 5: rv = 2 * (y * z - w0 * x); break;
+      case 6: rv = 2 * (x * z - w0 * y); break;
+      case 7: rv = 2 * (y * z + w0 * x); break;
+      case 8: rv = w0 * w0 - x * x - y * y + z * z; break;
+      default: break;
+    }
+    rv /= n2;
+    if (lane < 9) {
+      Q.rot[lane] = rv;
+      Q.rotf[lane] = (float)rv;
+    }
+  }
+  float tR = lane < C.nmr ? fabsf((float)Q.pose[7 + lane]) * C.mnorm_r[lane] : 0.f;
+  float tL = lane < C.nml ? fabsf((float)Q.pose[7 + C.nmr + lane]) * C.mnorm_l[lane] : 0.f;
+  for (int o = 16; o > 0; o >>= 1) {
+    tR += __shfl_xor_sync(0xffffffffu, tR, o);
+    tL += __shfl_xor_sync(0xffffffffu, tL, o);
+  }
+  __syncwarp();
+  if (lane < 3)
+    Q.gc[lane] = Q.rotf[3 * lane] * C.lig_ctr[0] + Q.rotf[3 * lane + 1] * C.lig_ctr[1] +
+                 Q.rotf[3 * lane + 2] * C.lig_ctr[2];
+  if (lane == 0) {
+    const float dR = tR * 1.0001f + 1e-4f, dL = tL * 1.0001f + 1e-4f;
+    Q.dR = dR;
+    Q.dL = dL;
+    // bound of |FP32 d2 - FP64 d2| for pairs within 15.1 A (coordinates centred on t)
+    const float RL = C.lig_radius + dL;
+    const float u32 = 5.9604645e-8f;
+    Q.B = 2.0f * (2.02f * u32 * (26.2f * (2.0f * RL + 15.1f) + 228.0f) + 3.0f * u32 * 228.0f) + 1e-6f;
+    // ligand reference point (prepare_gso_tasks.cc:460, :513, :524-526)
+    double rx = C.lig_ref[0], ry = C.lig_ref[1], rz = C.lig_ref[2];
+    quat_rotate(Q.q, Q.qi, rx, ry, rz);
+    double* ref = C.ref + (size_t)p * 3;
+    ref[0] = rx + Q.pose[0];
+    ref[1] = ry + Q.pose[1];
+    ref[2] = rz + Q.pose[2];
+  }
+}
+
+// bounding box of each group of 8 lanes of a tile (own: the lane's atom; an empty group's half extent is
+// -inf, so no point is near it)
+__device__ __forceinline__ void group_boxes(const float4& own, bool active, int lane, float4* box) {
+  float lo[3] = {own.x, own.y, own.z}, hi[3] = {own.x, own.y, own.z};
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    if (!active) {
+      lo[d] = 3e38f;
+      hi[d] = -3e38f;
+    }
+#pragma unroll
+    for (int o = 1; o < kGroup; o <<= 1) {
+      lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+      hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+    }
+  }
+  if ((lane & (kGroup - 1)) == 0) {
+    box[2 * (lane / kGroup)] = make_float4(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2]), 0.f);
+    box[2 * (lane / kGroup) + 1] =
+        make_float4(0.5f * (hi[0] - lo[0]), 0.5f * (hi[1] - lo[1]), 0.5f * (hi[2] - lo[2]), 0.f);
+  }
+}
+
+// squared distance of a point (negated) from group g's box
+__device__ __forceinline__ float box_distance2(const float4* box, int g, const float4& l) {
+  const float4 bc = box[2 * g], bh = box[2 * g + 1];
+  const float ex = fmaxf(fabsf(l.x + bc.x) - bh.x, 0.f), ey = fmaxf(fabsf(l.y + bc.y) - bh.y, 0.f),
+              ez = fmaxf(fabsf(l.z + bc.z) - bh.z, 0.f);
+  return fmaf(ez, ez, fmaf(ey, ey, ex * ex));
+}
+
+// half a bin less the bin coordinate's error: |d_fp32 - d| <= B / 30 inside the cutoff (B bounds d^2
+// there, its leading term is 2 d |error of the difference vector|), times the slope 2, plus FP32
+// roundings (square root 2^-22, coordinate up to 20).  Not above 0: no pair is settled in FP32
+__device__ __forceinline__ float settled_half(float B) { return 0.5f - (B * 0.0673f + 2e-5f); }
+
 }  // namespace
 
 // Variants differ only in warps per CTA and resident CTAs per SM: a tile is always processed by
@@ -168,72 +265,12 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) dfire_score_mixed_ker
       const int first = wi_local(work[item]), second = wi_local(work[item + np - 1]);
       item += np;
       const DevComplex& C = L.cplx[ci];
-      const int nslots = nslots_of(C), pl = C.pl, nlc = C.nlchunks;
+      const int nslots = nslots_of(C), nlc = C.nlchunks;
       if (warp < np) {
-        // pose prologue, one warp per pose: quaternion inverse (one division per lane, bit-identical to
-        // quat_inverse), rotation matrix, ANM displacement bounds, reference point
-        PoseBufs& Q = sh_p[warp];
-        const int p = warp == 0 ? first : second;
-        const double* pose_g = C.pos + (size_t)p * pl;
-        if (lane < pl) Q.pose[lane] = pose_g[lane];
-        __syncwarp();
-        const double w0 = Q.pose[3], x = Q.pose[4], y = Q.pose[5], z = Q.pose[6];
-        const double n2 = w0 * w0 + x * x + y * y + z * z;
-        if (lane < 4) {
-          const double qv = Q.pose[3 + lane];
-          Q.q[lane] = qv;
-          Q.qi[lane] = (lane == 0 ? qv : -qv) / n2;
-        }
-        {
-          // rotation matrix of the (possibly not normalised) quaternion, one element per lane
-          double rv = 0.0;
-          switch (lane) {
-            case 0: rv = w0 * w0 + x * x - y * y - z * z; break;
-            case 1: rv = 2 * (x * y - w0 * z); break;
-            case 2: rv = 2 * (x * z + w0 * y); break;
-            case 3: rv = 2 * (x * y + w0 * z); break;
-            case 4: rv = w0 * w0 - x * x + y * y - z * z; break;
-            case 5: rv = 2 * (y * z - w0 * x); break;
-            case 6: rv = 2 * (x * z - w0 * y); break;
-            case 7: rv = 2 * (y * z + w0 * x); break;
-            case 8: rv = w0 * w0 - x * x - y * y + z * z; break;
-            default: break;
-          }
-          rv /= n2;
-          if (lane < 9) {
-            Q.rot[lane] = rv;
-            Q.rotf[lane] = (float)rv;
-          }
-        }
-        float tR = lane < C.nmr ? fabsf((float)Q.pose[7 + lane]) * C.mnorm_r[lane] : 0.f;
-        float tL = lane < C.nml ? fabsf((float)Q.pose[7 + C.nmr + lane]) * C.mnorm_l[lane] : 0.f;
-        for (int o = 16; o > 0; o >>= 1) {
-          tR += __shfl_xor_sync(0xffffffffu, tR, o);
-          tL += __shfl_xor_sync(0xffffffffu, tL, o);
-        }
-        __syncwarp();
-        if (lane < 3)
-          Q.gc[lane] = Q.rotf[3 * lane] * C.lig_ctr[0] + Q.rotf[3 * lane + 1] * C.lig_ctr[1] +
-                       Q.rotf[3 * lane + 2] * C.lig_ctr[2];
-        if (lane == 0) {
-          const float dR = tR * 1.0001f + 1e-4f, dL = tL * 1.0001f + 1e-4f;
-          Q.dR = dR;
-          Q.dL = dL;
-          // bound of |FP32 d2 - FP64 d2| for pairs within 15.1 A (coordinates centred on t)
-          const float RL = C.lig_radius + dL;
-          const float u32 = 5.9604645e-8f;
-          Q.B = 2.0f * (2.02f * u32 * (26.2f * (2.0f * RL + 15.1f) + 228.0f) + 3.0f * u32 * 228.0f) + 1e-6f;
-          // ligand reference point (prepare_gso_tasks.cc:460, :513, :524-526)
-          double rx = C.lig_ref[0], ry = C.lig_ref[1], rz = C.lig_ref[2];
-          quat_rotate(Q.q, Q.qi, rx, ry, rz);
-          double* ref = C.ref + (size_t)p * 3;
-          ref[0] = rx + Q.pose[0];
-          ref[1] = ry + Q.pose[1];
-          ref[2] = rz + Q.pose[2];
-          if (warp == 0) {
-            sh_ntile = 0;
-            sh_next = 0;
-          }
+        pose_prologue(C, warp == 0 ? first : second, sh_p[warp], lane);
+        if (warp == 0 && lane == 0) {
+          sh_ntile = 0;
+          sh_next = 0;
         }
       }
       __syncthreads();
@@ -377,36 +414,11 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) dfire_score_mixed_ker
           const float reach2 = reach * reach;
           const float cut2 = 225.0f + Q.B;
           const float box_cut = 225.1f + Q.B;
-          // the bin coordinate's error: |d_fp32 - d| <= B / 30 inside the cutoff (B bounds d^2 there, its
-          // leading term is 2 d |error of the difference vector|), times the slope 2, plus FP32 roundings
-          // (square root 2^-22, coordinate up to 20).  If it reaches 0.5 no pair is settled in FP32
-          const float inner = 0.5f - (Q.B * 0.0673f + 2e-5f);
+          const float inner = settled_half(Q.B);
           const float4* const lig = ligS + p * (nls + 1);
           const float4* const rec = W.rec[p];
           __syncwarp();
-          {
-            // bounding box of each group of 8 lanes (an empty group's half extent is -inf: no candidate)
-            const float4 own = rec[lane];
-            float lo[3] = {own.x, own.y, own.z}, hi[3] = {own.x, own.y, own.z};
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-              if (!active) {
-                lo[d] = 3e38f;
-                hi[d] = -3e38f;
-              }
-#pragma unroll
-              for (int o = 1; o < kGroup; o <<= 1) {
-                lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-                hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
-              }
-            }
-            if ((lane & (kGroup - 1)) == 0) {
-              W.box[2 * (lane / kGroup)] =
-                  make_float4(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2]), 0.f);
-              W.box[2 * (lane / kGroup) + 1] =
-                  make_float4(0.5f * (hi[0] - lo[0]), 0.5f * (hi[1] - lo[1]), 0.5f * (hi[2] - lo[2]), 0.f);
-            }
-          }
+          group_boxes(rec[lane], active, lane, W.box);
           __syncwarp();
 
           unsigned nnear = 0, npairs = 0, nevals = 0;
@@ -450,10 +462,7 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) dfire_score_mixed_ker
               const float4 l4 = lig[s];
 #pragma unroll
               for (int g = 0; g < kGroups; ++g) {
-                const float4 bc = W.box[2 * g], bh = W.box[2 * g + 1];
-                const float ex = fmaxf(fabsf(l4.x + bc.x) - bh.x, 0.f), ey = fmaxf(fabsf(l4.y + bc.y) - bh.y, 0.f),
-                            ez = fmaxf(fabsf(l4.z + bc.z) - bh.z, 0.f);
-                const bool in = fmaf(ez, ez, fmaf(ey, ey, ex * ex)) <= box_cut;
+                const bool in = box_distance2(W.box, g, l4) <= box_cut;
                 const unsigned am = __ballot_sync(0xffffffffu, in);
                 if (in) W.list[g][cnt[g] + __popc(am & lt_mask)] = (unsigned short)s;
                 cnt[g] += __popc(am);

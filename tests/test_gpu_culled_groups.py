@@ -1,8 +1,8 @@
-"""The mixed DFIRE scorer at the edges of its groups (8 receptor atoms), tiles and chunks (32 atoms),
-candidate lists (160 places, so dense overlapping poses refill them) and two-pose batches, against
-the oracle.
+"""The culled DFIRE scorers at the edges of their groups (8 receptor atoms), tiles and chunks (32
+atoms), candidate lists (so dense overlapping poses refill them), two-pose batches and kernel shapes,
+against the oracle: FP64 bit for bit, mixed within a tolerance.
 
-Tolerance: both sides add the same FP64 table values (|v| < 6 here) in different orders, so they
+Tolerance of mixed: both sides add the same FP64 table values (|v| < 6 here) in different orders, so they
 differ by at most n * 2^-53 * sum|v| <= 6 n^2 2^-53 for n pairs; a wrong bin moves an energy by a
 difference of N(0,1) values."""
 import numpy as np
@@ -29,3 +29,16 @@ def test_groups_lists_and_pose_pairs(n_rec, n_lig, modes, tables):
         for k in (n, 5):
             _, en = dk.score_poses(0, poses[:k], sd.SD_PREC_MIXED)
             assert np.abs(en - ref[:k]).max() <= tol
+            _, en = dk.score_poses(0, poses[:k], sd.SD_PREC_FP64)
+            assert np.array_equal(en, ref[:k])
+
+
+@pytest.mark.parametrize("n_rec,n_lig", [(6001, 1766), (15999, 333), (17307, 1125), (21500, 500)])
+def test_fp64_kernel_shapes(n_rec, n_lig, tables):
+    """Receptors whose partial sums leave room for one CTA of 24, 16 or 8 warps per SM."""
+    c = sd.SyntheticComplex(n_rec, n_lig, 4, 1, seed=n_rec)
+    poses = c.poses.reshape(4, -1)
+    sc, ref = oracle_scores(OracleSystem(c, tables), poses)
+    with sd.Docking([c], tables) as dk:
+        got, en = dk.score_poses(0, poses, sd.SD_PREC_FP64)
+        assert np.array_equal(en, ref) and np.array_equal(got, sc)
