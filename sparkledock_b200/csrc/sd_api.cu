@@ -671,7 +671,9 @@ int enqueue_step(sd_ctx* c, int precision, int variant, int grid, size_t sm) {
   G.p.max_neighbors = c->params.max_neighbors;
   G.pos_prev = c->d_pos_prev;
   const int threads = (c->max_G + 31) / 32 * 32;
-  if ((rc = c->max_G > SD_MAX_G ? gso_launch_large(G, c->max_G, c->stream) : gso_launch(G, threads, c->stream)))
+  if ((rc = c->max_G > SD_MAX_G    ? gso_launch_large(G, c->max_G, c->stream)
+            : c->max_G > SD_WARP_G ? gso_launch(G, threads, c->stream)
+                                   : gso_launch_warp(G, c->max_G, c->nsm, c->stream)))
     return fail(rc, std::string("GSO kernel launch: ") + cudaGetErrorString(cudaGetLastError()));
   return SD_OK;
 }
@@ -813,6 +815,8 @@ int sd_ctx_create(const sd_complex_desc* complexes, int n_complexes, const sd_ta
   for (int p = 0; p < 2; ++p)
     if ((rc = cu(cudaMalloc(&c->d_work[p], sizeof(int) * std::max(1, c->total_glowworms)), "cudaMalloc"))) return bail(rc);
   if ((rc = cu(cudaMalloc(&c->d_swarm_map, sizeof(int) * c->total_swarms), "cudaMalloc"))) return bail(rc);
+  if (c->max_G <= SD_WARP_G && (rc = gso_prepare_warp()))
+    return bail(fail(rc, "GSO kernel: shared memory attribute"));
   if (c->max_G > SD_MAX_G) {
     if ((rc = cu(cudaMalloc(&c->d_pos_prev, sizeof(double) * SD_POSE_LEN(SD_MAX_MODES, SD_MAX_MODES) *
                                                (size_t)c->total_glowworms), "cudaMalloc")))

@@ -66,14 +66,6 @@ SD_HD dd dd_mul(dd a, dd b) {
   p.lo = fma_(a.lo, b.hi, p.lo);
   return fast_two_sum(p.hi, p.lo);
 }
-// a / d for an exactly representable double d
-SD_HD dd dd_div_d(dd a, double d) {
-  double q1 = a.hi / d;
-  dd p = two_prod(q1, d);
-  double r = ((a.hi - p.hi) - p.lo) + a.lo;
-  double q2 = r / d;
-  return fast_two_sum(q1, q2);
-}
 // 1 - a
 SD_HD dd one_minus(dd a) {
   dd s = two_sum(1.0, -a.hi);
@@ -81,26 +73,47 @@ SD_HD dd one_minus(dd a) {
   return fast_two_sum(s.hi, s.lo);
 }
 
-// sin(x) as double-double, |x| <= 2: x * (1 - x^2/(2*3) (1 - x^2/(4*5) (...)))
-SD_HD dd sin_dd(dd x) {
-  dd x2 = dd_mul(x, x);
-  dd p = {1.0, 0.0};
-  for (int k = 17; k >= 1; --k) {
-    double den = (double)(2 * k) * (double)(2 * k + 1);
-    p = one_minus(dd_div_d(dd_mul(x2, p), den));
-  }
-  return dd_mul(x, p);
+// 1 / d as double-double for an integer d below 2^11: the remainder 1 - hi d is exact (hi is split into
+// halves whose products with d are exact)
+constexpr dd reciprocal(double d) {
+  const double hi = 1.0 / d;
+  const double t = 134217729.0 * hi, h1 = t - (t - hi), h2 = hi - h1;
+  return {hi, ((1.0 - h1 * d) - h2 * d) / d};
 }
-// cos(x) as double-double, |x| <= 2: 1 - x^2/(1*2) (1 - x^2/(3*4) (...))
-SD_HD dd cos_dd(dd x) {
+constexpr int kTerms = 17;
+struct Terms {
+  dd cos_t[kTerms], sin_t[kTerms];  // 1 / ((2k-1) 2k) and 1 / (2k (2k+1)), k = 1 .. kTerms
+};
+constexpr Terms make_terms() {
+  Terms t{};
+  for (int k = 1; k <= kTerms; ++k) {
+    t.cos_t[k - 1] = reciprocal((2.0 * k - 1) * (2.0 * k));
+    t.sin_t[k - 1] = reciprocal((2.0 * k) * (2.0 * k + 1));
+  }
+  return t;
+}
+#if defined(__CUDACC__)
+static __device__ __constant__ const Terms c_terms = make_terms();
+#endif
+static constexpr Terms h_terms = make_terms();
+SD_HD const Terms& terms() {
+#if defined(__CUDA_ARCH__)
+  return c_terms;
+#else
+  return h_terms;
+#endif
+}
+
+// 1 - x^2 t_1 (1 - x^2 t_2 (...)) with the given reciprocals: cos(x) with cos_t, sin(x) / x with sin_t,
+// |x| <= 2 (the series is cut at x^35 / 35!)
+SD_HD dd series(dd x, const dd* t) {
   dd x2 = dd_mul(x, x);
   dd p = {1.0, 0.0};
-  for (int k = 17; k >= 1; --k) {
-    double den = (double)(2 * k - 1) * (double)(2 * k);
-    p = one_minus(dd_div_d(dd_mul(x2, p), den));
-  }
+  for (int k = kTerms - 1; k >= 0; --k) p = one_minus(dd_mul(dd_mul(x2, p), t[k]));
   return p;
 }
+SD_HD dd sin_dd(dd x) { return dd_mul(x, series(x, terms().sin_t)); }
+SD_HD dd cos_dd(dd x) { return series(x, terms().cos_t); }
 
 }  // namespace sdcr
 

@@ -22,6 +22,7 @@
 #define SD_MAX_LIG 65504        /* ligand atoms: the mixed scorer's 16-bit ligand slot indices */
 #define SD_MAX_REC (1 << 22)    /* receptor atoms */
 #define SD_MAX_G 1024           /* glowworms per swarm with one thread each (one CTA per swarm) */
+#define SD_WARP_G 512           /* glowworms per swarm with one warp each: their moved poses in shared memory */
 #define SD_MAX_GLOWWORMS 6144   /* glowworms per swarm: luciferin + reference points in shared memory */
 #define SD_CULL_MARGIN 0.05f    /* A, covers FP32 rounding of the conservative culling tests */
 #define SD_MAX_VARIANTS 16      /* compiled variants of the mixed DFIRE kernel (autotuner) */
@@ -164,7 +165,9 @@ int mixed_variant_warps(int v);
 int mixed_variant_min_blocks(int v);
 int gso_launch(const GsoLaunch& L, int threads, cudaStream_t st);
 int gso_launch_large(const GsoLaunch& L, int max_g, cudaStream_t st);
+int gso_launch_warp(const GsoLaunch& L, int max_g, int nsm, cudaStream_t st);
 int gso_prepare_large();
+int gso_prepare_warp();
 int bins_launch(const DevComplex* cplx, int c, const double* d_pose, int precision, int* d_bins, int nr, int nl,
                 int* d_fallback, cudaStream_t st);
 size_t pydock_smem_bytes(int precision, bool grad, int max_nl, int max_nr);
