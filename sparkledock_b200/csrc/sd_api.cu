@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -40,6 +41,14 @@ int fail(int code, const std::string& msg) {
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+};
+
+struct ScorePlan {
+  int grid = 0;            // 0: not made yet
+  size_t smem = 0;
+  bool spill = false;
+  size_t spill_stride = 0;
+  int poses = 1;           // per CTA
 };
 
 struct ComplexHost {
@@ -128,6 +137,9 @@ struct sd_ctx {
   DevBuf s_pose, s_score, s_ref, s_energy, s_work, s_grad, s_bins;
   // per-CTA global scratch of the spill instantiations (complexes too large for shared memory)
   DevBuf s_spill;
+  ScorePlan plan[3][SD_MAX_VARIANTS + 1], grad_plan[3];
+  void* h_stage = nullptr; // pinned, for small downloads
+  int* d_flag = nullptr;
   int smem_optin = 0;      // shared memory a CTA may use on this device (opt-in maximum)
   // step graph
   cudaGraphExec_t graph = nullptr;
@@ -413,33 +425,54 @@ int push_descriptors(sd_ctx* c) {
   return SD_OK;
 }
 
-// rebuild the first work list from moved/step of every complex
+// rebuild the first work list from moved/step of every complex (on the stream)
 int rebuild_worklist(sd_ctx* c) {
-  std::vector<int> work;
-  work.reserve(c->total_glowworms);
-  for (int ci = 0; ci < c->ncplx; ++ci) {
-    const DevComplex& D = c->cx[ci].d;
-    const size_t n = (size_t)D.S * D.G;
-    std::vector<int> moved(n), step(n);
-    SD_CUDA(cudaMemcpyAsync(moved.data(), D.moved, n * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    SD_CUDA(cudaMemcpyAsync(step.data(), D.step, n * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    SD_CUDA(cudaStreamSynchronize(c->stream));
-    for (size_t k = 0; k < n; ++k)
-      if (moved[k] || step[k] == 0) work.push_back(wi_pack(ci, (int)k));
-  }
-  StepCtl ctl;
-  SD_CUDA(cudaMemcpy(&ctl, c->d_ctl, sizeof ctl, cudaMemcpyDeviceToHost));
-  ctl.count[0] = (int)work.size();
-  ctl.count[1] = 0;
-  ctl.grab[0] = ctl.grab[1] = 0;
-  ctl.parity = 0;
-  ctl.done_blocks = 0;
-  if (!work.empty())
-    SD_CUDA(cudaMemcpyAsync(c->d_work[0], work.data(), work.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-  SD_CUDA(cudaMemcpyAsync(c->d_ctl, &ctl, sizeof ctl, cudaMemcpyHostToDevice, c->stream));
-  SD_CUDA(cudaStreamSynchronize(c->stream));
+  static_assert(offsetof(StepCtl, step) == 24, "count, grab, parity and done_blocks come first");
+  SD_CUDA(cudaMemsetAsync(c->d_ctl, 0, offsetof(StepCtl, step), c->stream));
+  if (worklist_launch(c->d_cplx, c->d_swarm_map, c->total_swarms, c->d_ctl, c->d_work[0], c->stream))
+    return fail(SD_ERR_CUDA, std::string("work list kernel: ") + cudaGetErrorString(cudaGetLastError()));
   return SD_OK;
 }
+
+// whether all n values are finite (v * 0 is 0 or NaN; eight independent sums, so it vectorises)
+bool all_finite(const double* v, size_t n) {
+  double a[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  size_t i = 0;
+  for (; i + 8 <= n; i += 8)
+    for (int k = 0; k < 8; ++k) a[k] += v[i + k] * 0.0;
+  for (; i < n; ++i) a[0] += v[i] * 0.0;
+  double s = 0;
+  for (double x : a) s += x;
+  return s == 0.0;
+}
+
+// n doubles into pinned host memory of the context (kept, up to 1 MiB) on the way to the caller's pageable
+// array, or straight there when they are more: a small download into pageable memory waits on its own
+constexpr size_t kStage = 1 << 20;
+struct Download {
+  sd_ctx* c;
+  size_t used = 0;
+  struct Part {
+    double* dst;
+    size_t at, n;
+  } part[2];
+  int parts = 0;
+  int add(double* dst, const void* src, size_t n) {
+    if (used + n * 8 > kStage || !c->h_stage) {
+      SD_CUDA(cudaMemcpyAsync(dst, src, n * 8, cudaMemcpyDeviceToHost, c->stream));
+      return SD_OK;
+    }
+    SD_CUDA(cudaMemcpyAsync((char*)c->h_stage + used, src, n * 8, cudaMemcpyDeviceToHost, c->stream));
+    part[parts++] = {dst, used, n};
+    used += n * 8;
+    return SD_OK;
+  }
+  int finish() {
+    SD_CUDA(cudaStreamSynchronize(c->stream));
+    for (int i = 0; i < parts; ++i) memcpy(part[i].dst, (char*)c->h_stage + part[i].at, part[i].n * 8);
+    return SD_OK;
+  }
+};
 
 // The spill scratch, grown to at least bytes.  The step graph holds the scratch's address, so a new
 // scratch means a new capture at the next step.
@@ -453,11 +486,10 @@ int grow_spill(sd_ctx* c, size_t bytes) {
   return ensure(c, c->s_spill, bytes);
 }
 
-// Launch shape of the scorer on this context: persistent grid (resident CTAs x SMs), dynamic shared
-// memory, threads.  When the per-pose arrays of the largest complex do not fit in the shared memory
-// a CTA may use, the spill instantiation is chosen (no dynamic shared memory) and the context's
-// spill scratch is sized to grid x per-CTA bytes; alloc = false refuses that instead of allocating.
-int configure_score(sd_ctx* c, int precision, int variant, int* grid, size_t* smem, bool alloc = true) {
+// Launch shape of the scorer on this context: persistent grid (resident CTAs x SMs) and dynamic shared
+// memory.  When the per-pose arrays of the largest complex do not fit in the shared memory a CTA may
+// use, the spill instantiation is chosen (only the warps' buffers in shared memory).
+int make_score_plan(sd_ctx* c, int precision, int variant, ScorePlan& plan) {
   const size_t need = score_smem_bytes(precision, c->scoring, c->max_nr, c->max_nl, 1);
   const void* k = score_kernel_ptr(precision, c->scoring, variant, false);
   cudaFuncAttributes fa;
@@ -470,41 +502,58 @@ int configure_score(sd_ctx* c, int precision, int variant, int* grid, size_t* sm
     sm = score_warp_bytes(precision, c->scoring, variant, true);
     threads = score_threads_of(precision, c->scoring, variant, true);
   }
+  // the kernel's limit is raised to what the device has, not to this plan's need: other contexts of the
+  // process set it too, and keep their plans
   int per_sm = 0;
+  cudaFuncAttributes ka;
+  SD_CUDA(cudaFuncGetAttributes(&ka, k));
+  SD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, c->smem_optin - (int)ka.sharedSizeBytes));
   auto occupancy = [&](size_t bytes) -> int {
-    SD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(bytes, 1)));
     SD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, bytes));
     return SD_OK;
   };
   int rc;
   if ((rc = occupancy(sm))) return rc;
   // two poses per CTA wherever their arrays leave as many CTAs resident as one pose's
-  c->score_poses = 1;
+  plan.poses = 1;
   if (!spill && precision == SD_PREC_MIXED && c->scoring == SD_SCORING_DFIRE) {
     const int one = per_sm;
     const size_t two = sm - need + score_smem_bytes(precision, c->scoring, c->max_nr, c->max_nl, 2);
     if (two + fa.sharedSizeBytes <= (size_t)c->smem_optin) {
       if ((rc = occupancy(two))) return rc;
       if (per_sm == one) {
-        c->score_poses = 2;
+        plan.poses = 2;
         sm = two;
       }
     }
-    if (c->score_poses == 1 && (rc = occupancy(sm))) return rc;
+    per_sm = one;
   }
   if (per_sm < 1) return fail(SD_ERR_ARG, "scoring kernel does not fit on an SM (shared memory)");
-  *grid = per_sm * c->nsm;
-  *smem = sm;
-  c->score_spill = spill;
-  if (spill) {
-    const size_t stride = (need + 255) & ~(size_t)255;
-    if (c->s_spill.bytes < stride * (size_t)*grid) {
-      if (!alloc) return fail(SD_ERR_NOTSUP, "complex too large for shared memory: its scorer needs the context's "
-                                             "global scratch, which this call may not allocate");
-      rc = grow_spill(c, stride * (size_t)*grid);
-      if (rc) return rc;
-    }
-    c->spill_stride = stride;
+  plan.smem = sm;
+  plan.spill = spill;
+  plan.spill_stride = spill ? (need + 255) & ~(size_t)255 : 0;
+  plan.grid = per_sm * c->nsm;
+  return SD_OK;
+}
+
+// The launch shape, made once per context, precision and variant (it depends on the context's largest
+// complex alone: 15 us of queries), and the context's spill scratch sized to it; alloc = false refuses
+// that instead of allocating.
+int configure_score(sd_ctx* c, int precision, int variant, int* grid, size_t* smem, bool alloc = true) {
+  ScorePlan& plan = c->plan[precision][precision == SD_PREC_FP64_REF ? 0 : variant];
+  if (!plan.grid) {
+    int rc = make_score_plan(c, precision, variant, plan);
+    if (rc) return rc;
+  }
+  *grid = plan.grid;
+  *smem = plan.smem;
+  c->score_poses = plan.poses;
+  c->score_spill = plan.spill;
+  c->spill_stride = plan.spill_stride;
+  if (plan.spill && c->s_spill.bytes < plan.spill_stride * (size_t)plan.grid) {
+    if (!alloc) return fail(SD_ERR_NOTSUP, "complex too large for shared memory: its scorer needs the context's "
+                                           "global scratch, which this call may not allocate");
+    return grow_spill(c, plan.spill_stride * (size_t)plan.grid);
   }
   return SD_OK;
 }
@@ -812,6 +861,12 @@ int sd_ctx_create(const sd_complex_desc* complexes, int n_complexes, const sd_ta
   if ((rc = cu(cudaMalloc(&c->d_lj_sigma, sizeof(double) * SD_LJ_TYPES), "cudaMalloc"))) return bail(rc);
   if ((rc = cu(cudaMalloc(&c->d_ctl, sizeof(StepCtl)), "cudaMalloc"))) return bail(rc);
   if ((rc = cu(cudaMalloc(&c->d_ctl_scratch, sizeof(StepCtl)), "cudaMalloc"))) return bail(rc);
+  if ((rc = cu(cudaMemset(c->d_ctl_scratch, 0, sizeof(StepCtl)), "cudaMemset"))) return bail(rc);
+  if ((rc = cu(cudaMalloc(&c->d_flag, sizeof(int)), "cudaMalloc"))) return bail(rc);
+  if (cudaMallocHost(&c->h_stage, kStage) != cudaSuccess) {
+    c->h_stage = nullptr;  // downloads then go straight to the caller
+    cudaGetLastError();
+  }
   for (int p = 0; p < 2; ++p)
     if ((rc = cu(cudaMalloc(&c->d_work[p], sizeof(int) * std::max(1, c->total_glowworms)), "cudaMalloc"))) return bail(rc);
   if ((rc = cu(cudaMalloc(&c->d_swarm_map, sizeof(int) * c->total_swarms), "cudaMalloc"))) return bail(rc);
@@ -872,6 +927,8 @@ int sd_ctx_destroy(sd_ctx* c) {
                 c->s_ref.p, c->s_energy.p, c->s_work.p, c->s_grad.p, c->s_bins.p, c->s_spill.p};
   for (void* p : ps)
     if (p) cudaFree(p);
+  if (c->d_flag) cudaFree(c->d_flag);
+  if (c->h_stage) cudaFreeHost(c->h_stage);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return SD_OK;
@@ -894,23 +951,31 @@ int sd_init_state(sd_ctx* c, int ci, const double* pos) {
   SD_CUDA(cudaSetDevice(c->device));
   const DevComplex& D = c->cx[ci].d;
   const size_t n = (size_t)D.S * D.G;
-  for (size_t i = 0; i < n * D.pl; ++i)
-    if (!std::isfinite(pos[i])) return fail(SD_ERR_NUMERIC, "sd_init_state: non-finite pose");
-  std::vector<double> luc(n, c->params.initial_luciferin), vis(n, c->params.initial_vision_range), zero(n, 0.0);
-  std::vector<int> izero(n, 0), sel(n);
-  for (size_t k = 0; k < n; ++k) sel[k] = (int)(k % D.G);
-  SD_CUDA(cudaMemcpyAsync(D.pos, pos, n * D.pl * 8, cudaMemcpyHostToDevice, c->stream));
-  SD_CUDA(cudaMemcpyAsync(D.luciferin, luc.data(), n * 8, cudaMemcpyHostToDevice, c->stream));
-  SD_CUDA(cudaMemcpyAsync(D.vision, vis.data(), n * 8, cudaMemcpyHostToDevice, c->stream));
-  SD_CUDA(cudaMemcpyAsync(D.scoring, zero.data(), n * 8, cudaMemcpyHostToDevice, c->stream));
-  SD_CUDA(cudaMemsetAsync(D.ref, 0, n * 3 * 8, c->stream));
-  SD_CUDA(cudaMemcpyAsync(D.step, izero.data(), n * 4, cudaMemcpyHostToDevice, c->stream));
-  SD_CUDA(cudaMemcpyAsync(D.moved, izero.data(), n * 4, cudaMemcpyHostToDevice, c->stream));
-  SD_CUDA(cudaMemcpyAsync(D.nnei, izero.data(), n * 4, cudaMemcpyHostToDevice, c->stream));
-  SD_CUDA(cudaMemcpyAsync(D.select, sel.data(), n * 4, cudaMemcpyHostToDevice, c->stream));
+  // the poses go to the stateless scratch first and are checked there, so that a refused call leaves the
+  // state as it was (checked on the host when there is no memory for that)
+  int rc;
+  const bool staged = ensure(c, c->s_pose, n * D.pl * 8) == SD_OK;
+  if (staged) {
+    int bad = 0;
+    SD_CUDA(cudaMemsetAsync(c->d_flag, 0, sizeof(int), c->stream));
+    SD_CUDA(cudaMemcpyAsync(c->s_pose.p, pos, n * D.pl * 8, cudaMemcpyHostToDevice, c->stream));
+    if ((rc = check_finite_launch((const double*)c->s_pose.p, n * D.pl, c->d_flag, c->stream)))
+      return fail(rc, "sd_init_state: kernel launch failed");
+    SD_CUDA(cudaMemcpyAsync(&bad, c->d_flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    SD_CUDA(cudaStreamSynchronize(c->stream));
+    if (bad) return fail(SD_ERR_NUMERIC, "sd_init_state: non-finite pose");
+    SD_CUDA(cudaMemcpyAsync(D.pos, c->s_pose.p, n * D.pl * 8, cudaMemcpyDeviceToDevice, c->stream));
+  } else {
+    cudaGetLastError();
+    if (!all_finite(pos, n * D.pl)) return fail(SD_ERR_NUMERIC, "sd_init_state: non-finite pose");
+    SD_CUDA(cudaMemcpyAsync(D.pos, pos, n * D.pl * 8, cudaMemcpyHostToDevice, c->stream));
+  }
+  if ((rc = init_state_launch(D, c->params.initial_luciferin, c->params.initial_vision_range, c->stream)))
+    return fail(rc, "sd_init_state: kernel launch failed");
+  if ((rc = rebuild_worklist(c))) return rc;
   SD_CUDA(cudaStreamSynchronize(c->stream));
   c->cx[ci].state_set = true;
-  return rebuild_worklist(c);
+  return SD_OK;
 }
 
 int sd_set_state(sd_ctx* c, int ci, const sd_swarm_state* st) {
@@ -932,9 +997,11 @@ int sd_set_state(sd_ctx* c, int ci, const sd_swarm_state* st) {
   SD_CUDA(cudaMemcpyAsync(D.nnei, st->nnei_len, n * 4, cudaMemcpyHostToDevice, c->stream));
   SD_CUDA(cudaMemcpyAsync(D.select, st->select, n * 4, cudaMemcpyHostToDevice, c->stream));
   SD_CUDA(cudaMemcpyAsync(D.ref, st->ligand_reference_pose, n * 3 * 8, cudaMemcpyHostToDevice, c->stream));
+  int rc = rebuild_worklist(c);
+  if (rc) return rc;
   SD_CUDA(cudaStreamSynchronize(c->stream));
   c->cx[ci].state_set = true;
-  return rebuild_worklist(c);
+  return SD_OK;
 }
 
 int sd_get_state(sd_ctx* c, int ci, sd_swarm_state* st) {
@@ -1086,30 +1153,20 @@ int sd_score_poses(sd_ctx* c, int ci, const double* poses, int n, int precision,
   if (n >= (1 << 24)) return fail(SD_ERR_ARG, "sd_score_poses: more than 2^24 poses");
   SD_CUDA(cudaSetDevice(c->device));
   const DevComplex& D = c->cx[ci].d;
-  for (size_t i = 0; i < (size_t)n * D.pl; ++i)
-    if (!std::isfinite(poses[i])) return fail(SD_ERR_NUMERIC, "sd_score_poses: non-finite pose");
+  if (!all_finite(poses, (size_t)n * D.pl)) return fail(SD_ERR_NUMERIC, "sd_score_poses: non-finite pose");
   int rc;
   if ((rc = ensure(c, c->s_pose, (size_t)n * D.pl * 8))) return rc;
   if ((rc = ensure(c, c->s_score, (size_t)n * 8))) return rc;
   if ((rc = ensure(c, c->s_energy, (size_t)n * 8))) return rc;
   if ((rc = ensure(c, c->s_ref, (size_t)n * 3 * 8))) return rc;
   if ((rc = ensure(c, c->s_work, (size_t)n * 4))) return rc;
-  std::vector<int> work(n);
-  for (int i = 0; i < n; ++i) work[i] = wi_pack(ci, i);
   DevComplex S = D;
   S.pos = (double*)c->s_pose.p;
   S.scoring = (double*)c->s_score.p;
   S.ref = (double*)c->s_ref.p;
-  StepCtl ctl;
-  SD_CUDA(cudaMemcpy(&ctl, c->d_ctl_scratch, sizeof ctl, cudaMemcpyDeviceToHost));
-  ctl.count[0] = n;
-  ctl.count[1] = 0;
-  ctl.grab[0] = ctl.grab[1] = 0;
-  ctl.parity = 0;
   SD_CUDA(cudaMemcpyAsync(c->s_pose.p, poses, (size_t)n * D.pl * 8, cudaMemcpyHostToDevice, c->stream));
-  SD_CUDA(cudaMemcpyAsync(c->s_work.p, work.data(), (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));
-  SD_CUDA(cudaMemcpyAsync(&c->d_cplx_scratch[ci], &S, sizeof S, cudaMemcpyHostToDevice, c->stream));
-  SD_CUDA(cudaMemcpyAsync(c->d_ctl_scratch, &ctl, sizeof ctl, cudaMemcpyHostToDevice, c->stream));
+  if ((rc = stateless_prepare_launch(c->d_ctl_scratch, c->d_cplx_scratch, S, (int*)c->s_work.p, ci, n, c->stream)))
+    return fail(rc, "stateless call: prepare kernel launch failed");
   int grid;
   size_t sm;
   const int variant = score_variant(c, precision, n, true);
@@ -1126,11 +1183,10 @@ int sd_score_poses(sd_ctx* c, int ci, const double* poses, int n, int precision,
   set_spill(c, L);
   if ((rc = score_launch(L, precision, c->scoring, grid, sm, c->stream, variant, c->score_spill)))
     return fail(rc, std::string("score kernel: ") + cudaGetErrorString(cudaGetLastError()));
-  SD_CUDA(cudaMemcpyAsync(score_out, c->s_score.p, (size_t)n * 8, cudaMemcpyDeviceToHost, c->stream));
-  if (energy_out)
-    SD_CUDA(cudaMemcpyAsync(energy_out, c->s_energy.p, (size_t)n * 8, cudaMemcpyDeviceToHost, c->stream));
-  SD_CUDA(cudaStreamSynchronize(c->stream));
-  return SD_OK;
+  Download down{c};
+  if ((rc = down.add(score_out, c->s_score.p, n))) return rc;
+  if (energy_out && (rc = down.add(energy_out, c->s_energy.p, n))) return rc;
+  return down.finish();
 }
 
 int sd_dfire_bins(sd_ctx* c, int ci, const double* pose, int precision, int* bins_out) {
@@ -1166,8 +1222,7 @@ int sd_pydock_grad(sd_ctx* c, int ci, const double* poses, int n, int precision,
   SD_CUDA(cudaSetDevice(c->device));
   const DevComplex& D = c->cx[ci].d;
   const int ng = 6 + D.nmr + D.nml;
-  for (size_t i = 0; i < (size_t)n * D.pl; ++i)
-    if (!std::isfinite(poses[i])) return fail(SD_ERR_NUMERIC, "sd_pydock_grad: non-finite pose");
+  if (!all_finite(poses, (size_t)n * D.pl)) return fail(SD_ERR_NUMERIC, "sd_pydock_grad: non-finite pose");
   int rc;
   if ((rc = ensure(c, c->s_pose, (size_t)n * D.pl * 8))) return rc;
   if ((rc = ensure(c, c->s_score, (size_t)n * 8))) return rc;
@@ -1175,40 +1230,39 @@ int sd_pydock_grad(sd_ctx* c, int ci, const double* poses, int n, int precision,
   if ((rc = ensure(c, c->s_ref, (size_t)n * 3 * 8))) return rc;
   if ((rc = ensure(c, c->s_work, (size_t)n * 4))) return rc;
   if ((rc = ensure(c, c->s_grad, (size_t)n * ng * 8))) return rc;
-  std::vector<int> work(n);
-  for (int i = 0; i < n; ++i) work[i] = wi_pack(ci, i);
   DevComplex S = D;
   S.pos = (double*)c->s_pose.p;
   S.scoring = (double*)c->s_score.p;
   S.ref = (double*)c->s_ref.p;
-  StepCtl ctl;
-  SD_CUDA(cudaMemcpy(&ctl, c->d_ctl_scratch, sizeof ctl, cudaMemcpyDeviceToHost));
-  ctl.count[0] = n;
-  ctl.count[1] = 0;
-  ctl.grab[0] = ctl.grab[1] = 0;
-  ctl.parity = 0;
   SD_CUDA(cudaMemcpyAsync(c->s_pose.p, poses, (size_t)n * D.pl * 8, cudaMemcpyHostToDevice, c->stream));
-  SD_CUDA(cudaMemcpyAsync(c->s_work.p, work.data(), (size_t)n * 4, cudaMemcpyHostToDevice, c->stream));
-  SD_CUDA(cudaMemcpyAsync(&c->d_cplx_scratch[ci], &S, sizeof S, cudaMemcpyHostToDevice, c->stream));
-  SD_CUDA(cudaMemcpyAsync(c->d_ctl_scratch, &ctl, sizeof ctl, cudaMemcpyHostToDevice, c->stream));
-  const size_t need = pydock_smem_bytes(precision, true, c->max_nl, c->max_nr);
-  const void* k = pydock_kernel_ptr(precision, true, false);
-  cudaFuncAttributes fa;
-  SD_CUDA(cudaFuncGetAttributes(&fa, k));
-  // a ligand too large for shared memory: the spill instantiation, per-CTA arrays in global scratch
-  const size_t warp_bytes = pydock_warp_bytes(precision, true);
-  const bool spill = warp_bytes + need + fa.sharedSizeBytes > (size_t)c->smem_optin;
-  const size_t sm = warp_bytes + (spill ? 0 : need);
-  if (spill) k = pydock_kernel_ptr(precision, true, true);
-  SD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(sm, 1)));
-  int per_sm = 0;
-  SD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, pydock_threads(precision, true), sm));
-  if (per_sm < 1) return fail(SD_ERR_ARG, "pyDock gradient kernel does not fit on an SM");
-  const size_t stride = (need + 255) & ~(size_t)255;
-  if (spill && (rc = grow_spill(c, stride * (size_t)per_sm * c->nsm))) return rc;
+  if ((rc = stateless_prepare_launch(c->d_ctl_scratch, c->d_cplx_scratch, S, (int*)c->s_work.p, ci, n, c->stream)))
+    return fail(rc, "stateless call: prepare kernel launch failed");
+  ScorePlan& plan = c->grad_plan[precision];
+  if (!plan.grid) {
+    const size_t need = pydock_smem_bytes(precision, true, c->max_nl, c->max_nr);
+    const void* k = pydock_kernel_ptr(precision, true, false);
+    cudaFuncAttributes fa;
+    SD_CUDA(cudaFuncGetAttributes(&fa, k));
+    // a ligand too large for shared memory: the spill instantiation, per-CTA arrays in global scratch
+    const size_t warp_bytes = pydock_warp_bytes(precision, true);
+    plan.spill = warp_bytes + need + fa.sharedSizeBytes > (size_t)c->smem_optin;
+    plan.smem = warp_bytes + (plan.spill ? 0 : need);
+    plan.spill_stride = plan.spill ? (need + 255) & ~(size_t)255 : 0;
+    if (plan.spill) {
+      k = pydock_kernel_ptr(precision, true, true);
+      SD_CUDA(cudaFuncGetAttributes(&fa, k));
+    }
+    SD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, c->smem_optin - (int)fa.sharedSizeBytes));
+    int per_sm = 0;
+    SD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, pydock_threads(precision, true), plan.smem));
+    if (per_sm < 1) return fail(SD_ERR_ARG, "pyDock gradient kernel does not fit on an SM");
+    plan.grid = per_sm * c->nsm;
+  }
+  const bool spill = plan.spill;
+  if (spill && (rc = grow_spill(c, plan.spill_stride * (size_t)plan.grid))) return rc;
   ScoreLaunch L{};
   L.spill = spill ? (unsigned char*)c->s_spill.p : nullptr;
-  L.spill_stride = spill ? stride : 0;
+  L.spill_stride = plan.spill_stride;
   L.force_scale = c->force_scale;
   L.cplx = c->d_cplx_scratch;
   L.ctl = c->d_ctl_scratch;
@@ -1218,13 +1272,12 @@ int sd_pydock_grad(sd_ctx* c, int ci, const double* poses, int n, int precision,
   L.lj_eps = c->d_lj_eps;
   L.lj_sigma = c->d_lj_sigma;
   L.energy_out = (double*)c->s_energy.p;
-  if ((rc = pydock_launch(L, precision, true, (double*)c->s_grad.p, per_sm * c->nsm, sm, c->stream, spill)))
+  if ((rc = pydock_launch(L, precision, true, (double*)c->s_grad.p, plan.grid, plan.smem, c->stream, spill)))
     return fail(rc, std::string("pyDock gradient kernel: ") + cudaGetErrorString(cudaGetLastError()));
-  if (energy_out)
-    SD_CUDA(cudaMemcpyAsync(energy_out, c->s_energy.p, (size_t)n * 8, cudaMemcpyDeviceToHost, c->stream));
-  SD_CUDA(cudaMemcpyAsync(grad_out, c->s_grad.p, (size_t)n * ng * 8, cudaMemcpyDeviceToHost, c->stream));
-  SD_CUDA(cudaStreamSynchronize(c->stream));
-  return SD_OK;
+  Download down{c};
+  if (energy_out && (rc = down.add(energy_out, c->s_energy.p, n))) return rc;
+  if ((rc = down.add(grad_out, c->s_grad.p, (size_t)n * ng))) return rc;
+  return down.finish();
 }
 
 int sd_refine_poses(sd_ctx* c, int ci, double* poses, int n, int iters, double step, int precision,

@@ -177,6 +177,12 @@ const void* pydock_kernel_ptr(int precision, bool grad, bool spill);
 int pydock_launch(const ScoreLaunch& L, int precision, bool grad, double* out_grad, int grid, size_t smem,
                   cudaStream_t st, bool spill);
 int pydock_threads(int precision, bool grad);
+int init_state_launch(const DevComplex& C, double luciferin, double vision, cudaStream_t st);
+int worklist_launch(const DevComplex* cplx, const int* swarm_map, int nswarms, StepCtl* ctl, int* work,
+                    cudaStream_t st);
+int stateless_prepare_launch(StepCtl* ctl, DevComplex* cplx, const DevComplex& desc, int* work, int ci, int n,
+                             cudaStream_t st);
+int check_finite_launch(const double* v, size_t n, int* bad, cudaStream_t st);
 void set_key_thresholds(const double* t64);
 size_t cluster_smem_bytes(int G, int nbb);
 int materialise_launch(const DevComplex* d_cplx, int ci, const int* d_poses, int n, const int* d_rslot, int nr, int nl,
