@@ -137,7 +137,7 @@ struct sd_ctx {
   DevBuf s_pose, s_score, s_ref, s_energy, s_work, s_grad, s_bins;
   // per-CTA global scratch of the spill instantiations (complexes too large for shared memory)
   DevBuf s_spill;
-  ScorePlan plan[3][SD_MAX_VARIANTS + 1], grad_plan[3];
+  ScorePlan plan[3][SD_MAX_VARIANTS + 1], grad_plan[3][2];
   void* h_stage = nullptr; // pinned, for small downloads
   int* d_flag = nullptr;
   int smem_optin = 0;      // shared memory a CTA may use on this device (opt-in maximum)
@@ -558,14 +558,20 @@ int configure_score(sd_ctx* c, int precision, int variant, int* grid, size_t* sm
   return SD_OK;
 }
 
-// the compiled variant of a precision's DFIRE kernel for a launch of at most `poses` poses; stateless:
-// not a GSO step, whose mixed variant the autotuner chose on its own poses
+// the few-poses shapes: at most one pose per SM, and receptors with a tile for most of the 24 warps
+bool few_poses(const sd_ctx* c, int poses) { return poses <= c->nsm && c->max_nr > 20 * SD_TILE; }
+
+// the compiled variant of a precision's kernel for a launch of at most `poses` poses; stateless: not a
+// GSO step, whose mixed variant the autotuner chose on its own poses
 int score_variant(const sd_ctx* c, int precision, int poses, bool stateless) {
-  if (precision == SD_PREC_FP64) return fp64_shape(c->max_nr, c->max_nl, c->smem_sm, poses, c->nsm);
-  if (precision != SD_PREC_MIXED || !stateless || poses > c->nsm) return c->mixed_variant;
-  const size_t cta = score_smem_bytes(precision, SD_SCORING_DFIRE, c->max_nr, c->max_nl, 1) +
-                     score_warp_bytes(precision, SD_SCORING_DFIRE, SD_MIXED_FEW, false) + 2048;
-  return cta <= (size_t)c->smem_optin ? SD_MIXED_FEW : c->mixed_variant;
+  bool few = few_poses(c, poses);
+  if (c->scoring == SD_SCORING_DFIRE) {
+    if (precision == SD_PREC_FP64) return fp64_shape(c->max_nr, c->max_nl, c->smem_sm, poses, c->nsm);
+    few &= precision == SD_PREC_MIXED && stateless;
+  }
+  const size_t cta = score_smem_bytes(precision, c->scoring, c->max_nr, c->max_nl, 1) +
+                     (few ? score_warp_bytes(precision, c->scoring, SD_FEW, false) : 0) + 12288;
+  return few && cta <= (size_t)c->smem_optin ? SD_FEW : c->mixed_variant;
 }
 
 // the spill scratch of the last configured launch (null pointers when it uses shared memory)
@@ -1237,24 +1243,27 @@ int sd_pydock_grad(sd_ctx* c, int ci, const double* poses, int n, int precision,
   SD_CUDA(cudaMemcpyAsync(c->s_pose.p, poses, (size_t)n * D.pl * 8, cudaMemcpyHostToDevice, c->stream));
   if ((rc = stateless_prepare_launch(c->d_ctl_scratch, c->d_cplx_scratch, S, (int*)c->s_work.p, ci, n, c->stream)))
     return fail(rc, "stateless call: prepare kernel launch failed");
-  ScorePlan& plan = c->grad_plan[precision];
+  const bool few = few_poses(c, n) && pydock_smem_bytes(precision, true, c->max_nl, c->max_nr) +
+                                              pydock_warp_bytes(precision, true, true) + 12288 <=
+                                          (size_t)c->smem_optin;
+  ScorePlan& plan = c->grad_plan[precision][few];
   if (!plan.grid) {
     const size_t need = pydock_smem_bytes(precision, true, c->max_nl, c->max_nr);
-    const void* k = pydock_kernel_ptr(precision, true, false);
+    const void* k = pydock_kernel_ptr(precision, true, false, few);
     cudaFuncAttributes fa;
     SD_CUDA(cudaFuncGetAttributes(&fa, k));
     // a ligand too large for shared memory: the spill instantiation, per-CTA arrays in global scratch
-    const size_t warp_bytes = pydock_warp_bytes(precision, true);
+    const size_t warp_bytes = pydock_warp_bytes(precision, true, few);
     plan.spill = warp_bytes + need + fa.sharedSizeBytes > (size_t)c->smem_optin;
     plan.smem = warp_bytes + (plan.spill ? 0 : need);
     plan.spill_stride = plan.spill ? (need + 255) & ~(size_t)255 : 0;
     if (plan.spill) {
-      k = pydock_kernel_ptr(precision, true, true);
+      k = pydock_kernel_ptr(precision, true, true, false);
       SD_CUDA(cudaFuncGetAttributes(&fa, k));
     }
     SD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, c->smem_optin - (int)fa.sharedSizeBytes));
     int per_sm = 0;
-    SD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, pydock_threads(precision, true), plan.smem));
+    SD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, pydock_threads(precision, true, few), plan.smem));
     if (per_sm < 1) return fail(SD_ERR_ARG, "pyDock gradient kernel does not fit on an SM");
     plan.grid = per_sm * c->nsm;
   }
@@ -1272,7 +1281,7 @@ int sd_pydock_grad(sd_ctx* c, int ci, const double* poses, int n, int precision,
   L.lj_eps = c->d_lj_eps;
   L.lj_sigma = c->d_lj_sigma;
   L.energy_out = (double*)c->s_energy.p;
-  if ((rc = pydock_launch(L, precision, true, (double*)c->s_grad.p, plan.grid, plan.smem, c->stream, spill)))
+  if ((rc = pydock_launch(L, precision, true, (double*)c->s_grad.p, plan.grid, plan.smem, c->stream, spill, few)))
     return fail(rc, std::string("pyDock gradient kernel: ") + cudaGetErrorString(cudaGetLastError()));
   Download down{c};
   if (energy_out && (rc = down.add(energy_out, c->s_energy.p, n))) return rc;

@@ -26,7 +26,7 @@
 #define SD_MAX_GLOWWORMS 6144   /* glowworms per swarm: luciferin + reference points in shared memory */
 #define SD_CULL_MARGIN 0.05f    /* A, covers FP32 rounding of the conservative culling tests */
 #define SD_MAX_VARIANTS 16      /* compiled variants of the mixed DFIRE kernel (autotuner) */
-#define SD_MIXED_FEW SD_MAX_VARIANTS  /* the mixed variant for stateless calls with few poses (not tuned) */
+#define SD_FEW SD_MAX_VARIANTS  /* the kernels' variant for at most one pose per SM (not tuned) */
 #define SD_NOALLOC_MAX_POSES 65536           /* poses per sd_score_poses_noalloc call */
 #define SD_NOALLOC_SCRATCH_BYTES (288 * 1024) /* its file-scope device scratch array */
 
@@ -171,12 +171,12 @@ int gso_prepare_warp();
 int bins_launch(const DevComplex* cplx, int c, const double* d_pose, int precision, int* d_bins, int nr, int nl,
                 int* d_fallback, cudaStream_t st);
 size_t pydock_smem_bytes(int precision, bool grad, int max_nl, int max_nr);
-size_t pydock_warp_bytes(int precision, bool grad);
+size_t pydock_warp_bytes(int precision, bool grad, bool few);
 float pydock_force_scale(double max_q_rec, double max_q_lig, const double* eps, const double* sigma, int max_nr);
-const void* pydock_kernel_ptr(int precision, bool grad, bool spill);
+const void* pydock_kernel_ptr(int precision, bool grad, bool spill, bool few);
 int pydock_launch(const ScoreLaunch& L, int precision, bool grad, double* out_grad, int grid, size_t smem,
-                  cudaStream_t st, bool spill);
-int pydock_threads(int precision, bool grad);
+                  cudaStream_t st, bool spill, bool few);
+int pydock_threads(int precision, bool grad, bool few);
 int init_state_launch(const DevComplex& C, double luciferin, double vision, cudaStream_t st);
 int worklist_launch(const DevComplex* cplx, const int* swarm_map, int nswarms, StepCtl* ctl, int* work,
                     cudaStream_t st);

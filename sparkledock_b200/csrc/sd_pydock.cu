@@ -41,8 +41,12 @@ namespace sd {
 namespace {
 
 // warps of a CTA: FP32 gradients 12, two CTAs per SM (their ligand forces take 24 bytes an atom, and
-// three CTAs of 8 warps would not fit beside ligands over 1,270 atoms); else 8, as many as fit
-__host__ __device__ constexpr int pd_warps(bool fp64, bool grad) { return grad && !fp64 ? 12 : 8; }
+// three CTAs of 8 warps would not fit beside ligands over 1,270 atoms); else 8, as many as fit.  few: at
+// most one pose per SM, so one CTA with all the warps that the registers allow, for a pose's time
+__host__ __device__ constexpr int pd_warps(bool fp64, bool grad, bool few) {
+  return few ? (grad && fp64 ? 16 : 24) : (grad && !fp64 ? 12 : 8);
+}
+__host__ __device__ constexpr int pd_ctas(bool grad, bool few) { return few ? 1 : (grad ? 2 : 4); }
 constexpr double kKe = 332.0636 / 4.0;
 
 // an atom in shared memory (position relative to t, the ligand's negated, charge): one 16-byte load in FP32
@@ -210,10 +214,10 @@ __device__ __forceinline__ T warp_sum(T v) {
 // L.energy_out (E) when set.  kSpill: the per-pose arrays live in this CTA's slice of the global
 // scratch L.spill instead of shared memory (ligands too large for it).  Four CTAs per SM (64
 // registers a thread) without forces: the pair terms are latency chains.
-template <class T, bool GRAD, bool kSpill>
-__global__ void __launch_bounds__(pd_warps(sizeof(T) == 8, GRAD) * 32, GRAD ? 2 : 4)
+template <class T, bool GRAD, bool kSpill, bool kFew>
+__global__ void __launch_bounds__(pd_warps(sizeof(T) == 8, GRAD, kFew) * 32, pd_ctas(GRAD, kFew))
 pydock_kernel(ScoreLaunch L, double* out_grad) {
-  constexpr int kWarps = pd_warps(sizeof(T) == 8, GRAD);
+  constexpr int kWarps = pd_warps(sizeof(T) == 8, GRAD, kFew);
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   PdWarp<T>& W = reinterpret_cast<PdWarp<T>*>(smem_dyn)[threadIdx.x >> 5];
   unsigned char* const smem =
@@ -605,9 +609,9 @@ size_t pydock_smem_bytes(int precision, bool grad, int max_nl, int max_nr) {
   return ts * 4 * (nls + 1) + (grad ? 24 * (nls + 4) : 0) + 16 * nlc + (nls + 1) +
          12 * ((max_nr + SD_TILE - 1) / SD_TILE) + 16;
 }
-size_t pydock_warp_bytes(int precision, bool grad) {
+size_t pydock_warp_bytes(int precision, bool grad, bool few) {
   const bool fp64 = precision != SD_PREC_MIXED;
-  return pd_warps(fp64, grad) * (fp64 ? sizeof(PdWarp<double>) : sizeof(PdWarp<float>));
+  return pd_warps(fp64, grad, few) * (fp64 ? sizeof(PdWarp<double>) : sizeof(PdWarp<float>));
 }
 
 // the scale of FP32 ligand forces: pair forces are at most 0.7 kKe q q' (electrostatics) plus 1.6 eps
@@ -627,25 +631,30 @@ float pydock_force_scale(double max_q_rec, double max_q_lig, const double* eps, 
   return std::ldexp(1.0f, std::min(100, std::max(-100, k)));
 }
 
-const void* pydock_kernel_ptr(int precision, bool grad, bool spill) {
-  if (precision == SD_PREC_MIXED) {
-    if (spill) return grad ? (const void*)pydock_kernel<float, true, true> : (const void*)pydock_kernel<float, false, true>;
-    return grad ? (const void*)pydock_kernel<float, true, false> : (const void*)pydock_kernel<float, false, false>;
-  }
-  if (spill) return grad ? (const void*)pydock_kernel<double, true, true> : (const void*)pydock_kernel<double, false, true>;
-  return grad ? (const void*)pydock_kernel<double, true, false> : (const void*)pydock_kernel<double, false, false>;
+template <class T, bool GRAD>
+static const void* kernel_of(bool spill, bool few) {
+  if (spill) return (const void*)pydock_kernel<T, GRAD, true, false>;
+  return few ? (const void*)pydock_kernel<T, GRAD, false, true> : (const void*)pydock_kernel<T, GRAD, false, false>;
+}
+
+// (the spill instantiation has the ordinary shape: few is ignored with it)
+const void* pydock_kernel_ptr(int precision, bool grad, bool spill, bool few) {
+  if (precision == SD_PREC_MIXED) return grad ? kernel_of<float, true>(spill, few) : kernel_of<float, false>(spill, few);
+  return grad ? kernel_of<double, true>(spill, few) : kernel_of<double, false>(spill, few);
 }
 
 int pydock_launch(const ScoreLaunch& L, int precision, bool grad, double* out_grad, int grid, size_t smem,
-                  cudaStream_t st, bool spill) {
+                  cudaStream_t st, bool spill, bool few) {
   ScoreLaunch l = L;
   void* args[] = {(void*)&l, (void*)&out_grad};
-  if (cudaLaunchKernel(pydock_kernel_ptr(precision, grad, spill), dim3(grid), dim3(pydock_threads(precision, grad)), args,
-                       smem, st) != cudaSuccess)
+  if (cudaLaunchKernel(pydock_kernel_ptr(precision, grad, spill, few), dim3(grid),
+                       dim3(pydock_threads(precision, grad, few && !spill)), args, smem, st) != cudaSuccess)
     return SD_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? SD_OK : SD_ERR_CUDA;
 }
 
-int pydock_threads(int precision, bool grad) { return pd_warps(precision != SD_PREC_MIXED, grad) * 32; }
+int pydock_threads(int precision, bool grad, bool few) {
+  return pd_warps(precision != SD_PREC_MIXED, grad, few) * 32;
+}
 
 }  // namespace sd

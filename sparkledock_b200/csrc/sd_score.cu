@@ -256,13 +256,13 @@ constexpr int kNumMixedVariants = sizeof(kMixedVariants) / sizeof(kMixedVariants
 static_assert(kNumMixedVariants <= SD_MAX_VARIANTS, "variant table");
 
 static const MixedVariant& mixed_variant(int v) {
-  return v == SD_MIXED_FEW ? kMixedFew : kMixedVariants[v < 0 || v >= kNumMixedVariants ? 0 : v];
+  return v == SD_FEW ? kMixedFew : kMixedVariants[v < 0 || v >= kNumMixedVariants ? 0 : v];
 }
 
 // bytes of the scorer's per-warp buffers, in dynamic shared memory in front of the per-pose arrays
 // (alone there in the spill instantiation)
 size_t score_warp_bytes(int precision, int scoring, int variant, bool spill) {
-  if (scoring == SD_SCORING_PYDOCK) return pydock_warp_bytes(precision, false);
+  if (scoring == SD_SCORING_PYDOCK) return pydock_warp_bytes(precision, false, !spill && variant == SD_FEW);
   if (precision == SD_PREC_FP64_REF) return 0;
   if (precision == SD_PREC_FP64) return sizeof(OrdBufs) * (spill ? kFp64Spill : kFp64Shapes[variant]).warps;
   return sizeof(WarpBufs) * (spill ? kMixedSpill.warps : mixed_variant(variant).warps);
@@ -286,13 +286,14 @@ size_t score_smem_bytes(int precision, int scoring, int max_nr, int max_nl, int 
 // the culled FP64 kernel's shape for these sizes and at most `poses` poses (1 KiB of each CTA is the
 // system's, 1 KiB covers the static arrays); the last one when none fits (the caller then spills)
 int fp64_shape(int max_nr, int max_nl, int smem_sm, int poses, int nsm) {
+  const int ntiles = (max_nr + SD_TILE - 1) / SD_TILE;  // a warp without a tile only waits
   int best = kNumFp64Shapes - 1;
   for (int v = kNumFp64Shapes - 1; v >= 0; --v) {
     const size_t cta = score_smem_bytes(SD_PREC_FP64, SD_SCORING_DFIRE, max_nr, max_nl, 1) +
                        score_warp_bytes(SD_PREC_FP64, SD_SCORING_DFIRE, v, false) + 2048;
     const bool few = poses <= kFp64Shapes[v].min_blocks * nsm;
     if (cta * kFp64Shapes[v].min_blocks > (size_t)smem_sm) continue;
-    if (!few || kFp64Shapes[v].warps > kFp64Shapes[best].warps) best = v;
+    if (!few || (kFp64Shapes[v].warps > kFp64Shapes[best].warps && kFp64Shapes[v].warps <= ntiles)) best = v;
   }
   return best;
 }
@@ -301,14 +302,14 @@ int mixed_variant_warps(int v) { return mixed_variant(v).warps; }
 int mixed_variant_min_blocks(int v) { return mixed_variant(v).min_blocks; }
 
 int score_threads_of(int precision, int scoring, int variant, bool spill) {
-  if (scoring == SD_SCORING_PYDOCK) return pydock_threads(precision, false);
+  if (scoring == SD_SCORING_PYDOCK) return pydock_threads(precision, false, !spill && variant == SD_FEW);
   if (precision == SD_PREC_FP64_REF) return kRefThreads;
   if (precision == SD_PREC_FP64) return (spill ? kFp64Spill : kFp64Shapes[variant]).warps * 32;
   return (spill ? kMixedSpill : mixed_variant(variant)).warps * 32;
 }
 
 const void* score_kernel_ptr(int precision, int scoring, int variant, bool spill) {
-  if (scoring == SD_SCORING_PYDOCK) return pydock_kernel_ptr(precision, false, spill);
+  if (scoring == SD_SCORING_PYDOCK) return pydock_kernel_ptr(precision, false, spill, variant == SD_FEW);
   switch (precision) {
     case SD_PREC_FP64_REF:
       return spill ? (const void*)dfire_score_ref_kernel<true> : (const void*)dfire_score_ref_kernel<false>;
@@ -319,7 +320,7 @@ const void* score_kernel_ptr(int precision, int scoring, int variant, bool spill
 
 int score_launch(const ScoreLaunch& L, int precision, int scoring, int grid, size_t smem, cudaStream_t st, int variant,
                  bool spill) {
-  if (scoring == SD_SCORING_PYDOCK) return pydock_launch(L, precision, false, nullptr, grid, smem, st, spill);
+  if (scoring == SD_SCORING_PYDOCK) return pydock_launch(L, precision, false, nullptr, grid, smem, st, spill, variant == SD_FEW);
   ScoreLaunch l = L;
   void* args[] = {(void*)&l};
   if (cudaLaunchKernel(score_kernel_ptr(precision, scoring, variant, spill), dim3(grid),
