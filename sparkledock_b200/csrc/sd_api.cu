@@ -134,7 +134,7 @@ struct sd_ctx {
   int total_swarms = 0;
   int max_nr = 0, max_nl = 0, max_G = 0;
   // stateless scratch
-  DevBuf s_pose, s_score, s_ref, s_energy, s_work, s_grad, s_bins;
+  DevBuf s_pose, s_score, s_ref, s_energy, s_work, s_grad, s_bins, s_final;
   // per-CTA global scratch of the spill instantiations (complexes too large for shared memory)
   DevBuf s_spill;
   ScorePlan plan[3][SD_MAX_VARIANTS + 1], grad_plan[3][2];
@@ -332,6 +332,10 @@ int setup_complex(sd_ctx* c, const sd_complex_desc& d, ComplexHost& h, int gbase
 
   int rc;
   if ((rc = upload(c, h, slots.data(), slots.size(), &D.r_orig))) return rc;
+  std::vector<int> rslot(d.n_rec);
+  for (int s = 0; s < nslots; ++s)
+    if (slots[s] >= 0) rslot[slots[s]] = s;
+  if ((rc = upload(c, h, rslot.data(), rslot.size(), &D.r_slot))) return rc;
   if ((rc = upload(c, h, rxyz.data(), rxyz.size(), &D.r_xyz))) return rc;
   if ((rc = upload(c, h, rmodes.data(), rmodes.size(), &D.r_modes))) return rc;
   if ((rc = upload(c, h, rmask.data(), rmask.size(), &D.r_mask))) return rc;
@@ -446,33 +450,36 @@ bool all_finite(const double* v, size_t n) {
   return s == 0.0;
 }
 
-// n doubles into pinned host memory of the context (kept, up to 1 MiB) on the way to the caller's pageable
-// array, or straight there when they are more: a small download into pageable memory waits on its own
+// Downloads through pinned host memory of the context (kept, 1 MiB) on the way to the caller's pageable
+// arrays, or straight there when they do not fit: a small download into pageable memory waits on its own
 constexpr size_t kStage = 1 << 20;
 struct Download {
   sd_ctx* c;
   size_t used = 0;
   struct Part {
-    double* dst;
-    size_t at, n;
-  } part[2];
+    void* dst;
+    size_t at, bytes;
+  } part[4];
   int parts = 0;
-  int add(double* dst, const void* src, size_t n) {
-    if (used + n * 8 > kStage || !c->h_stage) {
-      SD_CUDA(cudaMemcpyAsync(dst, src, n * 8, cudaMemcpyDeviceToHost, c->stream));
+  int add(void* dst, const void* src, size_t bytes) {
+    if (used + bytes > kStage || !c->h_stage) {
+      SD_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->stream));
       return SD_OK;
     }
-    SD_CUDA(cudaMemcpyAsync((char*)c->h_stage + used, src, n * 8, cudaMemcpyDeviceToHost, c->stream));
-    part[parts++] = {dst, used, n};
-    used += n * 8;
+    SD_CUDA(cudaMemcpyAsync((char*)c->h_stage + used, src, bytes, cudaMemcpyDeviceToHost, c->stream));
+    part[parts++] = {dst, used, bytes};
+    used += bytes;
     return SD_OK;
   }
   int finish() {
     SD_CUDA(cudaStreamSynchronize(c->stream));
-    for (int i = 0; i < parts; ++i) memcpy(part[i].dst, (char*)c->h_stage + part[i].at, part[i].n * 8);
+    for (int i = 0; i < parts; ++i) memcpy(part[i].dst, (char*)c->h_stage + part[i].at, part[i].bytes);
     return SD_OK;
   }
 };
+
+// coordinates of final poses on the device at a time (clustering, materialising), kept by the context
+constexpr size_t kFinalBytes = (size_t)256 << 20;
 
 // The spill scratch, grown to at least bytes.  The step graph holds the scratch's address, so a new
 // scratch means a new capture at the next step.
@@ -930,7 +937,7 @@ int sd_ctx_destroy(sd_ctx* c) {
     for (void* p : h.owned) cudaFree(p);
   void* ps[] = {c->d_cplx, c->d_cplx_scratch, c->d_table64, c->d_lj_eps, c->d_lj_sigma, c->d_ctl,
                 c->d_ctl_scratch, c->d_work[0], c->d_work[1], c->d_swarm_map, c->d_pos_prev, c->s_pose.p, c->s_score.p,
-                c->s_ref.p, c->s_energy.p, c->s_work.p, c->s_grad.p, c->s_bins.p, c->s_spill.p};
+                c->s_ref.p, c->s_energy.p, c->s_work.p, c->s_grad.p, c->s_bins.p, c->s_spill.p, c->s_final.p};
   for (void* p : ps)
     if (p) cudaFree(p);
   if (c->d_flag) cudaFree(c->d_flag);
@@ -1190,8 +1197,8 @@ int sd_score_poses(sd_ctx* c, int ci, const double* poses, int n, int precision,
   if ((rc = score_launch(L, precision, c->scoring, grid, sm, c->stream, variant, c->score_spill)))
     return fail(rc, std::string("score kernel: ") + cudaGetErrorString(cudaGetLastError()));
   Download down{c};
-  if ((rc = down.add(score_out, c->s_score.p, n))) return rc;
-  if (energy_out && (rc = down.add(energy_out, c->s_energy.p, n))) return rc;
+  if ((rc = down.add(score_out, c->s_score.p, (size_t)n * 8))) return rc;
+  if (energy_out && (rc = down.add(energy_out, c->s_energy.p, (size_t)n * 8))) return rc;
   return down.finish();
 }
 
@@ -1284,8 +1291,8 @@ int sd_pydock_grad(sd_ctx* c, int ci, const double* poses, int n, int precision,
   if ((rc = pydock_launch(L, precision, true, (double*)c->s_grad.p, plan.grid, plan.smem, c->stream, spill, few)))
     return fail(rc, std::string("pyDock gradient kernel: ") + cudaGetErrorString(cudaGetLastError()));
   Download down{c};
-  if (energy_out && (rc = down.add(energy_out, c->s_energy.p, n))) return rc;
-  if ((rc = down.add(grad_out, c->s_grad.p, (size_t)n * ng))) return rc;
+  if (energy_out && (rc = down.add(energy_out, c->s_energy.p, (size_t)n * 8))) return rc;
+  if ((rc = down.add(grad_out, c->s_grad.p, (size_t)n * ng * 8))) return rc;
   return down.finish();
 }
 
@@ -1358,51 +1365,29 @@ int sd_materialise_poses(sd_ctx* c, int ci, const int* poses, int n, double* rec
   const long long SG = (long long)D.S * D.G;
   for (int k = 0; k < n; ++k)
     if (poses[k] < 0 || poses[k] >= SG) return fail(SD_ERR_ARG, "sd_materialise_poses: pose index out of range");
-  const int nr = D.nr, nl = D.nl, nslots = D.ntiles * SD_TILE;
-  std::vector<int> orig(nslots), slot_of(nr, 0);
-  SD_CUDA(cudaMemcpy(orig.data(), D.r_orig, sizeof(int) * nslots, cudaMemcpyDeviceToHost));
-  for (int sl = 0; sl < nslots; ++sl)
-    if (orig[sl] >= 0) slot_of[orig[sl]] = sl;
-  // poses per launch: coordinates of at most 256 MiB on the device
+  const int nr = D.nr, nl = D.nl;
+  // poses per launch: coordinates of at most kFinalBytes in the context's workspace
   const size_t per_pose = (size_t)(nr + nl) * 3 * sizeof(double);
-  const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)n, ((size_t)256 << 20) / per_pose));
-  int *d_poses = nullptr, *d_slot = nullptr;
-  double* d_xyz = nullptr;
-  auto release = [&]() {
-    cudaFree(d_poses);
-    cudaFree(d_slot);
-    cudaFree(d_xyz);
-  };
-  auto cu = [&](cudaError_t e) {
-    if (e == cudaSuccess) return SD_OK;
-    release();
-    return fail(e == cudaErrorMemoryAllocation ? SD_ERR_OOM : SD_ERR_CUDA,
-                std::string("sd_materialise_poses: ") + cudaGetErrorString(e));
-  };
+  const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)n, kFinalBytes / per_pose));
   int rc;
-  if ((rc = cu(cudaMalloc(&d_poses, sizeof(int) * chunk)))) return rc;
-  if ((rc = cu(cudaMalloc(&d_slot, sizeof(int) * std::max(1, nr))))) return rc;
-  if ((rc = cu(cudaMalloc(&d_xyz, per_pose * chunk)))) return rc;
-  if ((rc = cu(cudaMemcpy(d_slot, slot_of.data(), sizeof(int) * nr, cudaMemcpyHostToDevice)))) return rc;
+  if ((rc = ensure(c, c->s_final, per_pose * chunk + sizeof(int) * (size_t)chunk))) return rc;
+  double* d_xyz = (double*)c->s_final.p;
+  int* d_poses = (int*)((char*)c->s_final.p + per_pose * chunk);
   for (int k0 = 0; k0 < n; k0 += chunk) {
     const int m = std::min(chunk, n - k0);
     double* d_rec = d_xyz;
     double* d_lig = d_xyz + (size_t)m * nr * 3;
-    if ((rc = cu(cudaMemcpyAsync(d_poses, poses + k0, sizeof(int) * m, cudaMemcpyHostToDevice, c->stream))))
-      return rc;
-    if ((rc = materialise_launch(c->d_cplx, ci, d_poses, m, d_slot, nr, nl, d_rec, d_lig, c->stream))) {
-      release();
+    SD_CUDA(cudaMemcpyAsync(d_poses, poses + k0, sizeof(int) * m, cudaMemcpyHostToDevice, c->stream));
+    if ((rc = materialise_launch(c->d_cplx, ci, d_poses, m, nr, nl, d_rec, d_lig, c->stream)))
       return fail(rc, "sd_materialise_poses: launch failed");
-    }
-    if (rec_xyz_out && (rc = cu(cudaMemcpyAsync(rec_xyz_out + (size_t)k0 * nr * 3, d_rec, sizeof(double) * m * nr * 3,
-                                                cudaMemcpyDeviceToHost, c->stream))))
-      return rc;
-    if (lig_xyz_out && (rc = cu(cudaMemcpyAsync(lig_xyz_out + (size_t)k0 * nl * 3, d_lig, sizeof(double) * m * nl * 3,
-                                                cudaMemcpyDeviceToHost, c->stream))))
-      return rc;
-    if ((rc = cu(cudaStreamSynchronize(c->stream)))) return rc;
+    if (rec_xyz_out)
+      SD_CUDA(cudaMemcpyAsync(rec_xyz_out + (size_t)k0 * nr * 3, d_rec, sizeof(double) * m * nr * 3,
+                              cudaMemcpyDeviceToHost, c->stream));
+    if (lig_xyz_out)
+      SD_CUDA(cudaMemcpyAsync(lig_xyz_out + (size_t)k0 * nl * 3, d_lig, sizeof(double) * m * nl * 3,
+                              cudaMemcpyDeviceToHost, c->stream));
+    SD_CUDA(cudaStreamSynchronize(c->stream));
   }
-  release();
   return SD_OK;
 }
 
@@ -1415,63 +1400,42 @@ int sd_cluster(sd_ctx* c, int ci, const int* rec_backbone, const int* lig_backbo
   if (!c->cx[ci].state_set) return fail(SD_ERR_STATE, "sd_cluster: no state");
   SD_CUDA(cudaSetDevice(c->device));
   const DevComplex& D = c->cx[ci].d;
-  const int S = D.S, G = D.G, nslots = D.ntiles * SD_TILE;
-  // receptor slot of each flagged atom (atoms are stored in spatial tile order)
-  std::vector<int> orig(nslots), slot_of(D.nr, -1), rb, lb;
-  SD_CUDA(cudaMemcpy(orig.data(), D.r_orig, sizeof(int) * nslots, cudaMemcpyDeviceToHost));
-  for (int sl = 0; sl < nslots; ++sl)
-    if (orig[sl] >= 0) slot_of[orig[sl]] = sl;
+  const int S = D.S, G = D.G;
+  std::vector<int> bb;  // flagged receptor atoms, then ligand atoms
   for (int i = 0; i < D.nr; ++i)
-    if (rec_backbone[i]) rb.push_back(slot_of[i]);
+    if (rec_backbone[i]) bb.push_back(i);
+  const int nbr = (int)bb.size();
   for (int j = 0; j < D.nl; ++j)
-    if (lig_backbone[j]) lb.push_back(j);
-  const int nbr = (int)rb.size(), nbl = (int)lb.size(), nbb = nbr + nbl;
+    if (lig_backbone[j]) bb.push_back(j);
+  const int nbb = (int)bb.size(), nbl = nbb - nbr;
   if (nbb == 0) return fail(SD_ERR_ARG, "sd_cluster: no backbone atoms flagged");
-  if (cluster_smem_bytes(G, nbb) > 227 * 1024) return fail(SD_ERR_NOTSUP, "sd_cluster: too many backbone atoms");
-  // swarms per launch: coordinates of at most ~1 GiB on the device
+  if (cluster_smem_bytes(G) + (size_t)nbb * 24 + 4 * (G & 1) > 227 * 1024)
+    return fail(SD_ERR_NOTSUP, "sd_cluster: too many backbone atoms");
+  // swarms per launch: coordinates of at most kFinalBytes in the context's workspace
   const size_t per_swarm = (size_t)G * nbb * 3 * sizeof(double);
-  const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)S, ((size_t)1 << 30) / per_swarm));
-  int* d_rb = nullptr;
-  int* d_lb = nullptr;
-  int* d_out = nullptr;
-  double* d_bb = nullptr;
-  auto release = [&]() {
-    cudaFree(d_rb);
-    cudaFree(d_lb);
-    cudaFree(d_out);
-    cudaFree(d_bb);
-  };
-  auto cu = [&](cudaError_t e) {
-    if (e == cudaSuccess) return SD_OK;
-    release();
-    return fail(e == cudaErrorMemoryAllocation ? SD_ERR_OOM : SD_ERR_CUDA, std::string("sd_cluster: ") + cudaGetErrorString(e));
-  };
+  const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)S, kFinalBytes / per_swarm));
+  const size_t n_out = (size_t)S + 3 * (size_t)S * G;
   int rc;
-  if ((rc = cu(cudaMalloc(&d_rb, sizeof(int) * std::max(1, nbr))))) return rc;
-  if ((rc = cu(cudaMalloc(&d_lb, sizeof(int) * std::max(1, nbl))))) return rc;
-  if ((rc = cu(cudaMalloc(&d_out, sizeof(int) * ((size_t)S + 3 * (size_t)S * G))))) return rc;
-  if ((rc = cu(cudaMalloc(&d_bb, per_swarm * chunk)))) return rc;
-  if (nbr && (rc = cu(cudaMemcpy(d_rb, rb.data(), sizeof(int) * nbr, cudaMemcpyHostToDevice)))) return rc;
-  if (nbl && (rc = cu(cudaMemcpy(d_lb, lb.data(), sizeof(int) * nbl, cudaMemcpyHostToDevice)))) return rc;
-  int* d_ncl = d_out;
-  int* d_rep = d_out + S;
+  if ((rc = ensure(c, c->s_final, per_swarm * chunk + sizeof(int) * (nbb + n_out)))) return rc;
+  double* d_bb = (double*)c->s_final.p;
+  int* d_idx = (int*)((char*)c->s_final.p + per_swarm * chunk);
+  int* d_ncl = d_idx + nbb;
+  int* d_rep = d_ncl + S;
   int* d_len = d_rep + (size_t)S * G;
   int* d_mem = d_len + (size_t)S * G;
+  SD_CUDA(cudaMemcpyAsync(d_idx, bb.data(), sizeof(int) * nbb, cudaMemcpyHostToDevice, c->stream));
   for (int s0 = 0; s0 < S; s0 += chunk) {
     const int ns = std::min(chunk, S - s0);
-    if ((rc = cluster_launch(c->d_cplx, ci, s0, ns, G, d_rb, nbr, d_lb, nbl, d_bb, d_ncl, d_rep, d_len, d_mem,
-                             c->stream))) {
-      release();
+    if ((rc = cluster_launch(c->d_cplx, ci, s0, ns, G, d_idx, nbr, d_idx + nbr, nbl, d_bb, d_ncl, d_rep, d_len, d_mem,
+                             c->stream)))
       return fail(rc, "sd_cluster: launch failed");
-    }
   }
-  if ((rc = cu(cudaStreamSynchronize(c->stream)))) return rc;
-  if ((rc = cu(cudaMemcpy(n_clusters, d_ncl, sizeof(int) * S, cudaMemcpyDeviceToHost)))) return rc;
-  if ((rc = cu(cudaMemcpy(cluster_rep, d_rep, sizeof(int) * S * G, cudaMemcpyDeviceToHost)))) return rc;
-  if ((rc = cu(cudaMemcpy(cluster_len, d_len, sizeof(int) * S * G, cudaMemcpyDeviceToHost)))) return rc;
-  if ((rc = cu(cudaMemcpy(member_of, d_mem, sizeof(int) * S * G, cudaMemcpyDeviceToHost)))) return rc;
-  release();
-  return SD_OK;
+  Download down{c};
+  if ((rc = down.add(n_clusters, d_ncl, sizeof(int) * S))) return rc;
+  if ((rc = down.add(cluster_rep, d_rep, sizeof(int) * S * G))) return rc;
+  if ((rc = down.add(cluster_len, d_len, sizeof(int) * S * G))) return rc;
+  if ((rc = down.add(member_of, d_mem, sizeof(int) * S * G))) return rc;
+  return down.finish();
 }
 
 }  // extern "C"

@@ -65,6 +65,7 @@ struct DevComplex {
   int gbase, sbase;     // first global glowworm / swarm index of this complex
   // receptor in tile order (slot = tile*32 + lane); padded slots have orig = -1
   const int* r_orig;
+  const int* r_slot;       // [nr] original receptor index -> slot
   const double* r_xyz;     // [3][nslots]
   const double* r_modes;   // [nmr][3][nslots]
   const int* r_mask;       // [nslots]
@@ -184,10 +185,10 @@ int stateless_prepare_launch(StepCtl* ctl, DevComplex* cplx, const DevComplex& d
                              cudaStream_t st);
 int check_finite_launch(const double* v, size_t n, int* bad, cudaStream_t st);
 void set_key_thresholds(const double* t64);
-size_t cluster_smem_bytes(int G, int nbb);
-int materialise_launch(const DevComplex* d_cplx, int ci, const int* d_poses, int n, const int* d_rslot, int nr, int nl,
-                       double* d_rec, double* d_lig, cudaStream_t st);
-int cluster_launch(const DevComplex* d_cplx, int ci, int s0, int ns, int G, const int* d_rb_slot, int nbr,
+size_t cluster_smem_bytes(int G);
+int materialise_launch(const DevComplex* d_cplx, int ci, const int* d_poses, int n, int nr, int nl, double* d_rec,
+                       double* d_lig, cudaStream_t st);
+int cluster_launch(const DevComplex* d_cplx, int ci, int s0, int ns, int G, const int* d_rb, int nbr,
                    const int* d_lb_idx, int nbl, double* d_bb, int* d_ncl, int* d_rep, int* d_len, int* d_member,
                    cudaStream_t st);
 
