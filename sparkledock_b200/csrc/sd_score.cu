@@ -219,9 +219,9 @@ struct MixedVariant {
 #define SD_MIXED(W, B) { (const void*)dfire_score_mixed_kernel<W, B, false>, W, B }
 // 24 or 28 warps per SM in all of them (80 or 72 registers a thread).  Fewer and larger CTAs hold fewer
 // copies of the ligand in shared memory and leave L1 more room for gathers in flight; smaller ones
-// lose less at the end of a batch.  Measured (M poses/s for 12x2, 14x2, 8x3, 6x4): 757/481 atoms 7.2,
-// 7.0, 9.3, 9.6; 3002/1274 2.94, 2.98, 2.39, 2.78; 6032/1766 1.90, 1.50, 1.76, 1.41; 17307/1125 2.49,
-// 2.57, 2.04, 2.32.  Variant 0 is the default before the autotuner has run.  The variants give
+// lose less at the end of a batch.  Measured (M poses/s for 12x2, 14x2, 8x3, 6x4): 757/481 atoms 7.4,
+// 7.2, 9.5, 9.7; 3002/1274 2.97, 3.01, 2.36, 2.78; 6032/1766 1.90, 1.50, 1.77, 1.41; 17307/1125 2.50,
+// 2.58, 2.04, 2.31.  Variant 0 is the default before the autotuner has run.  The variants give
 // bit-identical energies (same per-tile work and summation order), so the tuner's choice never changes
 // a result.
 static const MixedVariant kMixedVariants[] = {

@@ -20,8 +20,8 @@
 //    an approximate square root, the bin coordinate and its distance from the nearest edge.  A pair
 //    inside the cutoff and further from an edge than the proven FP32 error has its FP64 bin, and its
 //    value is gathered (through L2 only) and added by the next step, so that it is in flight while the
-//    next step is evaluated.  Pairs near an edge are found again after the group's loop and decided in
-//    FP64 from the exact transforms (counted as fallbacks).  Each lane sums its values in FP64 (Kahan
+//    next step is evaluated.  A bit per step notes a pair near an edge; such pairs are found again after
+//    the group's loop and decided in FP64 from the exact transforms (counted as fallbacks).  Each lane sums its values in FP64 (Kahan
 //    sums of an FP32-rounded table were measured to miss 1e-5 at 60k pairs per pose);
 //  * fixed summation order: a tile's lane sums are reduced by warp shuffles when the tile is done and
 //    stored in a per-pose shared slot of that tile; at the end one warp per pose adds the slots in a
@@ -35,8 +35,8 @@
 // the sectors (half of that before two poses shared them), and L1 must hold the gathers in flight, so
 // the shared memory a CTA takes costs speed too.  Measured on 8,000 to 20,000 poses, poses/s, against
 // the earlier kernel (FP16 pre-filter of tile x candidate pairs, a ring of in-cutoff pairs, one pose
-// per CTA): 3002/1274 2.36 M -> 2.97 M, 17307/1125 2.02 M -> 2.57 M, 6032/1766 1.34 M -> 1.90 M,
-// 757/481 6.9 M -> 9.5 M.
+// per CTA): 3002/1274 2.34 M -> 3.01 M, 17307/1125 2.02 M -> 2.58 M, 6032/1766 1.34 M -> 1.90 M,
+// 757/481 6.9 M -> 9.7 M.
 #pragma once
 
 namespace sd {
@@ -45,11 +45,10 @@ namespace {
 constexpr int kGroup = SD_GROUP;      // receptor atoms of a group (one row of 8 lanes)
 constexpr int kGroups = SD_TILE / kGroup;
 constexpr int kRow = 8;               // candidates of a step: 8 rows of 4 lanes, two atoms of the group per lane
-constexpr int kSteps = 1;             // steps in flight per block
-constexpr int kBlock = kSteps * kRow; // candidates of a block
 constexpr int kPoses = 2;             // poses of a batch: they share the reads of modes and tiles
 constexpr int kList = 160;            // candidates of a group between two drains of the lists
 constexpr int kNear = 16;             // pairs of a tile that may be decided in FP64 one by one
+static_assert(kList / kRow <= 32, "a bit per step");
 constexpr float kMagic = 12582912.0f; // 1.5 * 2^23: adding it rounds to an integer in the low bits
 constexpr int kMagicBits = 0x4B400000;
 
@@ -375,9 +374,7 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) dfire_score_mixed_ker
       __syncthreads();
       const int* tl = sorted ? tord : tlist;
       double acc = 0.0;           // per-lane FP64 sum of table values
-      double pv[2 * kSteps];      // values gathered by the previous block, added by the next
-#pragma unroll
-      for (int u = 0; u < 2 * kSteps; ++u) pv[u] = 0.0;
+      double pv[2] = {0.0, 0.0};  // values gathered by the previous step, added by the next
       const double* table = L.table64;
       unsigned pose_pairs = 0, pose_evals = 0;  // of this warp's tiles (pairs per lane)
 
@@ -477,11 +474,11 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) dfire_score_mixed_ker
               ncand = rest;
               __syncwarp();
               more = ncand > 0 || cm != 0 || cb < nlc;
-            } while (more && longest <= kList - 32 - kBlock);
-            // each list is padded with the far atom to whole blocks
+            } while (more && longest <= kList - 32 - kRow);
+            // each list is padded with the far atom to whole steps
 #pragma unroll
             for (int g = 0; g < kGroups; ++g) {
-              if (lane < kBlock) W.list[g][cnt[g] + lane] = (unsigned short)nls;
+              if (lane < kRow) W.list[g][cnt[g] + lane] = (unsigned short)nls;
               nevals += cnt[g] * __popc((act_mask >> (g * kGroup)) & 255u);
             }
             __syncwarp();
@@ -493,22 +490,17 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) dfire_score_mixed_ker
               const double* row1 = table + __float_as_int(r1.w);
               const unsigned short* list = W.list[g] + lane / 4;
               const int n = (int)(counts & 255u);
-              float far = 0.f;
-              for (int c = 0; c < n; c += kBlock) {
-                float d2[kSteps][2], mid[kSteps][2];
-                const double* at[kSteps][2];
+              unsigned near_steps = 0;  // steps of this list with a pair of this lane near an edge, the first highest
+              for (int c = 0; c < n; c += kRow) {
+                const float4 l = lig[list[c]];
+                float d2[2], mid[2];
+                int bin[2];
+                pair_terms(rx, ry, rz, l, d2, mid, bin);
+                near_steps += near_steps + (fmaxf(fabsf(mid[0]), fabsf(mid[1])) >= inner ? 1u : 0u);
+                const double* at[2] = {row0 + (__float_as_int(l.w) + bin[0]), row1 + (__float_as_int(l.w) + bin[1])};
 #pragma unroll
-                for (int u = 0; u < kSteps; ++u) {
-                  const float4 l = lig[list[c + u * kRow]];
-                  int bin[2];
-                  pair_terms(rx, ry, rz, l, d2[u], mid[u], bin);
-                  far = fmaxf(far, fmaxf(fabsf(mid[u][0]), fabsf(mid[u][1])));
-                  at[u][0] = row0 + (__float_as_int(l.w) + bin[0]);
-                  at[u][1] = row1 + (__float_as_int(l.w) + bin[1]);
-                }
-#pragma unroll
-                for (int u = 0; u < 2 * kSteps; ++u) {
-                  acc += pv[u];
+                for (int h = 0; h < 2; ++h) {
+                  acc += pv[h];
                   // a pair inside the cutoff and away from a bin's edge: its value, through L2 only (each
                   // is used once, and cached in L1 it would evict the atom and mode lines that the next
                   // tiles read again)
@@ -519,27 +511,29 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) dfire_score_mixed_ker
                       "mov.f64 %0, 0d0000000000000000;\n\t"
                       "@p ld.global.cg.f64 %0, [%6];\n\t"
                       "@p add.u32 %1, %1, 1;\n\t}"
-                      : "=&d"(pv[u]), "+r"(npairs)
-                      : "f"(d2[u >> 1][u & 1]), "f"(cut2), "f"(mid[u >> 1][u & 1]), "f"(inner), "l"(at[u >> 1][u & 1]));
+                      : "=&d"(pv[h]), "+r"(npairs)
+                      : "f"(d2[h]), "f"(cut2), "f"(mid[h]), "f"(inner), "l"(at[h]));
                 }
               }
-              if (__any_sync(0xffffffffu, far >= inner)) {
-                // some pair of the group is near an edge (one group in about ten): find such pairs again
-                for (int c = 0; c < n; c += kRow) {
-                  const int s = list[c];
-                  const float4 l = lig[s];
-                  float d2[2], mid[2];
-                  int bin[2];
-                  pair_terms(rx, ry, rz, l, d2, mid, bin);
+              near_steps = __reduce_or_sync(0xffffffffu, near_steps);
+              const int last = (n - 1) / kRow;  // below 32: kList / kRow steps at most
+              while (near_steps) {
+                // a step with such a pair (about twelve of a pose): find the pairs again
+                const int b = 31 - __clz(near_steps);
+                near_steps ^= 1u << b;
+                const int s = list[(last - b) * kRow];
+                const float4 l = lig[s];
+                float d2[2], mid[2];
+                int bin[2];
+                pair_terms(rx, ry, rz, l, d2, mid, bin);
 #pragma unroll
-                  for (int h = 0; h < 2; ++h) {
-                    const bool near = d2[h] <= cut2 && fabsf(mid[h]) >= inner;
-                    const unsigned nm = __ballot_sync(0xffffffffu, near);
-                    const unsigned place = nnear + __popc(nm & lt_mask);
-                    if (near && place < kNear)
-                      W.near[place] = (unsigned)s * 32u + (unsigned)(g * kGroup + (lane & 3) + 4 * h);
-                    nnear += __popc(nm);
-                  }
+                for (int h = 0; h < 2; ++h) {
+                  const bool near = d2[h] <= cut2 && fabsf(mid[h]) >= inner;
+                  const unsigned nm = __ballot_sync(0xffffffffu, near);
+                  const unsigned place = nnear + __popc(nm & lt_mask);
+                  if (near && place < kNear)
+                    W.near[place] = (unsigned)s * 32u + (unsigned)(g * kGroup + (lane & 3) + 4 * h);
+                  nnear += __popc(nm);
                 }
               }
             }
@@ -555,20 +549,17 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) dfire_score_mixed_ker
             // coordinates so large that FP32 decides nothing: the whole tile in FP64
             npairs = 0;
             acc = 0.0;
-#pragma unroll
-            for (int u = 0; u < 2 * kSteps; ++u) pv[u] = 0.0;
+            pv[0] = pv[1] = 0.0;
             if (active)
               for (int s = 0; s < nls; ++s)
                 if (C.l_perm[s] >= 0) acc += decide_pair(C, Q.pose, Q.q, Q.qi, sh_T, table, slot, s, sh_cnt);
           }
           __syncwarp();
-          // the tile's energy: the last block's gathers, then the lane sums in a fixed shuffle order,
+          // the tile's energy: the last step's gathers, then the lane sums in a fixed shuffle order,
           // into the tile's slot
-#pragma unroll
-          for (int u = 0; u < 2 * kSteps; ++u) {
-            acc += pv[u];
-            pv[u] = 0.0;
-          }
+          acc += pv[0];
+          acc += pv[1];
+          pv[0] = pv[1] = 0.0;
           double v = acc;
           for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
           if (lane == 0) tsum[p * tstride + k] = v;
