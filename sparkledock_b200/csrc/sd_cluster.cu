@@ -34,31 +34,43 @@ namespace sd {
 namespace {
 
 constexpr int kClusterThreads = 512;
+constexpr int kMatPoses = 4;
 constexpr int kLoads = 16;  // coordinates of each of two poses in flight per lane
 
-// coordinates [ns][G][nbb][3] of the backbone atoms of swarms s0 .. s0+ns-1 (receptor first)
-__global__ void materialise_backbone_kernel(const DevComplex* cplx, int ci, int s0, int ns, const int* rb_idx,
-                                            int nbr, const int* lb_idx, int nbl, double* out) {
+// coordinates [ns][G][nbb][3] of the backbone atoms of swarms s0 .. s0+ns-1 (receptor first).  A thread
+// takes an atom of kMatPoses consecutive glowworms: the backbone's slots are scattered, so each of an
+// atom's mode components is a sector of its own, and one read serves them all.  Measured on 402 x 200
+// glowworms x 534 atoms, the whole clustering call: 7.3 ms with one pose a thread, 4.4 ms with four, 4.3 ms
+// with eight; 130 x 200 x 154: 0.58, 0.46, 0.51 ms
+__global__ void __launch_bounds__(256) materialise_backbone_kernel(const DevComplex* cplx, int ci, int s0, int ns,
+                                                                   const int* rb_idx, int nbr, const int* lb_idx,
+                                                                   int nbl, double* out) {
   const DevComplex& C = cplx[ci];
-  const int nbb = nbr + nbl, G = C.G, nslots = nslots_of(C);
-  const long long total = (long long)ns * G * nbb;
+  const int nbb = nbr + nbl, n = ns * C.G, nslots = nslots_of(C);
+  const long long total = (long long)((n + kMatPoses - 1) / kMatPoses) * nbb;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
-    const int a = (int)(i % nbb);
-    const long long gg = i / nbb;  // glowworm within the chunk
-    const double* pose = C.pos + ((size_t)s0 * G + (size_t)gg) * C.pl;
-    double x, y, z;
+    const int a = (int)(i % nbb), g0 = (int)(i / nbb) * kMatPoses;  // glowworms of the chunk
+    const double* pose[kMatPoses];
+    double r[kMatPoses][3];
+#pragma unroll
+    for (int p = 0; p < kMatPoses; ++p) pose[p] = C.pos + ((size_t)s0 * C.G + min(g0 + p, n - 1)) * C.pl;
     if (a < nbr) {
-      receptor_exact(C, nslots, C.r_slot[rb_idx[a]], pose, x, y, z);
+      anm_exact(C.r_xyz, C.r_modes, C.r_mask, nslots, C.nmr, pose, 7, C.r_slot[rb_idx[a]], r);
     } else {
-      double q[4] = {pose[3], pose[4], pose[5], pose[6]}, qi[4];
-      quat_inverse(q, qi);
-      ligand_exact(C, C.l_slot[lb_idx[a - nbr]], pose, q, qi, x, y, z);
+      anm_exact(C.l_xyz, C.l_modes, C.l_mask, C.nlchunks * SD_TILE, C.nml, pose, 7 + C.nmr,
+                C.l_slot[lb_idx[a - nbr]], r);
+#pragma unroll
+      for (int p = 0; p < kMatPoses; ++p) ligand_place(pose[p], r[p][0], r[p][1], r[p][2]);
     }
-    double* o = out + (size_t)i * 3;
-    o[0] = x;
-    o[1] = y;
-    o[2] = z;
+#pragma unroll
+    for (int p = 0; p < kMatPoses; ++p) {
+      if (g0 + p >= n) break;
+      double* o = out + ((size_t)(g0 + p) * nbb + a) * 3;
+      o[0] = r[p][0];
+      o[1] = r[p][1];
+      o[2] = r[p][2];
+    }
   }
 }
 

@@ -51,6 +51,42 @@ __device__ __forceinline__ void anm_exact(const double* xyz, const double* modes
   }
 }
 
+// the same of kP poses (extents from pose[p] + e0) with one read of the modes
+template <int kP>
+__device__ __forceinline__ void anm_exact(const double* xyz, const double* modes, const int* mask, int n, int nm,
+                                          const double* const (&pose)[kP], int e0, int slot, double (&r)[kP][3]) {
+  const size_t st = n;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double v = xyz[slot + d * st];
+#pragma unroll
+    for (int p = 0; p < kP; ++p) r[p][d] = v;
+  }
+  if (mask[slot] != 1) return;
+  const double* M = modes + slot;
+#pragma unroll 2
+  for (int m = 0; m < nm; ++m, M += 3 * st) {
+    const double mx = M[0], my = M[st], mz = M[2 * st];
+#pragma unroll
+    for (int p = 0; p < kP; ++p) {
+      const double e = pose[p][e0 + m];
+      r[p][0] += mx * e;
+      r[p][1] += my * e;
+      r[p][2] += mz * e;
+    }
+  }
+}
+
+// a displaced ligand atom rotated and translated into the pose
+__device__ __forceinline__ void ligand_place(const double* pose, double& x, double& y, double& z) {
+  double q[4] = {pose[3], pose[4], pose[5], pose[6]}, qi[4];
+  quat_inverse(q, qi);
+  quat_rotate(q, qi, x, y, z);
+  x += pose[0];
+  y += pose[1];
+  z += pose[2];
+}
+
 // receptor atom in tile slot `slot`, extents e_rec = pose + 7
 __device__ __forceinline__ void receptor_exact(const DevComplex& C, int nslots, int slot, const double* pose,
                                                double& x, double& y, double& z) {

@@ -227,11 +227,11 @@ struct MixedVariant {
 static const MixedVariant kMixedVariants[] = {
     SD_MIXED(12, 2), SD_MIXED(14, 2), SD_MIXED(8, 3), SD_MIXED(6, 4),
 };
-// the spill instantiation of the mixed kernel: variant 0's shape (the per-tile work, and so every
-// energy, is the same in every variant)
 // stateless calls with at most one pose per SM: one CTA per SM with as many warps as fit, for a pose's
 // time (16 poses of 3002 / 1274 atoms, the whole call: 193 us with 12 warps, 164 us with 24)
 static const MixedVariant kMixedFew = {(const void*)dfire_score_mixed_kernel<24, 1, false>, 24, 1};
+// the spill instantiation of the mixed kernel: variant 0's shape (the per-tile work, and so every
+// energy, is the same in every variant)
 static const MixedVariant kMixedSpill = {(const void*)dfire_score_mixed_kernel<12, 2, true>, 12, 2};
 
 // shapes of the culled FP64 kernel, the smallest CTAs first: they lose least where warps wait for each

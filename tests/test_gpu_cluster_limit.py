@@ -35,3 +35,21 @@ def test_rmsd_at_the_limit(n_lig, every, tables):
     for s, n in enumerate(ref["n_clusters"]):
         assert np.array_equal(got["rep"][s, :n], ref["rep"][s, :n])
         assert np.array_equal(got["size"][s, :n], ref["size"][s, :n])
+
+
+@pytest.mark.parametrize("n_swarms,glowworms,modes", [(1, 1, 10), (1, 3, 0), (3, 21, 7), (2, 130, 10)])
+def test_ragged_swarms(n_swarms, glowworms, modes, tables):
+    """Final poses in batches over swarm boundaries, the last one short; receptor and ligand atoms."""
+    cx = sd.SyntheticComplex(100, 70, n_swarms, glowworms, modes, modes, seed=glowworms)
+    rng = np.random.default_rng(glowworms)
+    poses = np.array(cx.poses)
+    poses[:, :, :3] = poses[:, :1, :3] + rng.normal(size=poses[:, :, :3].shape)  # some pairs within 4 A
+    rb, lb = (np.arange(100) % 3 == 0).astype(np.int32), (np.arange(70) % 2 == 0).astype(np.int32)
+    with sd.Docking([cx], tables, precision=sd.SD_PREC_FP64) as dk:
+        dk.init_state(0, poses)
+        st = dk.get_state(0)
+        st.scoring[:] = rng.normal(size=st.scoring.shape)
+        dk.set_state(0, st)
+        got = dk.cluster(0, rb, lb)
+    ref = oracle_cluster(OracleSystem(cx, tables), poses, st.scoring, rb, lb)
+    assert np.array_equal(got["n_clusters"], ref["n_clusters"]) and np.array_equal(got["member"], ref["member"])
