@@ -53,20 +53,20 @@ METRIC = "scored poses/s and GSO steps/s on 1 B200, mixed vs FP64 at <=1e-5 rel 
 L2_FLUSH_BYTES = 256 << 20
 # DRAM traffic of one mixed DFIRE scorer launch after the L2 flush, from ncu
 # dram__bytes_read.sum + dram__bytes_write.sum of three launches (4,098 / 5,658 / 6,483 poses
-# rescored) on the 3002 / 1274-atom complex with 40 swarms: a fixed part (the L2-resident tables
+# rescored) on the 3002 / 1274-atom complex with 40 swarms: a fixed part (the L2-resident table
 # and atom arrays read once per launch) plus a part per rescored pose (pose in, score and
 # reference point out), a least-squares fit, as summarised with the scorer's launch list under profiles/
-DRAM_BYTES_PER_LAUNCH = 9.12e6
-DRAM_BYTES_PER_SCORED_POSE = 212.0
+DRAM_BYTES_PER_LAUNCH = 6.88e6
+DRAM_BYTES_PER_SCORED_POSE = 265.0
 # warp-instructions the mixed scorer issues per receptor-ligand pair inside the cutoff, from ncu
 # smsp__inst_executed.sum of one launch (3002 / 1274 atoms, 4,098 poses, 233.9 M pairs in the
 # cutoff), as summarised with its full capture under profiles/; one ceiling of the scorer is the
 # SMs' issue rate (148 SMs x 4 schedulers x clock) over this count
-WARP_INSTR_PER_PAIR = 5.96
+WARP_INSTR_PER_PAIR = 4.60
 # L1 data-pipe wavefronts per in-cutoff pair in the same launch (l1tex__data_pipe_lsu_wavefronts:
-# 228.5 M shared-memory wavefronts plus ~181.6 M global-load ones, nearly all table gathers, over
+# 122.6 M shared-memory wavefronts plus ~174 M global-load ones, mostly table gathers, over
 # 233.9 M pairs); the pipe retires one wavefront per SM per cycle, the other ceiling
-L1_WAVEFRONTS_PER_PAIR = 1.75
+L1_WAVEFRONTS_PER_PAIR = 1.27
 
 
 def make_complexes(cfg, seed0=100):

@@ -13,7 +13,7 @@
 //    atom count, square root; no superposition.  Coordinates are the final poses through the
 //    exact FP64 transforms (receptor ANM; ligand ANM, rotation, translation), as the reference
 //    materialises them for its lightdock_<g>.pdb files.
-// GPU work: one thread per (glowworm, backbone atom) materialises the coordinates; one CTA per
+// GPU work: one thread per backbone atom of four glowworms materialises the coordinates; one CTA per
 // swarm sorts and clusters, one warp per existing cluster comparing the current glowworm with its
 // representative.  Only the decision rmsd <= 4 is needed: a warp adds the squared differences in any
 // order, and where that sum is further from 16 x atoms than its rounding can be (1e-9 of it, 10^3 times
