@@ -115,6 +115,9 @@ __global__ void __launch_bounds__(kClusterThreads) bsas_kernel(const DevComplex*
     const double* cur = sbb + (size_t)g * m;
     const int ncl = sh_ncl;
     for (int c = warp; c < ncl; c += kClusterThreads / 32) {
+      // a cluster behind one that the glowworm is in by now cannot be the first (looked at from a warp's
+      // second cluster on; 402 swarms with 123 clusters each: 11.8 -> 9.7 ms)
+      if (c != warp && __any_sync(0xffffffffu, *(volatile int*)&sh_hit < c)) break;
       const double* r = sbb + (size_t)crep[c] * m;
       double sum = 0.0;
       for (int a0 = lane; a0 < m; a0 += 32 * kLoads) {
