@@ -551,7 +551,7 @@ int make_score_plan(sd_ctx* c, int precision, int variant, ScorePlan& plan) {
 // complex alone: 15 us of queries), and the context's spill scratch sized to it; alloc = false refuses
 // that instead of allocating.
 int configure_score(sd_ctx* c, int precision, int variant, int* grid, size_t* smem, bool alloc = true) {
-  ScorePlan& plan = c->plan[precision][precision == SD_PREC_FP64_REF ? 0 : variant];
+  ScorePlan& plan = c->plan[precision][variant];
   if (!plan.grid) {
     int rc = make_score_plan(c, precision, variant, plan);
     if (rc) return rc;
