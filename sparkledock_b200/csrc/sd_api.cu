@@ -246,6 +246,9 @@ void slot_modes(const double* modes, int nm, int n, const std::vector<int>& slot
   }
 }
 
+// coordinates of padded slots: outside every cutoff, also where FP32 coordinates cannot tell
+constexpr double kFar = 1e150;
+
 int setup_complex(sd_ctx* c, const sd_complex_desc& d, ComplexHost& h, int gbase, int sbase) {
   DevComplex& D = h.d;
   memset(&D, 0, sizeof D);
@@ -266,7 +269,7 @@ int setup_complex(sd_ctx* c, const sd_complex_desc& d, ComplexHost& h, int gbase
   const int nslots = (int)slots.size();
   D.ntiles = nslots / SD_TILE;
   h.nslots = nslots;
-  std::vector<double> rxyz((size_t)nslots * 3, 0.0), rmodes((size_t)std::max(1, D.nmr) * nslots * 3, 0.0);
+  std::vector<double> rxyz((size_t)nslots * 3, kFar), rmodes((size_t)std::max(1, D.nmr) * nslots * 3, 0.0);
   std::vector<int> rmask(nslots, 0), rrow(nslots, 0), rlj(nslots, 0);
   std::vector<float> rq(nslots, 0.f);
   std::vector<float4> tiles(D.ntiles);
@@ -375,7 +378,7 @@ int setup_complex(sd_ctx* c, const sd_complex_desc& d, ComplexHost& h, int gbase
       lch[t] = make_float4(cf[0], cf[1], cf[2], round_up_f(rad * (1 + 1e-6) + 1e-4));
     }
     const size_t nls = lslots.size();
-    std::vector<double> cxyz(nls * 3, 0.0), cmodes((size_t)std::max(1, D.nml) * nls * 3, 0.0);
+    std::vector<double> cxyz(nls * 3, kFar), cmodes((size_t)std::max(1, D.nml) * nls * 3, 0.0);
     std::vector<int> cmask(nls, 0), ccol(nls, 0), clj(nls, 0), slot_of(d.n_lig, 0);
     std::vector<float> cq(nls, 0.f);
     for (size_t s = 0; s < nls; ++s) {

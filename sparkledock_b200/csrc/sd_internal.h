@@ -63,7 +63,7 @@ struct DevComplex {
   int nr, nl, nmr, nml, S, G, pl;
   int ntiles;           // receptor tiles of SD_TILE slots
   int gbase, sbase;     // first global glowworm / swarm index of this complex
-  // receptor in tile order (slot = tile*32 + lane); padded slots have orig = -1
+  // receptor in tile order (slot = tile*32 + lane); padded slots far away, with r_orig = -1
   const int* r_orig;
   const int* r_slot;       // [nr] original receptor index -> slot
   const double* r_xyz;     // [3][nslots]
@@ -73,7 +73,7 @@ struct DevComplex {
   const float4* r_tile;    // [ntiles] centre (rest frame) + radius
   const float* r_q;        // [nslots] charge (pyDock)
   const int* r_lj;         // [nslots] LJ type (pyDock)
-  // ligand in spatial chunks of 32 (slot = chunk*32 + lane; padded slots 0, with l_perm = -1)
+  // ligand in spatial chunks of 32 (slot = chunk*32 + lane; padded slots far away, with l_perm = -1)
   int nlchunks;
   const int* l_perm;       // [nlchunks*32] slot -> original ligand index, or -1
   const int* l_slot;       // [nl] original ligand index -> slot

@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) dfire_score_fp64_kern
     const int* tl = sorted ? tord : tlist;
     const double tx = Q.pose[0], ty = Q.pose[1], tz = Q.pose[2];
     const float cut2 = 225.0f + Q.B, box_cut = 225.1f + Q.B, inner = settled_half(Q.B);
+    const bool settled = inner > 0.f;  // else every listed pair is decided in FP64
     unsigned pose_pairs = 0, pose_evals = 0;
 
     for (;;) {
@@ -216,17 +217,19 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) dfire_score_fp64_kern
             pair_terms(pack2(r0.x, r1.x), pack2(r0.y, r1.y), pack2(r0.z, r1.z), l, d2, mid, bin);
             double val[2];
             const bool ok0 = d2[0] <= cut2, ok1 = d2[1] <= cut2;
-            const bool near0 = ok0 && fabsf(mid[0]) >= inner, near1 = ok1 && fabsf(mid[1]) >= inner;
+            const bool near0 = (ok0 && fabsf(mid[0]) >= inner) || !settled,
+                       near1 = (ok1 && fabsf(mid[1]) >= inner) || !settled;
             const int i0 = __float_as_int(r0.w) + __float_as_int(l.w) + bin[0],
                       i1 = __float_as_int(r1.w) + __float_as_int(l.w) + bin[1];
             val[0] = ok0 && !near0 ? __ldcg(table + i0) : 0.0;
             val[1] = ok1 && !near1 ? __ldcg(table + i1) : 0.0;
             pose_pairs += (ok0 && !near0) + (ok1 && !near1);
             if (__any_sync(0xffffffffu, near0 || near1)) {
-              if (near0)
+              // (not the padding of the lists: unsettled, it is listed and near)
+              if (near0 && j < C.nl)
                 val[0] = decide_pair(C, Q.pose, Q.q, Q.qi, sh_T, table, k * SD_TILE + g * kGroup + (lane & 3),
                                      C.l_slot[j], sh_cnt);
-              if (near1)
+              if (near1 && j < C.nl)
                 val[1] = decide_pair(C, Q.pose, Q.q, Q.qi, sh_T, table, k * SD_TILE + g * kGroup + (lane & 3) + 4,
                                      C.l_slot[j], sh_cnt);
             }

@@ -216,7 +216,9 @@ __device__ __forceinline__ float box_distance2(const float4* box, int g, const f
 
 // half a bin less the bin coordinate's error: |d_fp32 - d| <= B / 30 inside the cutoff (B bounds d^2
 // there, its leading term is 2 d |error of the difference vector|), times the slope 2, plus FP32
-// roundings (square root 2^-22, coordinate up to 20).  Not above 0: no pair is settled in FP32
+// roundings (square root 2^-22, coordinate up to 20).  Not above 0 (atoms 5e5 A and more from t, up to a bound
+// that is infinite): no pair is settled in FP32, where a coordinate need not be finite and the far atoms that
+// fill the lists up are no longer far
 __device__ __forceinline__ float settled_half(float B) { return 0.5f - (B * 0.0673f + 2e-5f); }
 
 }  // namespace
@@ -540,13 +542,13 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) dfire_score_mixed_ker
             __syncwarp();
           } while (more);
           __syncwarp();
-          if (nnear <= kNear) {
+          if (nnear <= kNear && inner > 0.f) {
             for (int i = lane; i < (int)nnear; i += 32) {
               const unsigned e = W.near[i];
               acc += decide_pair(C, Q.pose, Q.q, Q.qi, sh_T, table, k * SD_TILE + (int)(e & 31), (int)(e >> 5), sh_cnt);
             }
           } else {
-            // coordinates so large that FP32 decides nothing: the whole tile in FP64
+            // too many, or coordinates so large that FP32 settles nothing: the whole tile in FP64
             npairs = 0;
             acc = 0.0;
             pv[0] = pv[1] = 0.0;
