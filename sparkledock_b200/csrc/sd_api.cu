@@ -152,6 +152,7 @@ struct sd_ctx {
   int score_poses = 1;       // poses per CTA of the last configured scorer launch
   // autotuner state (mixed-precision DFIRE kernel variants)
   int mixed_variant = 0;
+  int wide = 0;            // SD_WIDE when a ligand reaches far (DFIRE): part of the mixed kernel's variant
   int smem_sm = 0;         // shared memory of an SM
   bool tuned = false;
   double tune_ms[SD_MAX_VARIANTS] = {};
@@ -554,7 +555,7 @@ int make_score_plan(sd_ctx* c, int precision, int variant, ScorePlan& plan) {
 // complex alone: 15 us of queries), and the context's spill scratch sized to it; alloc = false refuses
 // that instead of allocating.
 int configure_score(sd_ctx* c, int precision, int variant, int* grid, size_t* smem, bool alloc = true) {
-  ScorePlan& plan = c->plan[precision][variant];
+  ScorePlan& plan = c->plan[precision][variant & ~SD_WIDE];
   if (!plan.grid) {
     int rc = make_score_plan(c, precision, variant, plan);
     if (rc) return rc;
@@ -585,7 +586,7 @@ int score_variant(const sd_ctx* c, int precision, int poses, bool stateless) {
   }
   const size_t cta = score_smem_bytes(precision, c->scoring, c->max_nr, c->max_nl, 1) +
                      (few ? score_warp_bytes(precision, c->scoring, SD_FEW, false) : 0) + 12288;
-  return few && cta <= (size_t)c->smem_optin ? SD_FEW : c->mixed_variant;
+  return (few && cta <= (size_t)c->smem_optin ? SD_FEW : c->mixed_variant) | (precision == SD_PREC_MIXED ? c->wide : 0);
 }
 
 // the spill scratch of the last configured launch (null pointers when it uses shared memory)
@@ -672,7 +673,7 @@ int autotune_mixed(sd_ctx* c) {
   for (int v = 0; v < nv && v < SD_MAX_VARIANTS; ++v) {
     int grid;
     size_t sm;
-    if (configure_score(c, SD_PREC_MIXED, v, &grid, &sm) != SD_OK) {
+    if (configure_score(c, SD_PREC_MIXED, v | c->wide, &grid, &sm) != SD_OK) {
       c->tune_ms[v] = -1;
       continue;
     }
@@ -687,7 +688,7 @@ int autotune_mixed(sd_ctx* c) {
       ctl.grab[0] = ctl.grab[1] = 0;
       SD_CUDA(cudaMemcpyAsync(c->d_ctl_scratch, &ctl, sizeof ctl, cudaMemcpyHostToDevice, c->stream));
       SD_CUDA(cudaEventRecord(e0, c->stream));
-      if ((rc = score_launch(L, SD_PREC_MIXED, c->scoring, grid, sm, c->stream, v, false)))
+      if ((rc = score_launch(L, SD_PREC_MIXED, c->scoring, grid, sm, c->stream, v | c->wide, false)))
         return fail(rc, std::string("autotune launch: ") + cudaGetErrorString(cudaGetLastError()));
       SD_CUDA(cudaEventRecord(e1, c->stream));
       SD_CUDA(cudaEventSynchronize(e1));
@@ -866,6 +867,7 @@ int sd_ctx_create(const sd_complex_desc* complexes, int n_complexes, const sd_ta
     c->max_nr = std::max(c->max_nr, complexes[i].n_rec);
     c->max_nl = std::max(c->max_nl, complexes[i].n_lig);
     c->max_G = std::max(c->max_G, complexes[i].n_glowworms);
+    if (scoring == SD_SCORING_DFIRE && wide_ligand(c->cx[i].d.lig_radius)) c->wide = SD_WIDE;
   }
   c->total_glowworms = gbase;
   c->total_swarms = sbase;

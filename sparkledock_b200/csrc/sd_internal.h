@@ -27,6 +27,7 @@
 #define SD_CULL_MARGIN 0.05f    /* A, covers FP32 rounding of the conservative culling tests */
 #define SD_MAX_VARIANTS 16      /* compiled variants of the mixed DFIRE kernel (autotuner) */
 #define SD_FEW SD_MAX_VARIANTS  /* the kernels' variant for at most one pose per SM (not tuned) */
+#define SD_WIDE 32              /* added to a variant of the mixed DFIRE kernel: its form for far-reaching ligands */
 #define SD_NOALLOC_MAX_POSES 65536           /* poses per sd_score_poses_noalloc call */
 #define SD_NOALLOC_SCRATCH_BYTES (288 * 1024) /* its file-scope device scratch array */
 
@@ -162,6 +163,7 @@ int score_threads_of(int precision, int scoring, int variant, bool spill);
 int fp64_shape(int max_nr, int max_nl, int smem_sm, int poses, int nsm);
 const void* score_kernel_ptr(int precision, int scoring, int variant, bool spill);
 int mixed_variant_count();
+bool wide_ligand(float radius);
 int mixed_variant_warps(int v);
 int mixed_variant_min_blocks(int v);
 int gso_launch(const GsoLaunch& L, int threads, cudaStream_t st);

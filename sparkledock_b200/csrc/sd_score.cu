@@ -216,7 +216,8 @@ struct MixedVariant {
   int warps;
   int min_blocks;
 };
-#define SD_MIXED(W, B) { (const void*)dfire_score_mixed_kernel<W, B, false>, W, B }
+#define SD_MIXED(W, B) { (const void*)dfire_score_mixed_kernel<W, B, false, false>, W, B }
+#define SD_MIXED_WIDE(W, B) { (const void*)dfire_score_mixed_kernel<W, B, false, true>, W, B }
 // 24 or 28 warps per SM in all of them (80 or 72 registers a thread).  Fewer and larger CTAs hold fewer
 // copies of the ligand in shared memory and leave L1 more room for gathers in flight; smaller ones
 // lose less at the end of a batch.  Measured (M poses/s for 12x2, 14x2, 8x3, 6x4): 757/481 atoms 7.4,
@@ -227,12 +228,15 @@ struct MixedVariant {
 static const MixedVariant kMixedVariants[] = {
     SD_MIXED(12, 2), SD_MIXED(14, 2), SD_MIXED(8, 3), SD_MIXED(6, 4),
 };
+static const MixedVariant kMixedWide[] = {
+    SD_MIXED_WIDE(12, 2), SD_MIXED_WIDE(14, 2), SD_MIXED_WIDE(8, 3), SD_MIXED_WIDE(6, 4),
+};
 // stateless calls with at most one pose per SM: one CTA per SM with as many warps as fit, for a pose's
 // time (16 poses of 3002 / 1274 atoms, the whole call: 193 us with 12 warps, 164 us with 24)
-static const MixedVariant kMixedFew = {(const void*)dfire_score_mixed_kernel<24, 1, false>, 24, 1};
+static const MixedVariant kMixedFew = SD_MIXED(24, 1), kMixedFewWide = SD_MIXED_WIDE(24, 1);
 // the spill instantiation of the mixed kernel: variant 0's shape (the per-tile work, and so every
 // energy, is the same in every variant)
-static const MixedVariant kMixedSpill = {(const void*)dfire_score_mixed_kernel<12, 2, true>, 12, 2};
+static const MixedVariant kMixedSpill = {(const void*)dfire_score_mixed_kernel<12, 2, true, true>, 12, 2};
 
 // shapes of the culled FP64 kernel, the smallest CTAs first: they lose least where warps wait for each
 // other at a pose's end, and the first whose CTAs are all resident for the context's largest complex is
@@ -253,11 +257,21 @@ static const MixedVariant kFp64Spill = {(const void*)dfire_score_fp64_kernel<12,
 constexpr int kNumFp64Shapes = sizeof(kFp64Shapes) / sizeof(kFp64Shapes[0]);
 
 constexpr int kNumMixedVariants = sizeof(kMixedVariants) / sizeof(kMixedVariants[0]);
+static_assert(sizeof(kMixedWide) == sizeof(kMixedVariants), "wide forms of all variants");
 static_assert(kNumMixedVariants <= SD_MAX_VARIANTS, "variant table");
 
 static const MixedVariant& mixed_variant(int v) {
-  return v == SD_FEW ? kMixedFew : kMixedVariants[v < 0 || v >= kNumMixedVariants ? 0 : v];
+  const bool wide = (v & SD_WIDE) != 0;
+  v &= ~SD_WIDE;
+  if (v == SD_FEW) return wide ? kMixedFewWide : kMixedFew;
+  if (v >= kNumMixedVariants) v = 0;
+  return wide ? kMixedWide[v] : kMixedVariants[v];
 }
+
+// whether tiles may meet more than kNear pairs near an edge: their share of the pairs grows with the ligand's
+// radius (1.8e-4 at 64 A, and a tile in an overlapping pose meets 12,800 pairs at most, so 2 of them; compact
+// ligands have 24 A at 1,274 atoms and 60 A at 20,000)
+bool wide_ligand(float radius) { return !(radius <= 64.f); }
 
 // bytes of the scorer's per-warp buffers, in dynamic shared memory in front of the per-pose arrays
 // (alone there in the spill instantiation)

@@ -47,8 +47,9 @@ constexpr int kGroups = SD_TILE / kGroup;
 constexpr int kRow = 8;               // candidates of a step: 8 rows of 4 lanes, two atoms of the group per lane
 constexpr int kPoses = 2;             // poses of a batch: they share the reads of modes and tiles
 constexpr int kList = 160;            // candidates of a group between two drains of the lists
-constexpr int kNear = 16;             // pairs of a tile that may be decided in FP64 one by one
+constexpr int kNear = 16;             // pairs of a tile decided in FP64 side by side (more: decide_near)
 static_assert(kList / kRow <= 32, "a bit per step");
+static_assert(kGroups * kList * 2 >= 64 * 4, "decide_near collects up to 63 pairs in the lists");
 constexpr float kMagic = 12582912.0f; // 1.5 * 2^23: adding it rounds to an integer in the low bits
 constexpr int kMagicBits = 0x4B400000;
 
@@ -221,13 +222,72 @@ __device__ __forceinline__ float box_distance2(const float4* box, int g, const f
 // fill the lists up are no longer far
 __device__ __forceinline__ float settled_half(float B) { return 0.5f - (B * 0.0673f + 2e-5f); }
 
+// The near pairs of a tile that has more than kNear of them, found again (one lane per receptor atom, the tile's
+// candidates in turn) and decided 32 side by side; buf: the warp's lists, which are done with by then.  600
+// poses of 3002 / 1274 atoms, the ligand moved away from its origin by 500, 4,000 and 16,000 A: 0.49, 0.79 and
+// 1.02 ms; 6.0, 50 and 92 ms with every pair of such tiles in FP64
+__device__ __noinline__ double decide_near(const DevComplex& C, const PoseBufs& Q, const float4* lig, const float4* chS,
+                                           const float4* rec, unsigned* buf, int k, const double* T,
+                                           const double* table, unsigned long long* cnt) {
+  const int lane = threadIdx.x & 31;
+  const float4 tile = C.r_tile[k], own = rec[lane];
+  const float cx = (float)((double)tile.x - Q.pose[0]), cy = (float)((double)tile.y - Q.pose[1]),
+              cz = (float)((double)tile.z - Q.pose[2]);
+  const float reach = 15.0f + Q.dR + SD_CULL_MARGIN + tile.w;
+  const float cut2 = 225.0f + Q.B, inner = settled_half(Q.B);
+  const float2x rx = pack2(own.x, own.x), ry = pack2(own.y, own.y), rz = pack2(own.z, own.z);
+  double v = 0.0;
+  int n = 0;
+  auto decide = [&]() {
+    __syncwarp();
+    if (lane < n)
+      v += decide_pair(C, Q.pose, Q.q, Q.qi, T, table, k * SD_TILE + (int)(buf[lane] & 31), (int)(buf[lane] >> 5), cnt);
+    __syncwarp();
+  };
+  for (int cb = 0; cb < C.nlchunks; cb += 32) {
+    bool cnear = false;
+    if (cb + lane < C.nlchunks) {
+      const float4 ch = chS[cb + lane];
+      const float ex = ch.x - cx, ey = ch.y - cy, ez = ch.z - cz, r = reach + ch.w;
+      cnear = ex * ex + ey * ey + ez * ez <= r * r;
+    }
+    for (unsigned cm = __ballot_sync(0xffffffffu, cnear); cm; cm &= cm - 1) {
+      const int sb = (cb + __ffs(cm) - 1) * SD_TILE;
+      const float4 la = lig[sb + lane];
+      const float ax = la.x + cx, ay = la.y + cy, az = la.z + cz;
+      const bool cand = fmaf(az, az, fmaf(ay, ay, ax * ax)) <= reach * reach;
+      for (unsigned am = __ballot_sync(0xffffffffu, cand); am; am &= am - 1) {
+        const int s = sb + __ffs(am) - 1;
+        float d2[2], mid[2];
+        int bin[2];
+        pair_terms(rx, ry, rz, lig[s], d2, mid, bin);
+        const bool near = d2[0] <= cut2 && fabsf(mid[0]) >= inner;
+        const unsigned nm = __ballot_sync(0xffffffffu, near);
+        if (near) buf[n + __popc(nm & ((1u << lane) - 1u))] = (unsigned)s * 32u + (unsigned)lane;
+        n += __popc(nm);
+        if (n >= 32) {
+          decide();
+          n -= 32;
+          const unsigned rest = lane < n ? buf[32 + lane] : 0u;
+          __syncwarp();
+          if (lane < n) buf[lane] = rest;
+        }
+      }
+    }
+  }
+  decide();
+  return v;
+}
+
 }  // namespace
 
 // Variants differ only in warps per CTA and resident CTAs per SM: a tile is always processed by
 // one warp in the same way, so they give identical energies.  kSpill: the per-pose arrays (tile
 // sums, transformed ligand, chunk spheres, tile lists) live in this CTA's slice of the global
-// scratch L.spill, for complexes too large for shared memory; the arithmetic is the same.
-template <int kWarps, int kMinBlocks, bool kSpill>
+// scratch L.spill, for complexes too large for shared memory; the arithmetic is the same.  kWide: for
+// ligands that reach far (wide_ligand), with decide_near, which costs the pair loop registers: 8,000 poses of
+// 3002 / 1274 atoms 2.89 -> 2.93 ms, 3,000 of 17307 / 1125 1.39 -> 1.41 ms
+template <int kWarps, int kMinBlocks, bool kSpill, bool kWide>
 __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) dfire_score_mixed_kernel(ScoreLaunch L) {
   constexpr int kSortMax = 512;        // near tiles ordered largest-first up to this many
   extern __shared__ __align__(16) unsigned char smem_dyn[];
@@ -542,13 +602,15 @@ __global__ void __launch_bounds__(kWarps * 32, kMinBlocks) dfire_score_mixed_ker
             __syncwarp();
           } while (more);
           __syncwarp();
-          if (nnear <= kNear && inner > 0.f) {
+          if (kWide && nnear > kNear && inner > 0.f) {
+            acc += decide_near(C, Q, lig, chS + p * nlc, rec, (unsigned*)W.list, k, sh_T, table, sh_cnt);
+          } else if (nnear <= kNear && inner > 0.f) {
             for (int i = lane; i < (int)nnear; i += 32) {
               const unsigned e = W.near[i];
               acc += decide_pair(C, Q.pose, Q.q, Q.qi, sh_T, table, k * SD_TILE + (int)(e & 31), (int)(e >> 5), sh_cnt);
             }
           } else {
-            // too many, or coordinates so large that FP32 settles nothing: the whole tile in FP64
+            // coordinates so large that FP32 settles nothing (without kWide also too many pairs): the whole tile in FP64
             npairs = 0;
             acc = 0.0;
             pv[0] = pv[1] = 0.0;
