@@ -130,6 +130,12 @@ __device__ __forceinline__ void anm_fused(const double* xyz, const double* modes
   }
 }
 
+// half extent of a group's box on an axis, wider by what the box test may lose in FP32 (three roundings of
+// 2^-24 of the largest coordinate: centre, extent and difference); -inf stays for an empty group (lo > hi)
+__device__ __forceinline__ float half_extent(float lo, float hi) {
+  return fmaf(5e-7f, fmaxf(fabsf(lo), fabsf(hi)), 0.5f * (hi - lo));
+}
+
 __device__ __forceinline__ int nslots_of(const DevComplex& C) { return C.ntiles * SD_TILE; }
 
 }  // namespace sd

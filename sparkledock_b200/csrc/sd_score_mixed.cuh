@@ -203,7 +203,7 @@ __device__ __forceinline__ void group_boxes(const float4& own, bool active, int 
   if ((lane & (kGroup - 1)) == 0) {
     box[2 * (lane / kGroup)] = make_float4(0.5f * (lo[0] + hi[0]), 0.5f * (lo[1] + hi[1]), 0.5f * (lo[2] + hi[2]), 0.f);
     box[2 * (lane / kGroup) + 1] =
-        make_float4(0.5f * (hi[0] - lo[0]), 0.5f * (hi[1] - lo[1]), 0.5f * (hi[2] - lo[2]), 0.f);
+        make_float4(half_extent(lo[0], hi[0]), half_extent(lo[1], hi[1]), half_extent(lo[2], hi[2]), 0.f);
   }
 }
 
