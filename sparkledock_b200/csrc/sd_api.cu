@@ -138,6 +138,7 @@ struct sd_ctx {
   // per-CTA global scratch of the spill instantiations (complexes too large for shared memory)
   DevBuf s_spill;
   ScorePlan plan[3][SD_MAX_VARIANTS + 1], grad_plan[3][2];
+  int few_fit[3] = {-1, -1, -1}, few_grad_fit[3] = {-1, -1, -1};  // by precision; see few_fits
   void* h_stage = nullptr; // pinned, for small downloads
   int* d_flag = nullptr;
   int smem_optin = 0;      // shared memory a CTA may use on this device (opt-in maximum)
@@ -576,17 +577,29 @@ int configure_score(sd_ctx* c, int precision, int variant, int* grid, size_t* sm
 // the few-poses shapes: at most one pose per SM, and receptors with a tile for most of the 24 warps
 bool few_poses(const sd_ctx* c, int poses) { return poses <= c->nsm && c->max_nr > 20 * SD_TILE; }
 
+// whether kernel k's few-poses shape fits in a CTA's shared memory with `dynamic` bytes beside its static arrays;
+// known: the answer, kept (-1: not asked yet)
+bool few_fits(const sd_ctx* c, const void* k, size_t dynamic, int* known) {
+  if (*known < 0) {
+    cudaFuncAttributes fa;
+    *known = cudaFuncGetAttributes(&fa, k) == cudaSuccess && dynamic + fa.sharedSizeBytes <= (size_t)c->smem_optin;
+  }
+  return *known != 0;
+}
+
 // the compiled variant of a precision's kernel for a launch of at most `poses` poses; stateless: not a
 // GSO step, whose mixed variant the autotuner chose on its own poses
-int score_variant(const sd_ctx* c, int precision, int poses, bool stateless) {
+int score_variant(sd_ctx* c, int precision, int poses, bool stateless) {
   bool few = few_poses(c, poses);
   if (c->scoring == SD_SCORING_DFIRE) {
     if (precision == SD_PREC_FP64) return fp64_shape(c->max_nr, c->max_nl, c->smem_sm, poses, c->nsm);
     few &= precision == SD_PREC_MIXED && stateless;
   }
-  const size_t cta = score_smem_bytes(precision, c->scoring, c->max_nr, c->max_nl, 1) +
-                     (few ? score_warp_bytes(precision, c->scoring, SD_FEW, false) : 0) + 12288;
-  return (few && cta <= (size_t)c->smem_optin ? SD_FEW : c->mixed_variant) | (precision == SD_PREC_MIXED ? c->wide : 0);
+  const int wide = precision == SD_PREC_MIXED ? c->wide : 0;
+  few = few && few_fits(c, score_kernel_ptr(precision, c->scoring, SD_FEW | wide, false),
+                        score_smem_bytes(precision, c->scoring, c->max_nr, c->max_nl, 1) +
+                            score_warp_bytes(precision, c->scoring, SD_FEW, false), &c->few_fit[precision]);
+  return (few ? SD_FEW : c->mixed_variant) | wide;
 }
 
 // the spill scratch of the last configured launch (null pointers when it uses shared memory)
@@ -1259,9 +1272,10 @@ int sd_pydock_grad(sd_ctx* c, int ci, const double* poses, int n, int precision,
   SD_CUDA(cudaMemcpyAsync(c->s_pose.p, poses, (size_t)n * D.pl * 8, cudaMemcpyHostToDevice, c->stream));
   if ((rc = stateless_prepare_launch(c->d_ctl_scratch, c->d_cplx_scratch, S, (int*)c->s_work.p, ci, n, c->stream)))
     return fail(rc, "stateless call: prepare kernel launch failed");
-  const bool few = few_poses(c, n) && pydock_smem_bytes(precision, true, c->max_nl, c->max_nr) +
-                                              pydock_warp_bytes(precision, true, true) + 12288 <=
-                                          (size_t)c->smem_optin;
+  const bool few = few_poses(c, n) && few_fits(c, pydock_kernel_ptr(precision, true, false, true),
+                                               pydock_smem_bytes(precision, true, c->max_nl, c->max_nr) +
+                                                   pydock_warp_bytes(precision, true, true),
+                                               &c->few_grad_fit[precision]);
   ScorePlan& plan = c->grad_plan[precision][few];
   if (!plan.grid) {
     const size_t need = pydock_smem_bytes(precision, true, c->max_nl, c->max_nr);
