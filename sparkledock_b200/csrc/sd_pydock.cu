@@ -191,6 +191,7 @@ constexpr int kGroups = SD_TILE / SD_GROUP;
 constexpr int kRow = SD_GROUP / 2;         // lanes of a row: one candidate, two atoms of the group per lane
 constexpr int kRows = 32 / kRow;           // candidates of a step
 constexpr int kPdList = 128;               // candidates of a group between two drains of the lists
+constexpr int kOrderMax = 512;             // near tiles that are ordered by distance
 
 // a warp's tile
 template <class T>
@@ -292,16 +293,16 @@ pydock_kernel(ScoreLaunch L, double* out_grad) {
     const double tx = sh_pose[0], ty = sh_pose[1], tz = sh_pose[2];
     const float dR = sh_bound[0], dL = sh_bound[1];
     // per-pose arrays: ligand atoms [nls + 1] (the last a far atom, the padding), GRAD: their forces
-    // [words][3][nls + 4], chunk spheres [nlc], near tiles [ntiles] as found, in order of distance, and
-    // their distances, LJ types [nls + 1]
+    // [words][3][nls + 4], chunk spheres [nlc], near tiles [ntiles] as found, the same in order of distance
+    // and their distances (each [kOrderMax] at most: more are not ordered), LJ types [nls + 1]
     LigAtom<T>* la = reinterpret_cast<LigAtom<T>*>(smem);
     Force<T>* fx = reinterpret_cast<Force<T>*>(la + nls + 1);  // GRAD only
     const int fstride = nls + 4;
     float4* chS = reinterpret_cast<float4*>(fx + (GRAD ? Force<T>::kWords * 3 * fstride : 0));
     int* tlist = reinterpret_cast<int*>(chS + nlc);
     int* tord = tlist + C.ntiles;
-    float* tdist = reinterpret_cast<float*>(tord + C.ntiles);
-    unsigned char* llj = reinterpret_cast<unsigned char*>(tdist + C.ntiles);
+    float* tdist = reinterpret_cast<float*>(tord + min(C.ntiles, kOrderMax));
+    unsigned char* llj = reinterpret_cast<unsigned char*>(tdist + min(C.ntiles, kOrderMax));
     if (tid == 0) {
       la[nls] = LigAtom<T>{(T)1e17, (T)1e17, (T)1e17, T(0)};
       llj[nls] = 0;
@@ -336,14 +337,14 @@ pydock_kernel(ScoreLaunch L, double* out_grad) {
       if (dd <= reach * reach) {
         const int at = atomicAdd(&sh_ntile, 1);
         tlist[at] = k;
-        tdist[at] = dd;
+        if (at < kOrderMax) tdist[at] = dd;
       }
     }
     __syncthreads();
     const int ntile = sh_ntile;
     // the tiles closest to the ligand centre (t) have the most pairs: taken first, the warps finish a
     // pose together
-    const bool sorted = ntile <= 512;
+    const bool sorted = ntile <= kOrderMax;
     if (sorted) {
       for (int t = tid; t < ntile; t += blockDim.x) {
         const float d = tdist[t];
@@ -604,10 +605,11 @@ pydock_kernel(ScoreLaunch L, double* out_grad) {
 // bytes of a CTA's per-pose arrays, and of its warps' buffers in front of them (always shared memory)
 size_t pydock_smem_bytes(int precision, bool grad, int max_nl, int max_nr) {
   const size_t nlc = (size_t)(max_nl + SD_TILE - 1) / SD_TILE, nls = nlc * SD_TILE;
+  const size_t nt = (size_t)(max_nr + SD_TILE - 1) / SD_TILE;
   const size_t ts = precision == SD_PREC_MIXED ? 4 : 8;
   // forces: 24 bytes an atom in both types
   return ts * 4 * (nls + 1) + (grad ? 24 * (nls + 4) : 0) + 16 * nlc + (nls + 1) +
-         12 * ((max_nr + SD_TILE - 1) / SD_TILE) + 16;
+         4 * nt + 8 * std::min<size_t>(nt, kOrderMax) + 16;
 }
 size_t pydock_warp_bytes(int precision, bool grad, bool few) {
   const bool fp64 = precision != SD_PREC_MIXED;
