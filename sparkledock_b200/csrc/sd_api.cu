@@ -602,6 +602,22 @@ int score_variant(sd_ctx* c, int precision, int poses, bool stateless) {
   return (few ? SD_FEW : c->mixed_variant) | wide;
 }
 
+// At creation: the spill scratch of scorers whose per-pose arrays fit in a CTA's shared memory by themselves but
+// not beside its warps' buffers, so that the no-allocation call never needs an allocating one before it there.
+// (Where the arrays alone are too large it does.)
+int reserve_spill(sd_ctx* c) {
+  for (int precision : {SD_PREC_FP64_REF, SD_PREC_FP64, SD_PREC_MIXED}) {
+    const size_t need = score_smem_bytes(precision, c->scoring, c->max_nr, c->max_nl, 1);
+    const int variant = score_variant(c, precision, 1 << 24, false);
+    const size_t room = score_warp_bytes(precision, c->scoring, variant, false) + (16 << 10);  // static arrays included
+    if (need > (size_t)c->smem_optin || need + room <= (size_t)c->smem_optin) continue;
+    int grid, rc;
+    size_t smem;
+    if ((rc = configure_score(c, precision, variant, &grid, &smem))) return rc;
+  }
+  return SD_OK;
+}
+
 // the spill scratch of the last configured launch (null pointers when it uses shared memory)
 void set_spill(const sd_ctx* c, ScoreLaunch& L) {
   L.poses_per_cta = c->score_poses;
@@ -945,6 +961,7 @@ int sd_ctx_create(const sd_complex_desc* complexes, int n_complexes, const sd_ta
     if ((rc = cu(cudaMemcpy(c->d_ctl, &ctl, sizeof ctl, cudaMemcpyHostToDevice), "upload"))) return bail(rc);
   }
   if ((rc = push_descriptors(c))) return bail(rc);
+  if ((rc = reserve_spill(c))) return bail(rc);
   if ((rc = cu(cudaStreamSynchronize(c->stream), "cudaStreamSynchronize"))) return bail(rc);
   *out = c;
   return SD_OK;

@@ -43,7 +43,9 @@ def test_few_poses_at_the_shape_limit(n_rec, n_lig, tables):
 
 
 # the arrays fit by themselves, but not beside the buffers of the warps
-@pytest.mark.parametrize("n_rec,n_lig,scoring", [(200000, 4600, sd.SD_SCORING_PYDOCK),
+@pytest.mark.parametrize("n_rec,n_lig,scoring", [(23100, 300, sd.SD_SCORING_DFIRE), (25900, 300, sd.SD_SCORING_DFIRE),
+                                                 (27600, 1, sd.SD_SCORING_DFIRE), (24000, 640, sd.SD_SCORING_DFIRE),
+                                                 (200000, 4600, sd.SD_SCORING_PYDOCK),
                                                  (200000, 4880, sd.SD_SCORING_PYDOCK)])
 def test_arrays_at_the_shared_memory_limit(n_rec, n_lig, scoring, tables):
     cx = sd.SyntheticComplex(n_rec, n_lig, 2, 1, 0, 0, seed=n_rec)
