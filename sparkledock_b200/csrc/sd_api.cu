@@ -153,6 +153,7 @@ struct sd_ctx {
   int score_poses = 1;       // poses per CTA of the last configured scorer launch
   // autotuner state (mixed-precision DFIRE kernel variants)
   int mixed_variant = 0;
+  bool forced = false;     // by the user: also where another shape would be taken
   int wide = 0;            // SD_WIDE when a ligand reaches far (DFIRE): part of the mixed kernel's variant
   int smem_sm = 0;         // shared memory of an SM
   bool tuned = false;
@@ -593,7 +594,7 @@ int score_variant(sd_ctx* c, int precision, int poses, bool stateless) {
   bool few = few_poses(c, poses);
   if (c->scoring == SD_SCORING_DFIRE) {
     if (precision == SD_PREC_FP64) return fp64_shape(c->max_nr, c->max_nl, c->smem_sm, poses, c->nsm);
-    few &= precision == SD_PREC_MIXED && stateless;
+    few &= precision == SD_PREC_MIXED && stateless && !c->forced;
   }
   const int wide = precision == SD_PREC_MIXED ? c->wide : 0;
   few = few && few_fits(c, score_kernel_ptr(precision, c->scoring, SD_FEW | wide, false),
@@ -634,7 +635,10 @@ int autotune_mixed(sd_ctx* c) {
   const int nv = mixed_variant_count();
   if (const char* f = getenv("SPARKLE_MIXED_VARIANT")) {
     const int v = atoi(f);
-    if (v >= 0 && v < nv) c->mixed_variant = v;
+    if (v >= 0 && v < nv) {
+      c->mixed_variant = v;
+      c->forced = true;
+    }
     return SD_OK;
   }
   if (const char* t = getenv("SPARKLE_TUNE"))
