@@ -149,7 +149,7 @@ struct sd_ctx {
   size_t score_smem = 0;
   bool score_spill = false;  // the last configured scorer launch uses the spill instantiation
   size_t spill_stride = 0;
-  float force_scale = 1.f;   // pyDock: fixed-point units of FP32 ligand forces
+  float force_scale = 0.f;   // pyDock: 1 / unit of the fixed-point FP32 ligand forces; 0: none is fine enough
   int score_poses = 1;       // poses per CTA of the last configured scorer launch
   // autotuner state (mixed-precision DFIRE kernel variants)
   int mixed_variant = 0;
@@ -957,12 +957,24 @@ int sd_ctx_create(const sd_complex_desc* complexes, int n_complexes, const sd_ta
         sig[i] = tables->lj_sigma[i];
       }
     if (scoring == SD_SCORING_PYDOCK) {
+      // the largest charges and the LJ types that occur
       double qr = 0, ql = 0;
+      unsigned tr = 0, tl = 0;
+      bool finite = true;
       for (int i = 0; i < n_complexes; ++i) {
-        for (int k = 0; k < complexes[i].n_rec; ++k) qr = std::max(qr, std::fabs(complexes[i].rec_charge[k]));
-        for (int k = 0; k < complexes[i].n_lig; ++k) ql = std::max(ql, std::fabs(complexes[i].lig_charge[k]));
+        const sd_complex_desc& d = complexes[i];
+        for (int k = 0; k < d.n_rec; ++k) {
+          finite &= std::isfinite(d.rec_charge[k]);
+          qr = std::max(qr, std::fabs(d.rec_charge[k]));
+          tr |= 1u << d.rec_lj_type[k];
+        }
+        for (int k = 0; k < d.n_lig; ++k) {
+          finite &= std::isfinite(d.lig_charge[k]);
+          ql = std::max(ql, std::fabs(d.lig_charge[k]));
+          tl |= 1u << d.lig_lj_type[k];
+        }
       }
-      c->force_scale = pydock_force_scale(qr, ql, eps.data(), sig.data(), c->max_nr);
+      if (finite) c->force_scale = pydock_force_scale(qr, ql, eps.data(), sig.data(), tr, tl, c->max_nr);
     }
     std::vector<int> smap(c->total_swarms);
     for (int ci = 0, s0 = 0; ci < n_complexes; ++ci)
@@ -1291,6 +1303,7 @@ int sd_pydock_grad(sd_ctx* c, int ci, const double* poses, int n, int precision,
     return fail(SD_ERR_ARG, "sd_pydock_grad: unknown precision");
   if (n == 0) return SD_OK;
   if (n >= (1 << 24)) return fail(SD_ERR_ARG, "sd_pydock_grad: more than 2^24 poses");
+  if (precision == SD_PREC_MIXED && !(c->force_scale > 0.f)) precision = SD_PREC_FP64;
   SD_CUDA(cudaSetDevice(c->device));
   const DevComplex& D = c->cx[ci].d;
   const int ng = 6 + D.nmr + D.nml;

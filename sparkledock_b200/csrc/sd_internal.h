@@ -175,7 +175,8 @@ int bins_launch(const DevComplex* cplx, int c, const double* d_pose, int precisi
                 int* d_fallback, cudaStream_t st);
 size_t pydock_smem_bytes(int precision, bool grad, int max_nl, int max_nr);
 size_t pydock_warp_bytes(int precision, bool grad, bool few);
-float pydock_force_scale(double max_q_rec, double max_q_lig, const double* eps, const double* sigma, int max_nr);
+float pydock_force_scale(double max_q_rec, double max_q_lig, const double* eps, const double* sigma,
+                         unsigned rec_types, unsigned lig_types, int max_nr);
 const void* pydock_kernel_ptr(int precision, bool grad, bool spill, bool few);
 int pydock_launch(const ScoreLaunch& L, int precision, bool grad, double* out_grad, int grid, size_t smem,
                   cudaStream_t st, bool spill, bool few);

@@ -616,21 +616,25 @@ size_t pydock_warp_bytes(int precision, bool grad, bool few) {
   return pd_warps(fp64, grad, few) * (fp64 ? sizeof(PdWarp<double>) : sizeof(PdWarp<float>));
 }
 
-// the scale of FP32 ligand forces: pair forces are at most 0.7 kKe q q' (electrostatics) plus 1.6 eps
-// (3072 / sig^2 + 26) (LJ: |6 s^5 - 3 s^2| <= 192, s^2 <= 4, within 8 A), times the receptor's atoms
-float pydock_force_scale(double max_q_rec, double max_q_lig, const double* eps, const double* sigma, int max_nr) {
-  double f = 0.7 * kKe * max_q_rec * max_q_lig;
+// The scale of FP32 ligand forces: pair forces are at most 0.7 kKe q q' (electrostatics) plus 1.6 eps
+// (3072 / sig^2 + 26) (LJ: |6 s^5 - 3 s^2| <= 192, s^2 <= 4, within 8 A; over the type pairs that occur: bit a of
+// rec_types, bit b of lig_types), times the receptor's atoms.  0 where the unit would be coarser than 2^-30
+// (charges of 100 and more on both sides, or a sigma below 0.01 A) or no bound exists: FP64 gradients then.
+float pydock_force_scale(double max_q_rec, double max_q_lig, const double* eps, const double* sigma,
+                         unsigned rec_types, unsigned lig_types, int max_nr) {
   double lj = 0;
   for (int a = 0; a < SD_LJ_TYPES; ++a)
     for (int b = 0; b < SD_LJ_TYPES; ++b) {
+      if (!(rec_types >> a & 1u) || !(lig_types >> b & 1u)) continue;
       const double e = std::sqrt(eps[a] * eps[b]), sg = 0.5 * (sigma[a] + sigma[b]);
       const double v = 1.6 * e * ((sg != 0 ? 3072.0 / (sg * sg) : 0.0) + 26.0);
-      if (std::isfinite(v)) lj = std::max(lj, v);
+      if (!std::isfinite(v)) return 0.f;
+      lj = std::max(lj, v);
     }
-  f = (f + lj) * std::max(8, max_nr);
-  if (!std::isfinite(f)) f = 1e30;
+  const double f = (0.7 * kKe * max_q_rec * max_q_lig + lj) * std::max(8, max_nr);
+  if (!(f <= 0x1p31)) return 0.f;
   const int k = (int)std::floor(61.0 - std::log2(std::max(f, 1e-9)));
-  return std::ldexp(1.0f, std::min(100, std::max(-100, k)));
+  return std::ldexp(1.0f, std::min(100, k));
 }
 
 template <class T, bool GRAD>
