@@ -132,7 +132,8 @@ __device__ __forceinline__ void pd_pairs(V2<T> x, V2<T> qq, const LjPair<T>* l0,
                                          V2<T>& dedx) {
   const V2<T> y = x + V2<T>(T(1));
   const V2<T> inv(T(1) / y.first(), T(1) / y.second());
-  const V2<T> el = qq * inv;
+  // (the cutoff holds for charges that are not finite too: 0 of the switch times them would not be 0)
+  const V2<T> el0 = qq * inv, el(x.first() < T(225) ? el0.first() : T(0), x.second() < T(225) ? el0.second() : T(0));
   const V2<T> a = V2<T>(T(225)) - x, c(T(1) / T(24389));  // (225 - 196)^3
   const V2<T> v = a * a * (V2<T>(T(225)) + V2<T>(T(2)) * x - V2<T>(T(588))) * c;
   const V2<T> dv = V2<T>(T(6)) * a * (V2<T>(T(196)) - x) * c;
