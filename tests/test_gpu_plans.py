@@ -35,3 +35,27 @@ def test_pydock_calls_of_both_shapes(first, precision, tol, tables):
         for n in (MANY, FEW, MANY, FEW) if first != "few" else (FEW, MANY, FEW):
             _, e = dk.score_poses(0, poses[:n], precision)
             assert (np.abs(e - ref[:n]) / scale[:n]).max() <= tol, f"{n} poses"
+
+
+@pytest.mark.parametrize("n", [1, 40, 5000])
+def test_results_of_repeated_calls(n, tables):
+    """Scores and energies, energies and gradients come to the host in one copy where they are small, through
+    pinned memory from the 16th call of a context on, and one by one where they are not (5,000 poses)."""
+    c = sd.SyntheticComplex(120, 60, n, 1, 10, 10, seed=3)
+    poses = c.poses.reshape(n, -1)
+    with sd.Docking([c], tables) as dk:
+        sc, en = dk.score_poses(0, poses, sd.SD_PREC_FP64)
+        assert np.array_equal(sc, -(0.0157 * en - 4.7)) and np.unique(en).size > n // 2
+        for _ in range(18):
+            s, e = dk.score_poses(0, poses, sd.SD_PREC_FP64)
+            assert np.array_equal(s, sc) and np.array_equal(e, en)
+    osys = OracleSystem(c, tables, scoring=1)
+    pick = np.unique([0, n // 2, n - 1])
+    ref = np.array([oracle_energy(osys, poses[k]) for k in pick])
+    grad = np.array([oracle_grad(osys, poses[k], 26) for k in pick])
+    top = np.maximum(np.abs(grad).max(axis=1), 1.0)
+    with sd.Docking([c], tables, scoring=sd.SD_SCORING_PYDOCK) as dk:
+        for _ in range(18):
+            e, g = dk.pydock_grad(0, poses, sd.SD_PREC_FP64)
+            assert (np.abs(e[pick] - ref) / np.maximum(np.abs(ref), top)).max() <= 1e-10
+            assert (np.abs(g[pick] - grad) / top[:, None]).max() <= 1e-10
