@@ -1296,12 +1296,15 @@ int sd_dfire_bins(sd_ctx* c, int ci, const double* pose, int precision, int* bin
   const size_t nb = (size_t)D.nr * D.nl;
   int rc;
   if ((rc = ensure(c, c->s_bins, nb * 4 + 64))) return rc;
-  if ((rc = ensure(c, c->s_pose, (size_t)D.pl * 8))) return rc;
+  if ((rc = ensure(c, c->s_pose, (size_t)(D.pl + 3) * 8))) return rc;  // the pose, its reference point
   SD_CUDA(cudaMemcpyAsync(c->s_pose.p, pose, (size_t)D.pl * 8, cudaMemcpyHostToDevice, c->stream));
   int* d_bins = (int*)c->s_bins.p;
   int* d_fb = (int*)((char*)c->s_bins.p + nb * 4);
   SD_CUDA(cudaMemsetAsync(d_fb, 0, 4, c->stream));
-  if ((rc = bins_launch(c->d_cplx, ci, (const double*)c->s_pose.p, precision, d_bins, D.nr, D.nl, d_fb, c->stream)))
+  DevComplex S = D;
+  S.pos = (double*)c->s_pose.p;
+  S.ref = (double*)c->s_pose.p + D.pl;
+  if ((rc = bins_launch(S, precision, d_bins, d_fb, c->stream)))
     return fail(rc, "bins kernel launch failed");
   SD_CUDA(cudaMemcpyAsync(bins_out, d_bins, nb * 4, cudaMemcpyDeviceToHost, c->stream));
   SD_CUDA(cudaStreamSynchronize(c->stream));

@@ -171,8 +171,7 @@ int gso_launch_large(const GsoLaunch& L, int max_g, cudaStream_t st);
 int gso_launch_warp(const GsoLaunch& L, int max_g, int nsm, cudaStream_t st);
 int gso_prepare_large();
 int gso_prepare_warp();
-int bins_launch(const DevComplex* cplx, int c, const double* d_pose, int precision, int* d_bins, int nr, int nl,
-                int* d_fallback, cudaStream_t st);
+int bins_launch(const DevComplex& C, int precision, int* d_bins, int* d_fallback, cudaStream_t st);
 size_t pydock_smem_bytes(int precision, bool grad, int max_nl, int max_nr);
 size_t pydock_warp_bytes(int precision, bool grad, bool few);
 float pydock_force_scale(double max_q_rec, double max_q_lig, const double* eps, const double* sigma,

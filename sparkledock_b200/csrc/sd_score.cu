@@ -23,18 +23,11 @@
 namespace sd {
 
 __constant__ double c_T[32];   // exact FP64 key thresholds: key(d2) = #{m>=1 : T[m] <= d2}
-__constant__ float c_Tf[32];   // same as float, with c_Tf[30] = 225 (cutoff)
 
 void set_key_thresholds(const double* t) {
   double T[32];
-  float Tf[32];
-  for (int m = 0; m < 32; ++m) {
-    T[m] = m < 30 ? t[m] : 1e300;
-    Tf[m] = m < 30 ? (float)t[m] : (m == 30 ? 225.0f : 3.0e38f);
-  }
-  Tf[0] = 0.0f;
+  for (int m = 0; m < 32; ++m) T[m] = m < 30 ? t[m] : 1e300;
   cudaMemcpyToSymbol(c_T, T, sizeof T);
-  cudaMemcpyToSymbol(c_Tf, Tf, sizeof Tf);
 }
 
 // dist_to_bins[key] - 1 (interface.h:30-35) for key 0..29; key 29 (d2 == 225) gives 20, which
@@ -343,62 +336,53 @@ int score_launch(const ScoreLaunch& L, int precision, int scoring, int grid, siz
   return cudaGetLastError() == cudaSuccess ? SD_OK : SD_ERR_CUDA;
 }
 
-// ---- per-pair bins of one pose (parity/debug): thread per pair ----
-__global__ void dfire_bins_kernel(const DevComplex* cplx, int ci, const double* pose, int precision, int* bins,
-                                  int* fallback) {
-  const DevComplex& C = cplx[ci];
-  const int nl = C.nl, nslots = nslots_of(C);
+// ---- per-pair bins of one pose (parity/debug), thread per pair, by the steps of the precision's scorer: FP32
+// terms and the exact transforms where they do not settle a pair, or the exact transforms alone (FP64_REF) ----
+// C: the complex with pos at the pose and ref at three doubles that the prologue may write
+__global__ void dfire_bins_kernel(DevComplex C, int precision, int* bins, int* fallback) {
+  __shared__ PoseBufs Q;
+  if (threadIdx.x < 32) pose_prologue(C, 0, Q, threadIdx.x);
+  __syncthreads();
+  const int nl = C.nl, nslots = nslots_of(C), nls = C.nlchunks * SD_TILE;
   const long long total = (long long)nslots * nl;
-  double q[4] = {pose[3], pose[4], pose[5], pose[6]}, qi[4];
-  quat_inverse(q, qi);
-  const double tx = pose[0], ty = pose[1], tz = pose[2];
-  float dL = 0.f;
-  for (int m = 0; m < C.nml; ++m) dL += fabsf((float)pose[7 + C.nmr + m]) * C.mnorm_l[m];
-  dL = dL * 1.0001f + 1e-4f;
-  const float RL = C.lig_radius + dL;
-  const float u32 = 5.9604645e-8f;
-  const float B = 2.0f * (2.02f * u32 * (26.2f * (2.0f * RL + 15.1f) + 228.0f) + 3.0f * u32 * 228.0f) + 1e-6f;
+  const float cut2 = 225.0f + Q.B, inner = settled_half(Q.B);
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
     const int slot = (int)(idx / nl), j = (int)(idx % nl);
     const int orig = C.r_orig[slot];
     if (orig < 0) continue;
-    double rx, ry, rz, lx, ly, lz;
-    receptor_exact(C, nslots, slot, pose, rx, ry, rz);
-    ligand_exact(C, C.l_slot[j], pose, q, qi, lx, ly, lz);
     int bin = -1;
-    if (precision != SD_PREC_MIXED) {
+    bool settled = false;
+    if (precision != SD_PREC_FP64_REF) {
+      double r[1][3], l[1][3];
+      anm_fused<1>(C.r_xyz, C.r_modes, C.r_mask, nslots, C.nmr, &Q.pose[7], 0, slot, r);
+      anm_fused<1>(C.l_xyz, C.l_modes, C.l_mask, nls, C.nml, &Q.pose[7 + C.nmr], 0, C.l_slot[j], l);
+      const float x = (float)(r[0][0] - Q.pose[0]), y = (float)(r[0][1] - Q.pose[1]), z = (float)(r[0][2] - Q.pose[2]);
+      const double* R = Q.rot;
+      const float4 lig = make_float4(-(float)fma(R[0], l[0][0], fma(R[1], l[0][1], R[2] * l[0][2])),
+                                     -(float)fma(R[3], l[0][0], fma(R[4], l[0][1], R[5] * l[0][2])),
+                                     -(float)fma(R[6], l[0][0], fma(R[7], l[0][1], R[8] * l[0][2])), 0.f);
+      float d2[2], mid[2];
+      int b[2];
+      pair_terms(pack2(x, x), pack2(y, y), pack2(z, z), lig, d2, mid, b);
+      settled = inner > 0.f && !(d2[0] <= cut2 && fabsf(mid[0]) >= inner);
+      if (settled && d2[0] <= cut2) bin = b[0] - kMagicBits;
+    }
+    if (!settled) {
+      if (precision != SD_PREC_FP64_REF) atomicAdd(fallback, 1);
+      double rx, ry, rz, lx, ly, lz;
+      receptor_exact(C, nslots, slot, Q.pose, rx, ry, rz);
+      ligand_exact(C, C.l_slot[j], Q.pose, Q.q, Q.qi, lx, ly, lz);
       const double ddx = rx - lx, ddy = ry - ly, ddz = rz - lz;
-      const double d2 = ddx * ddx + ddy * ddy + ddz * ddz;
-      if (d2 <= SD_CUTOFF2) bin = c_binlut[d2 == 0.0 ? 0 : exact_key(d2, c_T)];
-    } else {
-      const float ex = (float)(rx - tx) - (float)(lx - tx), ey = (float)(ry - ty) - (float)(ly - ty),
-                  ez = (float)(rz - tz) - (float)(lz - tz);
-      const float d2 = fmaf(ez, ez, fmaf(ey, ey, ex * ex));
-      if (d2 <= 225.0f + B) {
-        float f = sqrtf(d2) * 2.0f - 1.0f;
-        int key = (int)f;
-        key = key < 0 ? 0 : (key > 29 ? 29 : key);
-        const bool near = (d2 - c_Tf[key] <= B) || (c_Tf[key + 1] - d2 <= B);
-        if (near) {
-          atomicAdd(fallback, 1);
-          const double ddx = rx - lx, ddy = ry - ly, ddz = rz - lz;
-          const double e2 = ddx * ddx + ddy * ddy + ddz * ddz;
-          if (e2 <= SD_CUTOFF2) bin = c_binlut[e2 == 0.0 ? 0 : exact_key(e2, c_T)];
-        } else {
-          bin = c_binlut[key];
-        }
-      }
+      const double e2 = ddx * ddx + ddy * ddy + ddz * ddz;
+      if (e2 <= SD_CUTOFF2) bin = c_binlut[e2 == 0.0 ? 0 : exact_key(e2, c_T)];
     }
     bins[(size_t)orig * nl + j] = bin;
   }
 }
 
-int bins_launch(const DevComplex* cplx, int c, const double* d_pose, int precision, int* d_bins, int nr, int nl,
-                int* d_fallback, cudaStream_t st) {
-  (void)nr;
-  (void)nl;
-  dfire_bins_kernel<<<148 * 8, 256, 0, st>>>(cplx, c, d_pose, precision, d_bins, d_fallback);
+int bins_launch(const DevComplex& C, int precision, int* d_bins, int* d_fallback, cudaStream_t st) {
+  dfire_bins_kernel<<<148 * 8, 256, 0, st>>>(C, precision, d_bins, d_fallback);
   return cudaGetLastError() == cudaSuccess ? SD_OK : SD_ERR_CUDA;
 }
 

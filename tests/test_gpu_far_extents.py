@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 import sparkledock_b200 as sd
-from oracle_bind import OracleSystem, oracle_scores
+from oracle_bind import OracleSystem, oracle_bins, oracle_scores
 
 pytestmark = pytest.mark.gpu
 
@@ -36,3 +36,26 @@ def test_displacements_beyond_fp32(n_rec, n_lig, extent, tables):
             assert np.array_equal(en, ref[:k])
             _, en = dk.score_poses(0, poses[:k], sd.SD_PREC_MIXED)
             assert np.abs(en - ref[:k]).max() <= tol
+
+
+@pytest.mark.parametrize("extent", [0.0, 3.0, 1e4, 3e5, 1e6, 1e37, 1e39])
+def test_atoms_displaced_together(extent, tables):
+    """Receptor and ligand atoms displaced by the same vector, beyond what FP32 holds from 1e39 on: they meet
+    there, and the bins of the pairs, by the steps of each precision's scorer, are the oracle's."""
+    c = sd.SyntheticComplex(70, 41, 1, 1, n_modes_rec=1, n_modes_lig=1, seed=8)
+    c.rec_mask[:], c.lig_mask[:] = np.arange(70) % 2 == 0, np.arange(41) % 3 == 0
+    c.rec_modes[:], c.lig_modes[:] = (1.0, 0.0, 0.0), (1.0, 0.0, 0.0)
+    pose = np.zeros(c.pose_len)
+    pose[:3], pose[3], pose[7:] = (2.0, -1.0, 0.5), 1.0, extent
+    osys = OracleSystem(c, tables)
+    want, _, _, _, _ = oracle_bins(osys, pose)
+    both = np.ix_(c.rec_mask == 1, c.lig_mask == 1)
+    assert (want[both] >= 0).any()
+    _, ref = oracle_scores(osys, pose[None])
+    with sd.Docking([c], tables) as dk:
+        for precision in (sd.SD_PREC_FP64_REF, sd.SD_PREC_FP64, sd.SD_PREC_MIXED):
+            assert np.array_equal(dk.dfire_bins(0, pose, precision), want)
+        _, en = dk.score_poses(0, pose[None], sd.SD_PREC_FP64)
+        assert np.array_equal(en, ref)
+        _, en = dk.score_poses(0, pose[None], sd.SD_PREC_MIXED)
+        assert np.abs(en - ref).max() <= 6.0 * want.size ** 2 * 2.0 ** -53
