@@ -60,6 +60,7 @@ struct ComplexHost {
   int draws_steps = 0;   // columns uploaded
   int draws_used = 0;    // host mirror of draw_cursor
   bool state_set = false;
+  ScorePlan grad_plan[3][4];  // pyDock gradients, by precision and shape
   std::vector<void*> owned;
 };
 
@@ -144,7 +145,7 @@ struct sd_ctx {
   DevBuf s_pose, s_score, s_ref, s_work, s_grad, s_bins, s_final;
   // per-CTA global scratch of the spill instantiations (complexes too large for shared memory)
   DevBuf s_spill;
-  ScorePlan plan[3][SD_MAX_VARIANTS + 1], grad_plan[3][2];
+  ScorePlan plan[3][SD_MAX_VARIANTS + 1];
   int few_fit[3] = {-1, -1, -1}, few_grad_fit[3] = {-1, -1, -1};  // by precision; see few_fits
   void* h_stage = nullptr;   // pinned, for small downloads (made by the 16th of them)
   long long small_downloads = 0;
@@ -1339,28 +1340,29 @@ int sd_pydock_grad(sd_ctx* c, int ci, const double* poses, int n, int precision,
   SD_CUDA(cudaMemcpyAsync(c->s_pose.p, poses, (size_t)n * D.pl * 8, cudaMemcpyHostToDevice, c->stream));
   if ((rc = stateless_prepare_launch(c->d_ctl_scratch, c->d_cplx_scratch, S, (int*)c->s_work.p, ci, n, c->stream)))
     return fail(rc, "stateless call: prepare kernel launch failed");
-  const bool few = few_poses(c, n) && few_fits(c, pydock_kernel_ptr(precision, true, false, true),
+  const bool few = few_poses(c, n) && few_fits(c, pydock_kernel_ptr(precision, true, false, PD_FEW),
                                                pydock_smem_bytes(precision, true, c->max_nl, c->max_nr) +
-                                                   pydock_warp_bytes(precision, true, true),
+                                                   pydock_warp_bytes(precision, true, PD_FEW),
                                                &c->few_grad_fit[precision]);
-  ScorePlan& plan = c->grad_plan[precision][few];
+  const int shape = few ? PD_FEW : pydock_grad_shape(precision, D.nl, D.nr, n, c->smem_sm, c->nsm);
+  ScorePlan& plan = c->cx[ci].grad_plan[precision][shape];
   if (!plan.grid) {
-    const size_t need = pydock_smem_bytes(precision, true, c->max_nl, c->max_nr);
-    const void* k = pydock_kernel_ptr(precision, true, false, few);
+    const size_t need = pydock_smem_bytes(precision, true, D.nl, D.nr);
+    const void* k = pydock_kernel_ptr(precision, true, false, shape);
     cudaFuncAttributes fa;
     SD_CUDA(cudaFuncGetAttributes(&fa, k));
     // a ligand too large for shared memory: the spill instantiation, per-CTA arrays in global scratch
-    const size_t warp_bytes = pydock_warp_bytes(precision, true, few);
+    const size_t warp_bytes = pydock_warp_bytes(precision, true, shape);
     plan.spill = warp_bytes + need + fa.sharedSizeBytes > (size_t)c->smem_optin;
     plan.smem = warp_bytes + (plan.spill ? 0 : need);
     plan.spill_stride = plan.spill ? (need + 255) & ~(size_t)255 : 0;
     if (plan.spill) {
-      k = pydock_kernel_ptr(precision, true, true, false);
+      k = pydock_kernel_ptr(precision, true, true, PD_ORDINARY);
       SD_CUDA(cudaFuncGetAttributes(&fa, k));
     }
     SD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, c->smem_optin - (int)fa.sharedSizeBytes));
     int per_sm = 0;
-    SD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, pydock_threads(precision, true, few), plan.smem));
+    SD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, pydock_threads(precision, true, shape), plan.smem));
     if (per_sm < 1) return fail(SD_ERR_ARG, "pyDock gradient kernel does not fit on an SM");
     plan.grid = per_sm * c->nsm;
   }
@@ -1378,7 +1380,7 @@ int sd_pydock_grad(sd_ctx* c, int ci, const double* poses, int n, int precision,
   L.lj_eps = c->d_lj_eps;
   L.lj_sigma = c->d_lj_sigma;
   L.energy_out = (double*)c->s_grad.p;
-  if ((rc = pydock_launch(L, precision, true, (double*)c->s_grad.p + n, plan.grid, plan.smem, c->stream, spill, few)))
+  if ((rc = pydock_launch(L, precision, true, (double*)c->s_grad.p + n, plan.grid, plan.smem, c->stream, spill, shape)))
     return fail(rc, std::string("pyDock gradient kernel: ") + cudaGetErrorString(cudaGetLastError()));
   return download(c, c->s_grad.p, {{energy_out, (size_t)n * 8}, {grad_out, (size_t)n * ng * 8}});
 }

@@ -173,13 +173,15 @@ int gso_prepare_large();
 int gso_prepare_warp();
 int bins_launch(const DevComplex& C, int precision, int* d_bins, int* d_fallback, cudaStream_t st);
 size_t pydock_smem_bytes(int precision, bool grad, int max_nl, int max_nr);
-size_t pydock_warp_bytes(int precision, bool grad, bool few);
+enum PdShape { PD_ORDINARY = 0, PD_FEW, PD_MID, PD_SMALL };  // of the pyDock kernel (sd_pydock.cu)
+size_t pydock_warp_bytes(int precision, bool grad, int shape);
+int pydock_grad_shape(int precision, int nl, int nr, int poses, int smem_sm, int nsm);
 float pydock_force_scale(double max_q_rec, double max_q_lig, const double* eps, const double* sigma,
                          unsigned rec_types, unsigned lig_types, int max_nr);
-const void* pydock_kernel_ptr(int precision, bool grad, bool spill, bool few);
+const void* pydock_kernel_ptr(int precision, bool grad, bool spill, int shape);
 int pydock_launch(const ScoreLaunch& L, int precision, bool grad, double* out_grad, int grid, size_t smem,
-                  cudaStream_t st, bool spill, bool few);
-int pydock_threads(int precision, bool grad, bool few);
+                  cudaStream_t st, bool spill, int shape);
+int pydock_threads(int precision, bool grad, int shape);
 int init_state_launch(const DevComplex& C, double luciferin, double vision, cudaStream_t st);
 int worklist_launch(const DevComplex* cplx, const int* swarm_map, int nswarms, StepCtl* ctl, int* work,
                     cudaStream_t st);

@@ -40,13 +40,16 @@ namespace sd {
 
 namespace {
 
-// warps of a CTA: FP32 gradients 12, two CTAs per SM (their ligand forces take 24 bytes an atom, and
-// three CTAs of 8 warps would not fit beside ligands over 1,270 atoms); else 8, as many as fit.  few: at
-// most one pose per SM, so one CTA with all the warps that the registers allow, for a pose's time
-__host__ __device__ constexpr int pd_warps(bool fp64, bool grad, bool few) {
-  return few ? (grad && fp64 ? 16 : 24) : (grad && !fp64 ? 12 : 8);
+// Warps of a CTA and CTAs per SM of each shape.  PD_ORDINARY: 8 warps, as many CTAs as fit; FP32 gradients 12,
+// two CTAs (their ligand forces take 24 bytes an atom).  PD_MID and PD_SMALL: FP32 gradients of smaller
+// molecules (pydock_grad_shape).  PD_FEW: at most one pose per SM, so one CTA with all the warps that the
+// registers allow, for a pose's time
+__host__ __device__ constexpr int pd_warps(bool fp64, bool grad, int shape) {
+  return shape == PD_FEW ? (grad && fp64 ? 16 : 24) : shape == PD_MID ? 8 : shape == PD_SMALL ? 4 : grad && !fp64 ? 12 : 8;
 }
-__host__ __device__ constexpr int pd_ctas(bool grad, bool few) { return few ? 1 : (grad ? 2 : 4); }
+__host__ __device__ constexpr int pd_ctas(bool grad, int shape) {
+  return shape == PD_FEW ? 1 : shape == PD_MID ? 3 : shape == PD_SMALL ? 6 : grad ? 2 : 4;
+}
 constexpr double kKe = 332.0636 / 4.0;
 
 // an atom in shared memory (position relative to t, the ligand's negated, charge): one 16-byte load in FP32
@@ -216,10 +219,10 @@ __device__ __forceinline__ T warp_sum(T v) {
 // L.energy_out (E) when set.  kSpill: the per-pose arrays live in this CTA's slice of the global
 // scratch L.spill instead of shared memory (ligands too large for it).  Four CTAs per SM (64
 // registers a thread) without forces: the pair terms are latency chains.
-template <class T, bool GRAD, bool kSpill, bool kFew>
-__global__ void __launch_bounds__(pd_warps(sizeof(T) == 8, GRAD, kFew) * 32, pd_ctas(GRAD, kFew))
+template <class T, bool GRAD, bool kSpill, int kShape>
+__global__ void __launch_bounds__(pd_warps(sizeof(T) == 8, GRAD, kShape) * 32, pd_ctas(GRAD, kShape))
 pydock_kernel(ScoreLaunch L, double* out_grad) {
-  constexpr int kWarps = pd_warps(sizeof(T) == 8, GRAD, kFew);
+  constexpr int kWarps = pd_warps(sizeof(T) == 8, GRAD, kShape);
   extern __shared__ __align__(16) unsigned char smem_dyn[];
   PdWarp<T>& W = reinterpret_cast<PdWarp<T>*>(smem_dyn)[threadIdx.x >> 5];
   unsigned char* const smem =
@@ -612,9 +615,9 @@ size_t pydock_smem_bytes(int precision, bool grad, int max_nl, int max_nr) {
   return ts * 4 * (nls + 1) + (grad ? 24 * (nls + 4) : 0) + 16 * nlc + (nls + 1) +
          4 * nt + 8 * std::min<size_t>(nt, kOrderMax) + 16;
 }
-size_t pydock_warp_bytes(int precision, bool grad, bool few) {
+size_t pydock_warp_bytes(int precision, bool grad, int shape) {
   const bool fp64 = precision != SD_PREC_MIXED;
-  return pd_warps(fp64, grad, few) * (fp64 ? sizeof(PdWarp<double>) : sizeof(PdWarp<float>));
+  return pd_warps(fp64, grad, shape) * (fp64 ? sizeof(PdWarp<double>) : sizeof(PdWarp<float>));
 }
 
 // The scale of FP32 ligand forces: pair forces are at most 0.7 kKe q q' (electrostatics) plus 1.6 eps
@@ -638,30 +641,68 @@ float pydock_force_scale(double max_q_rec, double max_q_lig, const double* eps, 
   return std::ldexp(1.0f, std::min(100, k));
 }
 
-template <class T, bool GRAD>
-static const void* kernel_of(bool spill, bool few) {
-  if (spill) return (const void*)pydock_kernel<T, GRAD, true, false>;
-  return few ? (const void*)pydock_kernel<T, GRAD, false, true> : (const void*)pydock_kernel<T, GRAD, false, false>;
+// The shape of a gradient call of many poses: FP32 takes the one with the most warps resident on an SM beside the
+// arrays of a complex of this size (7 KiB of a CTA are its static arrays, 1 KiB the system's), the smallest
+// CTAs among equals, as a warp without a tile only waits.  4,096 poses, ms with 4 x 6, 8 x 3 and 12 x 2 warps x
+// CTAs: 200/100 atoms 0.42, 0.59, 0.76; 757/481 1.29, 1.35, 1.75; 1500/700 2.1, 1.88, 2.28; 3002/1274 5.4, 3.50,
+// 3.65; 3002/1766 9.8, 5.8, 4.72; 3002/2100 11.8, 6.9, 8.3; 3002/2500 24, 13.2, 9.7.  (12 warps for all sizes were
+// slower than the earlier kernel for the smallest: 0.76 against 0.69 ms.)
+// Where all poses are resident in that shape at once, the warps of a pose count: then the fewest rounds over the
+// warps that have a tile.  (757/481: 300 poses 0.34 ms in 4 x 6, 0.23 in 8 x 3, 0.27 in 12 x 2.)
+int pydock_grad_shape(int precision, int nl, int nr, int poses, int smem_sm, int nsm) {
+  if (precision != SD_PREC_MIXED) return PD_ORDINARY;
+  int ctas[4] = {}, best = PD_ORDINARY;
+  for (int shape : {PD_ORDINARY, PD_MID, PD_SMALL}) {
+    const size_t cta = pydock_smem_bytes(precision, true, nl, nr) + pydock_warp_bytes(precision, true, shape) + 8192;
+    ctas[shape] = std::min((int)(smem_sm / cta), pd_ctas(true, shape));
+    if (ctas[PD_ORDINARY] == 0) return PD_ORDINARY;  // the spill instantiation has more warps than what would fit
+    if (ctas[shape] * pd_warps(false, true, shape) >= ctas[best] * pd_warps(false, true, best)) best = shape;
+  }
+  if (poses > ctas[best] * nsm) return best;
+  const int ntiles = (nr + SD_TILE - 1) / SD_TILE;
+  double least = 1e300;
+  for (int shape : {PD_SMALL, PD_MID, PD_ORDINARY}) {
+    if (ctas[shape] == 0) continue;
+    const int rounds = (poses + ctas[shape] * nsm - 1) / (ctas[shape] * nsm);
+    const double time = (double)rounds / std::min(pd_warps(false, true, shape), ntiles);
+    if (time < least) {
+      least = time;
+      best = shape;
+    }
+  }
+  return best;
 }
 
-// (the spill instantiation has the ordinary shape: few is ignored with it)
-const void* pydock_kernel_ptr(int precision, bool grad, bool spill, bool few) {
-  if (precision == SD_PREC_MIXED) return grad ? kernel_of<float, true>(spill, few) : kernel_of<float, false>(spill, few);
-  return grad ? kernel_of<double, true>(spill, few) : kernel_of<double, false>(spill, few);
+template <class T, bool GRAD>
+static const void* kernel_of(bool spill, int shape) {
+  if (spill) return (const void*)pydock_kernel<T, GRAD, true, PD_ORDINARY>;
+  if constexpr (GRAD && sizeof(T) == 4) {
+    if (shape == PD_MID) return (const void*)pydock_kernel<T, GRAD, false, PD_MID>;
+    if (shape == PD_SMALL) return (const void*)pydock_kernel<T, GRAD, false, PD_SMALL>;
+  }
+  return shape == PD_FEW ? (const void*)pydock_kernel<T, GRAD, false, PD_FEW>
+                         : (const void*)pydock_kernel<T, GRAD, false, PD_ORDINARY>;
+}
+
+// (the spill instantiation has the ordinary shape: another is ignored with it)
+const void* pydock_kernel_ptr(int precision, bool grad, bool spill, int shape) {
+  if (precision == SD_PREC_MIXED)
+    return grad ? kernel_of<float, true>(spill, shape) : kernel_of<float, false>(spill, shape);
+  return grad ? kernel_of<double, true>(spill, shape) : kernel_of<double, false>(spill, shape);
 }
 
 int pydock_launch(const ScoreLaunch& L, int precision, bool grad, double* out_grad, int grid, size_t smem,
-                  cudaStream_t st, bool spill, bool few) {
+                  cudaStream_t st, bool spill, int shape) {
   ScoreLaunch l = L;
   void* args[] = {(void*)&l, (void*)&out_grad};
-  if (cudaLaunchKernel(pydock_kernel_ptr(precision, grad, spill, few), dim3(grid),
-                       dim3(pydock_threads(precision, grad, few && !spill)), args, smem, st) != cudaSuccess)
+  if (cudaLaunchKernel(pydock_kernel_ptr(precision, grad, spill, shape), dim3(grid),
+                       dim3(pydock_threads(precision, grad, spill ? PD_ORDINARY : shape)), args, smem, st) != cudaSuccess)
     return SD_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? SD_OK : SD_ERR_CUDA;
 }
 
-int pydock_threads(int precision, bool grad, bool few) {
-  return pd_warps(precision != SD_PREC_MIXED, grad, few) * 32;
+int pydock_threads(int precision, bool grad, int shape) {
+  return pd_warps(precision != SD_PREC_MIXED, grad, shape) * 32;
 }
 
 }  // namespace sd

@@ -269,7 +269,7 @@ bool wide_ligand(float radius) { return !(radius <= 64.f); }
 // bytes of the scorer's per-warp buffers, in dynamic shared memory in front of the per-pose arrays
 // (alone there in the spill instantiation)
 size_t score_warp_bytes(int precision, int scoring, int variant, bool spill) {
-  if (scoring == SD_SCORING_PYDOCK) return pydock_warp_bytes(precision, false, !spill && variant == SD_FEW);
+  if (scoring == SD_SCORING_PYDOCK) return pydock_warp_bytes(precision, false, !spill && variant == SD_FEW ? PD_FEW : PD_ORDINARY);
   if (precision == SD_PREC_FP64_REF) return 0;
   if (precision == SD_PREC_FP64) return sizeof(OrdBufs) * (spill ? kFp64Spill : kFp64Shapes[variant]).warps;
   return sizeof(WarpBufs) * (spill ? kMixedSpill.warps : mixed_variant(variant).warps);
@@ -309,14 +309,14 @@ int mixed_variant_warps(int v) { return mixed_variant(v).warps; }
 int mixed_variant_min_blocks(int v) { return mixed_variant(v).min_blocks; }
 
 int score_threads_of(int precision, int scoring, int variant, bool spill) {
-  if (scoring == SD_SCORING_PYDOCK) return pydock_threads(precision, false, !spill && variant == SD_FEW);
+  if (scoring == SD_SCORING_PYDOCK) return pydock_threads(precision, false, !spill && variant == SD_FEW ? PD_FEW : PD_ORDINARY);
   if (precision == SD_PREC_FP64_REF) return kRefThreads;
   if (precision == SD_PREC_FP64) return (spill ? kFp64Spill : kFp64Shapes[variant]).warps * 32;
   return (spill ? kMixedSpill : mixed_variant(variant)).warps * 32;
 }
 
 const void* score_kernel_ptr(int precision, int scoring, int variant, bool spill) {
-  if (scoring == SD_SCORING_PYDOCK) return pydock_kernel_ptr(precision, false, spill, variant == SD_FEW);
+  if (scoring == SD_SCORING_PYDOCK) return pydock_kernel_ptr(precision, false, spill, variant == SD_FEW ? PD_FEW : PD_ORDINARY);
   switch (precision) {
     case SD_PREC_FP64_REF:
       return spill ? (const void*)dfire_score_ref_kernel<true> : (const void*)dfire_score_ref_kernel<false>;
@@ -327,7 +327,8 @@ const void* score_kernel_ptr(int precision, int scoring, int variant, bool spill
 
 int score_launch(const ScoreLaunch& L, int precision, int scoring, int grid, size_t smem, cudaStream_t st, int variant,
                  bool spill) {
-  if (scoring == SD_SCORING_PYDOCK) return pydock_launch(L, precision, false, nullptr, grid, smem, st, spill, variant == SD_FEW);
+  if (scoring == SD_SCORING_PYDOCK)
+    return pydock_launch(L, precision, false, nullptr, grid, smem, st, spill, variant == SD_FEW ? PD_FEW : PD_ORDINARY);
   ScoreLaunch l = L;
   void* args[] = {(void*)&l};
   if (cudaLaunchKernel(score_kernel_ptr(precision, scoring, variant, spill), dim3(grid),
