@@ -60,7 +60,7 @@ struct ComplexHost {
   int draws_steps = 0;   // columns uploaded
   int draws_used = 0;    // host mirror of draw_cursor
   bool state_set = false;
-  ScorePlan grad_plan[3][4];  // pyDock gradients, by precision and shape
+  ScorePlan grad_plan[3][5];  // pyDock gradients, by precision and shape
   std::vector<void*> owned;
 };
 
@@ -1344,8 +1344,9 @@ int sd_pydock_grad(sd_ctx* c, int ci, const double* poses, int n, int precision,
                                                pydock_smem_bytes(precision, true, c->max_nl, c->max_nr) +
                                                    pydock_warp_bytes(precision, true, PD_FEW),
                                                &c->few_grad_fit[precision]);
-  const int shape = few ? PD_FEW : pydock_grad_shape(precision, D.nl, D.nr, n, c->smem_sm, c->nsm);
-  ScorePlan& plan = c->cx[ci].grad_plan[precision][shape];
+  const int choice = few ? PD_FEW : pydock_grad_shape(precision, D.nl, D.nr, n, c->smem_sm, c->nsm);
+  const int shape = choice == PD_SCRATCH ? PD_ORDINARY : choice;
+  ScorePlan& plan = c->cx[ci].grad_plan[precision][choice];
   if (!plan.grid) {
     const size_t need = pydock_smem_bytes(precision, true, D.nl, D.nr);
     const void* k = pydock_kernel_ptr(precision, true, false, shape);
@@ -1353,7 +1354,7 @@ int sd_pydock_grad(sd_ctx* c, int ci, const double* poses, int n, int precision,
     SD_CUDA(cudaFuncGetAttributes(&fa, k));
     // a ligand too large for shared memory: the spill instantiation, per-CTA arrays in global scratch
     const size_t warp_bytes = pydock_warp_bytes(precision, true, shape);
-    plan.spill = warp_bytes + need + fa.sharedSizeBytes > (size_t)c->smem_optin;
+    plan.spill = choice == PD_SCRATCH || warp_bytes + need + fa.sharedSizeBytes > (size_t)c->smem_optin;
     plan.smem = warp_bytes + (plan.spill ? 0 : need);
     plan.spill_stride = plan.spill ? (need + 255) & ~(size_t)255 : 0;
     if (plan.spill) {

@@ -173,7 +173,8 @@ int gso_prepare_large();
 int gso_prepare_warp();
 int bins_launch(const DevComplex& C, int precision, int* d_bins, int* d_fallback, cudaStream_t st);
 size_t pydock_smem_bytes(int precision, bool grad, int max_nl, int max_nr);
-enum PdShape { PD_ORDINARY = 0, PD_FEW, PD_MID, PD_SMALL };  // of the pyDock kernel (sd_pydock.cu)
+// shapes of the pyDock kernel (sd_pydock.cu); PD_SCRATCH: the ordinary one with its arrays in global scratch
+enum PdShape { PD_ORDINARY = 0, PD_FEW, PD_MID, PD_SMALL, PD_SCRATCH };
 size_t pydock_warp_bytes(int precision, bool grad, int shape);
 int pydock_grad_shape(int precision, int nl, int nr, int poses, int smem_sm, int nsm);
 float pydock_force_scale(double max_q_rec, double max_q_lig, const double* eps, const double* sigma,

@@ -649,16 +649,20 @@ float pydock_force_scale(double max_q_rec, double max_q_lig, const double* eps, 
 // slower than the earlier kernel for the smallest: 0.76 against 0.69 ms.)
 // Where all poses are resident in that shape at once, the warps of a pose count: then the fewest rounds over the
 // warps that have a tile.  (757/481: 300 poses 0.34 ms in 4 x 6, 0.23 in 8 x 3, 0.27 in 12 x 2.)
+// Where shared memory holds one CTA only, two with their arrays in global scratch (PD_SCRATCH) have more warps: 2,000
+// poses of 757/2500 atoms 3.85 -> 3.18 ms in FP32, 5.0 -> 3.3 ms in FP64, 50/3503 4.4 -> 2.4 ms in FP64.
 int pydock_grad_shape(int precision, int nl, int nr, int poses, int smem_sm, int nsm) {
-  if (precision != SD_PREC_MIXED) return PD_ORDINARY;
+  const size_t need = pydock_smem_bytes(precision, true, nl, nr);
   int ctas[4] = {}, best = PD_ORDINARY;
   for (int shape : {PD_ORDINARY, PD_MID, PD_SMALL}) {
-    const size_t cta = pydock_smem_bytes(precision, true, nl, nr) + pydock_warp_bytes(precision, true, shape) + 8192;
+    if (precision != SD_PREC_MIXED && shape != PD_ORDINARY) continue;
+    const size_t cta = need + pydock_warp_bytes(precision, true, shape) + (precision == SD_PREC_MIXED ? 8192 : 10240);
     ctas[shape] = std::min((int)(smem_sm / cta), pd_ctas(true, shape));
-    if (ctas[PD_ORDINARY] == 0) return PD_ORDINARY;  // the spill instantiation has more warps than what would fit
-    if (ctas[shape] * pd_warps(false, true, shape) >= ctas[best] * pd_warps(false, true, best)) best = shape;
+    const int warps = pd_warps(precision != SD_PREC_MIXED, true, shape);
+    if (ctas[shape] * warps >= ctas[best] * pd_warps(precision != SD_PREC_MIXED, true, best)) best = shape;
   }
-  if (poses > ctas[best] * nsm) return best;
+  if (ctas[PD_ORDINARY] == 0 || (ctas[best] == 1 && poses > nsm)) return PD_SCRATCH;
+  if (precision != SD_PREC_MIXED || poses > ctas[best] * nsm) return best;
   const int ntiles = (nr + SD_TILE - 1) / SD_TILE;
   double least = 1e300;
   for (int shape : {PD_SMALL, PD_MID, PD_ORDINARY}) {

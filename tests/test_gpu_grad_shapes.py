@@ -34,3 +34,21 @@ def test_shapes(n_rec, n_lig, beside, tables):
             if beside:  # between calls on the other complex
                 o = others[0].poses.reshape(1, -1)
                 dk.pydock_grad(0, np.repeat(o, n, axis=0), sd.SD_PREC_MIXED)
+
+
+@pytest.mark.parametrize("n_rec,n_lig", [(50, 1472), (50, 1536), (700, 1504), (47, 3456), (47, 3503), (47, 3560)])
+@pytest.mark.parametrize("n", [148, 149, 400])
+def test_fp64_beside_one_cta(n_rec, n_lig, n, tables):
+    """FP64 gradients where an SM's shared memory holds two CTAs' arrays, one, or none."""
+    c = sd.SyntheticComplex(n_rec, n_lig, n, 1, 2, 3, seed=n_rec + n_lig)
+    poses = np.array(c.poses.reshape(n, -1))
+    poses[:, :3] *= 0.7
+    pick = [0, 77, n - 1]
+    osys = OracleSystem(c, tables, scoring=1)
+    ref = np.array([oracle_energy(osys, poses[k]) for k in pick])
+    grad = np.array([oracle_grad(osys, poses[k], 11) for k in pick])
+    top = np.maximum(np.abs(grad).max(axis=1), 1.0)
+    with sd.Docking([c], tables, scoring=sd.SD_SCORING_PYDOCK) as dk:
+        e, g = dk.pydock_grad(0, poses, sd.SD_PREC_FP64)
+        assert (np.abs(g[pick] - grad) / top[:, None]).max() <= 1e-10
+        assert (np.abs(e[pick] - ref) / np.maximum(np.abs(ref), top)).max() <= 1e-10
