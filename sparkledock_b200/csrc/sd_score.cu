@@ -16,6 +16,8 @@
 // case the pair is decided in FP64 from the exact transforms.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "sd_internal.h"
 #include "sd_packed.cuh"
 #include "sd_pose.cuh"
@@ -231,18 +233,12 @@ static const MixedVariant kMixedFew = SD_MIXED(24, 1), kMixedFewWide = SD_MIXED_
 // energy, is the same in every variant)
 static const MixedVariant kMixedSpill = {(const void*)dfire_score_mixed_kernel<12, 2, true, true>, 12, 2};
 
-// shapes of the culled FP64 kernel, the smallest CTAs first: they lose least where warps wait for each
-// other at a pose's end, and the first whose CTAs are all resident for the context's largest complex is
-// taken (the v_i of a large receptor fill the shared memory; when none fits, the spill instantiation).
-// Measured (M poses/s for 4x6, 8x3, 12x2): 757/481 atoms 5.7, 5.2, 4.0; 1200/1400 - (does not fit), 1.90,
-// 1.86; 2516/1061 -, 1.98, 2.01; 3002/1274 -, -, 1.74.  With too few poses to fill the GPU the shape with
-// the most warps is taken instead: a pose's time counts then.
+// shapes of the culled FP64 kernel, the smallest CTAs first (fp64_shape)
 static const MixedVariant kFp64Shapes[] = {
     {(const void*)dfire_score_fp64_kernel<4, 6, false>, 4, 6},
     {(const void*)dfire_score_fp64_kernel<6, 4, false>, 6, 4},
     {(const void*)dfire_score_fp64_kernel<8, 3, false>, 8, 3},
     {(const void*)dfire_score_fp64_kernel<12, 2, false>, 12, 2},
-    {(const void*)dfire_score_fp64_kernel<24, 1, false>, 24, 1},
     {(const void*)dfire_score_fp64_kernel<16, 1, false>, 16, 1},
     {(const void*)dfire_score_fp64_kernel<8, 1, false>, 8, 1},
 };
@@ -290,17 +286,37 @@ size_t score_smem_bytes(int precision, int scoring, int max_nr, int max_nl, int 
   return (size_t)32 * max_nl + (size_t)8 * max_nr;
 }
 
-// the culled FP64 kernel's shape for these sizes and at most `poses` poses (1 KiB of each CTA is the
-// system's, 1 KiB covers the static arrays); the last one when none fits (the caller then spills)
+// The culled FP64 kernel's shape for these sizes and at most `poses` poses (1 KiB of each CTA is the system's, 1 KiB
+// covers the static arrays); the last one when none fits (the caller then spills).  Small CTAs lose least where
+// warps wait for each other at a pose's end, so the first whose CTAs are all resident is taken (the v_i of a large
+// receptor fill the shared memory).  Where it has all poses resident at once, a pose's time counts: the fewest
+// rounds over the warps that have a tile, among equals the fewest rounds, then the most registers.  Measured, M poses/s of
+// large calls with 4x6, 6x4, 8x3, 12x2, 16x1, 8x1 (* its CTAs are not all resident): 757/481 5.66, 5.60, 5.25,
+// 4.00, 2.58, 2.57; 1000/800 3.16*, 3.46, 3.42, 2.79, 1.82, 1.72; 1700/600 3.26*, 3.61, 3.74, 3.16, 2.08, 1.94;
+// 2516/1061 -, 1.82*, 2.04, 2.06, 1.42, 1.09; 3002/1274 -, -, 1.40*, 1.72, 1.26, 0.89; 12000/300 16x1 2.39, 8x1 2.16;
+// 21500/500 16x1 1.69 (spilled), 8x1 1.28.  Microseconds of 16 and 200 poses of 3002/1274: 12x2 199, 250; 16x1 174,
+// 275; 8x1 235, 387; of 200/100: 12x2 62, 70; 16x1 54, 80; 8x1 53, 78.  (24x1 was slower than 16x1 in all of them.)
 int fp64_shape(int max_nr, int max_nl, int smem_sm, int poses, int nsm) {
   const int ntiles = (max_nr + SD_TILE - 1) / SD_TILE;  // a warp without a tile only waits
-  int best = kNumFp64Shapes - 1;
-  for (int v = kNumFp64Shapes - 1; v >= 0; --v) {
+  auto fits = [&](int v) {
     const size_t cta = score_smem_bytes(SD_PREC_FP64, SD_SCORING_DFIRE, max_nr, max_nl, 1) +
                        score_warp_bytes(SD_PREC_FP64, SD_SCORING_DFIRE, v, false) + 2048;
-    const bool few = poses <= kFp64Shapes[v].min_blocks * nsm;
-    if (cta * kFp64Shapes[v].min_blocks > (size_t)smem_sm) continue;
-    if (!few || (kFp64Shapes[v].warps > kFp64Shapes[best].warps && kFp64Shapes[v].warps <= ntiles)) best = v;
+    return cta * kFp64Shapes[v].min_blocks <= (size_t)smem_sm;
+  };
+  int best = 0;
+  while (best < kNumFp64Shapes - 1 && !fits(best)) ++best;
+  if (poses > kFp64Shapes[best].min_blocks * nsm) return best;
+  int rounds = 0, eff = 0;
+  for (int v = best; v < kNumFp64Shapes; ++v) {
+    if (!fits(v)) continue;
+    const int slots = kFp64Shapes[v].min_blocks * nsm;
+    const int r = std::max(1, (poses + slots - 1 - slots / 16) / slots);  // a few more share the first round
+    const int e = std::min(kFp64Shapes[v].warps, ntiles);
+    if (eff == 0 || r * eff < rounds * e || (r * eff == rounds * e && r <= rounds)) {
+      rounds = r;
+      eff = e;
+      best = v;
+    }
   }
   return best;
 }
