@@ -629,7 +629,9 @@ bool few_fits(const sd_ctx* c, const void* k, size_t dynamic, int* known) {
 int score_variant(sd_ctx* c, int precision, int poses, bool stateless) {
   bool few = few_poses(c, poses);
   if (c->scoring == SD_SCORING_DFIRE) {
-    if (precision == SD_PREC_FP64) return fp64_shape(c->max_nr, c->max_nl, c->smem_sm, poses, c->nsm);
+    // (of a step's glowworms about 0.7 have moved and are rescored)
+    if (precision == SD_PREC_FP64)
+      return fp64_shape(c->max_nr, c->max_nl, c->smem_sm, stateless ? poses : (int)(0.7 * poses) + 1, c->nsm);
     few &= precision == SD_PREC_MIXED && stateless && !c->forced;
   }
   const int wide = precision == SD_PREC_MIXED ? c->wide : 0;

@@ -239,6 +239,7 @@ static const MixedVariant kFp64Shapes[] = {
     {(const void*)dfire_score_fp64_kernel<6, 4, false>, 6, 4},
     {(const void*)dfire_score_fp64_kernel<8, 3, false>, 8, 3},
     {(const void*)dfire_score_fp64_kernel<12, 2, false>, 12, 2},
+    {(const void*)dfire_score_fp64_kernel<24, 1, false>, 24, 1},
     {(const void*)dfire_score_fp64_kernel<16, 1, false>, 16, 1},
     {(const void*)dfire_score_fp64_kernel<8, 1, false>, 8, 1},
 };
@@ -295,10 +296,13 @@ size_t score_smem_bytes(int precision, int scoring, int max_nr, int max_nl, int 
 // 4.00, 2.58, 2.57; 1000/800 3.16*, 3.46, 3.42, 2.79, 1.82, 1.72; 1700/600 3.26*, 3.61, 3.74, 3.16, 2.08, 1.94;
 // 2516/1061 -, 1.82*, 2.04, 2.06, 1.42, 1.09; 3002/1274 -, -, 1.40*, 1.72, 1.26, 0.89; 12000/300 16x1 2.39, 8x1 2.16;
 // 21500/500 16x1 1.69 (spilled), 8x1 1.28.  Microseconds of 16 and 200 poses of 3002/1274: 12x2 199, 250; 16x1 174,
-// 275; 8x1 235, 387; of 200/100: 12x2 62, 70; 16x1 54, 80; 8x1 53, 78.  (24x1 was slower than 16x1 in all of them.)
+// 275; 8x1 235, 387; of 200/100: 12x2 62, 70; 16x1 54, 80; 8x1 53, 78.  24x1 has 80 registers a thread against 128
+// of 16x1 and is slower but for large ligands, which all threads place and list: 6 poses with 24x1 and 16x1 of
+// 3000/1274 174, 152; 700/4700 249, 238; 1500/2500 235, 202; 3000/2500 227, 241; 6000/4700 472, 497.
 int fp64_shape(int max_nr, int max_nl, int smem_sm, int poses, int nsm) {
   const int ntiles = (max_nr + SD_TILE - 1) / SD_TILE;  // a warp without a tile only waits
   auto fits = [&](int v) {
+    if (kFp64Shapes[v].warps == 24 && (max_nl <= 2048 || max_nr <= 1024)) return false;  // see above
     const size_t cta = score_smem_bytes(SD_PREC_FP64, SD_SCORING_DFIRE, max_nr, max_nl, 1) +
                        score_warp_bytes(SD_PREC_FP64, SD_SCORING_DFIRE, v, false) + 2048;
     return cta * kFp64Shapes[v].min_blocks <= (size_t)smem_sm;

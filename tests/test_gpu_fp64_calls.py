@@ -24,3 +24,15 @@ def test_every_number_of_poses_gives_the_same_bits(n_rec, n_lig, tables):
         for k in (1, 148, 149, 296, 297, 444, 592, 640, 888, 960):
             _, e = dk.score_poses(0, poses[:k], sd.SD_PREC_FP64)
             assert np.array_equal(e, e_all[:k]), f"{k} poses"
+
+
+@pytest.mark.parametrize("n_rec,n_lig", [(1024, 2500), (1025, 2048), (1025, 2049), (2000, 4700)])
+def test_large_ligands_of_few_poses(n_rec, n_lig, tables):
+    """24 warps a pose from 2,049 ligand and 1,025 receptor atoms on, else 16."""
+    c = sd.SyntheticComplex(n_rec, n_lig, 4, 1, 3, 3, seed=n_lig)
+    poses = np.array(c.poses.reshape(4, -1))
+    poses[:, :3] *= 0.8
+    _, ref = oracle_scores(OracleSystem(c, tables), poses)
+    with sd.Docking([c], tables) as dk:
+        _, e = dk.score_poses(0, poses, sd.SD_PREC_FP64)
+        assert np.array_equal(e, ref)
