@@ -479,6 +479,7 @@ pydock_kernel(ScoreLaunch L, double* out_grad) {
         __syncwarp();
         unsigned counts = cnt[0] | cnt[1] << 8 | cnt[2] << 16 | cnt[3] << 24;
         for (int g = 0; g < kGroups; ++g, counts >>= 8) {
+          if ((counts & 255u) == 0) continue;
           const LigAtom<T> ra = W.rec[g * SD_GROUP + atom], rb = W.rec[g * SD_GROUP + atom + kRow];
           const V2<T> rx(ra.x, rb.x), ry(ra.y, rb.y), rz(ra.z, rb.z), rq(ra.q, rb.q);
           // the LJ table is symmetric (products and sums of the two types' parameters), so it is read as
@@ -648,7 +649,7 @@ float pydock_force_scale(double max_q_rec, double max_q_lig, const double* eps, 
 // 3.65; 3002/1766 9.8, 5.8, 4.72; 3002/2100 11.8, 6.9, 8.3; 3002/2500 24, 13.2, 9.7.  (12 warps for all sizes were
 // slower than the earlier kernel for the smallest: 0.76 against 0.69 ms.)
 // Where all poses are resident in that shape at once, the warps of a pose count: then the fewest rounds over the
-// warps that have a tile.  (757/481: 300 poses 0.34 ms in 4 x 6, 0.23 in 8 x 3, 0.27 in 12 x 2.)
+// warps that have a part of it.  (757/481: 300 poses 0.34 ms in 4 x 6, 0.23 in 8 x 3, 0.27 in 12 x 2.)
 // Where shared memory holds one CTA only, two with their arrays in global scratch (PD_SCRATCH) have more warps: 2,000
 // poses of 757/2500 atoms 3.85 -> 3.18 ms in FP32, 5.0 -> 3.3 ms in FP64, 50/3503 4.4 -> 2.4 ms in FP64.
 int pydock_grad_shape(int precision, int nl, int nr, int poses, int smem_sm, int nsm) {
@@ -663,12 +664,12 @@ int pydock_grad_shape(int precision, int nl, int nr, int poses, int smem_sm, int
   }
   if (ctas[PD_ORDINARY] == 0 || (ctas[best] == 1 && poses > nsm)) return PD_SCRATCH;
   if (precision != SD_PREC_MIXED || poses > ctas[best] * nsm) return best;
-  const int ntiles = (nr + SD_TILE - 1) / SD_TILE;
+  const int parts = (nr + SD_TILE - 1) / SD_TILE;
   double least = 1e300;
   for (int shape : {PD_SMALL, PD_MID, PD_ORDINARY}) {
     if (ctas[shape] == 0) continue;
     const int rounds = (poses + ctas[shape] * nsm - 1) / (ctas[shape] * nsm);
-    const double time = (double)rounds / std::min(pd_warps(false, true, shape), ntiles);
+    const double time = (double)rounds / std::min(pd_warps(false, true, shape), parts);
     if (time < least) {
       least = time;
       best = shape;
