@@ -664,7 +664,8 @@ int pydock_grad_shape(int precision, int nl, int nr, int poses, int smem_sm, int
   }
   if (ctas[PD_ORDINARY] == 0 || (ctas[best] == 1 && poses > nsm)) return PD_SCRATCH;
   if (precision != SD_PREC_MIXED || poses > ctas[best] * nsm) return best;
-  const int parts = (nr + SD_TILE - 1) / SD_TILE;
+  // (tiles, or chunks of the ligand, whose atoms are placed and whose forces are projected by all warps)
+  const int parts = (std::max(nr, nl) + SD_TILE - 1) / SD_TILE;
   double least = 1e300;
   for (int shape : {PD_SMALL, PD_MID, PD_ORDINARY}) {
     if (ctas[shape] == 0) continue;
