@@ -709,7 +709,7 @@ def main():
         "metric": METRIC, "value": m["value"], "unit": "scored poses/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": t_ms / args.steps, "steps_per_s": args.steps / (t_ms / 1e3),
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "f16/f32 pair tests, f64 table sums and GSO" if cfg["precision"] == "mixed" else "f64",
+        "dtype": "f32 pair tests, f64 table sums and GSO" if cfg["precision"] == "mixed" else "f64",
         "data": "synthetic (seeded globules, N(0,1) DFIRE table)", "config": config,
         "gpu_launches": 2 * args.steps,
         "e2e": {"value": es / (et / 1e3), "unit": "scored poses/s", "h2d_bytes_per_step": e2e["h2d"],

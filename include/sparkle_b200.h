@@ -61,7 +61,7 @@ extern "C" {
 /* precision / algorithm of the pair stage */
 #define SD_PREC_FP64_REF 0   /* FP64, all Nr*Nl pairs, reference pair order: bit-exact energies */
 #define SD_PREC_FP64 1       /* FP64 with the cutoff cell culling; same order -> bit-exact */
-#define SD_PREC_MIXED 2      /* FP16/FP32 distances, exact bins (FP64 near-edge fallback), FP64 sums */
+#define SD_PREC_MIXED 2      /* FP32 distances, exact bins (FP64 decision near an edge), FP64 sums */
 
 /* One receptor/ligand complex and its swarms.  Mirrors the fields of the reference's
  * Complex (source/prep/include/complex.h:10-104: atom_coordinates, mask, modes, num_atoms)

@@ -611,7 +611,10 @@ int configure_score(sd_ctx* c, int precision, int variant, int* grid, size_t* sm
   return SD_OK;
 }
 
-// the few-poses shapes: at most one pose per SM, and receptors with a tile for most of the 24 warps
+// the few-poses shapes: at most one pose per SM, and receptors with a tile for most of the 24 warps.  148 poses with
+// the ordinary and the few-poses shape, us (mixed DFIRE, FP32 and FP64 pyDock energies, FP32 and FP64 gradients):
+// 2000/1000 atoms 150, 126; 240, 152; 263, 177; 277, 250; 353, 263.  757/378 89, 81; 117, 100; 139, 112; 158, 151;
+// 166, 154.  The gain ends slowly below the line: 320/160 84, 84; 77, 78; 89, 75; 115, 107; 116, 104
 bool few_poses(const sd_ctx* c, int poses) { return poses <= c->nsm && c->max_nr > 20 * SD_TILE; }
 
 // whether kernel k's few-poses shape fits in a CTA's shared memory with `dynamic` bytes beside its static arrays;
@@ -1501,6 +1504,7 @@ int sd_cluster(sd_ctx* c, int ci, const int* rec_backbone, const int* lig_backbo
     if (lig_backbone[j]) bb.push_back(j);
   const int nbb = (int)bb.size(), nbl = nbb - nbr;
   if (nbb == 0) return fail(SD_ERR_ARG, "sd_cluster: no backbone atoms flagged");
+  // (the limit is of an earlier kernel that kept a glowworm's atoms in shared memory; the calls it refuses stay refused)
   if (cluster_smem_bytes(G) + (size_t)nbb * 24 + 4 * (G & 1) > 227 * 1024)
     return fail(SD_ERR_NOTSUP, "sd_cluster: too many backbone atoms");
   // swarms per launch: coordinates of at most kBackboneBytes in the context's workspace

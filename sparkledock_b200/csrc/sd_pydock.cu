@@ -12,8 +12,8 @@
 //   dE/dt = sum_j F_j, dE/dw = sum_j (l_j - t) x F_j, dE/de_lig_m = sum_j mask_j (R M_mj).F_j,
 //   dE/de_rec_m = sum_i mask_i M_mi.G_i, with F_j = dE/dl_j, G_i = dE/dr_i (pair forces).
 //
-// Kernel: one CTA (8 warps) per pose at a time, persistent over a work list; receptor tiles of
-// 32 (one lane per atom) culled against the ligand sphere and against spatial ligand chunks, and
+// Kernel: one CTA (4 to 24 warps, PdShape) per pose at a time, persistent over a work list; receptor tiles
+// of 32 (one lane per atom) culled against the ligand sphere and against spatial ligand chunks, and
 // each tile's candidate ligand atoms against the bounding boxes of its four groups of 8 atoms (45 %
 // of a group's listed pairs are inside the cutoff, 21 % of a tile's).  A step evaluates 8 receptor
 // atoms x 8 candidates of one group, two atoms per lane (FP32 in packed instructions).  GRAD adds
@@ -25,8 +25,8 @@
 // What bounds it: instruction issue (0.7 of the slots) and, with forces, the latency of the shuffles
 // and shared atomics; memory traffic is small.  Measured on 3002 / 1274 atoms, 4,096 poses, the whole
 // call, against the earlier kernel (one candidate of a tile over all its lanes, 15 shuffles and 3
-// atomics for two candidates): FP32 gradients 6.1 -> 4.0 ms, FP32 energies 3.6 -> 2.0 ms, FP64 energies
-// 4.0 -> 2.6 ms, 2,000 FP64 gradients 4.7 -> 2.5 ms.
+// atomics for two candidates): FP32 gradients 5.94 -> 3.65 ms, FP32 energies 3.68 -> 1.89 ms; 2,000 FP64
+// energies 2.17 -> 1.33 ms, FP64 gradients 4.70 -> 2.43 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
