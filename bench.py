@@ -62,7 +62,7 @@ DRAM_BYTES_PER_SCORED_POSE = 265.0
 # smsp__inst_executed.sum of one launch (3002 / 1274 atoms, 4,098 poses, 233.9 M pairs in the
 # cutoff), as summarised with its full capture under profiles/; one ceiling of the scorer is the
 # SMs' issue rate (148 SMs x 4 schedulers x clock) over this count
-WARP_INSTR_PER_PAIR = 4.60
+WARP_INSTR_PER_PAIR = 4.61
 # L1 data-pipe wavefronts per in-cutoff pair in the same launch (l1tex__data_pipe_lsu_wavefronts:
 # 122.6 M shared-memory wavefronts plus ~174 M global-load ones, mostly table gathers, over
 # 233.9 M pairs); the pipe retires one wavefront per SM per cycle, the other ceiling

@@ -302,14 +302,16 @@ int sd_score_poses(sd_ctx* ctx, int complex_idx, const double* poses, int n, int
  * synchronisation would invalidate the capture; SD_ERR_ARG).  Poses must be finite: with
  * sync != 0 the call also counts non-finite pose values on the device and returns
  * SD_ERR_NUMERIC if there are any (the outputs of such a call are not meaningful); with sync == 0
- * nothing is checked.  These calls do not add to the counters of sd_get_stats.  The first call on
+ * nothing is checked.  A complex whose per-pose arrays exceed a CTA's shared memory needs the
+ * context's scratch, which an allocating scoring call makes: SD_ERR_NOTSUP before one.  These calls do not add to the counters of sd_get_stats.  The first call on
  * a device (and the first after a cudaDeviceReset) looks up the array's device address
  * (cudaGetSymbolAddress); make that first call before any stream capture. */
 int sd_score_poses_noalloc(sd_ctx* ctx, int complex_idx, const double* d_poses, int n, int precision,
                            double* d_score, double* d_energy, double* d_ref, int sync);
 
 /* Per-pair DFIRE bins of one pose (debug / parity): bins_out[i*n_lig + j] = table bin 0..19,
- * -1 when d^2 > 225.  Receptor order i and ligand order j are the caller's. */
+ * -1 when d^2 > 225, by the steps of the precision's scorer (FP64 and MIXED: FP32 terms, the exact
+ * transforms where they do not settle a pair).  Receptor order i and ligand order j are the caller's. */
 int sd_dfire_bins(sd_ctx* ctx, int complex_idx, const double* pose, int precision, int* bins_out);
 
 /* PYDOCK only: energy and its gradient with respect to the 6 rigid coordinates and the ANM

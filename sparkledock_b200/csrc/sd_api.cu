@@ -467,9 +467,9 @@ bool all_finite(const double* v, size_t n) {
 
 // Arrays that lie one after another on the device, to their places at the caller (null: not asked for).  Several
 // small ones come in one copy by way of host memory, as each copy into pageable memory waits on its own: two of
-// 64 KiB take 25 us, one of both 16 us.  That memory is pinned and kept from the context's 16th such call on: it
-// saves up to 80 us a call then (4,096 gradients of 757 / 481 atoms 1.84 -> 1.76 ms), but pinning takes 1 to 3 ms,
-// a third of a small context's creation, which few calls never earn back.
+// 64 KiB take 25 us, one of both 16 us.  That memory is pinned and kept from the context's 16th such call on, which
+// saves up to 80 us a call then (0.9 MB: 4,096 gradients of 26 components); pinning takes up to 3 ms (0.1
+// to 2.8 in different processes), which few calls would not earn back.
 constexpr size_t kOneCopy = 1 << 20;
 constexpr int kPinAfter = 16;
 struct Part {
